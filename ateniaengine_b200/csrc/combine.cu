@@ -8,6 +8,7 @@
 //
 // Also here: the small elementwise kernels of the library (int8 per-row quantiser, f32 to bf16 conversion).
 #include "common.cuh"
+#include "round_codes.cuh"
 
 namespace atenia {
 namespace {
@@ -80,32 +81,71 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineArgs a) {
 }
 
 // One block per row: scale = max|row| / 127 (1 for a zero row), q = clamp(round_half_away(w * (1/scale))).
-__global__ void __launch_bounds__(256) quantize_rows_kernel(const float* __restrict__ w, int64_t cols,
-                                                             int8_t* __restrict__ q, float* __restrict__ scales) {
-  __shared__ float red[8];
-  __shared__ float s_scale;
+// The row is read once: a thread keeps its (up to kQuantVecs) groups of four values in registers between the
+// maximum and the rounding; what a longer row has beyond that is read again.  HBM-bound, 5 bytes per weight.
+// VEC: every row starts on a 16-byte boundary (a thread's four values are one vector), else single values, a
+// block width apart.  Narrow rows take narrower blocks, so that several rows share an SM.  Measured on a B200:
+// 14336 x 4096 93 -> 50 us (floor 47), against a kernel that read every row twice with 4-byte loads.
+constexpr int kQuantVecs = 8;
+
+template <bool VEC>
+__global__ void __launch_bounds__(512) quantize_rows_kernel(const float* __restrict__ w, int64_t cols,
+                                                            int8_t* __restrict__ q, float* __restrict__ scales) {
+  __shared__ float red[16];
   const int64_t r = blockIdx.x;
   const float* row = w + r * cols;
+  int8_t* qrow = q + r * cols;
+  // value j of a thread's vector v
+  auto col_of = [&](int v, int j) -> int64_t {
+    const int64_t base = (int64_t)v * blockDim.x * 4;
+    return VEC ? base + threadIdx.x * 4 + j : base + threadIdx.x + (int64_t)j * blockDim.x;
+  };
+  auto load = [&](int v) -> float4 {
+    if (VEC) return col_of(v, 0) < cols ? *reinterpret_cast<const float4*>(row + col_of(v, 0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(col_of(v, 0) < cols ? row[col_of(v, 0)] : 0.f, col_of(v, 1) < cols ? row[col_of(v, 1)] : 0.f,
+                       col_of(v, 2) < cols ? row[col_of(v, 2)] : 0.f, col_of(v, 3) < cols ? row[col_of(v, 3)] : 0.f);
+  };
+  auto amax4 = [](float m, const float4& x) {
+    return fmaxf(fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y))), fmaxf(fabsf(x.z), fabsf(x.w)));
+  };
+  const int nvec = (int)((cols + (int64_t)blockDim.x * 4 - 1) / ((int64_t)blockDim.x * 4));
+  float4 keep[kQuantVecs];
   float amax = 0.f;
-  for (int64_t c = threadIdx.x; c < cols; c += blockDim.x) amax = fmaxf(amax, fabsf(row[c]));
+#pragma unroll
+  for (int v = 0; v < kQuantVecs; ++v) keep[v] = v < nvec ? load(v) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int v = 0; v < kQuantVecs; ++v) amax = amax4(amax, keep[v]);
+  for (int v = kQuantVecs; v < nvec; ++v) amax = amax4(amax, load(v));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float m = red[0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) m = fmaxf(m, red[i]);
-    float sc = m > 0.f ? __fdiv_rn(m, 127.0f) : 1.0f;
-    s_scale = sc;
-    scales[r] = sc;
-  }
-  __syncthreads();
-  const float inv = __fdiv_rn(1.0f, s_scale);
-  for (int64_t c = threadIdx.x; c < cols; c += blockDim.x) {
-    float v = roundf(__fmul_rn(row[c], inv));  // roundf: halves away from zero, like Rust's f32::round
+  float m = red[0];
+  for (int i = 1; i < (int)(blockDim.x >> 5); ++i) m = fmaxf(m, red[i]);
+  const float scale = m > 0.f ? __fdiv_rn(m, 127.0f) : 1.0f;
+  if (threadIdx.x == 0) scales[r] = scale;
+  const float inv = __fdiv_rn(1.0f, scale);
+  const float inv4[4] = {inv, inv, inv, inv};
+  auto exact = [&](float x, int) -> int {
+    float v = roundf(__fmul_rn(x, inv));  // roundf: halves away from zero, like Rust's f32::round
     v = fminf(fmaxf(v, -127.0f), 127.0f);
-    q[r * cols + c] = (int8_t)v;
-  }
+    return (int)v;
+  };
+  auto store = [&](int v, const float4& x) {
+    const float x4[4] = {x.x, x.y, x.z, x.w};
+    const uint32_t p = round_codes4(x4, inv4, exact);
+    if (VEC) {
+      if (col_of(v, 0) < cols) *reinterpret_cast<uint32_t*>(qrow + col_of(v, 0)) = p;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col_of(v, j) < cols) qrow[col_of(v, j)] = (int8_t)(p >> (8 * j));
+    }
+  };
+#pragma unroll
+  for (int v = 0; v < kQuantVecs; ++v)
+    if (v < nvec) store(v, keep[v]);
+  for (int v = kQuantVecs; v < nvec; ++v) store(v, load(v));
 }
 
 __global__ void f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int64_t n) {
@@ -154,7 +194,12 @@ extern "C" int atenia_quantize_per_row_i8(const float* w, int64_t rows, int64_t 
   if (!w || !q || !scales) return ATENIA_ERR_NULL;
   if (rows < 0 || cols <= 0 || rows > 0x7fffffff) return ATENIA_ERR_SHAPE;
   if (rows == 0) return ATENIA_OK;
-  atenia::quantize_rows_kernel<<<(unsigned)rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(w, cols, q, scales);
+  // the narrowest block whose registers hold a row (32 values per thread)
+  const int threads = cols <= 64 * 32 ? 64 : cols <= 128 * 32 ? 128 : cols <= 256 * 32 ? 256 : 512;
+  const bool vec = cols % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 3u) == 0;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (vec) atenia::quantize_rows_kernel<true><<<(unsigned)rows, threads, 0, s>>>(w, cols, q, scales);
+  else atenia::quantize_rows_kernel<false><<<(unsigned)rows, threads, 0, s>>>(w, cols, q, scales);
   atenia::count_launch();
   return (int)cudaGetLastError();
 }

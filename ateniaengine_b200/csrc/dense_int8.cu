@@ -3,80 +3,54 @@
 // (src/tensor/quantizer.rs:67-118 per channel, :176-246 per group; src/cuda/int8_to_bf16.cu:24-40,
 // :99-117).  The MoE tiers use the per-row layout of combine.cu instead.
 //
-// All three passes are streaming, HBM-bound work:
-//   amax      read K*N*4 bytes; a block covers 128 columns x up to 256 rows of one group, reduces its
-//             8 row lanes in shared memory and merges with atomicMax on the bit pattern (non-negative
-//             floats order like unsigned integers, so the result does not depend on scheduling)
-//   finalize  scale = max(amax / 127, 1e-12), in place
-//   quantize  read K*N*4, write K*N bytes: q = clamp(round_half_away(w / scale), -127, 127), NaN -> 0
-//   dequant   read K*N, write K*N*2 bytes: bf16 = high half of (float)q * scale (truncation, as the
-//             reference's kernel does)
+// Both directions are streaming, HBM-bound work (algorithmic bytes per weight: quantise 4 + 1, dequant 1 + 2):
+//   quantize_groups  a block owns 128 columns x one group; the group's values stay in registers between the
+//                    maximum and the rounding, so the matrix is read once (groups of at most 128 rows)
+//   quantize_tall    a cluster of eight blocks owns 64 columns x one taller group and reads it twice, the
+//                    second time from L2: 64 columns keep what all clusters have in flight (37 x 64 columns x
+//                    K x 4 bytes: 39 MB at K = 4096) below the L2 size
+//   dequant          a block owns 256 columns x 64 rows; a lane keeps its eight scales while the group lasts
+// Neither divides 64-bit indexes: an earlier form that walked the matrix as one flat list spent two 64-bit
+// divisions per vector and read the matrix in two launches.  Measured on a B200 at 4096 x 14336, groups of 128:
+// quantise (maximum, finalize and quantise kernels) 149 -> 68 us, dequant 42 -> 32 us; floors at the measured
+// copy rate 47 and 28 us.
+//   scale = max(amax / 127, 1e-12); q = clamp(round_half_away(w / scale), -127, 127), NaN -> 0;
+//   bf16 = high half of (float)q * scale (truncation, as the reference's kernel does)
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+#include "round_codes.cuh"
 
 namespace atenia {
 namespace {
 
-constexpr int COLS_PER_BLOCK = 128;  // 32 threads x 4 columns
-constexpr int ROW_LANES = 8;
-constexpr int ROWS_PER_BLOCK = 256;
+constexpr int COLS_PER_BLOCK = 128;  // 32 lanes x 4 columns
+constexpr int GROUP_ROWS_MAX = 128;  // tallest group that stays in registers: 16 warps x 8 rows
+constexpr int TALL_CTAS = 8;         // blocks per cluster
+constexpr int TALL_WARPS = 16;
+constexpr int TALL_COLS = 64;        // 16 lanes x 4 columns: a warp covers two rows
+constexpr int DEQ_COLS = 256, DEQ_ROWS = 64;
 
-struct Cols4 {
-  float v[4];
-};
-
-// Four consecutive columns of row r starting at c0; columns >= N read as 0.
-__device__ __forceinline__ Cols4 load_cols4(const float* __restrict__ w, int64_t r, int64_t c0, int64_t N, bool vec) {
-  Cols4 o;
-  if (vec) {
-    const float4 f = *reinterpret_cast<const float4*>(w + r * N + c0);
-    o.v[0] = f.x; o.v[1] = f.y; o.v[2] = f.z; o.v[3] = f.w;
+// Four columns of a row per lane (LANES lanes side by side): consecutive ones as one vector (VEC: every row
+// starts on a 16-byte boundary), else LANES apart.  Columns >= N read as 0.
+template <bool VEC, int LANES>
+__device__ __forceinline__ int64_t col_of(int64_t strip0, int lane, int j) {
+  return VEC ? strip0 + lane * 4 + j : strip0 + lane + LANES * j;
+}
+template <bool VEC, int LANES>
+__device__ __forceinline__ void load_cols4(float (&v)[4], const float* __restrict__ row, int64_t strip0, int lane,
+                                           int64_t N) {
+  if (VEC) {
+    const int64_t c = strip0 + lane * 4;
+    const float4 f = c < N ? *reinterpret_cast<const float4*>(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
   } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) o.v[j] = (c0 + j < N) ? w[r * N + c0 + j] : 0.f;
-  }
-  return o;
-}
-
-__global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ w, int64_t K, int64_t N, int64_t G,
-                                                    int64_t strips, int64_t chunks_per_group, int vec,
-                                                    unsigned int* __restrict__ amax_bits) {
-  __shared__ float red[ROW_LANES][COLS_PER_BLOCK];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t strip = blockIdx.x % strips, y = blockIdx.x / strips;
-  const int64_t g = y / chunks_per_group, ch = y % chunks_per_group;
-  const int64_t lo = g * G + ch * ROWS_PER_BLOCK;
-  int64_t hi = lo + ROWS_PER_BLOCK;
-  if (hi > (g + 1) * G) hi = (g + 1) * G;
-  if (hi > K) hi = K;
-  const int64_t c0 = strip * COLS_PER_BLOCK + tx * 4;
-  float m[4] = {0.f, 0.f, 0.f, 0.f};
-  if (c0 < N) {
-    for (int64_t r = lo + ty; r < hi; r += ROW_LANES) {
-      const Cols4 x = load_cols4(w, r, c0, N, vec != 0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float a = fabsf(x.v[j]);
-        if (a > m[j]) m[j] = a;  // a NaN never compares greater: skipped, as in the reference
-      }
+    for (int j = 0; j < 4; ++j) {
+      const int64_t c = strip0 + lane + LANES * j;
+      v[j] = c < N ? row[c] : 0.f;
     }
   }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) red[ty][tx * 4 + j] = m[j];
-  __syncthreads();
-  if (threadIdx.x < COLS_PER_BLOCK) {
-    const int64_t c = strip * COLS_PER_BLOCK + threadIdx.x;
-    if (c < N && lo < hi) {
-      float a = red[0][threadIdx.x];
-#pragma unroll
-      for (int l = 1; l < ROW_LANES; ++l) a = fmaxf(a, red[l][threadIdx.x]);
-      if (a > 0.f) atomicMax(&amax_bits[g * N + c], __float_as_uint(a));
-    }
-  }
-}
-
-__global__ void finalize_scales_kernel(float* __restrict__ scales, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i < n; i += (int64_t)gridDim.x * blockDim.x) scales[i] = fmaxf(__fdiv_rn(scales[i], 127.0f), 1e-12f);
 }
 
 __device__ __forceinline__ int quantize_one(float w, float s) {
@@ -86,27 +60,151 @@ __device__ __forceinline__ int quantize_one(float w, float s) {
   return (int)v;
 }
 
-__global__ void __launch_bounds__(256) quantize_kernel(const float* __restrict__ w, const float* __restrict__ scales,
-                                                        int64_t K, int64_t N, int64_t G, int vec,
-                                                        int8_t* __restrict__ q) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (vec) {
-    const int64_t n4 = K * N / 4;
-    for (; i < n4; i += stride) {
-      const int64_t e = i * 4, r = e / N, c = e % N;
-      const float4 x = *reinterpret_cast<const float4*>(w + e);
-      const float4 s = *reinterpret_cast<const float4*>(scales + (r / G) * N + c);
-      const uint32_t b0 = (uint32_t)quantize_one(x.x, s.x) & 0xffu, b1 = (uint32_t)quantize_one(x.y, s.y) & 0xffu,
-                     b2 = (uint32_t)quantize_one(x.z, s.z) & 0xffu, b3 = (uint32_t)quantize_one(x.w, s.w) & 0xffu;
-      *reinterpret_cast<uint32_t*>(q + e) = b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
-    }
+template <bool VEC, int LANES>
+__device__ __forceinline__ void store_codes4(const float (&w)[4], const float (&s)[4], const float (&inv)[4],
+                                             int8_t* __restrict__ row, int64_t strip0, int lane, int64_t N) {
+  const uint32_t p = round_codes4(w, inv, [&](float x, int j) { return quantize_one(x, s[j]); });
+  if (VEC) {
+    const int64_t c = strip0 + lane * 4;
+    if (c < N) *reinterpret_cast<uint32_t*>(row + c) = p;
   } else {
-    const int64_t n = K * N;
-    for (; i < n; i += stride) {
-      const int64_t r = i / N, c = i % N;
-      q[i] = (int8_t)quantize_one(w[i], scales[(r / G) * N + c]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t c = strip0 + lane + LANES * j;
+      if (c < N) row[c] = (int8_t)(p >> (8 * j));
     }
+  }
+}
+
+__device__ __forceinline__ void max_cols4(float (&m)[4], const float (&v)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float a = fabsf(v[j]);
+    if (a > m[j]) m[j] = a;  // a NaN never compares greater: skipped, as in the reference
+  }
+}
+__device__ __forceinline__ float scale_of(float amax) { return fmaxf(__fdiv_rn(amax, 127.0f), 1e-12f); }
+
+// RPT rows per thread: groups of at most WARPS * RPT rows.  Eight rows (32 registers) per thread at most: with
+// sixteen a third of the loads in flight per SM is lost (4096 x 14336, groups of 128: 83 against 68 us).
+template <bool VEC, int WARPS, int RPT>
+__global__ void __launch_bounds__(WARPS * 32) quantize_groups_kernel(const float* __restrict__ w, int64_t K,
+                                                                           int64_t N, int G, unsigned strips,
+                                                                           int8_t* __restrict__ q,
+                                                                           float* __restrict__ scales) {
+  __shared__ float red[WARPS][COLS_PER_BLOCK];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned g = blockIdx.x / strips;
+  const int64_t strip0 = (int64_t)(blockIdx.x - g * strips) * COLS_PER_BLOCK;
+  const int64_t lo = (int64_t)g * G;
+  const int rows = (int)(K - lo < G ? K - lo : G);
+  float v[RPT][4];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int r = warp + WARPS * i;
+    if (r < rows) load_cols4<VEC, 32>(v[i], w + (lo + r) * N, strip0, lane, N);
+    else v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
+  }
+  float m[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) max_cols4(m, v[i]);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) red[warp][lane + 32 * j] = m[j];  // [j][lane]: no bank conflict
+  __syncthreads();
+  float s[4], inv[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a = red[0][lane + 32 * j];
+#pragma unroll
+    for (int l = 1; l < WARPS; ++l) a = fmaxf(a, red[l][lane + 32 * j]);
+    s[j] = scale_of(a);
+    inv[j] = __frcp_rn(s[j]);
+  }
+  if (warp == 0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t c = col_of<VEC, 32>(strip0, lane, j);
+      if (c < N) scales[(int64_t)g * N + c] = s[j];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int r = warp + WARPS * i;
+    if (r < rows) store_codes4<VEC, 32>(v[i], s, inv, q + (lo + r) * N, strip0, lane, N);
+  }
+}
+
+template <bool VEC>
+__global__ void __cluster_dims__(TALL_CTAS, 1, 1) __launch_bounds__(TALL_WARPS * 32)
+quantize_tall_kernel(const float* __restrict__ w, int64_t K, int64_t N, int64_t G, int64_t strips,
+                     int8_t* __restrict__ q, float* __restrict__ scales) {
+  namespace cg = cooperative_groups;
+  constexpr int LANES = TALL_COLS / 4;
+  __shared__ float red[2 * TALL_WARPS][TALL_COLS];
+  __shared__ float part[TALL_COLS];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int lane = threadIdx.x % LANES, rl = threadIdx.x / LANES;  // column lane, row lane
+  const int64_t item = blockIdx.x / TALL_CTAS, g = item / strips, strip0 = (item - g * strips) * TALL_COLS;
+  const int64_t lo = g * G, hi = lo + G < K ? lo + G : K;
+  // row r of the group belongs to row lane r mod (TALL_CTAS * 2 * TALL_WARPS) of the cluster
+  const int64_t first = lo + (int64_t)cluster.block_rank() * 2 * TALL_WARPS + rl;
+  constexpr int64_t kStep = TALL_CTAS * 2 * TALL_WARPS;
+  float m[4] = {0.f, 0.f, 0.f, 0.f};
+  int64_t r = first;
+  for (; r + 3 * kStep < hi; r += 4 * kStep) {  // four rows in flight
+    float v[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) load_cols4<VEC, LANES>(v[i], w + (r + i * kStep) * N, strip0, lane, N);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) max_cols4(m, v[i]);
+  }
+  for (; r < hi; r += kStep) {
+    float v[4];
+    load_cols4<VEC, LANES>(v, w + r * N, strip0, lane, N);
+    max_cols4(m, v);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) red[rl][lane + LANES * j] = m[j];
+  __syncthreads();
+  if (threadIdx.x < TALL_COLS) {
+    float a = red[0][threadIdx.x];
+#pragma unroll 8
+    for (int l = 1; l < 2 * TALL_WARPS; ++l) a = fmaxf(a, red[l][threadIdx.x]);
+    part[threadIdx.x] = a;
+  }
+  cluster.sync();
+  if (threadIdx.x < TALL_COLS) {
+    float a = 0.f;
+#pragma unroll
+    for (int b = 0; b < TALL_CTAS; ++b) a = fmaxf(a, cluster.map_shared_rank(part, b)[threadIdx.x]);
+    red[0][threadIdx.x] = scale_of(a);
+  }
+  cluster.sync();  // also: no block leaves while another reads its part
+  float s[4], inv[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    s[j] = red[0][lane + LANES * j];
+    inv[j] = __frcp_rn(s[j]);
+  }
+  if (cluster.block_rank() == 0 && rl == 0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t c = col_of<VEC, LANES>(strip0, lane, j);
+      if (c < N) scales[g * N + c] = s[j];
+    }
+  }
+  r = first;
+  for (; r + 3 * kStep < hi; r += 4 * kStep) {
+    float v[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) load_cols4<VEC, LANES>(v[i], w + (r + i * kStep) * N, strip0, lane, N);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) store_codes4<VEC, LANES>(v[i], s, inv, q + (r + i * kStep) * N, strip0, lane, N);
+  }
+  for (; r < hi; r += kStep) {
+    float v[4];
+    load_cols4<VEC, LANES>(v, w + r * N, strip0, lane, N);
+    store_codes4<VEC, LANES>(v, s, inv, q + r * N, strip0, lane, N);
   }
 }
 
@@ -114,41 +212,88 @@ __device__ __forceinline__ uint32_t trunc_bf16(int q, float s) {
   return __float_as_uint(__fmul_rn((float)q, s)) >> 16;
 }
 
+// VEC: a lane's eight columns are consecutive (one 8-byte load, one 16-byte store), else 32 apart.
+template <bool VEC>
 __global__ void __launch_bounds__(256) dequant_kernel(const int8_t* __restrict__ q, const float* __restrict__ scales,
-                                                       int64_t K, int64_t N, int64_t G, int vec,
+                                                       int64_t K, int64_t N, int64_t G, unsigned strips,
                                                        uint16_t* __restrict__ out) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (vec) {
-    const int64_t n8 = K * N / 8;
-    for (; i < n8; i += stride) {
-      const int64_t e = i * 8, r = e / N, c = e % N;
-      const uint2 p = *reinterpret_cast<const uint2*>(q + e);
-      const float* srow = scales + (r / G) * N + c;
-      const float4 s0 = *reinterpret_cast<const float4*>(srow), s1 = *reinterpret_cast<const float4*>(srow + 4);
-      const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-      uint32_t h[8];
+  constexpr int RPT = DEQ_ROWS / 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned y = blockIdx.x / strips;
+  const int64_t strip0 = (int64_t)(blockIdx.x - y * strips) * DEQ_COLS, r0 = (int64_t)y * DEQ_ROWS;
+  auto col = [&](int j) -> int64_t { return VEC ? strip0 + lane * 8 + j : strip0 + lane + 32 * j; };
+  uint2 p[RPT];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t word = j < 4 ? p.x : p.y;
-        h[j] = trunc_bf16((int)(int8_t)((word >> (8 * (j & 3))) & 0xffu), s[j]);
-      }
-      *reinterpret_cast<uint4*>(out + e) =
-          make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+  for (int i = 0; i < RPT; ++i) {
+    const int64_t r = r0 + warp + 8 * i;
+    p[i] = make_uint2(0u, 0u);
+    if (r >= K) continue;
+    if (VEC) {
+      if (col(0) < N) p[i] = *reinterpret_cast<const uint2*>(q + r * N + col(0));
+    } else {
+      uint32_t h[2] = {0u, 0u};
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col(j) < N) h[j >> 2] |= (uint32_t)(uint8_t)q[r * N + col(j)] << (8 * (j & 3));
+      p[i] = make_uint2(h[0], h[1]);
     }
-  } else {
-    const int64_t n = K * N;
-    for (; i < n; i += stride) {
-      const int64_t r = i / N, c = i % N;
-      out[i] = (uint16_t)trunc_bf16((int)q[i], scales[(r / G) * N + c]);
+  }
+  float s[8];
+  int64_t g_have = -1, g_end = 0;  // the group whose scales are held, and its first row past the end
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int64_t r = r0 + warp + 8 * i;
+    if (r >= K) break;
+    if (g_have < 0 || r >= g_end) {  // (uniform over the warp)
+      g_have = r / G;
+      g_end = (g_have + 1) * G;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s[j] = 0.f;
+      if (VEC) {
+        if (col(0) < N) {
+          const float4* sp = reinterpret_cast<const float4*>(scales + g_have * N + col(0));
+          const float4 a = sp[0], b = sp[1];
+          s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w;
+          s[4] = b.x; s[5] = b.y; s[6] = b.z; s[7] = b.w;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (col(j) < N) s[j] = scales[g_have * N + col(j)];
+      }
+    }
+    uint32_t h[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t word = j < 4 ? p[i].x : p[i].y;
+      h[j] = trunc_bf16((int)(int8_t)((word >> (8 * (j & 3))) & 0xffu), s[j]);
+    }
+    if (VEC) {
+      if (col(0) < N)
+        *reinterpret_cast<uint4*>(out + r * N + col(0)) =
+            make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col(j) < N) out[r * N + col(j)] = (uint16_t)h[j];
     }
   }
 }
 
-inline unsigned grid_for(int64_t work_items) {
-  const int64_t blocks = (work_items + 255) / 256;
-  const int64_t cap = 148LL * 32;  // enough blocks in flight to cover HBM latency; the loops stride
-  return (unsigned)(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
+template <bool VEC>
+int launch_quantize(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, float* scales, cudaStream_t s) {
+  const int64_t groups = (K + G - 1) / G;
+  const bool tall = G > GROUP_ROWS_MAX;
+  const int cols = tall ? TALL_COLS : COLS_PER_BLOCK;
+  const int64_t strips = (N + cols - 1) / cols;
+  if (strips > 0x7fffffffLL / (tall ? TALL_CTAS : 1) / groups) return ATENIA_ERR_SHAPE;
+  const unsigned grid = (unsigned)(strips * groups * (tall ? TALL_CTAS : 1)), st = (unsigned)strips;
+  if (tall) quantize_tall_kernel<VEC><<<grid, TALL_WARPS * 32, 0, s>>>(w, K, N, G, strips, q, scales);
+  else if (G <= 32) quantize_groups_kernel<VEC, 8, 4><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
+  else if (G <= 64) quantize_groups_kernel<VEC, 8, 8><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
+  else quantize_groups_kernel<VEC, 16, 8><<<grid, 512, 0, s>>>(w, K, N, (int)G, st, q, scales);
+  count_launch();
+  return (int)cudaGetLastError();
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -164,25 +309,10 @@ int atenia_quantize_per_group_i8(const float* w, int64_t K, int64_t N, int64_t g
   if (K < 0 || N < 0 || group_size < 0) return ATENIA_ERR_SHAPE;
   if (K == 0 || N == 0) return ATENIA_OK;
   if (!w || !q || !scales) return ATENIA_ERR_NULL;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int64_t G = (group_size == 0 || group_size > K) ? K : group_size;
-  const int64_t groups = (K + G - 1) / G;
-  const int64_t strips = (N + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK;
-  const int64_t cpg = (G + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
-  const int64_t blocks = strips * groups * cpg;
-  if (blocks > 0x7fffffffLL || groups * N > 0x7fffffffLL * 4) return ATENIA_ERR_SHAPE;
-  ATENIA_CUDA_TRY(cudaMemsetAsync(scales, 0, (size_t)(groups * N) * sizeof(float), s));
-  const int vec_w = (N % 4 == 0 && aligned16(w)) ? 1 : 0;
-  amax_kernel<<<(unsigned)blocks, 256, 0, s>>>(w, K, N, G, strips, cpg, vec_w, reinterpret_cast<unsigned int*>(scales));
-  count_launch();
-  ATENIA_CUDA_TRY(cudaGetLastError());
-  finalize_scales_kernel<<<grid_for(groups * N), 256, 0, s>>>(scales, groups * N);
-  count_launch();
-  ATENIA_CUDA_TRY(cudaGetLastError());
-  const int vec_q = (vec_w && aligned16(scales) && (reinterpret_cast<uintptr_t>(q) & 3u) == 0) ? 1 : 0;
-  quantize_kernel<<<grid_for(vec_q ? K * N / 4 : K * N), 256, 0, s>>>(w, scales, K, N, G, vec_q, q);
-  count_launch();
-  return (int)cudaGetLastError();
+  const bool vec = N % 4 == 0 && aligned16(w) && (reinterpret_cast<uintptr_t>(q) & 3u) == 0;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return vec ? launch_quantize<true>(w, K, N, G, q, scales, s) : launch_quantize<false>(w, K, N, G, q, scales, s);
 }
 
 int atenia_int8_to_bf16_per_group(const int8_t* q, const float* scales, int64_t K, int64_t N, int64_t group_size,
@@ -192,11 +322,14 @@ int atenia_int8_to_bf16_per_group(const int8_t* q, const float* scales, int64_t 
   if (K == 0 || N == 0) return ATENIA_OK;
   if (!q || !scales || !out_bf16) return ATENIA_ERR_NULL;
   const int64_t G = (group_size == 0 || group_size > K) ? K : group_size;
-  const int vec = (N % 8 == 0 && aligned16(out_bf16) && aligned16(scales) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0)
-                      ? 1
-                      : 0;
-  dequant_kernel<<<grid_for(vec ? K * N / 8 : K * N), 256, 0, static_cast<cudaStream_t>(stream)>>>(q, scales, K, N, G,
-                                                                                                      vec, out_bf16);
+  const int64_t strips = (N + DEQ_COLS - 1) / DEQ_COLS, chunks = (K + DEQ_ROWS - 1) / DEQ_ROWS;
+  if (strips > 0x7fffffffLL / chunks) return ATENIA_ERR_SHAPE;
+  const unsigned grid = (unsigned)(strips * chunks);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (N % 8 == 0 && aligned16(out_bf16) && aligned16(scales) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0)
+    dequant_kernel<true><<<grid, 256, 0, s>>>(q, scales, K, N, G, (unsigned)strips, out_bf16);
+  else
+    dequant_kernel<false><<<grid, 256, 0, s>>>(q, scales, K, N, G, (unsigned)strips, out_bf16);
   count_launch();
   return (int)cudaGetLastError();
 }

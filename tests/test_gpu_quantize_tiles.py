@@ -1,0 +1,36 @@
+"""The quantisers at the edges of their tiles, bit for bit against the oracle: groups of 32 / 64 / 128 rows and
+one more, column strips of 128 and one more, rows of one block width and beyond what registers hold."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("K,N,g", [(33, 128, 32), (65, 129, 64), (127, 132, 64), (256, 127, 128), (129, 260, 129),
+                                   (257, 124, 0), (1281, 66, 0), (1000, 520, 300), (1, 5, 1)])
+def test_group_quantiser_and_dequant_at_tile_edges(K, N, g):
+    import torch
+    from ateniaengine_b200 import int8_to_bf16_per_group, quantize_per_group_i8
+    from oracle import oracle as orc
+    w = torch.randn((K, N), generator=torch.Generator().manual_seed(K + N)) * 0.02
+    q, s = quantize_per_group_i8(w.cuda(), g)
+    q_ref, s_ref = orc.absmax_per_group_symmetric(w.numpy(), g)
+    np.testing.assert_array_equal(s.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
+    np.testing.assert_array_equal(q.cpu().numpy(), q_ref)
+    out = int8_to_bf16_per_group(q, s, g).view(torch.int16).cpu().numpy().view(np.uint16)
+    np.testing.assert_array_equal(out, np.asarray(orc.int8_to_bf16_per_group(q_ref, s_ref, g), dtype=np.uint16))
+
+
+@pytest.mark.parametrize("rows,cols", [(3, 1), (5, 255), (4, 4096), (3, 4100), (3, 8195), (2, 16384), (2, 16400),
+                                       (2, 20001)])
+def test_row_quantiser_at_block_edges(rows, cols):
+    import torch
+    from ateniaengine_b200 import quantize_per_row_i8
+    from oracle import oracle as orc
+    w = torch.randn((rows, cols), generator=torch.Generator().manual_seed(rows * cols)) * 0.02
+    w[0] = 0.0
+    w[-1, -1] = 2.0  # the maximum in the last column
+    q, s = quantize_per_row_i8(w.cuda())
+    q_ref, s_ref = orc.quantize_per_row_i8(w.numpy())
+    np.testing.assert_array_equal(s.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
+    np.testing.assert_array_equal(q.cpu().numpy(), q_ref)
