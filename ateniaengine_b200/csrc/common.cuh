@@ -127,6 +127,14 @@ int launch_combine(const CombineArgs& a, cudaStream_t s);
 // B matrices are row-major [N, K] (K contiguous): the reference's weight layout.
 enum GemmMode { kSwiGLU = 0, kPlain = 1 };
 
+// Token rows of the CTA-pair kernel: the same buffer in boxes of several heights, of which a tile takes the
+// smallest that holds half of it.
+constexpr int kPairBoxes = 8;
+__host__ __device__ constexpr int pair_box_rows(int i) { return 16 * (i + 1); }
+struct PairRowMaps {
+  CUtensorMap box[kPairBoxes];
+};
+
 struct GroupedGemmArgs {
   CUtensorMap tmap_a;              // A [rows_cap, K] bf16, box {64, 128}, 128B swizzle
   const CUtensorMap* tmap_b0;      // device array [num_groups]
@@ -141,6 +149,7 @@ struct GroupedGemmArgs {
   const float* const* scale1;
   DeviceError* err;
   int max_rows;  // upper bound on total rows (sizes nothing; used by the checking kernel's grid)
+  const PairRowMaps* pair_rows;  // CTA-pair kernel only (host pointer, copied at the launch)
   int w8;        // B matrices are int8 (tensor maps of bytes), widened to bf16 inside the kernel
   float* splitk_ws;  // W8 tensor-memory kernel: workspace for stream-K partial sums (null: whole tiles only)
   // stream-K decode kernels: zeroed counters [kSplitKMaxTiles * 8] with which the kernel finishes the split
@@ -182,6 +191,7 @@ int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y,
 // Tensor-map encoding through the driver entry point (no link-time dependency on libcuda).
 int encode_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
                         uint32_t box_rows, uint32_t box_cols);
+int encode_pair_rows(PairRowMaps* out, const void* base, uint64_t rows, uint64_t cols);  // grouped_gemm_2cta.cu
 // int8 matrix [rows, cols]; unswizzled box, or 64-byte swizzle for the row-per-thread reads of the
 // TMEM-operand kernel
 int encode_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
@@ -217,7 +227,9 @@ struct DigitSource {
 };
 int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, int n_rows, int K, int plane_rows,
                            int8_t* planes, float* tok_scale, cudaStream_t s);
-// bf16 weights, CTA pairs (tcgen05 cta_group::2): 256-row tiles, each CTA stages half of the weight tile
+// bf16 weights, CTA pairs (tcgen05 cta_group::2), transposed product: pair_rows describes the token rows (tmap_a
+// is not read), tmap_b0 / tmap_b1 have boxes of kPairWeightRows (kSwiGLU) or 128 (kPlain) weight rows
+constexpr int kPairWeightRows = 64;
 int launch_grouped_gemm_2cta(const GroupedGemmArgs& a, int num_sms, cudaStream_t s);
 
 // Sub-batch sizes for the host-buffer operator (planner.cu): n tokens in pieces of at most cap tokens,

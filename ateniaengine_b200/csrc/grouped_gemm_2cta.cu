@@ -1,37 +1,52 @@
-// Grouped expert GEMM for bf16 weights with CTA pairs (tcgen05 cta_group::2).
+// Grouped expert GEMM for bf16 weights with CTA pairs (tcgen05 cta_group::2), transposed: the weights are
+// the M side, the token rows the N side of the MMA.
 //
-// Two CTAs on the two SMs of a TPC form a cluster and work on one 256-row x 256-column MMA tile:
-// each CTA stages its own 128 token rows (A) and only HALF of the weight tile (B: the gate rows in
-// rank 0 and the up rows in rank 1 for kSwiGLU; the two 128-row halves of W_down for kPlain).  One
-// thread of the leader CTA issues tcgen05.mma.cta_group::2 (M256 x N256 x K16), which reads A and B
-// from both CTAs' shared memory and accumulates each CTA's 128 rows in that CTA's tensor memory.
-// Per CTA a k-block costs 32 KiB of L2->shared traffic instead of 48 KiB, for the same math: the
-// single-CTA kernel is limited by how many bytes it can keep in flight, this one by the tensor pipe.
+// Two CTAs on the two SMs of a TPC form a cluster and compute D[f, t] = sum_k W[f, k] X[t, k] for 256 weight
+// rows (128 in each CTA's tensor memory) and a token tile of n <= 256 rows, n a multiple of 16.  Each CTA
+// stages its own 128 weight rows and half of the token tile; one thread of the leader CTA issues
+// tcgen05.mma.cta_group::2 (M256 x Nn x K16), which reads both operands from both CTAs' shared memory.
 //
+// Why transposed: the M side of an MMA costs 256 rows however few hold data, the N side costs what it is
+// wide.  A group of R rows is cut into ceil(R / 256) equal token tiles rounded up to 16 rows, so the padding
+// is below 16 rows per tile.
+//
+//   kSwiGLU : 256 weight rows = 128 features; a CTA's 128 rows are 64 rows of W_gate and the same 64 of W_up,
+//             so the epilogue warps of lane quarters q and q + 2 hold gate and up of the same features and
+//             exchange them through shared memory (f32), each finishing half of the tokens
+//   kPlain  : 256 weight rows = 256 features
+//   k-block : 64 (one 128-byte swizzle row): 16 KiB of weights + at most 16 KiB of tokens per CTA, 6 stages
+//
+// What bounds it: the tensor pipe and the board's power.  ncu, DeepSeek-V2-Lite shape, 8192 tokens, gate/up: the
+// pipe is busy 90 % of 524 k cycles (75 % of 626 k with the issuing lane under `lane == 0`, see uniform_warp;
+// 67 % of 701 k with two token tiles per weight tile and 16-byte stores through shared memory).  One forward on a
+// B200, before (token-major 256-row pair tiles from 512 rows per group, 128-row single-CTA tiles below) and now:
+// Mixtral shape 256 / 4096 tokens 548 -> 514 / 2710 -> 2605 us (power-capped), Qwen1.5-MoE shape 2048 tokens
+// 453 -> 410, DeepSeek-V2-Lite shape 61 / 8192 tokens 284 -> 263 / 1259 -> 1193, a 512-wide layer of 64 tokens
+// 53.6 -> 50.1.
 // No TMA multicast is used: every CTA fetches its own tiles (cp.async.bulk.tensor ... cta_group::2
 // only routes the completion to the leader's mbarrier).
 //
 // Barriers: full[s] lives in the leader and collects the bytes of both CTAs; empty[s] and
 // acc_full[b] exist in both CTAs and are signalled by tcgen05.commit with a CTA mask; acc_empty[b]
 // lives in the leader and is arrived on by the epilogue warps of both CTAs.
-// Tiles are pairs of 128-row m-tiles of one expert; a pair whose second half lies past the expert's
-// rows still runs (the MMA is one instruction for both) and masks its stores.
 #include "tc_common.cuh"
 
 namespace atenia {
 namespace {
 using namespace tc;
 
-constexpr int BN2 = 256;
-constexpr int PAIR_ROWS = 2 * BM;  // 256
+constexpr int TN2 = 256;     // token rows of a tile at most (MMA N)
 constexpr int STAGES2 = 6;
 constexpr int ACC_BUFS2 = 2;
 constexpr int TMEM_COLS2 = 512;
-constexpr int A_BYTES2 = BM * BK * 2;         // 16 KiB
-constexpr int BH_BYTES2 = (BN2 / 2) * BK * 2; // 16 KiB: this CTA's half of the weight tile
-constexpr int STAGE_BYTES2 = A_BYTES2 + BH_BYTES2;
-constexpr int NUM_THREADS2 = 192;
-constexpr int SMEM_BYTES2 = STAGES2 * STAGE_BYTES2 + 1024 + 256;
+constexpr int W_BYTES2 = BM * BK * 2;         // 16 KiB: this CTA's 128 weight rows
+constexpr int X_BYTES2 = (TN2 / 2) * BK * 2;  // 16 KiB: this CTA's half of the token tile
+constexpr int STAGE_BYTES2 = W_BYTES2 + X_BYTES2;
+constexpr int EPI_WARPS2 = 8;
+constexpr int NUM_THREADS2 = 64 + EPI_WARPS2 * 32;
+constexpr int EPI_WARP_BYTES2 = 2 * 1024;  // kSwiGLU: two buffers of 8 tokens x 32 features of f32 per warp
+constexpr int EPI_BYTES2 = EPI_WARPS2 * EPI_WARP_BYTES2;
+constexpr int SMEM_BYTES2 = STAGES2 * STAGE_BYTES2 + EPI_BYTES2 + 1024 + 256;
 
 struct __align__(8) Barriers2 {
   uint64_t full[STAGES2];
@@ -42,9 +57,47 @@ struct __align__(8) Barriers2 {
   int abort_flag;
 };
 
-// D f32, A = B = bf16, K-major, M = 256 (per pair), N = 256.
-constexpr uint32_t kInstrDesc2 = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(BN2 >> 3) << 17) |
-                                 (uint32_t(PAIR_ROWS >> 4) << 24);
+// D f32, A = B = bf16, K-major, M = 256 (per pair); N is added per tile.
+constexpr uint32_t kInstrDesc2 = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(256 >> 4) << 24);
+
+// ---- tile walk: the token tiles of one group are equal, so none is a nearly empty remainder ----
+struct PairCursor {
+  int group, base;  // current group, first tile index of it
+  int m_tiles, tile_rows;
+  int row_begin, row_end;
+};
+struct PairTile {
+  int group, row0, rows, f0;  // first row and rows of the tile, first feature
+  int n;                      // MMA N: rows rounded up to 16
+};
+__device__ __forceinline__ void pair_cursor_load(PairCursor& c, const int32_t* __restrict__ off) {
+  c.row_begin = off[c.group];
+  c.row_end = off[c.group + 1];
+  const int rows = c.row_end - c.row_begin;
+  c.m_tiles = (rows + TN2 - 1) / TN2;
+  c.tile_rows = c.m_tiles > 0 ? ((rows + c.m_tiles - 1) / c.m_tiles + 15) & ~15 : 16;
+}
+__device__ __forceinline__ bool pair_cursor_seek(PairCursor& c, int tile, int f_tiles, int num_groups,
+                                                 const int32_t* __restrict__ off, PairTile& out, int f_width) {
+  while (c.group < num_groups) {
+    const int here = c.m_tiles * f_tiles;
+    if (tile < c.base + here) {
+      const int local = tile - c.base;
+      const int ft = local / c.m_tiles;  // token tiles of one weight tile are neighbours: they share it in L2
+      const int mt = local - ft * c.m_tiles;
+      out.group = c.group;
+      out.row0 = c.row_begin + mt * c.tile_rows;
+      out.rows = min(c.row_end - out.row0, c.tile_rows);  // >= 1: tile_rows <= 256, so no tile starts past the end
+      out.n = (out.rows + 15) & ~15;
+      out.f0 = ft * f_width;
+      return true;
+    }
+    c.base += here;
+    c.group += 1;
+    if (c.group < num_groups) pair_cursor_load(c, off);
+  }
+  return false;
+}
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -64,20 +117,33 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The following run in a converged warp; one lane (always the same) issues the instruction.
 // TMA load whose completion bytes go to an mbarrier that may live in the peer CTA of the pair.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster, int x,
                                                  int y) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      "{\n\t.reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate) {
+// The four MMAs (K = 16 each, 32 bytes apart inside the swizzle row) of one k-block.
+__device__ __forceinline__ void tc_mma_bf16_pair_kblock(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                        uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred e, p, t;\n\t"
+      ".reg .b64 a, b;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "add.s64 a, %1, 2;\n\tadd.s64 b, %2, 2;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 4;\n\tadd.s64 b, %2, 4;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 6;\n\tadd.s64 b, %2, 6;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
@@ -85,33 +151,40 @@ __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t a_des
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
   const uint16_t mask = 3;
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+      "{\n\t.reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
       ::"r"(bar), "h"(mask)
       : "memory");
 }
 
+// the box (index of PairRowMaps) that holds the half sub-tile a CTA stages
+__device__ __forceinline__ int pair_box(int half_rows) { return (half_rows + 15) / 16 - 1; }
+
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS2, 1)
-grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const CUtensorMap* __restrict__ tmap_b0,
-                         const CUtensorMap* __restrict__ tmap_b1, const int32_t* __restrict__ group_offsets_g,
+grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUtensorMap* __restrict__ tmap_w0,
+                         const CUtensorMap* __restrict__ tmap_w1, const int32_t* __restrict__ group_offsets_g,
                          int num_groups, int N, int K, __nv_bfloat16* __restrict__ out, DeviceError* err) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int32_t goff_s[kMaxGroupsShared + 1];
   const int32_t* group_offsets = stage_group_offsets(group_offsets_g, num_groups, goff_s);
-  constexpr int BN_OUT = (MODE == kSwiGLU) ? BN2 / 2 : BN2;
+  constexpr int F_CTA = (MODE == kSwiGLU) ? BM / 2 : BM;  // output features per CTA
+  constexpr int F_PAIR = 2 * F_CTA;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
-  Barriers2* bars = reinterpret_cast<Barriers2*>(smem_aligned + STAGES2 * STAGE_BYTES2);
+  uint8_t* epi = smem_aligned + STAGES2 * STAGE_BYTES2;
+  Barriers2* bars = reinterpret_cast<Barriers2*>(epi + EPI_BYTES2);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   const int num_kb = (K + BK - 1) / BK;
-  const int n_tiles = (N + BN_OUT - 1) / BN_OUT;
+  const int f_tiles = (N + F_PAIR - 1) / F_PAIR;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES2; ++s) {
@@ -120,7 +193,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const CUten
     }
     for (int b = 0; b < ACC_BUFS2; ++b) {
       mbar_init(smem_u32(&bars->acc_full[b]), 1);
-      mbar_init(smem_u32(&bars->acc_empty[b]), 8);  // 4 epilogue warps of each CTA
+      mbar_init(smem_u32(&bars->acc_empty[b]), 2 * EPI_WARPS2);  // the epilogue warps of both CTAs
     }
     bars->abort_flag = 0;
     fence_barrier_init();
@@ -138,93 +211,96 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const CUten
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
-  TileCursor cur;
+  PairCursor cur;
   cur.group = 0;
   cur.base = 0;
-  if (num_groups > 0) cursor_load(cur, group_offsets, PAIR_ROWS);
-  TileCoord tc;
+  if (num_groups > 0) pair_cursor_load(cur, group_offsets);
+  PairTile tc;
 
   if (warp == 0) {
     // ================= TMA producer (both CTAs) =================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int last_group = -1;
-      uint32_t armed = 0;
-      bool ok = true;
-      for (int tile = pair; ok && cursor_seek(cur, tile, n_tiles, num_groups, group_offsets, tc, BN_OUT, PAIR_ROWS);
-           tile += num_pairs) {
-        // this CTA's half of the weight tile
-        const CUtensorMap* mb;
-        int nb;
-        if (MODE == kSwiGLU) {
-          mb = leader ? &tmap_b0[tc.group] : &tmap_b1[tc.group];
-          nb = tc.n0;
-        } else {
-          mb = &tmap_b0[tc.group];
-          nb = tc.n0 + (leader ? 0 : BN2 / 2);
+    int stage = 0;
+    uint32_t phase = 0;
+    int last_group = -1;
+    uint32_t armed = 0;  // stages with a copy possibly in flight
+    bool ok = true;
+    for (int tile = pair; ok && pair_cursor_seek(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
+         tile += num_pairs) {
+      const CUtensorMap* m0 = &tmap_w0[tc.group];
+      const CUtensorMap* m1 = MODE == kSwiGLU ? &tmap_w1[tc.group] : m0;
+      if (tc.group != last_group) {
+        tmap_acquire(m0);
+        if (MODE == kSwiGLU) tmap_acquire(m1);
+        last_group = tc.group;
+      }
+      const int box = pair_box(tc.n / 2);
+      const CUtensorMap* mx = &tmaps_x.box[box];
+      const int f_row = tc.f0 + (int)rank * F_CTA;
+      const int x_row = tc.row0 + (int)rank * (tc.n / 2);
+      const uint32_t tx = 2 * (W_BYTES2 + pair_box_rows(box) * BK * 2);  // bytes of both CTAs
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag)) {
+          if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1100 + stage);
+          *abort_flag = 1;
+          ok = false;
         }
-        if (tc.group != last_group) {
-          tmap_acquire(mb);
-          last_group = tc.group;
-        }
-        const int my_row0 = tc.row0 + (int)rank * BM;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag)) {
-            report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1100 + stage);
-            *abort_flag = 1;
-            ok = false;
-            break;
-          }
-          const uint32_t full_local = smem_u32(&bars->full[stage]);
-          const uint32_t full_leader = mapa(full_local, 0);
-          const uint32_t sa = smem_base + stage * STAGE_BYTES2;
-          const uint32_t sb = sa + A_BYTES2;
-          if (leader) mbar_expect_tx(full_local, 2 * STAGE_BYTES2);  // bytes of both CTAs
-          tma_load_2d_pair(sa, &tmap_a, full_leader, kb * BK, my_row0);
-          tma_load_2d_pair(sb, mb, full_leader, kb * BK, nb);
-          armed |= 1u << stage;
-          if (++stage == STAGES2) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        const uint32_t full_local = smem_u32(&bars->full[stage]);
+        const uint32_t full_leader = mapa(full_local, 0);
+        const uint32_t dst = smem_base + stage * STAGE_BYTES2;
+        if (leader) mbar_expect_tx_one(full_local, tx);
+        tma_load_2d_pair(dst, m0, full_leader, kb * BK, f_row);
+        if (MODE == kSwiGLU) tma_load_2d_pair(dst + W_BYTES2 / 2, m1, full_leader, kb * BK, f_row);
+        tma_load_2d_pair(dst + W_BYTES2, mx, full_leader, kb * BK, x_row);
+        armed |= 1u << stage;
+        if (++stage == STAGES2) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      (void)armed;
+    }
+    if (*abort_flag && leader && lane == 0) {
+      // let the copies already issued (both CTAs') land before the pair's shared memory is released
+      for (int s = 0; s < STAGES2; ++s) {
+        if (!(armed & (1u << s))) continue;
+        const uint32_t par = s < stage ? phase : phase ^ 1u;
+        for (int i = 0; i < (1 << 16) && !mbar_try_wait(smem_u32(&bars->full[s]), par); ++i) {}
+      }
     }
   } else if (warp == 1) {
     // ================= MMA issuer (leader CTA only) =================
-    if (leader && lane == 0) {
+    if (leader) {
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t acc_phase[ACC_BUFS2] = {0, 0};
+      uint32_t acc_phase = 0;  // bit b: accumulator b
       int it = 0;
       bool ok = true;
-      for (int tile = pair; ok && cursor_seek(cur, tile, n_tiles, num_groups, group_offsets, tc, BN_OUT, PAIR_ROWS);
+      for (int tile = pair; ok && pair_cursor_seek(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
            tile += num_pairs, ++it) {
         const int acc = it & 1;
-        if (!mbar_wait(smem_u32(&bars->acc_empty[acc]), acc_phase[acc] ^ 1u, abort_flag)) {
-          report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1200 + acc);
+        if (!mbar_wait(smem_u32(&bars->acc_empty[acc]), ((acc_phase >> acc) & 1u) ^ 1u, abort_flag)) {
+          if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1200 + acc);
           *abort_flag = 1;
-          break;
+          ok = false;
         }
-        acc_phase[acc] ^= 1u;
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        acc_phase ^= 1u << acc;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN2;
+        const uint32_t d_tmem = tmem_base + acc * TN2;
+        const uint32_t idesc = kInstrDesc2 | (uint32_t(tc.n >> 3) << 17);
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag)) {
-            report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1300 + stage);
+            if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1300 + stage);
             *abort_flag = 1;
             ok = false;
-            break;
           }
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           tc_fence_after();
           const uint32_t sa = smem_base + stage * STAGE_BYTES2;
-          const uint64_t da = make_smem_desc(sa);
-          const uint64_t db = make_smem_desc(sa + A_BYTES2);
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            tc_mma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, kInstrDesc2, (kb > 0 || k > 0) ? 1u : 0u);
+          tc_mma_bf16_pair_kblock(d_tmem, make_smem_desc(sa), make_smem_desc(sa + W_BYTES2), idesc, kb > 0 ? 1u : 0u);
           tc_commit_pair(smem_u32(&bars->empty[stage]));
           if (++stage == STAGES2) {
             stage = 0;
@@ -235,59 +311,76 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const CUten
       }
     }
   } else {
-    // ================= epilogue (warps 2..5 of both CTAs) =================
-    const int quarter = warp & 3;
-    const int row_in_tile = quarter * 32 + lane;
-    uint32_t acc_phase[ACC_BUFS2] = {0, 0};
+    // ================= epilogue (warps 2..9 of both CTAs) =================
+    // A lane holds one weight row; the columns are token rows.  A value is stored from where it is, two bytes
+    // per lane and 64 contiguous bytes per warp and token: passing the tile through shared memory for 16-byte
+    // stores costs the MMAs more shared-memory cycles than it saves stores.
+    // kSwiGLU: the warps of quarters q (gates) and q + 2 (ups) swap eight tokens of f32 first: the gate warp
+    // finishes tokens 0..7 of a chunk of 16, the up warp tokens 8..15.
+    const int quarter = warp & 3;         // TMEM lanes [32 * quarter, 32 * quarter + 32)
+    const int first = ((warp - 2) >> 2);  // two warps per quarter take the 16-token chunks in turn
+    float* mine = reinterpret_cast<float*>(epi + (warp - 2) * EPI_WARP_BYTES2);
+    const bool up = MODE == kSwiGLU && quarter >= 2;
+    // the other warp of the pair: same `first`, quarter +- 2 (warps 2..5 hold quarters 2, 3, 0, 1)
+    const float* theirs = reinterpret_cast<const float*>(epi + ((warp - 2) ^ 2) * EPI_WARP_BYTES2);
+    const int f_lane = (int)rank * F_CTA + (MODE == kSwiGLU ? (quarter & 1) * 32 : quarter * 32) + lane;
+    const uint32_t pair_bar = 1 + first * 2 + (quarter & 1);
+    int flip = 0;
+    uint32_t acc_phase = 0;
     int it = 0;
-    for (int tile = pair; cursor_seek(cur, tile, n_tiles, num_groups, group_offsets, tc, BN_OUT, PAIR_ROWS);
+    for (int tile = pair; pair_cursor_seek(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
          tile += num_pairs, ++it) {
       const int acc = it & 1;
-      if (!mbar_wait(smem_u32(&bars->acc_full[acc]), acc_phase[acc], abort_flag)) {
+      bool ready = mbar_wait(smem_u32(&bars->acc_full[acc]), (acc_phase >> acc) & 1u, abort_flag);
+      if (MODE == kSwiGLU) {
+        // the two warps of a pair leave together or not at all: one of them alone would hold the other in bar.sync
+        uint32_t both;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.ne.b32 p, %1, 0;\n\t"
+            "bar.red.and.pred q, %2, 64, p;\n\t"
+            "selp.b32 %0, 1, 0, q;\n\t}"
+            : "=r"(both)
+            : "r"((uint32_t)ready), "r"(pair_bar)
+            : "memory");
+        ready = both != 0;
+      }
+      if (!ready) {
         if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1400 + acc);
         *abort_flag = 1;
         break;
       }
-      acc_phase[acc] ^= 1u;
+      acc_phase ^= 1u << acc;
       tc_fence_after();
-      const int grow = tc.row0 + (int)rank * BM + row_in_tile;
-      const bool row_ok = grow < tc.row_end;
-      const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc * BN2;
-      __nv_bfloat16* orow = out + (size_t)grow * N;
-      if (MODE == kSwiGLU) {
+      const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc * TN2;
+      const bool f_ok = tc.f0 + f_lane < N;
+      const int t_half = up ? 8 : 0;
+      __nv_bfloat16* dst = out + (size_t)(tc.row0 + t_half) * N + tc.f0 + f_lane;
+      const int rows = f_ok ? tc.rows - t_half : 0;  // tokens of the tile this lane may store
 #pragma unroll 1
-        for (int c = 0; c < BN_OUT; c += 16) {
-          uint32_t g[16], u[16];
-          tc_ld16(taddr + c, g);
-          tc_ld16(taddr + BN_OUT + c, u);
-          tc_ld_wait();
-          const int n = tc.n0 + c;
-          if (row_ok && n < N) {
-            uint32_t p[8];
+      for (int c = 16 * first; c < tc.n; c += 32) {
+        uint32_t v[16];
+        tc_ld16(taddr + c, v);
+        tc_ld_wait();
+        __nv_bfloat16* d = dst + (size_t)c * N;
+        if (MODE == kSwiGLU) {
+          float* ex = mine + flip * 256;
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              p[j] = pack_bf16x2(silu_mul(__uint_as_float(g[2 * j]), __uint_as_float(u[2 * j])),
-                                 silu_mul(__uint_as_float(g[2 * j + 1]), __uint_as_float(u[2 * j + 1])));
-            uint4* dst = reinterpret_cast<uint4*>(orow + n);
-            dst[0] = make_uint4(p[0], p[1], p[2], p[3]);
-            dst[1] = make_uint4(p[4], p[5], p[6], p[7]);
-          }
-        }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < BN_OUT; c += 16) {
-          uint32_t v[16];
-          tc_ld16(taddr + c, v);
-          tc_ld_wait();
-          const int n = tc.n0 + c;
-          if (row_ok && n < N) {
-            uint32_t p[8];
+          for (int j = 0; j < 8; ++j) ex[j * 32 + lane] = __uint_as_float(up ? v[j] : v[8 + j]);
+          asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
+          const float* ox = theirs + flip * 256;
+          flip ^= 1;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) p[j] = pack_bf16x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-            uint4* dst = reinterpret_cast<uint4*>(orow + n);
-            dst[0] = make_uint4(p[0], p[1], p[2], p[3]);
-            dst[1] = make_uint4(p[4], p[5], p[6], p[7]);
+          for (int j = 0; j < 8; ++j) {
+            const float o = ox[j * 32 + lane];
+            const float g = up ? o : __uint_as_float(v[j]);
+            const float u = up ? __uint_as_float(v[8 + j]) : o;
+            if (c + j < rows) d[(size_t)j * N] = __float2bfloat16(silu_mul(g, u));
           }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < rows) d[(size_t)j * N] = __float2bfloat16(__uint_as_float(v[j]));
         }
       }
       tc_fence_before();
@@ -315,16 +408,24 @@ int launch_2cta_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   }
   const int grid = num_sms & ~1;  // whole pairs
   grouped_gemm_2cta_kernel<MODE><<<dim3(grid), dim3(NUM_THREADS2), SMEM_BYTES2, s>>>(
-      a.tmap_a, a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out,
+      *a.pair_rows, a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out,
       a.err);
   return (int)cudaGetLastError();
 }
 
 }  // namespace
 
+int encode_pair_rows(PairRowMaps* out, const void* base, uint64_t rows, uint64_t cols) {
+  int rc = ATENIA_OK;
+  for (int i = 0; i < kPairBoxes && !rc; ++i)
+    rc = encode_tmap_2d_bf16(&out->box[i], base, rows, cols, pair_box_rows(i), BK);
+  return rc;
+}
+
 int launch_grouped_gemm_2cta(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   if (a.num_groups <= 0) return ATENIA_OK;
   if (a.N % 16 != 0 || a.K % 16 != 0) return ATENIA_ERR_SHAPE;
+  if (!a.pair_rows) return ATENIA_ERR_NULL;
   if (a.w8) return ATENIA_ERR_UNSUPPORTED;  // INT8 weights: w8_gemm.cu / w8_gemm_m256.cu
   int rc = a.mode == kSwiGLU ? launch_2cta_one<kSwiGLU>(a, num_sms, s) : launch_2cta_one<kPlain>(a, num_sms, s);
   count_launch();

@@ -7,6 +7,13 @@
 
 namespace atenia {
 struct EpComm;  // ep.cu: an NCCL communicator, destroyed with its last holder
+
+// Tensor maps of one bf16 row buffer: boxes of 128 rows, and those of the CTA-pair kernel (encoded for bf16
+// layers only: INT8 weights never take it)
+struct RowMaps {
+  CUtensorMap tile{};
+  PairRowMaps pair{};
+};
 }
 
 struct AteniaMoeLayer {
@@ -27,8 +34,7 @@ struct AteniaMoeLayer {
   // tile kernel of w8_gemm_m256.cu for large ones), 1 = always the small-group kernel,
   // 2 = always the 128-row shared-memory widening kernel (grouped_gemm.cu)
   int w8_mode = 0;
-  // bf16: 0 = pick per call (CTA-pair kernel once groups average >= 512 rows), 1 = always pairs,
-  // 2 = always the single-CTA kernel
+  // bf16: 0, 1 = the CTA-pair kernel, 2 = the single-CTA kernel of grouped_gemm.cu (cross-checks)
   int pair_mode = 0;
   // bf16 stream-K decode kernel: -1 = calls of at most 16 rows, 1 = every call of at most 128 rows
   // (ATENIA_MOE_BF16_DECODE=1), 0 = never (=0, or INT8 weights)
@@ -54,6 +60,10 @@ struct AteniaMoeLayer {
   CUtensorMap* d_tm_up = nullptr;
   CUtensorMap* d_tm_down = nullptr;
   CUtensorMap* d_tm_shared = nullptr;  // [3]: gate, up, down
+  // bf16 only: gate and up in boxes of kPairWeightRows rows, for the CTA-pair kernel
+  CUtensorMap* d_tm_gate_box = nullptr;    // [n_groups]
+  CUtensorMap* d_tm_up_box = nullptr;
+  CUtensorMap* d_tm_shared_box = nullptr;  // [2]: gate, up
   // INT8 only: the same matrices described with the 64-byte swizzle the tensor-memory kernel reads
   CUtensorMap* d_tm_gate_sw = nullptr;
   CUtensorMap* d_tm_up_sw = nullptr;
@@ -104,7 +114,7 @@ struct AteniaMoeLayer {
   atenia::DigitSource i8_src{};  // the caller's batch and the permutation, when the digit kernel does the row gather
   bool i8_src_set = false;
   float* splitk_ws_shared = nullptr;  // the same for the shared expert's launches (INT8 with a shared expert)
-  CUtensorMap tm_x_perm{}, tm_h{}, tm_h_shared{};
+  atenia::RowMaps tm_x_perm{}, tm_h{}, tm_h_shared{};
 
   // expert parallelism
   std::shared_ptr<atenia::EpComm> ep;  // layers of one stack may share a communicator (atenia_moe_ep_attach)
@@ -117,7 +127,7 @@ struct AteniaMoeLayer {
   int32_t* d_counts_all = nullptr;     // [world, E] rows per (source rank, expert)
   int32_t* h_counts_all = nullptr;     // pinned host copy
   int32_t* d_group_offsets = nullptr;  // [world * e_local + 1]
-  CUtensorMap tm_recv_x{}, tm_recv_h{};
+  atenia::RowMaps tm_recv_x{}, tm_recv_h{};
   // direct exchange (atenia_moe_ep_ipc_import): rows are stored straight into the owner's receive
   // buffer and results straight back into the source's y_perm through peer mappings
   bool ep_direct = false;
@@ -163,7 +173,7 @@ bool ep_ready(const AteniaMoeLayer* L);
 // ATENIA_ERR_NCCL, so a collective whose peer never arrives cannot block the host for ever.
 int ep_bounded_wait(AteniaMoeLayer* L, cudaStream_t s);
 void ep_destroy(AteniaMoeLayer* L);
-int run_expert_gemms(AteniaMoeLayer* L, const CUtensorMap& tm_a, const CUtensorMap& tm_mid,
+int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_mid,
                      const __nv_bfloat16* a_ptr, __nv_bfloat16* mid, __nv_bfloat16* out,
                      const int32_t* group_offsets, int num_groups, int max_rows, cudaStream_t s);
 }  // namespace atenia

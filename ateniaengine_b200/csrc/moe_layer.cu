@@ -47,7 +47,7 @@ int validate_config(const AteniaMoeConfig& c) {
 
 }  // namespace
 
-int run_expert_gemms(AteniaMoeLayer* L, const CUtensorMap& tm_a, const CUtensorMap& tm_mid,
+int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_mid,
                      const __nv_bfloat16* a_ptr, __nv_bfloat16* mid, __nv_bfloat16* out,
                      const int32_t* group_offsets, int num_groups, int max_rows, cudaStream_t s) {
   const AteniaMoeConfig& c = L->cfg;
@@ -60,12 +60,14 @@ int run_expert_gemms(AteniaMoeLayer* L, const CUtensorMap& tm_a, const CUtensorM
   // shared-memory widening kernel of grouped_gemm.cu (tests, A/B runs).
   const bool m256 = q && large && L->w8_mode != 1 && L->w8_mode != 2 && !L->use_check_gemm;
   const bool tmem = q && !m256 && (L->w8_mode == 1 || (L->w8_mode != 2 && !large));
-  // bf16: 256-row CTA-pair tiles pay off once an average group fills a few of them; a call of at most
+  // bf16: the CTA-pair kernel at every size above that of the decode kernel (its token tiles follow the row
+  // count: 61 tokens of a DeepSeek-V2-Lite shape 263 us against 284 with the single-CTA kernel, 64 tokens of a
+  // 512-wide layer 50 against 54); a call of at most
   // 16 rows (decode) takes the stream-K kernel of bf16_decode_gemm.cu, which spreads the few tiles
   // there are over all SMs (bf16_decode 1 / 0 pins it on for every call of at most 128 rows / off).
   const bool dec = !q && !L->use_check_gemm && L->splitk_ws &&
                    (L->bf16_decode == 1 ? max_rows <= 128 : (L->bf16_decode < 0 && max_rows <= 16));
-  const bool pairs = !q && !dec && (L->pair_mode == 1 || (L->pair_mode == 0 && max_rows >= 512 * num_groups));
+  const bool pairs = !q && !dec && L->pair_mode != 2;
   // a call of at most two rows in all (decode at batch 1) is a stream over the touched experts' weights:
   // the CUDA-core matrix-vector kernel (ATENIA_MOE_GEMV=0 keeps the tensor-core kernels: A/B runs)
   // INT8, calls of at most i8_rows rows (decode): the codes multiplied as integers against digit planes of
@@ -137,9 +139,10 @@ int run_expert_gemms(AteniaMoeLayer* L, const CUtensorMap& tm_a, const CUtensorM
     if (rc) return rc;
   } else {
     GroupedGemmArgs g1{};
-    g1.tmap_a = tm_a;
-    g1.tmap_b0 = tmem ? L->d_tm_gate_sw : L->d_tm_gate;
-    g1.tmap_b1 = tmem ? L->d_tm_up_sw : L->d_tm_up;
+    g1.tmap_a = tm_a.tile;
+    g1.pair_rows = &tm_a.pair;
+    g1.tmap_b0 = tmem ? L->d_tm_gate_sw : pairs ? L->d_tm_gate_box : L->d_tm_gate;
+    g1.tmap_b1 = tmem ? L->d_tm_up_sw : pairs ? L->d_tm_up_box : L->d_tm_up;
     g1.group_offsets = group_offsets;
     g1.num_groups = num_groups;
     g1.N = c.d_ff;
@@ -168,7 +171,8 @@ int run_expert_gemms(AteniaMoeLayer* L, const CUtensorMap& tm_a, const CUtensorM
     if (rc) return rc;
   } else {
     GroupedGemmArgs g2{};
-    g2.tmap_a = tm_mid;
+    g2.tmap_a = tm_mid.tile;
+    g2.pair_rows = &tm_mid.pair;
     g2.tmap_b0 = tmem ? L->d_tm_down_sw : L->d_tm_down;
     g2.tmap_b1 = g2.tmap_b0;
     g2.group_offsets = group_offsets;
@@ -207,7 +211,7 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   // 256-row-tile kernel above)
   const bool m256 = q && T >= 256 && L->w8_mode != 1 && L->w8_mode != 2 && !L->use_check_gemm;
   const bool tmem = q && !m256 && (L->w8_mode == 1 || (L->w8_mode != 2 && T < 256));
-  const bool pairs = !q && (L->pair_mode == 1 || (L->pair_mode == 0 && T >= 512));
+  const bool pairs = !q && L->pair_mode != 2;
   const bool gemv = L->use_gemv && T <= L->gemv_rows && !L->use_check_gemm;
   if (L->timing) cudaEventRecord(L->ev[3], s);
   if (L->use_check_gemm || gemv) {
@@ -228,9 +232,12 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
     return ATENIA_OK;
   }
   GroupedGemmArgs g1{};
-  int rc = encode_tmap_2d_bf16(&g1.tmap_a, xb, (uint64_t)T, (uint64_t)c.d_model, 128, 64);
+  PairRowMaps x_rows;
+  int rc = pairs ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model)
+                 : encode_tmap_2d_bf16(&g1.tmap_a, xb, (uint64_t)T, (uint64_t)c.d_model, 128, 64);
   if (rc) return rc;
-  g1.tmap_b0 = tmem ? L->d_tm_shared_sw : L->d_tm_shared;
+  g1.pair_rows = &x_rows;
+  g1.tmap_b0 = tmem ? L->d_tm_shared_sw : pairs ? L->d_tm_shared_box : L->d_tm_shared;
   g1.tmap_b1 = g1.tmap_b0 + 1;
   g1.group_offsets = L->shared_offsets;
   g1.num_groups = 1;
@@ -250,7 +257,8 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   if (rc) return rc;
   if (L->timing) cudaEventRecord(L->ev[4], s);
   GroupedGemmArgs g2{};
-  g2.tmap_a = L->tm_h_shared;
+  g2.tmap_a = L->tm_h_shared.tile;
+  g2.pair_rows = &L->tm_h_shared.pair;
   g2.tmap_b0 = (tmem ? L->d_tm_shared_sw : L->d_tm_shared) + 2;
   g2.tmap_b1 = g2.tmap_b0;
   g2.group_offsets = L->shared_offsets;
@@ -370,6 +378,11 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
   TRY_ALLOC(L->d_tm_up, (size_t)L->n_groups);
   TRY_ALLOC(L->d_tm_down, (size_t)L->n_groups);
   TRY_ALLOC(L->d_tm_shared, 3);
+  if (c.weight_dtype == ATENIA_W_BF16) {
+    TRY_ALLOC(L->d_tm_gate_box, (size_t)L->n_groups);
+    TRY_ALLOC(L->d_tm_up_box, (size_t)L->n_groups);
+    TRY_ALLOC(L->d_tm_shared_box, 2);
+  }
   if (L->bf16_decode != 0 || c.weight_dtype == ATENIA_W_INT8_ROW) {
     TRY_ALLOC(L->splitk_ws, (size_t)L->num_sms * 2 * kW8SplitKSlotFloats);
     // ATENIA_MOE_SPLITK_FIXUP=0: a second kernel adds the pieces of split tiles (A/B runs)
@@ -449,14 +462,19 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
     atenia_moe_destroy(L);
     return (int)e;
   }
-  rc = encode_tmap_2d_bf16(&L->tm_x_perm, L->x_perm, R, d, 128, 64);
-  if (!rc && L->h) rc = encode_tmap_2d_bf16(&L->tm_h, L->h, R, F, 128, 64);
+  auto row_maps = [&](RowMaps& m, const void* base, size_t rows, size_t cols) -> int {
+    int e = encode_tmap_2d_bf16(&m.tile, base, rows, cols, 128, 64);
+    if (!e && c.weight_dtype == ATENIA_W_BF16) e = encode_pair_rows(&m.pair, base, rows, cols);
+    return e;
+  };
+  rc = row_maps(L->tm_x_perm, L->x_perm, R, d);
+  if (!rc && L->h) rc = row_maps(L->tm_h, L->h, R, F);
   if (!rc && L->dq_x) rc = encode_tmap_2d_u8(&L->tm_dq_x, L->dq_x, (uint64_t)4 * L->i8_rows, d, 16, 128, 2);
   if (!rc && L->dq_h) rc = encode_tmap_2d_u8(&L->tm_dq_h, L->dq_h, (uint64_t)4 * L->i8_rows, F, 16, 128, 2);
-  if (!rc && L->has_shared) rc = encode_tmap_2d_bf16(&L->tm_h_shared, L->h_shared, Tm, Fs, 128, 64);
+  if (!rc && L->has_shared) rc = row_maps(L->tm_h_shared, L->h_shared, Tm, Fs);
   if (!rc && c.ep_world > 1) {
-    rc = encode_tmap_2d_bf16(&L->tm_recv_x, L->recv_x, (uint64_t)L->recv_cap, d, 128, 64);
-    if (!rc) rc = encode_tmap_2d_bf16(&L->tm_recv_h, L->recv_h, (uint64_t)L->recv_cap, F, 128, 64);
+    rc = row_maps(L->tm_recv_x, L->recv_x, (size_t)L->recv_cap, d);
+    if (!rc) rc = row_maps(L->tm_recv_h, L->recv_h, (size_t)L->recv_cap, F);
   }
   if (rc) {
     atenia_moe_destroy(L);
@@ -486,7 +504,7 @@ int atenia_moe_destroy(AteniaMoeLayer* L) {
                   L->h, L->y_perm, L->x_bf16, L->h_shared, L->y_shared, L->d_err, L->d_tm_gate, L->d_tm_up,
                   L->d_tm_down, L->d_tm_shared, L->d_sc_gate, L->d_sc_up, L->d_sc_down, L->d_sc_shared,
                   L->d_p_gate, L->d_p_up, L->d_p_down, L->d_p_shared, L->d_tm_gate_sw, L->d_tm_up_sw,
-                  L->d_tm_down_sw, L->d_tm_shared_sw,
+                  L->d_tm_down_sw, L->d_tm_shared_sw, L->d_tm_gate_box, L->d_tm_up_box, L->d_tm_shared_box,
                   L->splitk_ws, L->splitk_cnt, L->splitk_ws_shared, L->d_tm_gate_i8, L->d_tm_up_i8, L->d_tm_down_i8, L->dq_x, L->dq_h,
                   L->dq_ts_x, L->dq_ts_h, L->d_escore, L->logits_ws, L->recv_x, L->recv_h, L->recv_y, L->d_counts_all,
                   L->d_group_offsets, L->d_peer_recv_x, L->d_peer_y_perm, L->d_dst_base, L->d_src_base,
@@ -543,7 +561,7 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
   };
 
   const int G = L->n_groups, El = L->e_local;
-  std::vector<CUtensorMap> tg(G), tu(G), td(G), tgs(G), tus(G), tds(G), tgi(G), tui(G), tdi(G);
+  std::vector<CUtensorMap> tg(G), tu(G), td(G), tgs(G), tus(G), tds(G), tgi(G), tui(G), tdi(G), tgb(G), tub(G);
   std::vector<const void*> pg(G), pu(G), pd(G);
   std::vector<const float*> sg(G, nullptr), su(G, nullptr), sd(G, nullptr);
   for (int e = 0; e < El; ++e) {
@@ -556,6 +574,8 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
     if (!rc && q) rc = encode(&tgs[e], pg[e], F, d, 1);
     if (!rc && q) rc = encode(&tus[e], pu[e], F, d, 1);
     if (!rc && q) rc = encode(&tds[e], pd[e], d, F, 1);
+    if (!rc && !q) rc = encode_tmap_2d_bf16(&tgb[e], pg[e], F, d, kPairWeightRows, 64);
+    if (!rc && !q) rc = encode_tmap_2d_bf16(&tub[e], pu[e], F, d, kPairWeightRows, 64);
     // integer-MMA decode kernel: 128 codes of 128 rows per box, 128-byte swizzle
     if (!rc && q) rc = encode_tmap_2d_u8(&tgi[e], pg[e], F, d, 128, 128, 2);
     if (!rc && q) rc = encode_tmap_2d_u8(&tui[e], pu[e], F, d, 128, 128, 2);
@@ -579,6 +599,8 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
     tgi[g] = tgi[g % El];
     tui[g] = tui[g % El];
     tdi[g] = tdi[g % El];
+    tgb[g] = tgb[g % El];
+    tub[g] = tub[g % El];
     pg[g] = pg[g % El];
     pu[g] = pu[g % El];
     pd[g] = pd[g % El];
@@ -597,6 +619,9 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
     ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_gate_i8, tgi.data(), mb, cudaMemcpyHostToDevice));
     ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_up_i8, tui.data(), mb, cudaMemcpyHostToDevice));
     ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_down_i8, tdi.data(), mb, cudaMemcpyHostToDevice));
+  } else {
+    ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_gate_box, tgb.data(), mb, cudaMemcpyHostToDevice));
+    ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_up_box, tub.data(), mb, cudaMemcpyHostToDevice));
   }
   ATENIA_CUDA_TRY(cudaMemcpy(L->d_p_gate, pg.data(), pb, cudaMemcpyHostToDevice));
   ATENIA_CUDA_TRY(cudaMemcpy(L->d_p_up, pu.data(), pb, cudaMemcpyHostToDevice));
@@ -605,7 +630,7 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
   ATENIA_CUDA_TRY(cudaMemcpy(L->d_sc_up, su.data(), pb, cudaMemcpyHostToDevice));
   ATENIA_CUDA_TRY(cudaMemcpy(L->d_sc_down, sd.data(), pb, cudaMemcpyHostToDevice));
   if (L->has_shared) {
-    CUtensorMap ts[3], tss[3];
+    CUtensorMap ts[3], tss[3], tsb[2];
     const void* ps[3];
     const float* ss[3] = {q ? w->shared_s_gate : nullptr, q ? w->shared_s_up : nullptr,
                           q ? w->shared_s_down : nullptr};
@@ -615,11 +640,14 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
     int rc = encode(&ts[0], ps[0], Fs, d);
     if (!rc) rc = encode(&ts[1], ps[1], Fs, d);
     if (!rc) rc = encode(&ts[2], ps[2], d, Fs);
+    if (!rc && !q) rc = encode_tmap_2d_bf16(&tsb[0], ps[0], Fs, d, kPairWeightRows, 64);
+    if (!rc && !q) rc = encode_tmap_2d_bf16(&tsb[1], ps[1], Fs, d, kPairWeightRows, 64);
     if (!rc && q) rc = encode(&tss[0], ps[0], Fs, d, 1);
     if (!rc && q) rc = encode(&tss[1], ps[1], Fs, d, 1);
     if (!rc && q) rc = encode(&tss[2], ps[2], d, Fs, 1);
     if (rc) return rc;
     if (q) ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_shared_sw, tss, sizeof(tss), cudaMemcpyHostToDevice));
+    else ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_shared_box, tsb, sizeof(tsb), cudaMemcpyHostToDevice));
     ATENIA_CUDA_TRY(cudaMemcpy(L->d_tm_shared, ts, sizeof(ts), cudaMemcpyHostToDevice));
     ATENIA_CUDA_TRY(cudaMemcpy(L->d_p_shared, ps, sizeof(ps), cudaMemcpyHostToDevice));
     ATENIA_CUDA_TRY(cudaMemcpy(L->d_sc_shared, ss, sizeof(ss), cudaMemcpyHostToDevice));

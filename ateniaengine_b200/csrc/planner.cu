@@ -98,6 +98,11 @@ uint64_t layer_workspace_bytes(const AteniaMoeConfig& c, int world) {
   t.add(groups * tm);
   t.add(groups * tm);
   t.add(3 * tm);
+  if (!q) {  // gate and up in the boxes of the CTA-pair kernel
+    t.add(groups * tm);
+    t.add(groups * tm);
+    t.add(2 * tm);
+  }
   t.add((uint64_t)148 * 2 * kW8SplitKSlotFloats * 4);  // stream-K partial sums, one pair of slots per SM
   t.add((uint64_t)kSplitKMaxTiles * 8 * 4);            // arrival counters of split tiles
   if (q) {

@@ -744,7 +744,7 @@ def main():
     if shape.int8:
         kname = "grouped_gemm_w8_tmem_kernel" if rows_slow < 256 * groups else "grouped_gemm_w8_m256_kernel"
     else:
-        kname = "grouped_gemm_2cta_kernel" if rows_slow >= 512 * groups else "grouped_gemm_tcgen05_kernel"
+        kname = "grouped_gemm_2cta_kernel"
     # dominant kernel: the routed gate/up + SwiGLU grouped GEMM of the rank with the most rows
     flops1 = 4.0 * rows_slow * shape.d_model * shape.d_ff  # gate and up: 2 * 2 * rows * d * F
     achieved = flops1 / (g1_slow * 1e-3) / 1e12
