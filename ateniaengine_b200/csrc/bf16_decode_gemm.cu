@@ -74,12 +74,14 @@ __device__ __forceinline__ uint32_t idesc_dec(int n) {
 __device__ __forceinline__ uint32_t idesc_dec_i8(int n) {
   return (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(DROWS >> 4) << 24);
 }
-__device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+// (a converged warp, one lane issues)
+__device__ __forceinline__ void tc_mma_i8_one(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                           uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred e, p;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+      "@e tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
@@ -179,7 +181,7 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
   BarriersDec* bars = reinterpret_cast<BarriersDec*>(smem_aligned + D_STAGES * D_STAGE_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const int num_kb = (K + BKE - 1) / BKE;
   const int n_tiles = (N + BN_OUT - 1) / BN_OUT;
@@ -214,10 +216,7 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
 
   if (warp == 0) {
     // ================= TMA producer =================
-    // All lanes of the warp walk the same piece list.  Lane 0 waits for the stage and arms its barrier;
-    // then lane c issues copy c of the stage (0 and 1: the two weight tiles, 2 and up: the token rows), so
-    // that the issue latencies of a stage's copies overlap instead of adding up in one thread (a stage of
-    // the INT8 form has up to ten copies).  Measured: no different from one issuing thread.
+    // (the warp stays converged, one lane issues: see uniform_warp)
     {
       uint32_t idx = 0;
       int last_group = -1;
@@ -227,15 +226,12 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
         const CUtensorMap* m0 = &tmap_w0[tc.group];
         const CUtensorMap* m1 = (MODE == kSwiGLU) ? &tmap_w1[tc.group] : m0;
         if (tc.group != last_group) {
-          if (lane == 0) tmap_acquire(m0);
-          if (lane == 1) tmap_acquire(m1);
+          tmap_acquire(m0);
+          if (MODE == kSwiGLU) tmap_acquire(m1);
           last_group = tc.group;
         }
         const int n1 = (MODE == kSwiGLU) ? tc.n0 : tc.n0 + DROWS;
-        // copies of token rows per stage, and the stage's bytes
         const int tokp = (it.rows() + 15) & ~15;
-        const int cpp = tokp / 16;  // INT8: copies per digit plane (16 rows each)
-        const int n_x = I8 ? kDigitPlanes * cpp : 1;
         const uint32_t bytes = I8 ? 2 * D_W_BYTES + kDigitPlanes * tokp * 128 : (uint32_t)D_STAGE_BYTES;
         for (int kb = it.kb0; kb < it.kb0 + it.nkb; ++kb, ++idx) {
           const int stage = idx % STAGES;
@@ -253,22 +249,17 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
           }
           const uint32_t full = smem_u32(&bars->full[stage]);
           const uint32_t sw = smem_base + stage * STAGE_BYTES;
-          if (lane == 0) mbar_expect_tx(full, bytes);
-          __syncwarp();
-          if (lane == 0) {
-            tma_load_2d(sw, m0, full, kb * BKE, tc.n0);
-          } else if (lane == 1) {
-            tma_load_2d(sw + D_W_BYTES, m1, full, kb * BKE, n1);
-          } else if (lane - 2 < n_x) {
-            const int c = lane - 2;
-            if (I8) {
-              // digit plane p, token rows 16 cc .. 16 cc + 15 of the tile: MMA columns p * tokp + 16 cc ...
-              const int p = c / cpp, cc = (c - p * cpp) * 16;
-              tma_load_2d(sw + 2 * D_W_BYTES + (p * tokp + cc) * 128, &tmap_x, full, kb * BKE,
-                          p * plane_rows + tc.row0 + cc);
-            } else {
-              tma_load_2d(sw + 2 * D_W_BYTES, &tmap_x, full, kb * BKE, tc.row0);
-            }
+          mbar_expect_tx_one(full, bytes);
+          tma_load_2d_one(sw, m0, full, kb * BKE, tc.n0);
+          tma_load_2d_one(sw + D_W_BYTES, m1, full, kb * BKE, n1);
+          if (I8) {
+            // digit plane p, token rows cc .. cc + 15 of the tile: MMA columns p * tokp + cc ...
+            for (int p = 0; p < kDigitPlanes; ++p)
+              for (int cc = 0; cc < tokp; cc += 16)
+                tma_load_2d_one(sw + 2 * D_W_BYTES + (p * tokp + cc) * 128, &tmap_x, full, kb * BKE,
+                                p * plane_rows + tc.row0 + cc);
+          } else {
+            tma_load_2d_one(sw + 2 * D_W_BYTES, &tmap_x, full, kb * BKE, tc.row0);
           }
           armed |= 1u << stage;
         }
@@ -286,17 +277,20 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
     }
   } else if (warp == 1) {
     // ================= MMA issuer =================
-    if (lane == 0) {
+    // (the warp stays converged: see uniform_warp)
+    {
       uint32_t idx = 0;
       int acc = 0;
-      uint32_t acc_phase[2] = {0, 0};
+      uint32_t acc_phase = 0;  // bit b: accumulator b
       bool ok = true;
       while (ok && it.next()) {
-        if (!mbar_wait(smem_u32(&bars->acc_empty[acc]), acc_phase[acc] ^ 1u, abort_flag)) {
-          report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 2700 + acc);
+        if (!mbar_wait(smem_u32(&bars->acc_empty[acc]), ((acc_phase >> acc) & 1u) ^ 1u, abort_flag)) {
+          if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 2700 + acc);
           *abort_flag = 1;
-          break;
+          ok = false;
         }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         tc_fence_after();
         const int tokp = (it.rows() + 15) & ~15;
         const uint32_t idesc = I8 ? idesc_dec_i8(kDigitPlanes * tokp) : idesc_dec(tokp);
@@ -305,11 +299,12 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
           const int stage = idx % STAGES;
           const uint32_t phase = (idx / STAGES) & 1u;
           if (!mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag)) {
-            report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 2710 + stage);
+            if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 2710 + stage);
             *abort_flag = 1;
             ok = false;
-            break;
           }
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           tc_fence_after();
           const uint32_t sw = smem_base + stage * STAGE_BYTES;
           const uint64_t da0 = make_smem_desc(sw), da1 = make_smem_desc(sw + D_W_BYTES);
@@ -319,17 +314,17 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
             const uint32_t accum = (kb > it.kb0 || k > 0) ? 1u : 0u;
             // 16 bf16 (32 int8) of K = 32 bytes along a swizzled row = 2 in descriptor address units
             if (I8) {
-              tc_mma_i8(d0, da0 + 2 * k, db + 2 * k, idesc, accum);
-              tc_mma_i8(d1, da1 + 2 * k, db + 2 * k, idesc, accum);
+              tc_mma_i8_one(d0, da0 + 2 * k, db + 2 * k, idesc, accum);
+              tc_mma_i8_one(d1, da1 + 2 * k, db + 2 * k, idesc, accum);
             } else {
-              tc_mma_bf16(d0, da0 + 2 * k, db + 2 * k, idesc, accum);
-              tc_mma_bf16(d1, da1 + 2 * k, db + 2 * k, idesc, accum);
+              tc_mma_bf16_one(d0, da0 + 2 * k, db + 2 * k, idesc, accum);
+              tc_mma_bf16_one(d1, da1 + 2 * k, db + 2 * k, idesc, accum);
             }
           }
-          tc_commit(smem_u32(&bars->empty[stage]));
+          tc_commit_one(smem_u32(&bars->empty[stage]));
         }
-        if (ok) tc_commit(smem_u32(&bars->acc_full[acc]));
-        acc_phase[acc] ^= 1u;
+        if (ok) tc_commit_one(smem_u32(&bars->acc_full[acc]));
+        acc_phase ^= 1u << acc;
         acc ^= 1;
       }
     }
