@@ -19,6 +19,9 @@
 //   TMEM      = columns [0,256) rows 0..127 of the tile, [256,512) rows 128..255
 //   warps     : 0 TMA, 1 MMA + TMEM alloc, 2..5 epilogue of the first accumulator, 6..13 and 14..21 the
 //               two widening groups (alternate k-blocks, one buffer each), 22..25 epilogue of the second
+// The issuing warps stay converged (see uniform_warp): Mixtral shape, 4096 tokens, gate/up 1654 -> 1583 us, down
+// 794 -> 770, a forward 2893 -> 2791.  (A CTA-pair form with the weights as the M side and widening warps in both
+// CTAs was measured at 1823 us for gate/up: its chain of widening, remote arrival, MMA and commit is too long.)
 // (q * s) . x = s * (q . x) exactly and |q| <= 127 is exact in bf16: the MMA runs on the codes and the
 // per-row scale multiplies the accumulator column in the epilogue.  All waits are bounded.
 #include "tc_common.cuh"
@@ -71,7 +74,7 @@ grouped_gemm_w8_m256_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
   BarriersM256* bars = reinterpret_cast<BarriersM256*>(smem_aligned + M_CONV_OFF + M_CONV * M_B_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const int num_kb = (K + BK - 1) / BK;
   const int n_tiles = (N + BN_OUT - 1) / BN_OUT;
@@ -109,8 +112,8 @@ grouped_gemm_w8_m256_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
   TileCoord tc;
 
   if (warp == 0) {
-    // ================= TMA producer =================
-    if (lane == 0) {
+    // ================= TMA producer (the warp stays converged: see uniform_warp) =================
+    {
       uint32_t gk = 0;  // k-blocks issued so far, across tiles
       int last_group = -1;
       uint32_t armed = 0;
@@ -129,23 +132,24 @@ grouped_gemm_w8_m256_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
           const int stage = gk % M_STAGES;
           const uint32_t phase = (gk / M_STAGES) & 1u;
           if (!mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag)) {
-            report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 3100 + stage);
+            if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 3100 + stage);
             *abort_flag = 1;
             ok = false;
-            break;
           }
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           const uint32_t full = smem_u32(&bars->full[stage]);
           const uint32_t sa = smem_base + stage * M_STAGE_BYTES;
           const uint32_t sq = sa + M_A_BYTES;
-          mbar_expect_tx(full, M_STAGE_BYTES);
-          tma_load_2d(sa, &tmap_a, full, kb * BK, tc.row0);
-          tma_load_2d(sa + M_A_BYTES / 2, &tmap_a, full, kb * BK, tc.row0 + 128);
-          tma_load_2d(sq, mb0, full, kb * BK, tc.n0);
-          tma_load_2d(sq + M_Q_BYTES / 2, mb1, full, kb * BK, n1);
+          mbar_expect_tx_one(full, M_STAGE_BYTES);
+          tma_load_2d_one(sa, &tmap_a, full, kb * BK, tc.row0);
+          tma_load_2d_one(sa + M_A_BYTES / 2, &tmap_a, full, kb * BK, tc.row0 + 128);
+          tma_load_2d_one(sq, mb0, full, kb * BK, tc.n0);
+          tma_load_2d_one(sq + M_Q_BYTES / 2, mb1, full, kb * BK, n1);
           armed |= 1u << stage;
         }
       }
-      if (*abort_flag) {
+      if (*abort_flag && lane == 0) {
         // copies already issued must land before the CTA's shared memory is released
         const int stage = gk % M_STAGES;
         const uint32_t phase = (gk / M_STAGES) & 1u;
@@ -158,18 +162,20 @@ grouped_gemm_w8_m256_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer =================
-    if (lane == 0) {
+    // ================= MMA issuer (the warp stays converged) =================
+    {
       uint32_t gk = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x;
            ok && cursor_seek(cur, tile, n_tiles, num_groups, group_offsets, tc, BN_OUT, M_ROWS); tile += gridDim.x) {
         if (!mbar_wait(smem_u32(&bars->acc_empty), acc_phase ^ 1u, abort_flag)) {
-          report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 3200);
+          if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 3200);
           *abort_flag = 1;
-          break;
+          ok = false;
         }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         acc_phase ^= 1u;
         tc_fence_after();
         for (int kb = 0; kb < num_kb; ++kb, ++gk) {
@@ -177,11 +183,12 @@ grouped_gemm_w8_m256_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
           const uint32_t phase = (gk / M_STAGES) & 1u, cphase = (gk / M_CONV) & 1u;
           if (!mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag) ||
               !mbar_wait(smem_u32(&bars->conv_full[cstage]), cphase, abort_flag)) {
-            report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 3300 + stage);
+            if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 3300 + stage);
             *abort_flag = 1;
             ok = false;
-            break;
           }
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           tc_fence_after();
           const uint32_t sa = smem_base + stage * M_STAGE_BYTES;
           const uint64_t da0 = make_smem_desc(sa), da1 = make_smem_desc(sa + M_A_BYTES / 2);
@@ -190,13 +197,13 @@ grouped_gemm_w8_m256_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint32_t accum = (kb > 0 || k > 0) ? 1u : 0u;
             // 16 bf16 of K = 32 bytes inside the swizzled row: +2 in descriptor address units
-            tc_mma_bf16(tmem_base, da0 + 2 * k, db + 2 * k, kInstrDescM, accum);
-            tc_mma_bf16(tmem_base + M_BN, da1 + 2 * k, db + 2 * k, kInstrDescM, accum);
+            tc_mma_bf16_one(tmem_base, da0 + 2 * k, db + 2 * k, kInstrDescM, accum);
+            tc_mma_bf16_one(tmem_base + M_BN, da1 + 2 * k, db + 2 * k, kInstrDescM, accum);
           }
-          tc_commit(smem_u32(&bars->empty[stage]));
-          tc_commit(smem_u32(&bars->conv_empty[cstage]));
+          tc_commit_one(smem_u32(&bars->empty[stage]));
+          tc_commit_one(smem_u32(&bars->conv_empty[cstage]));
         }
-        if (ok) tc_commit(smem_u32(&bars->acc_full));
+        if (ok) tc_commit_one(smem_u32(&bars->acc_full));
       }
     }
   } else if (warp >= M_FIRST_CONV_WARP && warp < M_SECOND_EPI_WARP) {
