@@ -181,6 +181,10 @@ int launch_grouped_gemm_check(const GroupedGemmCheckArgs& a, cudaStream_t s);
 // four rows per group, but from three rows on the tensor-core kernels are as fast).
 int launch_grouped_gemv(const GroupedGemmCheckArgs& a, cudaStream_t s);
 constexpr int kGemvMaxRows = 2;
+// rows x d x F above which a bf16 call of at most kGemvMaxRows rows takes the stream-K kernel instead.  One token,
+// top-2 of 8 experts on a B200, matrix-vector / stream-K: d 4096, F 3584 66.0 / 69.3 us, F 7168 97.3 / 97.8,
+// F 14336 157.3 / 147.4.
+constexpr int64_t kGemvMaxWeights = (int64_t)1 << 26;
 
 int launch_f32_to_bf16(const float* src, __nv_bfloat16* dst, int64_t n, cudaStream_t s);
 // p[0] = a, p[1] = b on the stream (the one-group offsets of the shared expert's GEMMs)

@@ -200,7 +200,8 @@ void launch_gv(const GroupedGemmCheckArgs& a, dim3 grid, dim3 block, cudaStream_
 // have at most kGvMaxRows rows in total (a.max_rows), so that every group has at most that many.  The
 // layer sends calls of at most kGemvMaxRows = 2 rows here: measured on B200 (Mixtral shape, one token)
 // bf16 0.189 -> 0.183 ms, INT8 0.174 -> 0.166 ms, a DeepSeek-shaped layer with its shared expert
-// 0.182 -> 0.156 ms; with four rows the tensor-core decode kernels are as fast or faster.
+// 0.182 -> 0.156 ms; with four rows the tensor-core decode kernels are as fast or faster, and so is the bf16
+// one at one row of large experts (kGemvMaxWeights).
 int launch_grouped_gemv(const GroupedGemmCheckArgs& a, cudaStream_t s) {
   if (a.num_groups <= 0 || a.max_rows <= 0) return ATENIA_OK;
   if (a.max_rows > kGvMaxRows || a.K % 16 != 0) return ATENIA_ERR_SHAPE;

@@ -76,7 +76,9 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   // 0.160 (matrix-vector kernel) / 0.300 / 0.525 ms (tensor-memory kernel).  ATENIA_MOE_W8_I8=0 or a pinned
   // w8_mode keep the widening kernels (tests, A/B runs).
   const bool i8dec = q && L->w8_i8 && L->dq_x && max_rows <= L->i8_rows && !L->use_check_gemm && L->w8_mode == 0;
-  const bool gemv = L->use_gemv && max_rows <= L->gemv_rows && !L->use_check_gemm && !i8dec;
+  // bf16 from kGemvMaxWeights weights on: the stream-K kernel, whose launch costs more and whose stream is faster
+  const bool dec_few = dec && (int64_t)max_rows * c.d_model * c.d_ff >= kGemvMaxWeights;
+  const bool gemv = L->use_gemv && max_rows <= L->gemv_rows && !L->use_check_gemm && !i8dec && !dec_few;
   if (L->timing) cudaEventRecord(L->ev[0], s);
   // (set by the forward when it left the row gather to the digit kernel; consumed here)
   const bool gather_here = L->i8_src_set && a_ptr == L->x_perm;
@@ -712,9 +714,11 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   // The shared expert needs only this call's tokens, so its GEMMs run on the layer's second stream from
   // the start of the forward, beside the routing phase (an FP64-bound router, an HBM-bound gather: the
   // tensor cores are idle there) and, under expert parallelism, beside the exchanges; the combine waits
-  // for them.  f32 input is converted to bf16 first.  Tiny batches keep the one-stream order (the two
-  // event hops would cost more than the overlap gives); ATENIA_MOE_SHARED_ASIDE=0 turns it off.
-  const bool shared_aside = L->has_shared && T >= 64 && L->aux_stream && L->shared_aside;
+  // for them.  f32 input is converted to bf16 first.  Calls of the matrix-vector kernel keep the one-stream
+  // order: there the two event hops cost what the overlap gives (DeepSeek-V2-Lite shape, 1 token: 89.3 us aside,
+  // 88.6 in order; 3 tokens 99 / 126, 61 tokens 229 / 253; Qwen1.5-MoE shape, 16 tokens 172 / 198).
+  // ATENIA_MOE_SHARED_ASIDE=0 turns it off.
+  const bool shared_aside = L->has_shared && T > L->gemv_rows && L->aux_stream && L->shared_aside;
   if (shared_aside) {
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
     if (x_f32) {
