@@ -209,6 +209,7 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  chain_wait();  // (everything above touches only this CTA's shared and tensor memory)
 
   DecPieces it;
   it.init(splitk != 0, num_kb, n_tiles, num_groups, BN_OUT, group_offsets, TROWS);
@@ -513,6 +514,7 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
     }
   }
 
+  chain_next();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -621,11 +623,10 @@ int launch_dec_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   // hundred rows on the last warp's serial sum costs what the launch saved, so the reduce kernel stays.
   const bool fixup = splitk && a.splitk_cnt != nullptr && a.max_rows <= kFixupMaxRows &&
                      max_tok_tiles * n_tiles <= kSplitKMaxTiles;
-  grouped_gemm_decode_kernel<MODE, I8><<<dim3(num_sms), dim3(D_THREADS), D_SMEM_BYTES, s>>>(
-      a.tmap_a, a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out,
-      a.err, splitk ? 1 : 0, a.splitk_ws, a.scale0, a.scale1, a.tok_scale, a.plane_rows,
-      fixup ? a.splitk_cnt : nullptr);
-  int rc = (int)cudaGetLastError();
+  int rc = launch_chained(a.chained, grouped_gemm_decode_kernel<MODE, I8>, dim3(num_sms), dim3(D_THREADS), D_SMEM_BYTES, s, a.tmap_a,
+                          a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K,
+                          a.out, a.err, splitk ? 1 : 0, a.splitk_ws, a.scale0, a.scale1, a.tok_scale, a.plane_rows,
+                          fixup ? a.splitk_cnt : nullptr);
   if (rc || !splitk || fixup) return rc;
   decode_splitk_reduce_kernel<MODE, I8><<<dim3(max_tok_tiles * n_tiles), dim3(DROWS, kReduceTokLanes), 0, s>>>(
       a.group_offsets, a.num_groups, a.N, a.K, a.out, a.splitk_ws, num_sms, a.scale0, a.scale1, a.tok_scale);
@@ -674,6 +675,8 @@ __global__ void __launch_bounds__(kQThreads) quantize_digits_kernel(DigitSource 
                                                                     int K, int plane_rows, int8_t* __restrict__ planes,
                                                                     float* __restrict__ tok_scale) {
   const int row = blockIdx.x;
+  chain_next();
+  chain_wait();
   // rows the dispatch did not place (invalid expert ids) hold nothing: skip them
   const int placed = n_rows_dev ? (*n_rows_dev < n_rows ? *n_rows_dev : n_rows) : n_rows;
   if (row >= placed) return;
@@ -765,9 +768,9 @@ int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, in
                            int8_t* planes, float* tok_scale, cudaStream_t s) {
   if (n_rows <= 0) return ATENIA_OK;
   if (K % 16 != 0 || n_rows > plane_rows || !src.x || (src.perm && src.k < 1)) return ATENIA_ERR_SHAPE;
-  quantize_digits_kernel<<<n_rows, kQThreads, 0, s>>>(src, n_rows_dev, n_rows, K, plane_rows, planes, tok_scale);
   count_launch();
-  return (int)cudaGetLastError();
+  return launch_chained(true, quantize_digits_kernel, dim3(n_rows), dim3(kQThreads), 0, s, src, n_rows_dev, n_rows, K, plane_rows,
+                        planes, tok_scale);
 }
 
 }  // namespace atenia

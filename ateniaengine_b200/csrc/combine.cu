@@ -20,6 +20,8 @@ template <int K>
 __global__ void __launch_bounds__(256) combine_kernel(CombineArgs a) {
   const int t = blockIdx.x;
   const int nvec = a.d / 8;
+  chain_next();
+  chain_wait();
   int rows[K];
   float w[K];
 #pragma unroll
@@ -160,12 +162,14 @@ int launch_combine(const CombineArgs& a, cudaStream_t s) {
   // d / 8 vectors per token: narrow rows take narrower blocks
   const int nvec = a.d / 8;
   const int threads = nvec >= 256 ? 256 : nvec >= 128 ? 128 : 64;
-  if (a.k <= 2) combine_kernel<2><<<a.T, threads, 0, s>>>(a);
-  else if (a.k <= 4) combine_kernel<4><<<a.T, threads, 0, s>>>(a);
-  else if (a.k <= 6) combine_kernel<6><<<a.T, threads, 0, s>>>(a);
-  else combine_kernel<8><<<a.T, threads, 0, s>>>(a);
+  auto launch = [&](auto kernel) { return launch_chained(a.chained, kernel, dim3(a.T), dim3(threads), 0, s, a); };
+  int rc;
+  if (a.k <= 2) rc = launch(combine_kernel<2>);
+  else if (a.k <= 4) rc = launch(combine_kernel<4>);
+  else if (a.k <= 6) rc = launch(combine_kernel<6>);
+  else rc = launch(combine_kernel<8>);
   count_launch();
-  return (int)cudaGetLastError();
+  return rc;
 }
 
 __global__ void set_pair_kernel(int32_t* p, int32_t a, int32_t b) {

@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(kGvWarps * 32, MAXR <= 2 ? 2 : 1) grouped_gemv
   using Step = GvStep<NM, W8>;
   constexpr int CH = 16 * Step::U;               // k per lane and step
   const int g = blockIdx.y;
+  chain_next();
+  chain_wait();
   const int r0 = a.group_offsets[g];
   int R = a.group_offsets[g + 1] - r0;
   if (R <= 0) return;
@@ -189,9 +191,9 @@ __global__ void __launch_bounds__(kGvWarps * 32, MAXR <= 2 ? 2 : 1) grouped_gemv
 }
 
 template <int MODE, bool W8>
-void launch_gv(const GroupedGemmCheckArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
-  if (a.max_rows <= 2) grouped_gemv_kernel<MODE, W8, 2><<<grid, block, 0, s>>>(a);
-  else grouped_gemv_kernel<MODE, W8, 4><<<grid, block, 0, s>>>(a);
+int launch_gv(const GroupedGemmCheckArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
+  if (a.max_rows <= 2) return launch_chained(a.chained, grouped_gemv_kernel<MODE, W8, 2>, grid, block, 0, s, a);
+  return launch_chained(a.chained, grouped_gemv_kernel<MODE, W8, 4>, grid, block, 0, s, a);
 }
 
 }  // namespace
@@ -207,15 +209,9 @@ int launch_grouped_gemv(const GroupedGemmCheckArgs& a, cudaStream_t s) {
   if (a.max_rows > kGvMaxRows || a.K % 16 != 0) return ATENIA_ERR_SHAPE;
   if (a.b_is_int8 && (!a.scale0 || (a.mode == kSwiGLU && !a.scale1))) return ATENIA_ERR_NULL;
   const dim3 grid((a.N + kGvRowsPerBlock - 1) / kGvRowsPerBlock, a.num_groups), block(kGvWarps * 32);
-  if (a.mode == kSwiGLU) {
-    if (a.b_is_int8) launch_gv<kSwiGLU, true>(a, grid, block, s);
-    else launch_gv<kSwiGLU, false>(a, grid, block, s);
-  } else {
-    if (a.b_is_int8) launch_gv<kPlain, true>(a, grid, block, s);
-    else launch_gv<kPlain, false>(a, grid, block, s);
-  }
   count_launch();
-  return (int)cudaGetLastError();
+  if (a.mode == kSwiGLU) return a.b_is_int8 ? launch_gv<kSwiGLU, true>(a, grid, block, s) : launch_gv<kSwiGLU, false>(a, grid, block, s);
+  return a.b_is_int8 ? launch_gv<kPlain, true>(a, grid, block, s) : launch_gv<kPlain, false>(a, grid, block, s);
 }
 
 }  // namespace atenia

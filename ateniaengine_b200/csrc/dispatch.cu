@@ -114,7 +114,9 @@ __global__ void __launch_bounds__(kSmallDispatchMax) dispatch_small_kernel(Dispa
   __shared__ int warp_cnt[kSmallDispatchMax / 32][kMaxE];  // entries of expert e in warp w, then their base
   __shared__ int offsets[kMaxE + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  chain_next();
   for (int j = threadIdx.x; j < nwarps * kMaxE; j += blockDim.x) (&warp_cnt[0][0])[j] = 0;
+  chain_wait();
   __syncthreads();
   const int i = threadIdx.x;
   int e = -1;
@@ -183,7 +185,9 @@ dispatch_cluster_kernel(DispatchArgs a) {
   const int per = ((a.n + kDispatchCtas - 1) / kDispatchCtas + 31) & ~31;
   const int begin = rank * per < a.n ? rank * per : a.n;
   const int end = begin + per < a.n ? begin + per : a.n;
+  chain_next();
   if (threadIdx.x < kMaxE) hist[threadIdx.x] = 0;
+  chain_wait();
   __syncthreads();
   for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
     const int e = a.topk_idx[i];
@@ -301,6 +305,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32) gather_rows_kernel(const vo
                                                                          int total_rows) {
   const int lane = threadIdx.x & 31;
   const int nvec = d / 8;
+  chain_next();
+  chain_wait();
   const int n_placed = n_rows > 0 ? *placed : 0;
   for (int r = blockIdx.x * kGatherWarps + (threadIdx.x >> 5); r < total_rows; r += gridDim.x * kGatherWarps) {
     int src_t, dst_r;
@@ -353,14 +359,12 @@ int launch_dispatch(const DispatchArgs& a, cudaStream_t s) {
   if (a.E > kMaxE) return ATENIA_ERR_UNSUPPORTED;
   if (a.n > 0 && a.n <= kSmallDispatchMax) {
     const int threads = ((a.n + 31) / 32 * 32) < a.E ? ((a.E + 31) / 32 * 32) : ((a.n + 31) / 32 * 32);
-    dispatch_small_kernel<<<1, threads, 0, s>>>(a);
     count_launch();
-    return (int)cudaGetLastError();
+    return launch_chained(a.chained, dispatch_small_kernel, dim3(1), dim3(threads), 0, s, a);
   }
   if (a.n > kSmallDispatchMax && a.n <= kClusterDispatchMax) {
-    dispatch_cluster_kernel<<<kDispatchCtas, kSmallDispatchMax, 0, s>>>(a);
     count_launch();
-    return (int)cudaGetLastError();
+    return launch_chained(a.chained, dispatch_cluster_kernel, dim3(kDispatchCtas), dim3(kSmallDispatchMax), 0, s, a);
   }
   const int nblk = (a.n + kDispatchChunk - 1) / kDispatchChunk;
   if (nblk > 0) {
@@ -377,17 +381,16 @@ int launch_dispatch(const DispatchArgs& a, cudaStream_t s) {
 }
 
 int launch_gather_rows(const void* x, int x_is_f32, const int32_t* perm, const int32_t* placed, int n_rows, int k,
-                       int d, __nv_bfloat16* x_perm, __nv_bfloat16* x_bf16, int T, cudaStream_t s) {
+                       int d, __nv_bfloat16* x_perm, __nv_bfloat16* x_bf16, int T, bool chained, cudaStream_t s) {
   const int extra = x_bf16 ? T : 0;
   const int total = n_rows + extra;
   if (total <= 0) return ATENIA_OK;
   // enough blocks to keep every SM's memory pipeline full; the kernel loops over the rest
   const int want = (total + kGatherWarps - 1) / kGatherWarps;
   const int cap = 148 * 8;
-  gather_rows_kernel<<<want < cap ? want : cap, kGatherWarps * 32, 0, s>>>(x, x_is_f32, perm, placed, n_rows, k, d, x_perm,
-                                                                          x_bf16, T, total);
   count_launch();
-  return (int)cudaGetLastError();
+  return launch_chained(chained, gather_rows_kernel, dim3(want < cap ? want : cap), dim3(kGatherWarps * 32), 0, s, x, x_is_f32, perm,
+                        placed, n_rows, k, d, x_perm, x_bf16, T, total);
 }
 
 }  // namespace atenia

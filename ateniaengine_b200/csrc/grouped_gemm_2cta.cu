@@ -168,7 +168,6 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
                          int num_groups, int N, int K, __nv_bfloat16* __restrict__ out, DeviceError* err) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int32_t goff_s[kMaxGroupsShared + 1];
-  const int32_t* group_offsets = stage_group_offsets(group_offsets_g, num_groups, goff_s);
   constexpr int F_CTA = (MODE == kSwiGLU) ? BM / 2 : BM;  // output features per CTA
   constexpr int F_PAIR = 2 * F_CTA;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -205,6 +204,8 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  chain_wait();  // (everything above touches only this CTA's shared and tensor memory)
+  const int32_t* group_offsets = stage_group_offsets(group_offsets_g, num_groups, goff_s);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before anyone signals them
@@ -389,6 +390,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
     }
   }
 
+  chain_next();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // neither CTA leaves while its peer may still signal or read it
@@ -407,10 +409,8 @@ int launch_2cta_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
                                          SMEM_BYTES2));
   }
   const int grid = num_sms & ~1;  // whole pairs
-  grouped_gemm_2cta_kernel<MODE><<<dim3(grid), dim3(NUM_THREADS2), SMEM_BYTES2, s>>>(
-      *a.pair_rows, a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out,
-      a.err);
-  return (int)cudaGetLastError();
+  return launch_chained(a.chained, grouped_gemm_2cta_kernel<MODE>, dim3(grid), dim3(NUM_THREADS2), SMEM_BYTES2, s, *a.pair_rows, a.tmap_b0,
+                        MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out, a.err);
 }
 
 }  // namespace

@@ -89,6 +89,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
                                     L->i8_rows, L->dq_x, L->dq_ts_x, s);
     if (rc) return rc;
     GroupedGemmArgs g1{};
+    g1.chained = L->gemm_chained;
     g1.tmap_a = L->tm_dq_x;
     g1.tmap_b0 = L->d_tm_gate_i8;
     g1.tmap_b1 = L->d_tm_up_i8;
@@ -136,11 +137,12 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   if (L->use_check_gemm || gemv) {
     GroupedGemmCheckArgs k1{a_ptr, L->d_p_gate, L->d_p_up, q ? 1 : 0, q ? L->d_sc_gate : nullptr,
                             q ? L->d_sc_up : nullptr, group_offsets, num_groups, c.d_ff, c.d_model,
-                            kSwiGLU, mid, max_rows};
+                            kSwiGLU, mid, max_rows, L->gemm_chained};
     int rc = gemv ? launch_grouped_gemv(k1, s) : launch_grouped_gemm_check(k1, s);
     if (rc) return rc;
   } else {
     GroupedGemmArgs g1{};
+    g1.chained = L->gemm_chained;
     g1.tmap_a = tm_a.tile;
     g1.pair_rows = &tm_a.pair;
     g1.tmap_b0 = tmem ? L->d_tm_gate_sw : pairs ? L->d_tm_gate_box : L->d_tm_gate;
@@ -168,11 +170,12 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   if (L->timing) cudaEventRecord(L->ev[1], s);
   if (L->use_check_gemm || gemv) {
     GroupedGemmCheckArgs k2{mid, L->d_p_down, nullptr, q ? 1 : 0, q ? L->d_sc_down : nullptr, nullptr,
-                            group_offsets, num_groups, c.d_model, c.d_ff, kPlain, out, max_rows};
+                            group_offsets, num_groups, c.d_model, c.d_ff, kPlain, out, max_rows, L->gemm_chained};
     int rc = gemv ? launch_grouped_gemv(k2, s) : launch_grouped_gemm_check(k2, s);
     if (rc) return rc;
   } else {
     GroupedGemmArgs g2{};
+    g2.chained = L->gemm_chained;
     g2.tmap_a = tm_mid.tile;
     g2.pair_rows = &tm_mid.pair;
     g2.tmap_b0 = tmem ? L->d_tm_down_sw : L->d_tm_down;
@@ -219,12 +222,12 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   if (L->use_check_gemm || gemv) {
     GroupedGemmCheckArgs k1{xb, L->d_p_shared, L->d_p_shared + 1, q ? 1 : 0, q ? L->d_sc_shared : nullptr,
                             q ? L->d_sc_shared + 1 : nullptr, L->shared_offsets, 1, c.shared_d_ff, c.d_model,
-                            kSwiGLU, L->h_shared, T};
+                            kSwiGLU, L->h_shared, T, L->gemm_chained};
     int rc = gemv ? launch_grouped_gemv(k1, s) : launch_grouped_gemm_check(k1, s);
     if (rc) return rc;
     if (L->timing) cudaEventRecord(L->ev[4], s);
     GroupedGemmCheckArgs k2{L->h_shared, L->d_p_shared + 2, nullptr, q ? 1 : 0, q ? L->d_sc_shared + 2 : nullptr,
-                            nullptr, L->shared_offsets, 1, c.d_model, c.shared_d_ff, kPlain, L->y_shared, T};
+                            nullptr, L->shared_offsets, 1, c.d_model, c.shared_d_ff, kPlain, L->y_shared, T, L->gemm_chained};
     rc = gemv ? launch_grouped_gemv(k2, s) : launch_grouped_gemm_check(k2, s);
     if (rc) return rc;
     if (L->timing) {
@@ -234,6 +237,7 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
     return ATENIA_OK;
   }
   GroupedGemmArgs g1{};
+  g1.chained = L->gemm_chained;
   PairRowMaps x_rows;
   int rc = pairs ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model)
                  : encode_tmap_2d_bf16(&g1.tmap_a, xb, (uint64_t)T, (uint64_t)c.d_model, 128, 64);
@@ -259,6 +263,7 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   if (rc) return rc;
   if (L->timing) cudaEventRecord(L->ev[4], s);
   GroupedGemmArgs g2{};
+  g2.chained = L->gemm_chained;
   g2.tmap_a = L->tm_h_shared.tile;
   g2.pair_rows = &L->tm_h_shared.pair;
   g2.tmap_b0 = (tmem ? L->d_tm_shared_sw : L->d_tm_shared) + 2;
@@ -719,6 +724,11 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   // 88.6 in order; 3 tokens 99 / 126, 61 tokens 229 / 253; Qwen1.5-MoE shape, 16 tokens 172 / 198).
   // ATENIA_MOE_SHARED_ASIDE=0 turns it off.
   const bool shared_aside = L->has_shared && T > L->gemv_rows && L->aux_stream && L->shared_aside;
+  // Blocks of a chained kernel sit on the SMs while they wait.  Beside a shared expert that is affordable while the
+  // row gather (8 rows a block) brings at most two blocks to an SM; more would keep its GEMMs out (Qwen1.5-MoE shape,
+  // 2048 tokens, 345 -> 370 us).
+  const bool chained = !shared_aside || n <= 16 * L->num_sms;
+  L->gemm_chained = !shared_aside;
   if (shared_aside) {
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
     if (x_f32) {
@@ -757,6 +767,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   ra.sk_gate = L->sk_gate;
   ra.sk_counters = L->sk_counters;
   ra.sk_tokens = L->sk_tokens;
+  ra.chained = chained;
   int rc = launch_router(ra, s);
   if (rc) return rc;
   if (v3) {
@@ -783,6 +794,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   da.extra_offsets = shared_aside ? nullptr : L->shared_offsets;
   da.T = T;
   da.err = L->d_err;
+  da.chained = chained && !sel_idx;
   rc = launch_dispatch(da, s);
   if (rc) return rc;
 
@@ -793,7 +805,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   const bool i8_gather = c.weight_dtype == ATENIA_W_INT8_ROW && L->w8_i8 && L->dq_x && n <= L->i8_rows &&
                          !L->use_check_gemm && L->w8_mode == 0 && (c.ep_world == 1 || L->ep_replicated);
   rc = launch_gather_rows(x, x_f32, L->perm, L->expert_offsets + c.num_experts, (direct || i8_gather) ? 0 : n, k,
-                          c.d_model, L->x_perm, need_xb ? L->x_bf16 : nullptr, T, s);
+                          c.d_model, L->x_perm, need_xb ? L->x_bf16 : nullptr, T, chained, s);
   if (rc) return rc;
   L->i8_src = DigitSource{x, x_f32 ? 1 : 0, L->perm, k, T};
   L->i8_src_set = i8_gather;
@@ -838,6 +850,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   ca.T = T;
   ca.k = k;
   ca.d = c.d_model;
+  ca.chained = !shared_aside;
   rc = launch_combine(ca, s);
   if (rc) return rc;
   if (L->timing) {

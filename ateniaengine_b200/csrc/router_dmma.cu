@@ -81,6 +81,8 @@ __device__ __forceinline__ double x_elem(const uint32_t (&w)[N], int j) {
 // rounding to f32 and the routing of each token by one warp (route_one_warp).
 template <int E_T, int MT, int NTW, bool XF, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) router_dmma_direct_kernel(RouterArgs a, int kw) {
+  chain_next();
+  chain_wait();
   constexpr int NT = E_T / 8;
   constexpr int NW_N = NT / NTW;
   constexpr int NW_K = WARPS / NW_N;
@@ -234,9 +236,8 @@ int launch_form(const RouterArgs& a, cudaStream_t s) {
   // k-range of a k-slice: d over the slices, rounded up to whole 32-k steps
   const int kw = ((a.d + NW_K - 1) / NW_K + 31) / 32 * 32;
   const int grid = (a.T + kTok - 1) / kTok;
-  if (a.x_is_f32) router_dmma_direct_kernel<E_T, MT, NTW, true, WARPS><<<grid, WARPS * 32, 0, s>>>(a, kw);
-  else router_dmma_direct_kernel<E_T, MT, NTW, false, WARPS><<<grid, WARPS * 32, 0, s>>>(a, kw);
-  return (int)cudaGetLastError();
+  if (a.x_is_f32) return launch_chained(a.chained, router_dmma_direct_kernel<E_T, MT, NTW, true, WARPS>, dim3(grid), dim3(WARPS * 32), 0, s, a, kw);
+  return launch_chained(a.chained, router_dmma_direct_kernel<E_T, MT, NTW, false, WARPS>, dim3(grid), dim3(WARPS * 32), 0, s, a, kw);
 }
 
 // Two forms.  A batch whose 8-token CTAs fit the SMs in one round is bound by the latency of its

@@ -39,6 +39,8 @@ __global__ void __launch_bounds__(kSkWarps * 32) router_splitk_kernel(RouterArgs
   const int k0 = slice * kSkSlice + lane * 4;
   const bool k_ok = k0 < d;  // d is a multiple of 16: four consecutive k are all in or all out
 
+  chain_next();
+  chain_wait();
   double xk[kSkTok][4];
 #pragma unroll
   for (int t = 0; t < kSkTok; ++t) {
@@ -164,8 +166,7 @@ template <int E_T>
 int launch_one(const RouterArgs& a, cudaStream_t s) {
   const int ksplit = (a.d + kSkSlice - 1) / kSkSlice;
   const int n_tb = (a.T + kSkTok - 1) / kSkTok;
-  router_splitk_kernel<E_T><<<dim3(ksplit, n_tb), kSkWarps * 32, 0, s>>>(a, ksplit, n_tb);
-  return (int)cudaGetLastError();
+  return launch_chained(a.chained, router_splitk_kernel<E_T>, dim3(ksplit, n_tb), dim3(kSkWarps * 32), 0, s, a, ksplit, n_tb);
 }
 
 }  // namespace

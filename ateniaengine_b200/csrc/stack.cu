@@ -44,6 +44,8 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float*
                                                                      float* __restrict__ y, int d) {
   __shared__ float red[kNormThreads / 32];
   __shared__ float s_inv;
+  atenia::chain_next();
+  atenia::chain_wait();
   const float* row = x + (size_t)blockIdx.x * d;
   float* yrow = y + (size_t)blockIdx.x * d;
   // 16-byte vectors when every row starts on a 16-byte boundary
@@ -100,9 +102,8 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float*
 namespace atenia {
 int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y, int T, int d, cudaStream_t s) {
   if (T <= 0) return ATENIA_OK;
-  rmsnorm_rows_kernel<<<T, kNormThreads, 0, s>>>(x, gamma, eps, y, d);
   count_launch();
-  return (int)cudaGetLastError();
+  return launch_chained(true, rmsnorm_rows_kernel, dim3(T), dim3(kNormThreads), 0, s, x, gamma, eps, y, d);
 }
 }  // namespace atenia
 
