@@ -1,5 +1,5 @@
 // Grouped expert GEMM at decode sizes, sm_100a: bf16 weights (groups of at most 128 rows) and INT8
-// weights multiplied as integers (calls of at most 128 rows).
+// weights multiplied as integers (calls of at most 256 rows).
 //
 // At a batch of a few tokens the work is streaming the touched experts' weights once; what decides
 // the speed is whether every SM streams the same number of bytes.  The 128-row-tile kernels of

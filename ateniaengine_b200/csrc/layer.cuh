@@ -100,10 +100,10 @@ struct AteniaMoeLayer {
   atenia::DeviceError* d_err = nullptr;
   float* splitk_ws = nullptr;  // stream-K partial sums of the decode kernels, 2 slots per SM
   unsigned int* splitk_cnt = nullptr;  // [kSplitKMaxTiles * 8] arrival counters of split tiles (zero between launches)
-  // INT8, integer-MMA decode kernel: weight maps (box {128, 128}, 128B swizzle), digit planes [4][128][K] of
+  // INT8, integer-MMA decode kernel: weight maps (box {128, 128}, 128B swizzle), digit planes [4][i8_rows][K] of
   // the token rows and of the intermediate rows with their row scales, and the planes' tensor maps
   bool w8_i8 = true;
-  int i8_rows = 128;  // rows of one digit plane = the largest call the kernel takes
+  int i8_rows = 0;  // rows of one digit plane = the largest call the kernel takes
   CUtensorMap* d_tm_gate_i8 = nullptr;
   CUtensorMap* d_tm_up_i8 = nullptr;
   CUtensorMap* d_tm_down_i8 = nullptr;
