@@ -37,12 +37,8 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustain
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the routed gate/up + SwiGLU kernel the
 # workload selects, from one-pass ncu captures of this command (kernel name -> bytes).
 NCU_TRAFFIC_BYTES = {
-    # CTA-pair kernel: 1.966 GB read + 228 MB written at 4096 tokens; 1.908 GB + 29.6 MB at 512
-    "mixtral:4096:grouped_gemm_2cta_kernel": 2.194e9,
-    "mixtral:512:grouped_gemm_2cta_kernel": 1.938e9,
-    # single-CTA kernel: 1.95 GB read + 227.5 MB written at 4096 tokens; 1.904 GB + 29.9 MB at 512
-    "mixtral:4096:grouped_gemm_tcgen05_kernel": 2.18e9,
-    "mixtral:512:grouped_gemm_tcgen05_kernel": 1.934e9,
+    # CTA-pair kernel: 2.274 GB read + 231 MB written at 4096 tokens
+    "mixtral:4096:grouped_gemm_2cta_kernel": 2.504e9,
     # 256-row INT8 kernel: 1.013 GB read + 223 MB written at 4096 tokens
     "mixtral_int8:4096:grouped_gemm_w8_m256_kernel": 1.236e9,
 }
