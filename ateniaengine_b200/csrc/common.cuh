@@ -75,7 +75,9 @@ int launch_chained(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, si
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = chained ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();  // returned here: not again by the next plain launch's check
+  return (int)e;
 }
 
 #define ATENIA_CUDA_TRY(expr)                \

@@ -5,7 +5,8 @@
 // The only order it defines is therefore "tokens ascending, experts ascending inside a token", and
 // the permutation emitted here is the stable counting sort of the flat entry list i = t*k + s by
 // expert id: expert_offsets[e] = number of entries with a smaller expert, and the rows of one
-// expert keep ascending i.  Three launches: per-block histogram, scan, stable placement.
+// expert keep ascending i.  Three launches (per-block histogram, scan, stable placement) above 16384
+// entries, one below.
 #include "common.cuh"
 
 namespace atenia {

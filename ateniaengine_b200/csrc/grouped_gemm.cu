@@ -2,6 +2,8 @@
 //
 // One launch covers every expert of a layer.  A persistent grid (one CTA per SM) walks a tile list
 // derived on the device from the dispatch offsets, so the host never reads routing results.
+// The forward takes the kernels of grouped_gemm_2cta.cu, w8_gemm.cu and w8_gemm_m256.cu; this one is their
+// cross-check (ATENIA_MOE_PAIR_MODE=2, ATENIA_MOE_W8_MODE=2).
 //
 //   tile            = 128 rows of one expert  x  BN_OUT output columns
 //   kSwiGLU         : B tile = 128 rows of W_gate || 128 rows of W_up  -> one M128 x N256 MMA,
