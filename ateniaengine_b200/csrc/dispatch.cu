@@ -195,6 +195,7 @@ dispatch_cluster_kernel(DispatchArgs a) {
     if (e >= 0 && e < a.E) atomicAdd(&hist[e], 1);
     else report_error(a.err, ATENIA_ERR_ROUTING, 2002);
   }
+  __syncwarp();  // (.aligned: the lanes of a warp arrive together, and the loop lets them leave apart)
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   int before = 0, total = 0;
@@ -212,6 +213,7 @@ dispatch_cluster_kernel(DispatchArgs a) {
     totals[threadIdx.x] = total;
   }
   // (waited for at the end: no CTA leaves while another may read its histogram)
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   __syncthreads();
   if (warp == 0) {  // exclusive scan of the totals, four experts per lane
@@ -286,6 +288,7 @@ dispatch_cluster_kernel(DispatchArgs a) {
     }
     __syncwarp();  // (a warp's row is cleared by the warp itself)
   }
+  __syncwarp();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

@@ -105,6 +105,7 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -333,6 +334,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
          tile += num_pairs, ++it) {
       const int acc = it & 1;
       bool ready = mbar_wait(smem_u32(&bars->acc_full[acc]), (acc_phase >> acc) & 1u, abort_flag);
+      __syncwarp();  // (each lane polled by itself; the barriers and tensor-memory loads below want the warp as one)
       if (MODE == kSwiGLU) {
         // the two warps of a pair leave together or not at all: one of them alone would hold the other in bar.sync
         uint32_t both;
