@@ -310,6 +310,7 @@ int atenia_quantize_per_group_i8(const float* w, int64_t K, int64_t N, int64_t g
   if (K == 0 || N == 0) return ATENIA_OK;
   if (!w || !q || !scales) return ATENIA_ERR_NULL;
   const int64_t G = (group_size == 0 || group_size > K) ? K : group_size;
+  if ((K + G - 1) / G > 0x7fffffffLL * 4 / N) return ATENIA_ERR_SHAPE;  // scales
   const bool vec = N % 4 == 0 && aligned16(w) && (reinterpret_cast<uintptr_t>(q) & 3u) == 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return vec ? launch_quantize<true>(w, K, N, G, q, scales, s) : launch_quantize<false>(w, K, N, G, q, scales, s);
