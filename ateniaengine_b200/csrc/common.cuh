@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "../../include/atenia_moe.h"
+#include "pair_tiles.cuh"
 
 namespace atenia {
 
@@ -164,10 +165,7 @@ int launch_combine(const CombineArgs& a, cudaStream_t s);
 // B matrices are row-major [N, K] (K contiguous): the reference's weight layout.
 enum GemmMode { kSwiGLU = 0, kPlain = 1 };
 
-// Token rows of the CTA-pair kernel: the same buffer in boxes of several heights, of which a tile takes the
-// smallest that holds half of it.
-constexpr int kPairBoxes = 8;
-__host__ __device__ constexpr int pair_box_rows(int i) { return 16 * (i + 1); }
+// Token rows of the CTA-pair kernel: the same buffer in boxes of several heights (pair_tiles.cuh).
 struct PairRowMaps {
   CUtensorMap box[kPairBoxes];
 };
@@ -234,7 +232,8 @@ int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y,
 // Tensor-map encoding through the driver entry point (no link-time dependency on libcuda).
 int encode_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
                         uint32_t box_rows, uint32_t box_cols);
-int encode_pair_rows(PairRowMaps* out, const void* base, uint64_t rows, uint64_t cols);  // grouped_gemm_2cta.cu
+// grouped_gemm_2cta.cu; `boxes` (bit i: box i) are encoded, a launch reads no others
+int encode_pair_rows(PairRowMaps* out, const void* base, uint64_t rows, uint64_t cols, unsigned boxes = kPairAllBoxes);
 // int8 matrix [rows, cols]; unswizzled box, or 64-byte swizzle for the row-per-thread reads of the
 // TMEM-operand kernel
 int encode_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,

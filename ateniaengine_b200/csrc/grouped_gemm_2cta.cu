@@ -35,7 +35,7 @@ namespace atenia {
 namespace {
 using namespace tc;
 
-constexpr int TN2 = 256;     // token rows of a tile at most (MMA N)
+constexpr int TN2 = kPairTokens;
 constexpr int STAGES2 = 6;
 constexpr int ACC_BUFS2 = 2;
 constexpr int TMEM_COLS2 = 512;
@@ -74,8 +74,8 @@ __device__ __forceinline__ void pair_cursor_load(PairCursor& c, const int32_t* _
   c.row_begin = off[c.group];
   c.row_end = off[c.group + 1];
   const int rows = c.row_end - c.row_begin;
-  c.m_tiles = (rows + TN2 - 1) / TN2;
-  c.tile_rows = c.m_tiles > 0 ? ((rows + c.m_tiles - 1) / c.m_tiles + 15) & ~15 : 16;
+  c.m_tiles = pair_tiles(rows);
+  c.tile_rows = pair_tile_rows(rows, c.m_tiles);
 }
 __device__ __forceinline__ bool pair_cursor_seek(PairCursor& c, int tile, int f_tiles, int num_groups,
                                                  const int32_t* __restrict__ off, PairTile& out, int f_width) {
@@ -88,7 +88,7 @@ __device__ __forceinline__ bool pair_cursor_seek(PairCursor& c, int tile, int f_
       out.group = c.group;
       out.row0 = c.row_begin + mt * c.tile_rows;
       out.rows = min(c.row_end - out.row0, c.tile_rows);  // >= 1: tile_rows <= 256, so no tile starts past the end
-      out.n = (out.rows + 15) & ~15;
+      out.n = pair_tile_n(out.rows);
       out.f0 = ft * f_width;
       return true;
     }
@@ -158,9 +158,6 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
       ::"r"(bar), "h"(mask)
       : "memory");
 }
-
-// the box (index of PairRowMaps) that holds the half sub-tile a CTA stages
-__device__ __forceinline__ int pair_box(int half_rows) { return (half_rows + 15) / 16 - 1; }
 
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS2, 1)
@@ -235,7 +232,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
         if (MODE == kSwiGLU) tmap_acquire(m1);
         last_group = tc.group;
       }
-      const int box = pair_box(tc.n / 2);
+      const int box = pair_tile_box(tc.n);
       const CUtensorMap* mx = &tmaps_x.box[box];
       const int f_row = tc.f0 + (int)rank * F_CTA;
       const int x_row = tc.row0 + (int)rank * (tc.n / 2);
@@ -417,10 +414,10 @@ int launch_2cta_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
 
 }  // namespace
 
-int encode_pair_rows(PairRowMaps* out, const void* base, uint64_t rows, uint64_t cols) {
+int encode_pair_rows(PairRowMaps* out, const void* base, uint64_t rows, uint64_t cols, unsigned boxes) {
   int rc = ATENIA_OK;
   for (int i = 0; i < kPairBoxes && !rc; ++i)
-    rc = encode_tmap_2d_bf16(&out->box[i], base, rows, cols, pair_box_rows(i), BK);
+    if (boxes >> i & 1u) rc = encode_tmap_2d_bf16(&out->box[i], base, rows, cols, pair_box_rows(i), BK);
   return rc;
 }
 

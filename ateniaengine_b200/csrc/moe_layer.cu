@@ -238,8 +238,9 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   }
   GroupedGemmArgs g1{};
   g1.chained = L->gemm_chained;
-  PairRowMaps x_rows;
-  int rc = pairs ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model)
+  // (the one group has T rows: only the boxes of its tiles, since the caller's x makes this part of every call)
+  PairRowMaps x_rows{};
+  int rc = pairs ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model, pair_boxes_of_group(T))
                  : encode_tmap_2d_bf16(&g1.tmap_a, xb, (uint64_t)T, (uint64_t)c.d_model, 128, 64);
   if (rc) return rc;
   g1.pair_rows = &x_rows;
