@@ -675,8 +675,8 @@ __global__ void __launch_bounds__(kQThreads) quantize_digits_kernel(DigitSource 
                                                                     int K, int plane_rows, int8_t* __restrict__ planes,
                                                                     float* __restrict__ tok_scale) {
   const int row = blockIdx.x;
-  chain_next();
   chain_wait();
+  chain_next();  // (after the wait: the GEMM behind takes every SM, so it may come no earlier than these rows)
   // rows the dispatch did not place (invalid expert ids) hold nothing: skip them
   const int placed = n_rows_dev ? (*n_rows_dev < n_rows ? *n_rows_dev : n_rows) : n_rows;
   if (row >= placed) return;
@@ -765,11 +765,11 @@ int launch_grouped_gemm_w8_i8_decode(const GroupedGemmArgs& a, int num_sms, cuda
 }
 
 int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, int n_rows, int K, int plane_rows,
-                           int8_t* planes, float* tok_scale, cudaStream_t s) {
+                           int8_t* planes, float* tok_scale, bool chained, cudaStream_t s) {
   if (n_rows <= 0) return ATENIA_OK;
   if (K % 16 != 0 || n_rows > plane_rows || !src.x || (src.perm && src.k < 1)) return ATENIA_ERR_SHAPE;
   count_launch();
-  return launch_chained(true, quantize_digits_kernel, dim3(n_rows), dim3(kQThreads), 0, s, src, n_rows_dev, n_rows, K, plane_rows,
+  return launch_chained(chained, quantize_digits_kernel, dim3(n_rows), dim3(kQThreads), 0, s, src, n_rows_dev, n_rows, K, plane_rows,
                         planes, tok_scale);
 }
 

@@ -56,9 +56,15 @@ inline bool first_use_on_current_device(bool (&flags)[kMaxDevices]) {
 // launched plainly and wait for everything before them as usual.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// A kernel that takes a whole SM must not sit there waiting while another stream's work could run (`chained` false:
-// Qwen1.5-MoE shape, 2048 tokens, 342 -> 372 us when the routed GEMM displaced the shared expert's), and a captured
-// launch stays plain: a graph's own edges are as fast (eight INT8 layers, 8 tokens: 1657 -> 1688 us chained).
+// A kernel that takes whole SMs must not sit there waiting while another stream's work could run.  So the kernels
+// before the first GEMM of a forward (row gather, digit quantiser) call chain_next() after their chain_wait(): the GEMM
+// comes no earlier than the rows it reads are being written, and not already beside the router (one token of the
+// Mixtral shape 137.3 -> 134.8 us for it, other sizes the same).  Beside a layer's own shared expert the GEMMs are
+// not chained at all (`chained` false: Qwen1.5-MoE shape, 2048 tokens, 342 -> 372 us when the routed GEMM displaced the
+// shared expert's), and a captured launch stays plain: a graph's own edges are as fast (eight INT8 layers, 8 tokens:
+// 1657 -> 1688 us chained).  Two layers on two streams, in all ms for the same calls, chained / plain: Mixtral shape of
+// 1024 tokens beside a 64-expert layer of 64 44.2 / 46.7, 4096 beside 64 42.5 / 49.2, 64 beside 16 33.5 / 35.6.
+// ATENIA_MOE_CHAINED=0 makes every launch of a layer plain.
 template <typename... P, typename... A>
 int launch_chained(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   if (chained) {
@@ -227,7 +233,8 @@ int launch_f32_to_bf16(const float* src, __nv_bfloat16* dst, int64_t n, cudaStre
 // p[0] = a, p[1] = b on the stream (the one-group offsets of the shared expert's GEMMs)
 int launch_set_pair(int32_t* p, int32_t a, int32_t b, cudaStream_t s);
 // y = (x * inv_rms(x)) * gamma per row (stack.cu); gamma may be null (unit gain)
-int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y, int T, int d, cudaStream_t s);
+int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y, int T, int d, bool chained,
+                        cudaStream_t s);
 
 // Tensor-map encoding through the driver entry point (no link-time dependency on libcuda).
 int encode_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
@@ -270,7 +277,7 @@ struct DigitSource {
   int n_src_rows;
 };
 int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, int n_rows, int K, int plane_rows,
-                           int8_t* planes, float* tok_scale, cudaStream_t s);
+                           int8_t* planes, float* tok_scale, bool chained, cudaStream_t s);
 // bf16 weights, CTA pairs (tcgen05 cta_group::2), transposed product: pair_rows describes the token rows (tmap_a
 // is not read), tmap_b0 / tmap_b1 have boxes of kPairWeightRows (kSwiGLU) or 128 (kPlain) weight rows
 constexpr int kPairWeightRows = 64;

@@ -309,8 +309,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32) gather_rows_kernel(const vo
                                                                          int total_rows) {
   const int lane = threadIdx.x & 31;
   const int nvec = d / 8;
-  chain_next();
   chain_wait();
+  chain_next();  // (after the wait: the GEMM behind takes every SM, so it may come no earlier than these rows)
   const int n_placed = n_rows > 0 ? *placed : 0;
   for (int r = blockIdx.x * kGatherWarps + (threadIdx.x >> 5); r < total_rows; r += gridDim.x * kGatherWarps) {
     int src_t, dst_r;

@@ -28,6 +28,7 @@ struct AteniaMoeLayer {
   bool use_gemv = true;         // small calls take the matrix-vector kernel (decode_gemv.cu)
   int gemv_rows = 2;   // calls of at most this many rows take it
   bool timing = false;
+  bool chained = true;          // launches may start early (ATENIA_MOE_CHAINED=0: plain launches)
   bool gemm_chained = false;    // of the current forward: its GEMMs may start early (nothing runs beside them)
   const float* residual = nullptr;  // set by a stack around one forward: added by the combine kernel
   float* block_normed = nullptr;    // [max_tokens, d] f32, allocated by the first atenia_moe_block_forward

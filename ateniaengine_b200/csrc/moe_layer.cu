@@ -86,7 +86,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   if (i8dec) {
     const DigitSource own{a_ptr, 0, nullptr, 1, max_rows};
     int rc = launch_quantize_digits(gather_here ? L->i8_src : own, group_offsets + num_groups, max_rows, c.d_model,
-                                    L->i8_rows, L->dq_x, L->dq_ts_x, s);
+                                    L->i8_rows, L->dq_x, L->dq_ts_x, L->gemm_chained, s);
     if (rc) return rc;
     GroupedGemmArgs g1{};
     g1.chained = L->gemm_chained;
@@ -113,7 +113,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     if (L->timing) cudaEventRecord(L->ev[1], s);
     const DigitSource mid_rows{mid, 0, nullptr, 1, max_rows};
     rc = launch_quantize_digits(mid_rows, group_offsets + num_groups, max_rows, c.d_ff, L->i8_rows, L->dq_h, L->dq_ts_h,
-                                s);
+                                L->gemm_chained, s);
     if (rc) return rc;
     GroupedGemmArgs g2 = g1;
     g2.tmap_a = L->tm_dq_h;
@@ -321,6 +321,7 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
   L->w8_mode = std::getenv("ATENIA_MOE_W8_MODE") ? std::atoi(std::getenv("ATENIA_MOE_W8_MODE")) : 0;
   L->pair_mode = std::getenv("ATENIA_MOE_PAIR_MODE") ? std::atoi(std::getenv("ATENIA_MOE_PAIR_MODE")) : 0;
   L->shared_aside = !(std::getenv("ATENIA_MOE_SHARED_ASIDE") && std::atoi(std::getenv("ATENIA_MOE_SHARED_ASIDE")) == 0);
+  L->chained = !(std::getenv("ATENIA_MOE_CHAINED") && std::atoi(std::getenv("ATENIA_MOE_CHAINED")) == 0);
   L->use_gemv = !(std::getenv("ATENIA_MOE_GEMV") && std::atoi(std::getenv("ATENIA_MOE_GEMV")) == 0);
   // ATENIA_MOE_W8_I8=0: INT8 decode calls keep the widening kernels; ATENIA_MOE_W8_I8_ROWS moves the row
   // count up to which the integer-MMA decode kernel is taken (16 .. kI8DecodeMaxRows; A/B runs)
@@ -728,8 +729,8 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   // Blocks of a chained kernel sit on the SMs while they wait.  Beside a shared expert that is affordable while the
   // row gather (8 rows a block) brings at most two blocks to an SM; more would keep its GEMMs out (Qwen1.5-MoE shape,
   // 2048 tokens, 345 -> 370 us).
-  const bool chained = !shared_aside || n <= 16 * L->num_sms;
-  L->gemm_chained = !shared_aside;
+  const bool chained = L->chained && (!shared_aside || n <= 16 * L->num_sms);
+  L->gemm_chained = L->chained && !shared_aside;
   if (shared_aside) {
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
     if (x_f32) {
@@ -851,7 +852,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   ca.T = T;
   ca.k = k;
   ca.d = c.d_model;
-  ca.chained = !shared_aside;
+  ca.chained = L->gemm_chained;
   rc = launch_combine(ca, s);
   if (rc) return rc;
   if (L->timing) {
@@ -884,7 +885,7 @@ int atenia_moe_block_forward(AteniaMoeLayer* L, const float* x, const float* gam
                                (size_t)L->cfg.max_tokens * (size_t)L->cfg.d_model * sizeof(float)));
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int rc = launch_rmsnorm_rows(x, gamma, eps, L->block_normed, T, L->cfg.d_model, s);
+  int rc = launch_rmsnorm_rows(x, gamma, eps, L->block_normed, T, L->cfg.d_model, L->chained, s);
   if (rc) return rc;
   L->residual = x;  // added last by the combine kernel: out = x + MoE(h)
   rc = forward_impl(L, L->block_normed, ATENIA_IO_F32, T, out, ATENIA_IO_F32, nullptr, stream, nullptr, nullptr);

@@ -100,10 +100,11 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float*
 }  // namespace
 
 namespace atenia {
-int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y, int T, int d, cudaStream_t s) {
+int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y, int T, int d, bool chained,
+                        cudaStream_t s) {
   if (T <= 0) return ATENIA_OK;
   count_launch();
-  return launch_chained(true, rmsnorm_rows_kernel, dim3(T), dim3(kNormThreads), 0, s, x, gamma, eps, y, d);
+  return launch_chained(chained, rmsnorm_rows_kernel, dim3(T), dim3(kNormThreads), 0, s, x, gamma, eps, y, d);
 }
 }  // namespace atenia
 
@@ -127,7 +128,7 @@ int run_layers(AteniaMoeStack* S, const void* x, int x_dtype, int T, void* out, 
     const void* in = cur;
     if (S->prenorm) {
       const float* g = S->gammas.empty() ? nullptr : S->gammas[(size_t)l];
-      int nrc = atenia::launch_rmsnorm_rows(static_cast<const float*>(cur), g, S->eps, S->normed, T, S->d_model, s);
+      int nrc = atenia::launch_rmsnorm_rows(static_cast<const float*>(cur), g, S->eps, S->normed, T, S->d_model, L->chained, s);
       if (nrc) return nrc;
       in = S->normed;
     }
