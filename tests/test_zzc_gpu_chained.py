@@ -8,8 +8,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-#: entries of the permutation below and above the sizes at which the routing kernels stop being chained beside a shared
-#: expert (16 per SM) and at which the dispatch changes its kernel (1024)
+#: below and above the sizes at which the routing kernels stop being chained beside a shared expert (four tokens per
+#: SM) and at which the dispatch changes its kernel (1024 entries)
 BATCHES = [1, 400, 9, 130, 700, 2, 333, 64, 257, 16, 500, 1]
 V3 = {"n_group": 4, "topk_group": 2, "scaling": 2.5, "e_score_bias": None}
 
