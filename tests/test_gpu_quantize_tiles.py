@@ -34,3 +34,28 @@ def test_row_quantiser_at_block_edges(rows, cols):
     q_ref, s_ref = orc.quantize_per_row_i8(w.numpy())
     np.testing.assert_array_equal(s.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
     np.testing.assert_array_equal(q.cpu().numpy(), q_ref)
+
+
+@pytest.mark.parametrize("K,N,g", [
+    (8250, 256, 129), (8250, 253, 129),                       # one block per item
+    (33000, 256, 1024), (16384, 252, 1024), (1281, 66, 700),  # clusters of two, four and two
+    (4500, 130, 0), (4500, 132, 4097),                        # clusters of eight
+    (16400, 132, 0), (16390, 67, 0),                          # three passes: few items
+    (20001, 8, 16), (20001, 7, 16), (1100, 100, 1),           # three passes: small items
+    (300, 160, 64), (70, 264, 0), (513, 24, 100)])            # narrow strips: flat dequant
+def test_group_quantiser_forms(K, N, g):
+    import torch
+    from ateniaengine_b200 import int8_to_bf16_per_group, quantize_per_group_i8
+    from oracle import oracle as orc
+    w = torch.randn((K, N), generator=torch.Generator().manual_seed(K + N)) * 0.02
+    w[0, :3] = torch.tensor([float("inf"), float("nan"), 0.0])
+    w[:, N // 2] = 0.0
+    q, s = quantize_per_group_i8(w.cuda(), g)
+    q_ref, s_ref = orc.absmax_per_group_symmetric(w.numpy(), g)
+    np.testing.assert_array_equal(s.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
+    np.testing.assert_array_equal(q.cpu().numpy(), q_ref)
+    out = int8_to_bf16_per_group(q, s, g).view(torch.int16).cpu().numpy().view(np.uint16)
+    ref = np.asarray(orc.int8_to_bf16_per_group(q_ref, s_ref, g), dtype=np.uint16)
+    nan = (ref & 0x7FFF) > 0x7F80  # code 0 x scale inf: any NaN pattern
+    np.testing.assert_array_equal((out & 0x7FFF) > 0x7F80, nan)
+    np.testing.assert_array_equal(out[~nan], ref[~nan])
