@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "../../include/atenia_moe.h"
+#include "kernel_choice.cuh"
 #include "pair_tiles.cuh"
 
 namespace atenia {
@@ -262,8 +263,8 @@ int launch_grouped_gemm_bf16_decode(const GroupedGemmArgs& a, int num_sms, cudaS
 // launch_quantize_digits.  tmap_a is the digit-plane map (uint8, box {128, 16}, 128B swizzle; plane p of
 // row r at row p * plane_rows + r), tmap_b0 / tmap_b1 int8 maps with box {128, 128} and the 128B swizzle.
 constexpr int kI8DecodeMaxRows = 512;      // largest call (rows of one digit plane) a layer may be set up for
-// ... and what a layer takes unless told otherwise.  Mixtral shape, integer-MMA / tensor-memory kernel, a forward of 65,
-// 128, 256 tokens (130, 256, 512 rows): 266 / 370, 348 / 387, 526 / 391 us.
+// ... and what it is set up for unless told otherwise (512 rows of the Mixtral shape: 526 us, tensor-memory kernel 391).
+// Which calls take it up to there: i8_decode_pays (kernel_choice.cuh).
 constexpr int kI8DecodeDefaultRows = 256;
 int launch_grouped_gemm_w8_i8_decode(const GroupedGemmArgs& a, int num_sms, cudaStream_t s);
 // planes [4][plane_rows][K] int8 and tok_scale [plane_rows] of n_rows rows; n_rows_dev (device, may be null)

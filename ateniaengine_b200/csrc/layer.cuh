@@ -105,6 +105,7 @@ struct AteniaMoeLayer {
   // the token rows and of the intermediate rows with their row scales, and the planes' tensor maps
   bool w8_i8 = true;
   int i8_rows = 0;  // rows of one digit plane = the largest call the kernel takes
+  bool i8_rows_pinned = false;  // ATENIA_MOE_W8_I8_ROWS: every call of at most i8_rows rows takes it
   CUtensorMap* d_tm_gate_i8 = nullptr;
   CUtensorMap* d_tm_up_i8 = nullptr;
   CUtensorMap* d_tm_down_i8 = nullptr;

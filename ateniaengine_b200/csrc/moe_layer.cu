@@ -45,6 +45,14 @@ int validate_config(const AteniaMoeConfig& c) {
   return ATENIA_OK;
 }
 
+// Does an INT8 call of `rows` rows take the integer-MMA decode kernel?  Asked by the forward, which then leaves the row
+// gather to that kernel's digit pass, and by the GEMMs.
+bool takes_i8_decode(const AteniaMoeLayer* L, int rows) {
+  const AteniaMoeConfig& c = L->cfg;
+  return c.weight_dtype == ATENIA_W_INT8_ROW && L->w8_i8 && L->dq_x && rows <= L->i8_rows && !L->use_check_gemm &&
+         L->w8_mode == 0 && (L->i8_rows_pinned || i8_decode_pays(rows, c.num_experts, c.d_model, c.d_ff, L->has_shared));
+}
+
 }  // namespace
 
 int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_mid,
@@ -68,15 +76,15 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   const bool dec = !q && !L->use_check_gemm && L->splitk_ws &&
                    (L->bf16_decode == 1 ? max_rows <= 128 : (L->bf16_decode < 0 && max_rows <= 16));
   const bool pairs = !q && !dec && L->pair_mode != 2;
-  // a call of at most two rows in all (decode at batch 1) is a stream over the touched experts' weights:
-  // the CUDA-core matrix-vector kernel (ATENIA_MOE_GEMV=0 keeps the tensor-core kernels: A/B runs)
-  // INT8, calls of at most i8_rows rows (decode): the codes multiplied as integers against digit planes of
+  // INT8, small calls (takes_i8_decode): the codes multiplied as integers against digit planes of
   // the token rows (bf16_decode_gemm.cu, I8 form) -- nothing is widened and the kernel streams weights like
   // the bf16 one.  Measured on B200, Mixtral shape, 1 / 8 / 64 tokens: 0.145 / 0.221 / 0.390 ms against
   // 0.160 (matrix-vector kernel) / 0.300 / 0.525 ms (tensor-memory kernel).  ATENIA_MOE_W8_I8=0 or a pinned
   // w8_mode keep the widening kernels (tests, A/B runs).
-  const bool i8dec = q && L->w8_i8 && L->dq_x && max_rows <= L->i8_rows && !L->use_check_gemm && L->w8_mode == 0;
-  // bf16 from kGemvMaxWeights weights on: the stream-K kernel, whose launch costs more and whose stream is faster
+  const bool i8dec = takes_i8_decode(L, max_rows);
+  // a call of at most two rows in all (decode at batch 1) is a stream over the touched experts' weights:
+  // the CUDA-core matrix-vector kernel (ATENIA_MOE_GEMV=0 keeps the tensor-core kernels: A/B runs); bf16 from
+  // kGemvMaxWeights weights on: the stream-K kernel, whose launch costs more and whose stream is faster
   const bool dec_few = dec && (int64_t)max_rows * c.d_model * c.d_ff >= kGemvMaxWeights;
   const bool gemv = L->use_gemv && max_rows <= L->gemv_rows && !L->use_check_gemm && !i8dec && !dec_few;
   if (L->timing) cudaEventRecord(L->ev[0], s);
@@ -427,6 +435,7 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
     r = r < 16 ? 16 : (r > kI8DecodeMaxRows ? kI8DecodeMaxRows : r);
     const int cap = (int)((R + 15) / 16 * 16);  // never more planes than the layer has rows
     L->i8_rows = r < cap ? r : cap;
+    L->i8_rows_pinned = e != nullptr;
   }
     TRY_ALLOC(L->d_tm_gate_i8, (size_t)L->n_groups);
     TRY_ALLOC(L->d_tm_up_i8, (size_t)L->n_groups);
@@ -806,8 +815,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   // the direct expert-parallel exchange gathers rows straight into the owners' buffers
   const bool direct = c.ep_world > 1 && !L->ep_replicated && L->ep_direct;
   // an INT8 decode call (integer-MMA kernel) never reads x_perm: its digit kernel gathers the rows itself
-  const bool i8_gather = c.weight_dtype == ATENIA_W_INT8_ROW && L->w8_i8 && L->dq_x && n <= L->i8_rows &&
-                         !L->use_check_gemm && L->w8_mode == 0 && (c.ep_world == 1 || L->ep_replicated);
+  const bool i8_gather = takes_i8_decode(L, n) && (c.ep_world == 1 || L->ep_replicated);
   rc = launch_gather_rows(x, x_f32, L->perm, L->expert_offsets + c.num_experts, (direct || i8_gather) ? 0 : n, k,
                           c.d_model, L->x_perm, need_xb ? L->x_bf16 : nullptr, T, chained, s);
   if (rc) return rc;

@@ -1,0 +1,6 @@
+// Test-only: compiles the kernel-choice rules with a host compiler.  Not part of the product library.
+#include "../ateniaengine_b200/csrc/kernel_choice.cuh"
+
+extern "C" int choice_i8_decode(int rows, int experts, int d, int F, int shared) {
+  return atenia::i8_decode_pays(rows, experts, d, F, shared != 0);
+}

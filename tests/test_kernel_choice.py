@@ -1,0 +1,38 @@
+"""The rules that pick an expert GEMM kernel from sizes, compiled for the host, against the calls they were measured on."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    so = tmp_path_factory.mktemp("choice") / "libchoiceprobe.so"
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-shared", "-fPIC",
+                           os.path.join(ROOT, "tests", "kernel_choice_probe.cpp"), "-o", str(so)])
+    return C.CDLL(str(so))
+
+
+# rows, experts, d, F, shared expert, us of the integer-MMA kernel, us of the widening kernel
+I8 = [(130, 8, 4096, 14336, 0, 267, 377), (192, 8, 4096, 14336, 0, 284, 379), (256, 8, 4096, 14336, 0, 319, 389),
+      (192, 16, 4096, 7168, 0, 280, 380), (160, 4, 4096, 14336, 0, 271, 280), (224, 4, 4096, 14336, 0, 219, 284),
+      (192, 3, 4096, 14336, 0, 267, 243), (250, 3, 4096, 14336, 0, 292, 247), (192, 2, 4096, 14336, 0, 228, 220),
+      (256, 2, 4096, 14336, 0, 277, 227), (250, 1, 4096, 14336, 0, 233, 212), (130, 8, 2048, 7168, 0, 118, 156),
+      (224, 8, 3072, 8192, 0, 191, 205), (192, 8, 2048, 4096, 0, 98, 101), (250, 8, 2048, 4096, 0, 106, 103),
+      (192, 4, 2048, 4096, 0, 88, 84), (192, 64, 2048, 1408, 0, 194, 187), (132, 60, 2048, 1408, 1, 203, 228),
+      (256, 60, 2048, 1408, 1, 230, 263), (192, 8, 1024, 2816, 0, 76, 72), (192, 8, 1024, 1024, 0, 56, 44),
+      (192, 128, 2048, 768, 0, 257, 200), (192, 8, 512, 1408, 0, 62, 43), (252, 32, 2048, 1408, 0, 120, 118)]
+
+
+@pytest.mark.parametrize("rows,experts,d,F,shared,i8,wide", I8)
+def test_integer_mma_decode_kernel_is_taken_where_it_is_the_faster_one(lib, rows, experts, d, F, shared, i8, wide):
+    assert bool(lib.choice_i8_decode(rows, experts, d, F, shared)) == (i8 < wide)
+
+
+def test_up_to_128_rows_the_integer_mma_decode_kernel_is_always_taken(lib):
+    for rows in (1, 16, 127, 128):
+        for experts, d, F in [(1, 16, 16), (8, 4096, 14336), (128, 64, 64)]:
+            assert lib.choice_i8_decode(rows, experts, d, F, 0) and lib.choice_i8_decode(rows, experts, d, F, 1)
