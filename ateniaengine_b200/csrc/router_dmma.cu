@@ -230,28 +230,30 @@ __global__ void __launch_bounds__(WARPS * 32) router_dmma_direct_kernel(RouterAr
 }
 
 template <int E_T, int MT, int NTW, int WARPS>
-int launch_form(const RouterArgs& a, cudaStream_t s) {
+int launch_form(const RouterArgs& a, bool chained, cudaStream_t s) {
   constexpr int NW_K = WARPS / ((E_T / 8) / NTW);
   constexpr int kTok = 8 * MT;
   // k-range of a k-slice: d over the slices, rounded up to whole 32-k steps
   const int kw = ((a.d + NW_K - 1) / NW_K + 31) / 32 * 32;
   const int grid = (a.T + kTok - 1) / kTok;
-  if (a.x_is_f32) return launch_chained(a.chained, router_dmma_direct_kernel<E_T, MT, NTW, true, WARPS>, dim3(grid), dim3(WARPS * 32), 0, s, a, kw);
-  return launch_chained(a.chained, router_dmma_direct_kernel<E_T, MT, NTW, false, WARPS>, dim3(grid), dim3(WARPS * 32), 0, s, a, kw);
+  if (a.x_is_f32) return launch_chained(chained, router_dmma_direct_kernel<E_T, MT, NTW, true, WARPS>, dim3(grid), dim3(WARPS * 32), 0, s, a, kw);
+  return launch_chained(chained, router_dmma_direct_kernel<E_T, MT, NTW, false, WARPS>, dim3(grid), dim3(WARPS * 32), 0, s, a, kw);
 }
 
 // Two forms.  A batch whose 8-token CTAs fit the SMs in one round is bound by the latency of its
 // dependent load -> multiply steps, not by a pipe: 16 warps per CTA cut the k-range, and with it the
 // number of steps, of every warp in half (DeepSeek-V2-Lite shape, 1024 tokens: router 41 -> 22 us).
-// Larger batches take 16 tokens and 8 warps per CTA, 2 to 3 CTAs per SM.
+// Larger batches take 16 tokens and 8 warps per CTA, 2 to 3 CTAs per SM.  They are launched plainly: CTAs placed while
+// the kernel before still runs go two and three to the SMs that free up first, and the others stay empty (128 experts of
+// 2048 x 768, 1500 / 2048 tokens, a forward with the router plain / chained: 357 / 377, 382 / 397 us).
 constexpr int kSmallBatchCtas = 148;
 
 template <int E_T>
 int launch_direct(const RouterArgs& a, cudaStream_t s) {
   constexpr int NT = E_T / 8;
   constexpr int NTW = NT < 2 ? NT : 2;
-  if ((a.T + 7) / 8 <= kSmallBatchCtas) return launch_form<E_T, 1, NTW, 2 * kDW>(a, s);
-  return launch_form<E_T, 2, NTW, kDW>(a, s);
+  if ((a.T + 7) / 8 <= kSmallBatchCtas) return launch_form<E_T, 1, NTW, 2 * kDW>(a, a.chained, s);
+  return launch_form<E_T, 2, NTW, kDW>(a, false, s);
 }
 
 }  // namespace
