@@ -2,8 +2,9 @@
 //
 // One launch covers every expert of a layer.  A persistent grid (one CTA per SM) walks a tile list
 // derived on the device from the dispatch offsets, so the host never reads routing results.
-// The forward takes the kernels of grouped_gemm_2cta.cu, w8_gemm.cu and w8_gemm_m256.cu; this one is their
-// cross-check (ATENIA_MOE_PAIR_MODE=2, ATENIA_MOE_W8_MODE=2).
+// bf16 calls of many rows take it for products over a short k (pair_pays, kernel_choice.cuh); otherwise the forward takes
+// the kernels of grouped_gemm_2cta.cu, w8_gemm.cu and w8_gemm_m256.cu, and this one is their cross-check
+// (ATENIA_MOE_PAIR_MODE=2, ATENIA_MOE_W8_MODE=2).
 //
 //   tile            = 128 rows of one expert  x  BN_OUT output columns
 //   kSwiGLU         : B tile = 128 rows of W_gate || 128 rows of W_up  -> one M128 x N256 MMA,
@@ -81,7 +82,6 @@ grouped_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
                             DeviceError* err) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int32_t goff_s[kMaxGroupsShared + 1];
-  const int32_t* group_offsets = stage_group_offsets(group_offsets_g, num_groups, goff_s);
   constexpr int BN_OUT = (MODE == kSwiGLU) ? BN / 2 : BN;
   // 1024-byte alignment is required by the 128B swizzle atoms.
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -124,6 +124,8 @@ grouped_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  chain_wait();  // (everything above touches only this CTA's shared and tensor memory)
+  const int32_t* group_offsets = stage_group_offsets(group_offsets_g, num_groups, goff_s);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -373,6 +375,7 @@ grouped_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
     }
   }
 
+  chain_next();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -430,10 +433,9 @@ static int launch_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
     ATENIA_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_tcgen05_kernel<MODE, W8>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   }
-  grouped_gemm_tcgen05_kernel<MODE, W8><<<dim3(num_sms), dim3(kThreads), kSmem, s>>>(
-      a.tmap_a, a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out,
-      a.scale0, a.scale1, a.err);
-  return (int)cudaGetLastError();
+  return launch_chained(a.chained, grouped_gemm_tcgen05_kernel<MODE, W8>, dim3(num_sms), dim3(kThreads), kSmem, s, a.tmap_a,
+                        a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K,
+                        a.out, a.scale0, a.scale1, a.err);
 }
 
 int launch_grouped_gemm_tcgen05(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {

@@ -31,4 +31,16 @@ inline bool i8_decode_pays(int rows, int experts, int d, int F, bool shared) {
   return shared && weights >= (int64_t)1 << 21 && r <= 5 * e;
 }
 
+// bf16 products above decode size: does the CTA-pair kernel (grouped_gemm_2cta.cu) pay against the single-CTA one
+// (grouped_gemm.cu)?  The pair kernel's tile is 256 weight rows x up to 256 tokens and leaves tensor memory two bytes a
+// lane; over a short k that store takes longer than the MMAs.  One product on a B200, pair / single-CTA, us:
+//   k 512   8 experts, n 1408, 32 / 64 / 256 rows an expert 16 / 14, 17 / 14, 27 / 20; n 512, 64 rows 13 / 14; 128 experts, n 512,
+//           16 / 100 / 512 rows 49 / 43, 64 / 46, 143 / 97
+//   k 1024  8 experts, n 1024, 64 / 128 / 256 rows 16 / 18, 18 / 18, 27 / 25; 32 experts, n 2816, 64 / 256 / 1024 rows 74 / 72, 128 /
+//           120, 388 / 344; 128 experts, n 512, 100 / 256 rows 77 / 68, 109 / 97
+//   k 1408  (n 2048) 32 experts, 64 / 256 rows 45 / 43, 69 / 73; 128 experts, 100 / 256 157 / 142, 216 / 255
+//   k 2048  8 experts, n 512, 64 rows 18 / 22; 32 experts, n 1408, 64 / 256 / 1024 rows 74 / 78, 109 / 117, 293 / 345
+constexpr int kPairMinK = 1024, kPairFewRows = 1024;
+inline bool pair_pays(int rows, int k) { return k > kPairMinK || rows < kPairFewRows; }
+
 }  // namespace atenia

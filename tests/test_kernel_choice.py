@@ -36,3 +36,15 @@ def test_up_to_128_rows_the_integer_mma_decode_kernel_is_always_taken(lib):
     for rows in (1, 16, 127, 128):
         for experts, d, F in [(1, 16, 16), (8, 4096, 14336), (128, 64, 64)]:
             assert lib.choice_i8_decode(rows, experts, d, F, 0) and lib.choice_i8_decode(rows, experts, d, F, 1)
+
+
+# experts, rows an expert, k, us of the CTA-pair kernel, us of the single-CTA kernel
+PAIRS = [(8, 256, 512, 27, 20), (8, 1024, 512, 51, 38), (32, 100, 512, 37, 31), (128, 16, 512, 49, 43), (128, 512, 512, 143, 97),
+         (8, 256, 1024, 27, 25), (32, 256, 1024, 128, 120), (32, 1024, 1024, 388, 344), (128, 100, 1024, 77, 68),
+         (8, 64, 512, 13, 14), (8, 64, 1024, 16, 18), (32, 256, 1408, 69, 73), (128, 256, 1408, 216, 255), (8, 64, 2048, 18, 22),
+         (32, 64, 2048, 74, 78), (32, 1024, 2048, 293, 345)]
+
+
+@pytest.mark.parametrize("experts,rows,k,pair,single", PAIRS)
+def test_pair_kernel_is_taken_where_it_is_the_faster_one(lib, experts, rows, k, pair, single):
+    assert bool(lib.choice_pairs(experts * rows, k)) == (pair < single)
