@@ -11,7 +11,7 @@
 //   quantize_passes  maxima, scales and codes in three launches over the whole grid, for matrices whose groups
 //                    and strips are too few or too small for the kernels above
 //   dequant          a block owns 256 columns x 64 rows; a lane keeps its eight scales while the group lasts;
-//                    narrow matrices take a flat walk
+//                    narrow matrices and groups of few rows take a flat walk
 // The three passes and the flat walk spend two 64-bit divisions per vector, the others none.  Measured on a B200
 // at 4096 x 14336, groups of 128: quantise 149 (three passes) -> 68 us, dequant 42 (flat) -> 32 us; floors at the
 // measured copy rate 47 and 28 us.
@@ -225,10 +225,17 @@ __global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ w, 
   if (hi > (g + 1) * G) hi = (g + 1) * G;
   if (hi > K) hi = K;
   float m[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int64_t r = lo + warp; r < hi; r += 8) {
-    float v[4];
-    load_cols4<VEC, 32>(v, w + r * N, strip0, lane, N);
-    max_cols4(m, v);
+  if (!VEC || strip0 + lane * 4 < N) {
+    for (int64_t r = lo + warp; r < hi; r += 8) {
+      float v[4];
+      if (VEC) {
+        const float4 f = *reinterpret_cast<const float4*>(w + r * N + strip0 + lane * 4);
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+      } else {
+        load_cols4<false, 32>(v, w + r * N, strip0, lane, N);
+      }
+      max_cols4(m, v);
+    }
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) red[warp][VEC ? lane * 4 + j : lane + 32 * j] = m[j];
@@ -343,11 +350,21 @@ __global__ void __launch_bounds__(256) dequant_kernel(const int8_t* __restrict__
   }
 }
 
-// Strips that few columns fill: the same over one flat list, so that every lane has columns (rows of whole vectors).
+// Strips that few columns fill, and groups of few rows: the same over one flat list.
+template <bool VEC>
 __global__ void __launch_bounds__(256) dequant_flat_kernel(const int8_t* __restrict__ q, const float* __restrict__ scales,
                                                            int64_t K, int64_t N, int64_t G, uint16_t* __restrict__ out) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x, n8 = K * N / 8;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += stride) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (!VEC) {
+    const int64_t n = K * N;
+    for (; i < n; i += stride) {
+      const int64_t r = i / N, c = i % N;
+      out[i] = (uint16_t)trunc_bf16((int)q[i], scales[(r / G) * N + c]);
+    }
+    return;
+  }
+  for (const int64_t n8 = K * N / 8; i < n8; i += stride) {
     const int64_t e = i * 8, r = e / N, c = e % N;
     const uint2 p = *reinterpret_cast<const uint2*>(q + e);
     const float* srow = scales + (r / G) * N + c;
@@ -408,7 +425,7 @@ int launch_quantize_tall(const float* w, int64_t K, int64_t N, int64_t G, int8_t
 //                    184 / 188 / 182 / 282
 //   small items      a block of the groups kernel costs what its launch costs.  1048576 x 8, groups of 128 142 / 63 three
 //                    passes, 262144 x 8 39.9 / 27.7, 262144 x 16 by 64 35.8 / 34.1, 262144 x 32 by 64 35.8 / 40.7, 262144 x
-//                    32 by 1 898 / 370, 65536 x 8 17.2 / 25.2
+//                    32 by 1 898 / 370, 65536 x 8 17.2 / 25.2; 4096 x 14336 by 1 1151 / 1048, by 2 598 / 598
 template <bool VEC>
 int launch_quantize(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, float* scales, cudaStream_t s) {
   const int64_t groups = (K + G - 1) / G;
@@ -423,7 +440,7 @@ int launch_quantize(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, 
                        : launch_quantize_tall<VEC, 8>(w, K, N, G, q, scales, s);
   }
   const int64_t strips = (N + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK;
-  if (N < COLS_PER_BLOCK && N * G <= 1024 && groups > 1024) return launch_quantize_passes<VEC>(w, K, N, G, q, scales, s);
+  if (groups > 1024 && (G == 1 || (N < COLS_PER_BLOCK && N * G <= 1024))) return launch_quantize_passes<VEC>(w, K, N, G, q, scales, s);
   const unsigned grid = (unsigned)(strips * groups), st = (unsigned)strips;
   if (G <= 32) quantize_groups_kernel<VEC, 8, 4><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
   else if (G <= 64) quantize_groups_kernel<VEC, 8, 8><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
@@ -465,9 +482,13 @@ int atenia_int8_to_bf16_per_group(const int8_t* q, const float* scales, int64_t 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool vec = N % 8 == 0 && aligned16(out_bf16) && aligned16(scales) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
   // strips filled to less than five eighths: the flat walk (262144 rows, strips / flat: 32 columns 27.4 / 14.3 us, 128
-  // 29.4 / 22.9, 160 31.3 / 29.4, 192 31.5 / 33.6; 131072 x 264 29.5 / 24.6; unaligned rows gain nothing: x 100 68 / 81)
-  if (vec && 8 * N <= 5 * DEQ_COLS * strips)
-    dequant_flat_kernel<<<grid_for(K * N / 8), 256, 0, s>>>(q, scales, K, N, G, out_bf16);
+  // 29.4 / 22.9, 160 31.3 / 29.4, 192 31.5 / 33.6; 131072 x 264 29.5 / 24.6; unaligned rows gain nothing: x 100 68 / 81);
+  // and groups of under 16 rows, whose scales a lane holds for one row in eight (4096 x 14336 by 1 / 8 / 16 72.6 / 64.3,
+  // 60.3 / 45.9, 43.2 / 43.9; 300000 x 100 by 8 120 / 109)
+  if (vec && (G < 16 || 8 * N <= 5 * DEQ_COLS * strips))
+    dequant_flat_kernel<true><<<grid_for(K * N / 8), 256, 0, s>>>(q, scales, K, N, G, out_bf16);
+  else if (G < 16)
+    dequant_flat_kernel<false><<<grid_for(K * N), 256, 0, s>>>(q, scales, K, N, G, out_bf16);
   else if (vec)
     dequant_kernel<true><<<grid, 256, 0, s>>>(q, scales, K, N, G, (unsigned)strips, out_bf16);
   else

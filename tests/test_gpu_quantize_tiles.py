@@ -41,8 +41,8 @@ def test_row_quantiser_at_block_edges(rows, cols):
     (33000, 256, 1024), (16384, 252, 1024), (1281, 66, 700),  # clusters of two, four and two
     (4500, 130, 0), (4500, 132, 4097),                        # clusters of eight
     (16400, 132, 0), (16390, 67, 0),                          # three passes: few items
-    (20001, 8, 16), (20001, 7, 16), (1100, 100, 1),           # three passes: small items
-    (300, 160, 64), (70, 264, 0), (513, 24, 100)])            # narrow strips: flat dequant
+    (20001, 8, 16), (20001, 7, 16), (1100, 100, 1), (1030, 260, 1),  # three passes: small items
+    (300, 160, 64), (70, 264, 0), (513, 24, 100), (90, 520, 15), (90, 517, 15)])  # flat dequant: narrow, small groups
 def test_group_quantiser_forms(K, N, g):
     import torch
     from ateniaengine_b200 import int8_to_bf16_per_group, quantize_per_group_i8
