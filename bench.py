@@ -275,6 +275,22 @@ def host_threads():
         return max(1, os.cpu_count() or 1)
 
 
+def gate_up_kernel(shape, rows, groups):
+    """The kernel a routed gate/up product of `rows` rows takes (run_expert_gemms; the lines of csrc/kernel_choice.cuh)."""
+    weights, E = shape.d_model * shape.d_ff, shape.num_experts
+    if shape.int8:
+        few = (rows < 64 * E if weights >= 1 << 25 else rows <= 30 * E if weights >= 1 << 23
+               else shape.shared_d_ff > 0 and weights >= 1 << 21 and rows <= 5 * E)
+        if rows <= 128 or (rows <= 256 and few):
+            return "grouped_gemm_decode_kernel"
+        return "grouped_gemm_w8_tmem_kernel" if rows < 256 * groups else "grouped_gemm_w8_m256_kernel"
+    if rows <= 2 and rows * weights < 1 << 26:
+        return "grouped_gemv_kernel"
+    if rows <= 16:
+        return "grouped_gemm_decode_kernel"
+    return "grouped_gemm_2cta_kernel" if shape.d_model > 1024 or rows < 1024 else "grouped_gemm_tcgen05_kernel"
+
+
 def layer_roofline(shape, T, touched, peaks, int8):
     """Whole-forward target on one GPU: the slower of the expert flops at the measured tensor peak and
     the bytes that must cross HBM (weights of the experts that got a row, router, activations in and
@@ -737,10 +753,7 @@ def main():
     rows_slow = per_rank[slow][0]
     g1_slow, g2_slow = per_rank[slow][1], per_rank[slow][2]
     groups = (shape.num_experts // args.gpus) * (args.gpus if args.gpus > 1 and not direct else 1)
-    if shape.int8:
-        kname = "grouped_gemm_w8_tmem_kernel" if rows_slow < 256 * groups else "grouped_gemm_w8_m256_kernel"
-    else:
-        kname = "grouped_gemm_2cta_kernel"
+    kname = gate_up_kernel(shape, rows_slow, groups)
     # dominant kernel: the routed gate/up + SwiGLU grouped GEMM of the rank with the most rows
     flops1 = 4.0 * rows_slow * shape.d_model * shape.d_ff  # gate and up: 2 * 2 * rows * d * F
     achieved = flops1 / (g1_slow * 1e-3) / 1e12

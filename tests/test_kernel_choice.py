@@ -48,3 +48,23 @@ PAIRS = [(8, 256, 512, 27, 20), (8, 1024, 512, 51, 38), (32, 100, 512, 37, 31), 
 @pytest.mark.parametrize("experts,rows,k,pair,single", PAIRS)
 def test_pair_kernel_is_taken_where_it_is_the_faster_one(lib, experts, rows, k, pair, single):
     assert bool(lib.choice_pairs(experts * rows, k)) == (pair < single)
+
+
+def test_the_benchmark_names_the_kernel_that_runs(lib):
+    import sys
+    sys.path.insert(0, ROOT)
+    import bench
+    from ateniaengine_b200.synth import MoeShape
+
+    for d, F, E, k, Fs in [(512, 1408, 8, 2, 0), (1024, 512, 128, 8, 0), (2048, 1408, 60, 4, 5632), (2048, 4096, 8, 2, 0),
+                           (4096, 14336, 8, 2, 0), (4096, 14336, 2, 2, 0)]:
+        for rows in (1, 2, 3, 16, 17, 128, 129, 192, 240, 256, 257, 1023, 1024, 4096, 70000):
+            name = bench.gate_up_kernel(MoeShape("s", d, F, E, k, True, Fs, int8=True), rows, E)
+            assert (name == "grouped_gemm_decode_kernel") == (rows <= 256 and bool(lib.choice_i8_decode(rows, E, d, F, Fs > 0)))
+            if name != "grouped_gemm_decode_kernel":
+                assert name == ("grouped_gemm_w8_m256_kernel" if rows >= 256 * E else "grouped_gemm_w8_tmem_kernel")
+            name = bench.gate_up_kernel(MoeShape("s", d, F, E, k, True, Fs), rows, E)
+            if rows > 16:
+                assert (name == "grouped_gemm_2cta_kernel") == bool(lib.choice_pairs(rows, d))
+            else:
+                assert name == ("grouped_gemv_kernel" if rows <= 2 and rows * d * F < 1 << 26 else "grouped_gemm_decode_kernel")
