@@ -212,40 +212,59 @@ quantize_tall_kernel(const float* __restrict__ w, int64_t K, int64_t N, int64_t 
 // narrow, to fill the SMs above: maxima of 128 columns x up to 256 rows of one group merged by atomicMax on the bit
 // pattern (non-negative floats order like unsigned integers, so the result does not depend on scheduling), scales in
 // place, codes.
-constexpr int CHUNK_ROWS = 256;
+constexpr int CHUNK_ROWS = 256, CHUNK_LANES = 8;
 
-template <bool VEC>
+struct Quad {
+  float v[4];
+};
+
+// Four consecutive columns of row r starting at c0; columns >= N read as 0.
+__device__ __forceinline__ Quad load_quad(const float* __restrict__ w, int64_t r, int64_t c0, int64_t N, bool vec) {
+  Quad o;
+  if (vec) {
+    const float4 f = *reinterpret_cast<const float4*>(w + r * N + c0);
+    o.v[0] = f.x; o.v[1] = f.y; o.v[2] = f.z; o.v[3] = f.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.v[j] = (c0 + j < N) ? w[r * N + c0 + j] : 0.f;
+  }
+  return o;
+}
+
 __global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ w, int64_t K, int64_t N, int64_t G,
-                                                   int64_t strips, int64_t chunks, unsigned int* __restrict__ amax_bits) {
-  __shared__ float red[8][COLS_PER_BLOCK];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t y = blockIdx.x / strips, strip0 = (blockIdx.x - y * strips) * COLS_PER_BLOCK;
-  const int64_t g = y / chunks, lo = g * G + (y - g * chunks) * CHUNK_ROWS;
+                                                    int64_t strips, int64_t chunks_per_group, int vec,
+                                                    unsigned int* __restrict__ amax_bits) {
+  __shared__ float red[CHUNK_LANES][COLS_PER_BLOCK];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t strip = blockIdx.x % strips, y = blockIdx.x / strips;
+  const int64_t g = y / chunks_per_group, ch = y % chunks_per_group;
+  const int64_t lo = g * G + ch * CHUNK_ROWS;
   int64_t hi = lo + CHUNK_ROWS;
   if (hi > (g + 1) * G) hi = (g + 1) * G;
   if (hi > K) hi = K;
+  const int64_t c0 = strip * COLS_PER_BLOCK + tx * 4;
   float m[4] = {0.f, 0.f, 0.f, 0.f};
-  if (!VEC || strip0 + lane * 4 < N) {
-    for (int64_t r = lo + warp; r < hi; r += 8) {
-      float v[4];
-      if (VEC) {
-        const float4 f = *reinterpret_cast<const float4*>(w + r * N + strip0 + lane * 4);
-        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-      } else {
-        load_cols4<false, 32>(v, w + r * N, strip0, lane, N);
+  if (c0 < N) {
+    for (int64_t r = lo + ty; r < hi; r += CHUNK_LANES) {
+      const Quad x = load_quad(w, r, c0, N, vec != 0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = fabsf(x.v[j]);
+        if (a > m[j]) m[j] = a;  // a NaN never compares greater: skipped, as in the reference
       }
-      max_cols4(m, v);
     }
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) red[warp][VEC ? lane * 4 + j : lane + 32 * j] = m[j];
+  for (int j = 0; j < 4; ++j) red[ty][tx * 4 + j] = m[j];
   __syncthreads();
-  const int64_t c = strip0 + threadIdx.x;
-  if (threadIdx.x < COLS_PER_BLOCK && c < N && lo < hi) {
-    float a = red[0][threadIdx.x];
+  if (threadIdx.x < COLS_PER_BLOCK) {
+    const int64_t c = strip * COLS_PER_BLOCK + threadIdx.x;
+    if (c < N && lo < hi) {
+      float a = red[0][threadIdx.x];
 #pragma unroll
-    for (int l = 1; l < 8; ++l) a = fmaxf(a, red[l][threadIdx.x]);
-    if (a > 0.f) atomicMax(&amax_bits[g * N + c], __float_as_uint(a));
+      for (int l = 1; l < CHUNK_LANES; ++l) a = fmaxf(a, red[l][threadIdx.x]);
+      if (a > 0.f) atomicMax(&amax_bits[g * N + c], __float_as_uint(a));
+    }
   }
 }
 
@@ -254,12 +273,12 @@ __global__ void finalize_scales_kernel(float* __restrict__ scales, int64_t n) {
   for (; i < n; i += (int64_t)gridDim.x * blockDim.x) scales[i] = scale_of(scales[i]);
 }
 
-template <bool VEC>
 __global__ void __launch_bounds__(256) quantize_flat_kernel(const float* __restrict__ w, const float* __restrict__ scales,
-                                                            int64_t K, int64_t N, int64_t G, int8_t* __restrict__ q) {
+                                                        int64_t K, int64_t N, int64_t G, int vec,
+                                                        int8_t* __restrict__ q) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (VEC) {
+  if (vec) {
     const int64_t n4 = K * N / 4;
     for (; i < n4; i += stride) {
       const int64_t e = i * 4, r = e / N, c = e % N;
@@ -389,20 +408,20 @@ inline unsigned grid_for(int64_t work_items) {
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <bool VEC>
 int launch_quantize_passes(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, float* scales, cudaStream_t s) {
   const int64_t groups = (K + G - 1) / G, strips = (N + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK;
   const int64_t chunks = (G + CHUNK_ROWS - 1) / CHUNK_ROWS;
   ATENIA_CUDA_TRY(cudaMemsetAsync(scales, 0, (size_t)(groups * N) * sizeof(float), s));
-  amax_kernel<VEC><<<(unsigned)(strips * groups * chunks), 256, 0, s>>>(w, K, N, G, strips, chunks,
-                                                                        reinterpret_cast<unsigned int*>(scales));
+  const int vec_w = (N % 4 == 0 && aligned16(w)) ? 1 : 0;
+  amax_kernel<<<(unsigned)(strips * groups * chunks), 256, 0, s>>>(w, K, N, G, strips, chunks, vec_w,
+                                                                   reinterpret_cast<unsigned int*>(scales));
   count_launch();
   ATENIA_CUDA_TRY(cudaGetLastError());
   finalize_scales_kernel<<<grid_for(groups * N), 256, 0, s>>>(scales, groups * N);
   count_launch();
   ATENIA_CUDA_TRY(cudaGetLastError());
-  if (VEC && aligned16(scales)) quantize_flat_kernel<true><<<grid_for(K * N / 4), 256, 0, s>>>(w, scales, K, N, G, q);
-  else quantize_flat_kernel<false><<<grid_for(K * N), 256, 0, s>>>(w, scales, K, N, G, q);
+  const int vec_q = (vec_w && aligned16(scales) && (reinterpret_cast<uintptr_t>(q) & 3u) == 0) ? 1 : 0;
+  quantize_flat_kernel<<<grid_for(vec_q ? K * N / 4 : K * N), 256, 0, s>>>(w, scales, K, N, G, vec_q, q);
   count_launch();
   return (int)cudaGetLastError();
 }
@@ -410,7 +429,7 @@ int launch_quantize_passes(const float* w, int64_t K, int64_t N, int64_t G, int8
 template <bool VEC, int CTAS>
 int launch_quantize_tall(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, float* scales, cudaStream_t s) {
   const int64_t strips = (N + TALL_COLS - 1) / TALL_COLS, items = strips * ((K + G - 1) / G);
-  if (items > 0x7fffffffLL / CTAS) return launch_quantize_passes<VEC>(w, K, N, G, q, scales, s);
+  if (items > 0x7fffffffLL / CTAS) return launch_quantize_passes(w, K, N, G, q, scales, s);
   quantize_tall_kernel<VEC, CTAS><<<(unsigned)(items * CTAS), TALL_WARPS * 32, 0, s>>>(w, K, N, G, strips, q, scales);
   count_launch();
   return (int)cudaGetLastError();
@@ -418,20 +437,20 @@ int launch_quantize_tall(const float* w, int64_t K, int64_t N, int64_t G, int8_t
 
 // Where the lines lie (B200, us; the Python call costs about 15, so short ones are all launch):
 //   few tall items   a cluster walks K / 256 rows per lane whatever the width.  Eight items or fewer of more than
-//                    16384 rows, clusters / three passes: 16384 x 256 25.5 / 27.4, 32768 x 64 42.2 / 23.5, 65536 x 512
-//                    125 / 91, 262144 x 128 388 / 91; 16 items: 65536 x 1024 155 / 163
-//   blocks per item  clusters of 1 / 2 / 8 blocks and three passes, 8192 x 14336: groups of 256 169 / 234 / 905 / 285,
-//                    of 512 146 / 179 / 528 / 284, of 1024 154 / 152 / 298 / 284, of 2048 183 / 160 / 219 / 283, of 4096
-//                    184 / 188 / 182 / 282
-//   small items      a block of the groups kernel costs what its launch costs.  1048576 x 8, groups of 128 142 / 63 three
-//                    passes, 262144 x 8 39.9 / 27.7, 262144 x 16 by 64 35.8 / 34.1, 262144 x 32 by 64 35.8 / 40.7, 262144 x
-//                    32 by 1 898 / 370, 65536 x 8 17.2 / 25.2; 4096 x 14336 by 1 1151 / 1048, by 2 598 / 598
+//                    16384 rows, clusters / three passes: 16384 x 256 19.2 / 24.7, 32768 x 64 31.6 / 25.0, 65536 x 512
+//                    112 / 89, 262144 x 128 382 / 89; 16 items: 65536 x 1024 136 / 160
+//   blocks per item  8192 x 14336, the cluster taken / clusters of eight / three passes: groups of 256 163 / 836 / 271, of
+//                    512 141 / 530 / 268 (one block), of 1024 148 / 279 / 268, of 2048 156 / 201 / 267 (two), of 4096 165 /
+//                    165 / 267; 2048 x 4096 by 256 17.4 / 56.4 / 32.1
+//   small items      a block of the groups kernel costs what its launch costs.  Groups kernel / three passes: 1048576 x 8 by
+//                    128 142 / 59, 262144 x 8 by 128 39.9 / 27.0, 262144 x 16 by 64 35.8 / 34.6, 262144 x 32 by 64 35.8 /
+//                    40.7, 262144 x 32 by 1 899 / 406, 65536 x 8 by 128 17.6 / 26.1; 4096 x 14336 by 1 1151 / 1048, by 2 598 / 598
 template <bool VEC>
 int launch_quantize(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, float* scales, cudaStream_t s) {
   const int64_t groups = (K + G - 1) / G;
   if (G > GROUP_ROWS_MAX) {
     const int64_t items = groups * ((N + TALL_COLS - 1) / TALL_COLS);
-    if (items <= 8 && G > 16384) return launch_quantize_passes<VEC>(w, K, N, G, q, scales, s);
+    if (items <= 8 && G > 16384) return launch_quantize_passes(w, K, N, G, q, scales, s);
     int ctas = G >= 4096 ? 8 : G >= 1024 ? 2 : 1;
     while (ctas < 8 && items * ctas < 256 && G >= ctas * 256) ctas *= 2;  // (fill the SMs with 128 rows a block or more)
     return ctas == 1   ? launch_quantize_tall<VEC, 1>(w, K, N, G, q, scales, s)
@@ -440,7 +459,7 @@ int launch_quantize(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, 
                        : launch_quantize_tall<VEC, 8>(w, K, N, G, q, scales, s);
   }
   const int64_t strips = (N + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK;
-  if (groups > 1024 && (G == 1 || (N < COLS_PER_BLOCK && N * G <= 1024))) return launch_quantize_passes<VEC>(w, K, N, G, q, scales, s);
+  if (groups > 1024 && (G == 1 || (N < COLS_PER_BLOCK && N * G <= 1024))) return launch_quantize_passes(w, K, N, G, q, scales, s);
   const unsigned grid = (unsigned)(strips * groups), st = (unsigned)strips;
   if (G <= 32) quantize_groups_kernel<VEC, 8, 4><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
   else if (G <= 64) quantize_groups_kernel<VEC, 8, 8><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
