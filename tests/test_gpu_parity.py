@@ -153,7 +153,7 @@ def test_w8a16_structure(dev):
 @pytest.mark.parametrize("mode", ["0", "1", "2"])
 def test_w8a16_every_kernel(dev, monkeypatch, mode):
     """ATENIA_MOE_W8_MODE pins the INT8 kernel family (0: by size -- the integer-MMA decode kernel up to
-    128 rows, weights widened into tensor memory for small groups, 256-row tiles widened into shared memory
+    128 rows (256 with large experts), weights widened into tensor memory for small groups, 256-row tiles widened into shared memory
     for large ones; 1: always the tensor-memory kernel; 2: 128-row tiles widened into shared memory); each
     must meet the bar at small and large group sizes."""
     monkeypatch.setenv("ATENIA_MOE_W8_MODE", mode)
@@ -204,7 +204,7 @@ def test_tensor_core_kernel_agrees_with_cuda_core_check(dev, monkeypatch):
 
 @pytest.mark.parametrize("T", [5, 300, 1100])
 def test_cta_pair_kernel_matches_single_cta_kernel(dev, monkeypatch, T):
-    """ATENIA_MOE_PAIR_MODE pins the bf16 kernel (1: CTA pairs with 256-row tiles, 2: single CTA).
+    """ATENIA_MOE_PAIR_MODE pins the bf16 kernel (1: CTA pairs, equal token tiles of at most 256 rows, 2: single CTA).
     Both see the same rows and accumulate over k in the same order."""
     synth = _synth()
     shape = synth.small(synth.SHAPES["deepseek_v2_lite"], d_model=512, d_ff=384, shared_d_ff=256)

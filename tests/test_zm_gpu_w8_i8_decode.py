@@ -1,5 +1,5 @@
 """The INT8 decode kernel that multiplies the codes as integers (tcgen05 kind::i8, the token rows as four
-planes of base-128 digits; the default for INT8 calls of at most 128 rows) against the oracle and against the
+planes of base-128 digits; the default for INT8 calls of at most 128 rows, and of up to 256 with large experts) against the oracle and against the
 tensor-memory decode kernel it replaced (ATENIA_MOE_W8_I8=0)."""
 from dataclasses import replace
 

@@ -1,5 +1,8 @@
-"""The CTA-pair kernel at the edges of its tiles: groups of 0, 1, 15 .. 17, 255 .. 257, 511 .. 513 rows (token tiles
-are equal parts of at most 256 rows, rounded up to 16), features and k that fill no tile, both weight types."""
+"""Expert GEMM kernels at the edges of their tiles, features and k that fill no tile.  bf16: the CTA-pair kernel (pinned:
+by default products of 1024 rows or more over k of at most 1024 take the single-CTA kernel, which runs on the same
+groups), 0, 1, 15 .. 17, 255 .. 257, 511 .. 513 rows (token tiles are equal parts of at most 256 rows, rounded up to 16).  INT8 takes
+other kernels on the same groups: the integer-MMA decode kernel up to 128 rows in all (token tiles of 32 rows), the
+tensor-memory kernel (128 rows) above, the 256-row-tile kernel from 256 rows a group on; their own edges follow."""
 import numpy as np
 import pytest
 import torch
@@ -14,8 +17,41 @@ TOL = 2 * 2.0 ** -9
 @pytest.mark.parametrize("sizes", [[1, 15, 16, 17, 0, 31, 33, 7], [255, 256, 257, 0, 1, 240, 273, 16],
                                    [511, 512, 513, 0, 769, 1030, 2, 300]])
 @pytest.mark.parametrize("d,F", [(272, 144), (512, 1408)])
-def test_groups_at_tile_edges(sizes, d, F, int8):
-    from ateniaengine_b200 import moe, synth
+def test_groups_at_tile_edges(monkeypatch, sizes, d, F, int8):
+    if not int8:
+        monkeypatch.setenv("ATENIA_MOE_PAIR_MODE", "1")
+    _check_groups(sizes, d, F, int8)
+
+
+@pytest.mark.parametrize("sizes", [[511, 512, 513, 0, 769, 1030, 2, 300], [128, 127, 129, 0, 255, 257, 127, 0],
+                                   [128, 127, 129, 0, 255, 257, 128, 0]])
+@pytest.mark.parametrize("d,F", [(272, 144), (1024, 1040), (1040, 1024)])
+def test_short_k_by_the_default_rule(sizes, d, F):
+    """1023, 1024 and more rows, k of 1024 and the next: both products on either kernel."""
+    _check_groups(sizes, d, F, False)
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("sizes", [[31, 32, 33, 32], [31, 32, 33, 0, 33], [64, 65, 63, 33, 31], [64, 65, 63, 33, 32],
+                                   [127, 128, 129, 1], [255, 256, 257, 512]])
+def test_int8_groups_at_tile_edges(monkeypatch, sizes, pinned):
+    """Totals of 128, 129, 256, 257, 385 and 1280 rows: by the default rule (small experts: integer-MMA up to 128 rows,
+    then the widening kernels) and with the integer-MMA kernel for every call of at most 512 rows."""
+    if pinned:
+        monkeypatch.setenv("ATENIA_MOE_W8_I8_ROWS", "512")
+    _check_groups(sizes, 272, 144, True)
+
+
+@pytest.mark.parametrize("sizes", [[33, 32, 31, 1, 16, 17, 0, 0], [33, 32, 31, 1, 64, 31, 0, 0],
+                                   [65, 33, 32, 31, 64, 15, 0, 0], [64, 65, 31, 32, 33, 31, 0, 0]])
+def test_int8_large_experts_by_the_default_rule(sizes):
+    """130, 192 and 240 rows in eight experts large enough for the integer-MMA kernel above 128 rows, and 256, which are
+    more than 30 an expert and take the tensor-memory kernel."""
+    _check_groups(sizes, 2048, 4096, True)
+
+
+def _check_groups(sizes, d, F, int8):
+    from ateniaengine_b200 import synth
 
     dev = torch.device("cuda:0")
     shape = synth.MoeShape("edges", d, F, len(sizes), 1, True, int8=int8)

@@ -14,13 +14,13 @@ BATCHES = [1, 400, 9, 130, 700, 2, 333, 64, 257, 16, 500, 1]
 V3 = {"n_group": 4, "topk_group": 2, "scaling": 2.5, "e_score_bias": None}
 
 
-def _pair(monkeypatch, name, shared, v3=None):
+def _pair(monkeypatch, name, shared, v3=None, seed=2):
     """The same layer twice: launched as it is by default, and plainly."""
     from ateniaengine_b200 import moe, synth
 
     dev = torch.device("cuda:0")
     shape = synth.small(synth.SHAPES[name], d_model=512, d_ff=384, shared_d_ff=shared)
-    w = synth.make_weights(shape, 2, dev)
+    w = synth.make_weights(shape, seed, dev)
 
     def make():
         if v3 is None:
@@ -73,23 +73,24 @@ def test_back_to_back_equals_plain_launches(monkeypatch, name, shared, v3):
 @pytest.mark.parametrize("name,shared", [("mixtral", 0), ("qwen_moe", 256), ("mixtral_int8", 0)])
 @pytest.mark.parametrize("T", [1, 9, 400, 700])
 def test_calls_that_feed_one_another(monkeypatch, name, shared, T):
-    """Each call reads what the one before wrote, into two buffers in turn."""
+    """Two layers in turn, each call reading what the one before wrote, in two buffers."""
     layer, plain, _ = _pair(monkeypatch, name, shared)
+    second, plain_second, _ = _pair(monkeypatch, name, shared, seed=3)
     gamma = torch.ones(512, device="cuda:0")
     x = torch.randn((T, 512), generator=torch.Generator(device="cuda:0").manual_seed(T), device="cuda:0")
 
-    def chain(which):
+    def chain(*layers):
         bufs = [x.clone(), torch.zeros_like(x)]
         torch.cuda.synchronize()
         for i in range(8):
-            which.block_forward(bufs[i & 1], gamma=gamma, out=bufs[1 - (i & 1)])
+            layers[i >> 1 & 1].block_forward(bufs[i & 1], gamma=gamma, out=bufs[1 - (i & 1)])
         torch.cuda.synchronize()
         return bufs[0]
 
-    want = chain(plain)
+    want = chain(plain, plain_second)
     assert torch.isfinite(want).all()
     for _ in range(4):
-        assert torch.equal(chain(layer), want)
+        assert torch.equal(chain(layer, second), want)
 
 
 def test_given_selections_back_to_back(monkeypatch):
