@@ -61,8 +61,8 @@ __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.laun
 // before the first GEMM of a forward (row gather, digit quantiser) call chain_next() after their chain_wait(): the GEMM
 // comes no earlier than the rows it reads are being written, and not already beside the router (one token of the
 // Mixtral shape 137.3 -> 134.8 us for it, other sizes the same).  Beside a layer's own shared expert the GEMMs are
-// not chained at all (`chained` false: Qwen1.5-MoE shape, 2048 tokens, 342 -> 372 us when the routed GEMM displaced the
-// shared expert's), and a captured launch stays plain: a graph's own edges are as fast (eight INT8 layers, 8 tokens:
+// not chained at all (`chained` false: Qwen1.5-MoE shape, 2048 tokens, in bursts after a pause, 342 -> 372 us when the
+// routed GEMM displaced the shared expert's), and a captured launch stays plain: a graph's own edges are as fast (eight INT8 layers, 8 tokens:
 // 1657 -> 1688 us chained).  Two layers on two streams, in all ms for the same calls, chained / plain: Mixtral shape of
 // 1024 tokens beside a 64-expert layer of 64 44.2 / 46.7, 4096 beside 64 42.5 / 49.2, 64 beside 16 33.5 / 35.6.
 // ATENIA_MOE_CHAINED=0 makes every launch of a layer plain.

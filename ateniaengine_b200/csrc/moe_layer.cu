@@ -741,7 +741,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   // ATENIA_MOE_SHARED_ASIDE=0 turns it off.
   const bool shared_aside = L->has_shared && T > L->gemv_rows && L->aux_stream && L->shared_aside;
   // Blocks of a chained kernel sit on the SMs while they wait.  Beside a shared expert that is affordable up to about
-  // four tokens per SM; from there on they keep its GEMMs out.  A forward with plain / chained routing kernels, us:
+  // four tokens per SM; from there on they keep its GEMMs out.  20 forwards after a pause, plain / chained routing kernels, us each:
   // DeepSeek-V2-Lite shape, 197 / 592 / 1578 tokens 233.9 / 228.0, 255.3 / 250.8, 313.7 / 340.1; Qwen1.5-MoE shape, 148 /
   // 592 / 1776 tokens 234.3 / 223.7, 249.0 / 249.3, 327.6 / 351.8; 16 experts top-1 of 1024 x 2048, 592 / 2368 tokens
   // 81.0 / 76.2, 109.5 / 113.8; 8 experts top-2 of 4096 x 4096, 592 / 1184 tokens 221.2 / 223.4, 339.7 / 343.4.

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kSkWarps * 32) router_splitk_kernel(RouterArgs
     }
   }
   double* part = a.sk_part + ((size_t)slice * n_tb + tb) * kSkTok * E_T;
-  // sums of eight tokens over the lanes; the lanes 4 t .. 4 t + 3 end with token fold_token(lane)
+  // sums of eight tokens over the lanes; the lanes 4 t .. 4 t + 3 end with that of token t
   static_assert(kSkTok == 8, "three halving levels");
   auto fold8 = [&](double (&v)[kSkTok]) {
 #pragma unroll
