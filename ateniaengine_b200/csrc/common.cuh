@@ -283,6 +283,8 @@ int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, in
 // is not read), tmap_b0 / tmap_b1 have boxes of kPairWeightRows (kSwiGLU) or 128 (kPlain) weight rows
 constexpr int kPairWeightRows = 64;
 int launch_grouped_gemm_2cta(const GroupedGemmArgs& a, int num_sms, cudaStream_t s);
+// bf16 weights, CTA pairs, token rows as the M side (grouped_gemm_pair_rows.cu): tensor maps of the single-CTA kernel
+int launch_grouped_gemm_pair_rows(const GroupedGemmArgs& a, int num_sms, cudaStream_t s);
 
 // Sub-batch sizes for the host-buffer operator (planner.cu): n tokens in pieces of at most cap tokens,
 // chosen with a cost model of the copies and the forward; one piece means "do not overlap".  `fit`

@@ -2,7 +2,7 @@
 //
 // One launch covers every expert of a layer.  A persistent grid (one CTA per SM) walks a tile list
 // derived on the device from the dispatch offsets, so the host never reads routing results.
-// bf16 calls of many rows take it for products over a short k (pair_pays, kernel_choice.cuh); otherwise the forward takes
+// bf16 calls of many rows in small groups take it for products over a short k (bf16_product_kernel, kernel_choice.cuh); otherwise the forward takes
 // the kernels of grouped_gemm_2cta.cu, w8_gemm.cu and w8_gemm_m256.cu, and this one is their cross-check
 // (ATENIA_MOE_PAIR_MODE=2, ATENIA_MOE_W8_MODE=2).
 //

@@ -31,8 +31,8 @@ inline bool i8_decode_pays(int rows, int experts, int d, int F, bool shared) {
   return shared && weights >= (int64_t)1 << 21 && r <= 5 * e;
 }
 
-// bf16 products above decode size: does the CTA-pair kernel (grouped_gemm_2cta.cu) pay against the single-CTA one
-// (grouped_gemm.cu)?  The pair kernel's tile is 256 weight rows x up to 256 tokens and leaves tensor memory two bytes a
+// bf16 products above decode size: the CTA-pair kernel (grouped_gemm_2cta.cu) against the single-CTA one
+// (grouped_gemm.cu).  The pair kernel's tile is 256 weight rows x up to 256 tokens and leaves tensor memory two bytes a
 // lane; over a short k that store takes longer than the MMAs.  One product on a B200, pair / single-CTA, us:
 //   k 512   8 experts, n 1408, 32 / 64 / 256 rows an expert 16 / 14, 17 / 14, 27 / 20; n 512, 64 rows 13 / 14; 128 experts, n 512,
 //           16 / 100 / 512 rows 49 / 43, 64 / 46, 143 / 97
@@ -40,7 +40,15 @@ inline bool i8_decode_pays(int rows, int experts, int d, int F, bool shared) {
 //           120, 388 / 344; 128 experts, n 512, 100 / 256 rows 77 / 68, 109 / 97
 //   k 1408  (n 2048) 32 experts, 64 / 256 rows 45 / 43, 69 / 73; 128 experts, 100 / 256 157 / 142, 216 / 255
 //   k 2048  8 experts, n 512, 64 rows 18 / 22; 32 experts, n 1408, 64 / 256 / 1024 rows 74 / 78, 109 / 117, 293 / 345
-constexpr int kPairMinK = 1024, kPairFewRows = 1024;
-inline bool pair_pays(int rows, int k) { return k > kPairMinK || rows < kPairFewRows; }
+// Groups of 512 rows or more take the pair kernel with the rows as its M side (grouped_gemm_pair_rows.cu).
+// A shared expert's gate/up product (`beside` the routing kernels, on the second stream) keeps the transposed pairs up to 4096
+// tokens; a forward with it there / on the single-CTA kernel, us: 32 experts top-4 of 1024 x 1024, shared 4096, 1184 / 2048 / 3000 /
+// 4096 tokens 119 / 134, 163 / 173, 215 / 222, 268 / 261; of 512 x 1408, shared 2816, 1024 / 3000 86 / 100, 140 / 146; 16 experts
+// top-1 of 1024 x 2048, shared 2048, 1500 / 4096 96 / 102, 147 / 159.
+enum Bf16Kernel { kBf16Pairs = 0, kBf16Single = 1, kBf16PairRows = 2 };
+inline Bf16Kernel bf16_product_kernel(int rows, int groups, int k, bool beside) {
+  if (k > 1024 || rows < (beside ? 4096 : 1024)) return kBf16Pairs;
+  return (int64_t)rows >= (int64_t)512 * groups ? kBf16PairRows : kBf16Single;
+}
 
 }  // namespace atenia

@@ -36,8 +36,8 @@ struct AteniaMoeLayer {
   // tile kernel of w8_gemm_m256.cu for large ones), 1 = always the small-group kernel,
   // 2 = always the 128-row shared-memory widening kernel (grouped_gemm.cu)
   int w8_mode = 0;
-  // bf16: 0 = pick per product (pair_pays), 1 = always the CTA-pair kernel, 2 = always the single-CTA kernel of
-  // grouped_gemm.cu
+  // bf16: 0 = pick per product (bf16_product_kernel), 1 = always the CTA-pair kernel, 2 = always the single-CTA kernel
+  // of grouped_gemm.cu, 3 = always the pair kernel of grouped_gemm_pair_rows.cu
   int pair_mode = 0;
   // bf16 stream-K decode kernel: -1 = calls of at most 16 rows, 1 = every call of at most 128 rows
   // (ATENIA_MOE_BF16_DECODE=1), 0 = never (=0, or INT8 weights)

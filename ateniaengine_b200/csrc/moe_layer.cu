@@ -53,9 +53,15 @@ bool takes_i8_decode(const AteniaMoeLayer* L, int rows) {
          L->w8_mode == 0 && (L->i8_rows_pinned || i8_decode_pays(rows, c.num_experts, c.d_model, c.d_ff, L->has_shared));
 }
 
-// Does a bf16 product of `rows` rows over `k` take the CTA-pair kernel?
-bool takes_pairs(const AteniaMoeLayer* L, int rows, int k) {
-  return L->pair_mode == 1 || (L->pair_mode != 2 && pair_pays(rows, k));
+// The kernel of a bf16 product of `rows` rows over `k`
+Bf16Kernel bf16_kernel(const AteniaMoeLayer* L, int rows, int groups, int k, bool beside) {
+  if (L->pair_mode >= 1 && L->pair_mode <= 3) return (Bf16Kernel)(L->pair_mode - 1);
+  return bf16_product_kernel(rows, groups, k, beside);
+}
+int launch_bf16_product(Bf16Kernel kernel, const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
+  return kernel == kBf16Pairs      ? launch_grouped_gemm_2cta(a, num_sms, s)
+         : kernel == kBf16PairRows ? launch_grouped_gemm_pair_rows(a, num_sms, s)
+                                   : launch_grouped_gemm_tcgen05(a, num_sms, s);
 }
 
 }  // namespace
@@ -75,12 +81,14 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   const bool tmem = q && !m256 && (L->w8_mode == 1 || (L->w8_mode != 2 && !large));
   // bf16: the CTA-pair kernel above the size of the decode kernel (its token tiles follow the row
   // count: 61 tokens of a DeepSeek-V2-Lite shape 263 us against 284 with the single-CTA kernel, 64 tokens of a
-  // 512-wide layer 50 against 54) but for products of many rows over a short k (pair_pays); a call of at most
+  // 512-wide layer 50 against 54) but for products of many rows over a short k
+  // (bf16_product_kernel); a call of at most
   // 16 rows (decode) takes the stream-K kernel of bf16_decode_gemm.cu, which spreads the few tiles
   // there are over all SMs (bf16_decode 1 / 0 pins it on for every call of at most 128 rows / off).
   const bool dec = !q && !L->use_check_gemm && L->splitk_ws &&
                    (L->bf16_decode == 1 ? max_rows <= 128 : (L->bf16_decode < 0 && max_rows <= 16));
-  const bool pairs1 = !q && !dec && takes_pairs(L, max_rows, c.d_model), pairs2 = !q && !dec && takes_pairs(L, max_rows, c.d_ff);
+  const Bf16Kernel bf1 = q ? kBf16Single : bf16_kernel(L, max_rows, num_groups, c.d_model, false),
+                   bf2 = q ? kBf16Single : bf16_kernel(L, max_rows, num_groups, c.d_ff, false);
   // INT8, small calls (takes_i8_decode): the codes multiplied as integers against digit planes of
   // the token rows (bf16_decode_gemm.cu, I8 form) -- nothing is widened and the kernel streams weights like
   // the bf16 one.  Measured on B200, Mixtral shape, 1 / 8 / 64 tokens: 0.145 / 0.221 / 0.390 ms against
@@ -158,8 +166,8 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     g1.chained = L->gemm_chained;
     g1.tmap_a = tm_a.tile;
     g1.pair_rows = &tm_a.pair;
-    g1.tmap_b0 = tmem ? L->d_tm_gate_sw : pairs1 ? L->d_tm_gate_box : L->d_tm_gate;
-    g1.tmap_b1 = tmem ? L->d_tm_up_sw : pairs1 ? L->d_tm_up_box : L->d_tm_up;
+    g1.tmap_b0 = tmem ? L->d_tm_gate_sw : !q && !dec && bf1 == kBf16Pairs ? L->d_tm_gate_box : L->d_tm_gate;
+    g1.tmap_b1 = tmem ? L->d_tm_up_sw : !q && !dec && bf1 == kBf16Pairs ? L->d_tm_up_box : L->d_tm_up;
     g1.group_offsets = group_offsets;
     g1.num_groups = num_groups;
     g1.N = c.d_ff;
@@ -176,8 +184,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     int rc = m256 ? launch_grouped_gemm_w8_m256(g1, L->num_sms, s)
                   : dec ? launch_grouped_gemm_bf16_decode(g1, L->num_sms, s)
                   : tmem ? launch_grouped_gemm_w8_tmem(g1, L->num_sms, s)
-                         : pairs1 ? launch_grouped_gemm_2cta(g1, L->num_sms, s)
-                                  : launch_grouped_gemm_tcgen05(g1, L->num_sms, s);
+                         : launch_bf16_product(bf1, g1, L->num_sms, s);
     if (rc) return rc;
   }
   if (L->timing) cudaEventRecord(L->ev[1], s);
@@ -209,8 +216,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     int rc = m256 ? launch_grouped_gemm_w8_m256(g2, L->num_sms, s)
                   : dec ? launch_grouped_gemm_bf16_decode(g2, L->num_sms, s)
                   : tmem ? launch_grouped_gemm_w8_tmem(g2, L->num_sms, s)
-                         : pairs2 ? launch_grouped_gemm_2cta(g2, L->num_sms, s)
-                                  : launch_grouped_gemm_tcgen05(g2, L->num_sms, s);
+                         : launch_bf16_product(bf2, g2, L->num_sms, s);
     if (rc) return rc;
   }
   if (L->timing) {
@@ -229,7 +235,8 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   // 256-row-tile kernel above)
   const bool m256 = q && T >= 256 && L->w8_mode != 1 && L->w8_mode != 2 && !L->use_check_gemm;
   const bool tmem = q && !m256 && (L->w8_mode == 1 || (L->w8_mode != 2 && T < 256));
-  const bool pairs1 = !q && takes_pairs(L, T, c.d_model), pairs2 = !q && takes_pairs(L, T, c.shared_d_ff);
+  const Bf16Kernel bf1 = q ? kBf16Single : bf16_kernel(L, T, 1, c.d_model, true),
+                   bf2 = q ? kBf16Single : bf16_kernel(L, T, 1, c.shared_d_ff, false);
   const bool gemv = L->use_gemv && T <= L->gemv_rows && !L->use_check_gemm;
   if (L->timing) cudaEventRecord(L->ev[3], s);
   if (L->use_check_gemm || gemv) {
@@ -253,11 +260,11 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   g1.chained = L->gemm_chained;
   // (the one group has T rows: only the boxes of its tiles, since the caller's x makes this part of every call)
   PairRowMaps x_rows{};
-  int rc = pairs1 ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model, pair_boxes_of_group(T))
-                  : encode_tmap_2d_bf16(&g1.tmap_a, xb, (uint64_t)T, (uint64_t)c.d_model, 128, 64);
+  int rc = bf1 == kBf16Pairs ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model, pair_boxes_of_group(T))
+                             : encode_tmap_2d_bf16(&g1.tmap_a, xb, (uint64_t)T, (uint64_t)c.d_model, 128, 64);
   if (rc) return rc;
   g1.pair_rows = &x_rows;
-  g1.tmap_b0 = tmem ? L->d_tm_shared_sw : pairs1 ? L->d_tm_shared_box : L->d_tm_shared;
+  g1.tmap_b0 = tmem ? L->d_tm_shared_sw : bf1 == kBf16Pairs ? L->d_tm_shared_box : L->d_tm_shared;
   g1.tmap_b1 = g1.tmap_b0 + 1;
   g1.group_offsets = L->shared_offsets;
   g1.num_groups = 1;
@@ -272,8 +279,7 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   g1.w8 = q;
   g1.splitk_ws = L->splitk_ws_shared;  // its own: these launches may run beside the routed GEMMs
   rc = m256 ? launch_grouped_gemm_w8_m256(g1, L->num_sms, s)
-       : tmem ? launch_grouped_gemm_w8_tmem(g1, L->num_sms, s)
-                  : pairs1 ? launch_grouped_gemm_2cta(g1, L->num_sms, s) : launch_grouped_gemm_tcgen05(g1, L->num_sms, s);
+       : tmem ? launch_grouped_gemm_w8_tmem(g1, L->num_sms, s) : launch_bf16_product(bf1, g1, L->num_sms, s);
   if (rc) return rc;
   if (L->timing) cudaEventRecord(L->ev[4], s);
   GroupedGemmArgs g2{};
@@ -294,8 +300,7 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   g2.w8 = q;
   g2.splitk_ws = L->splitk_ws_shared;
   rc = m256 ? launch_grouped_gemm_w8_m256(g2, L->num_sms, s)
-       : tmem ? launch_grouped_gemm_w8_tmem(g2, L->num_sms, s)
-                  : pairs2 ? launch_grouped_gemm_2cta(g2, L->num_sms, s) : launch_grouped_gemm_tcgen05(g2, L->num_sms, s);
+       : tmem ? launch_grouped_gemm_w8_tmem(g2, L->num_sms, s) : launch_bf16_product(bf2, g2, L->num_sms, s);
   if (rc) return rc;
   if (L->timing) {
     cudaEventRecord(L->ev[5], s);

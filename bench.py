@@ -288,7 +288,9 @@ def gate_up_kernel(shape, rows, groups):
         return "grouped_gemv_kernel"
     if rows <= 16:
         return "grouped_gemm_decode_kernel"
-    return "grouped_gemm_2cta_kernel" if shape.d_model > 1024 or rows < 1024 else "grouped_gemm_tcgen05_kernel"
+    if shape.d_model > 1024 or rows < 1024:
+        return "grouped_gemm_2cta_kernel"
+    return "grouped_gemm_pair_rows_kernel" if rows >= 512 * groups else "grouped_gemm_tcgen05_kernel"
 
 
 def layer_roofline(shape, T, touched, peaks, int8):

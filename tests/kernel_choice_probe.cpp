@@ -4,4 +4,6 @@
 extern "C" int choice_i8_decode(int rows, int experts, int d, int F, int shared) {
   return atenia::i8_decode_pays(rows, experts, d, F, shared != 0);
 }
-extern "C" int choice_pairs(int rows, int k) { return atenia::pair_pays(rows, k); }
+extern "C" int choice_bf16(int rows, int groups, int k, int beside) {
+  return atenia::bf16_product_kernel(rows, groups, k, beside != 0);
+}

@@ -38,16 +38,27 @@ def test_up_to_128_rows_the_integer_mma_decode_kernel_is_always_taken(lib):
             assert lib.choice_i8_decode(rows, experts, d, F, 0) and lib.choice_i8_decode(rows, experts, d, F, 1)
 
 
+PAIRS, SINGLE, PAIR_ROWS = 0, 1, 2
+
 # experts, rows an expert, k, us of the CTA-pair kernel, us of the single-CTA kernel
-PAIRS = [(8, 256, 512, 27, 20), (8, 1024, 512, 51, 38), (32, 100, 512, 37, 31), (128, 16, 512, 49, 43), (128, 512, 512, 143, 97),
-         (8, 256, 1024, 27, 25), (32, 256, 1024, 128, 120), (32, 1024, 1024, 388, 344), (128, 100, 1024, 77, 68),
-         (8, 64, 512, 13, 14), (8, 64, 1024, 16, 18), (32, 256, 1408, 69, 73), (128, 256, 1408, 216, 255), (8, 64, 2048, 18, 22),
-         (32, 64, 2048, 74, 78), (32, 1024, 2048, 293, 345)]
+PRODUCTS = [(8, 256, 512, 27, 20), (32, 100, 512, 37, 31), (128, 16, 512, 49, 43), (128, 256, 512, 96, 66), (8, 256, 1024, 27, 25),
+            (32, 256, 1024, 128, 120), (128, 100, 1024, 77, 68), (8, 64, 512, 13, 14), (8, 64, 1024, 16, 18),
+            (32, 256, 1408, 69, 73), (128, 256, 1408, 216, 255), (8, 64, 2048, 18, 22), (32, 64, 2048, 74, 78),
+            (32, 1024, 2048, 293, 345)]
 
 
-@pytest.mark.parametrize("experts,rows,k,pair,single", PAIRS)
+@pytest.mark.parametrize("experts,rows,k,pair,single", PRODUCTS)
 def test_pair_kernel_is_taken_where_it_is_the_faster_one(lib, experts, rows, k, pair, single):
-    assert bool(lib.choice_pairs(experts * rows, k)) == (pair < single)
+    assert lib.choice_bf16(experts * rows, experts, k, 0) == (PAIRS if pair < single else SINGLE)
+
+
+def test_large_groups_and_the_shared_expert(lib):
+    for k in (16, 512, 1024):
+        assert lib.choice_bf16(8 * 512, 8, k, 0) == PAIR_ROWS and lib.choice_bf16(8 * 512 - 1, 8, k, 0) == SINGLE
+        assert lib.choice_bf16(1023, 1, k, 0) == PAIRS and lib.choice_bf16(1024, 1, k, 0) == PAIR_ROWS
+        assert lib.choice_bf16(4095, 1, k, 1) == PAIRS and lib.choice_bf16(4096, 1, k, 1) == PAIR_ROWS
+    for rows, groups in [(17, 1), (4096, 8), (1 << 30, 1), (1 << 30, 128)]:
+        assert lib.choice_bf16(rows, groups, 1040, 0) == PAIRS and lib.choice_bf16(rows, groups, 1040, 1) == PAIRS
 
 
 def test_the_benchmark_names_the_kernel_that_runs(lib):
@@ -65,6 +76,7 @@ def test_the_benchmark_names_the_kernel_that_runs(lib):
                 assert name == ("grouped_gemm_w8_m256_kernel" if rows >= 256 * E else "grouped_gemm_w8_tmem_kernel")
             name = bench.gate_up_kernel(MoeShape("s", d, F, E, k, True, Fs), rows, E)
             if rows > 16:
-                assert (name == "grouped_gemm_2cta_kernel") == bool(lib.choice_pairs(rows, d))
+                assert name == ("grouped_gemm_2cta_kernel", "grouped_gemm_tcgen05_kernel",
+                                "grouped_gemm_pair_rows_kernel")[lib.choice_bf16(rows, E, d, 0)]
             else:
                 assert name == ("grouped_gemv_kernel" if rows <= 2 and rows * d * F < 1 << 26 else "grouped_gemm_decode_kernel")

@@ -1,6 +1,5 @@
 """Expert GEMM kernels at the edges of their tiles, features and k that fill no tile.  bf16: the CTA-pair kernel (pinned:
-by default products of 1024 rows or more over k of at most 1024 take the single-CTA kernel, which runs on the same
-groups), 0, 1, 15 .. 17, 255 .. 257, 511 .. 513 rows (token tiles are equal parts of at most 256 rows, rounded up to 16).  INT8 takes
+by default products of 1024 rows or more over k of at most 1024 take other kernels, which run on the same groups), 0, 1, 15 .. 17, 255 .. 257, 511 .. 513 rows (token tiles are equal parts of at most 256 rows, rounded up to 16).  INT8 takes
 other kernels on the same groups: the integer-MMA decode kernel up to 128 rows in all (token tiles of 32 rows), the
 tensor-memory kernel (128 rows) above, the 256-row-tile kernel from 256 rows a group on; their own edges follow."""
 import numpy as np
@@ -24,11 +23,27 @@ def test_groups_at_tile_edges(monkeypatch, sizes, d, F, int8):
 
 
 @pytest.mark.parametrize("sizes", [[511, 512, 513, 0, 769, 1030, 2, 300], [128, 127, 129, 0, 255, 257, 127, 0],
-                                   [128, 127, 129, 0, 255, 257, 128, 0]])
+                                   [128, 127, 129, 0, 255, 257, 128, 0], [513, 512, 600, 500, 511, 900, 640, 1]])
 @pytest.mark.parametrize("d,F", [(272, 144), (1024, 1040), (1040, 1024)])
 def test_short_k_by_the_default_rule(sizes, d, F):
-    """1023, 1024 and more rows, k of 1024 and the next: both products on either kernel."""
+    """1023, 1024 and more rows, 512 a group on average and fewer, k of 1024 and the next."""
     _check_groups(sizes, d, F, False)
+
+
+@pytest.mark.parametrize("T", [700, 2600])
+def test_bf16_kernels_agree_bit_for_bit(monkeypatch, T):
+    """All three add over k in the same order; a shared expert runs on each as well."""
+    from ateniaengine_b200 import synth
+
+    dev = torch.device("cuda:0")
+    shape = synth.MoeShape("edges", 528, 400, 5, 2, False, 272)
+    w = synth.make_weights(shape, 5, dev)
+    x = synth.make_activations(shape, 5, dev, tokens=T)
+    outs = []
+    for mode in ("1", "2", "3", "0"):
+        monkeypatch.setenv("ATENIA_MOE_PAIR_MODE", mode)
+        outs.append(synth.build_layer(shape, w, max_tokens=T).forward(x, out_dtype=torch.float32, sync=True))
+    assert all(torch.equal(outs[0], y) for y in outs[1:])
 
 
 @pytest.mark.parametrize("pinned", [False, True])
