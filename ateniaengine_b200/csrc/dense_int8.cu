@@ -4,16 +4,16 @@
 // :99-117).  The MoE tiers use the per-row layout of combine.cu instead.
 //
 // Both directions are streaming, HBM-bound work (algorithmic bytes per weight: quantise 4 + 1, dequant 1 + 2):
-//   quantize_groups  a block owns 128 columns x one group; the group's values stay in registers between the
+//   quantize_groups  a block owns 32 to 128 columns x one group; the group's values stay in registers between the
 //                    maximum and the rounding, so the matrix is read once (groups of at most 128 rows)
 //   quantize_tall    a cluster of one to eight blocks owns 64 columns x one taller group and reads it twice, the
 //                    second time from L2 where it fits
 //   quantize_passes  maxima, scales and codes in three launches over the whole grid, for matrices whose groups
-//                    and strips are too few or too small for the kernels above
+//                    and strips are too few for the kernel above
 //   dequant          a block owns 256 columns x 64 rows; a lane keeps its eight scales while the group lasts;
 //                    narrow matrices and groups of few rows take a flat walk
 // The three passes and the flat walk spend two 64-bit divisions per vector, the others none.  Measured on a B200
-// at 4096 x 14336, groups of 128: quantise 149 (three passes) -> 68 us, dequant 42 (flat) -> 32 us; floors at the
+// at 4096 x 14336, groups of 128: quantise 149 (three passes) -> 51 us, dequant 42 (flat) -> 32 us; floors at the
 // measured copy rate 47 and 28 us.
 //   scale = max(amax / 127, 1e-12); q = clamp(round_half_away(w / scale), -127, 127), NaN -> 0;
 //   bf16 = high half of (float)q * scale (truncation, as the reference's kernel does)
@@ -25,8 +25,8 @@
 namespace atenia {
 namespace {
 
-constexpr int COLS_PER_BLOCK = 128;  // 32 lanes x 4 columns
-constexpr int GROUP_ROWS_MAX = 128;  // tallest group that stays in registers: 16 warps x 8 rows
+constexpr int COLS_PER_BLOCK = 128;  // three passes: 32 lanes x 4 columns
+constexpr int GROUP_ROWS_MAX = 128;  // tallest group that stays in registers: 16 row lanes x 8 rows
 constexpr int TALL_WARPS = 16;
 constexpr int TALL_COLS = 64;        // 16 lanes x 4 columns: a warp covers two rows
 constexpr int DEQ_COLS = 256, DEQ_ROWS = 64;
@@ -61,7 +61,7 @@ __device__ __forceinline__ int quantize_one(float w, float s) {
 }
 
 template <bool VEC, int LANES>
-__device__ __forceinline__ void store_codes4(const float (&w)[4], const float (&s)[4], const float (&inv)[4],
+__device__ __forceinline__ void store_codes4(const float (&w)[4], const float* s, const float (&inv)[4],
                                              int8_t* __restrict__ row, int64_t strip0, int lane, int64_t N) {
   const uint32_t p = round_codes4(w, inv, [&](float x, int j) { return quantize_one(x, s[j]); });
   if (VEC) {
@@ -79,58 +79,60 @@ __device__ __forceinline__ void store_codes4(const float (&w)[4], const float (&
 __device__ __forceinline__ void max_cols4(float (&m)[4], const float (&v)[4]) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float a = fabsf(v[j]);
-    if (a > m[j]) m[j] = a;  // a NaN never compares greater: skipped, as in the reference
+    m[j] = fmaxf(m[j], fabsf(v[j]));  // (fmaxf returns the other operand for a NaN: skipped, as in the reference)
   }
 }
 __device__ __forceinline__ float scale_of(float amax) { return fmaxf(__fdiv_rn(amax, 127.0f), 1e-12f); }
 
-// RPT rows per thread: groups of at most WARPS * RPT rows.  Eight rows (32 registers) per thread at most: with
-// sixteen a third of the loads in flight per SM is lost (4096 x 14336, groups of 128: 83 against 68 us).
-template <bool VEC, int WARPS, int RPT>
-__global__ void __launch_bounds__(WARPS * 32) quantize_groups_kernel(const float* __restrict__ w, int64_t K,
-                                                                           int64_t N, int G, unsigned strips,
-                                                                           int8_t* __restrict__ q,
-                                                                           float* __restrict__ scales) {
-  __shared__ float red[WARPS][COLS_PER_BLOCK];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// A block of LANES x RL threads owns 4 LANES columns x one group of at most RL * GROUP_RPT rows.  HBM-bound as long as other
+// blocks of the SM load while one rounds and stores, so blocks are small (many per SM, each at another point) and the
+// rounding is kept short: one thread per column turns the RL partial maxima into the scale and its reciprocal, not every
+// thread for its own four.  B200, 4096 x 14336 f32 (floor 45 us at the measured copy rate), blocks of 512 threads x 128
+// columns with the scales in every thread / these: groups of 128 67.4 / 51.2 us, 100 75.7 / 55.6, 64 55.6 / 49.5, 48
+// 63.8 / 55.6, 32 63.9 / 49.4, 20 84.9 / 59.3.  Sixteen rows per thread lose (128: 61), blocks twice as wide too (128: 53.4).
+constexpr int GROUP_RPT = 8;
+template <bool VEC, int LANES, int RL>
+__global__ void __launch_bounds__(LANES * RL) quantize_groups_kernel(const float* __restrict__ w, int64_t K, int64_t N,
+                                                                     int G, unsigned strips, int8_t* __restrict__ q,
+                                                                     float* __restrict__ scales) {
+  constexpr int COLS = LANES * 4;
+  __shared__ float red[RL][COLS];
+  __shared__ float4 scale_s[LANES], inv_s[LANES];
+  const int lane = threadIdx.x % LANES, rl = threadIdx.x / LANES;
   const unsigned g = blockIdx.x / strips;
-  const int64_t strip0 = (int64_t)(blockIdx.x - g * strips) * COLS_PER_BLOCK;
+  const int64_t strip0 = (int64_t)(blockIdx.x - g * strips) * COLS;
   const int64_t lo = (int64_t)g * G;
   const int rows = (int)(K - lo < G ? K - lo : G);
-  float v[RPT][4];
+  float v[GROUP_RPT][4];
 #pragma unroll
-  for (int i = 0; i < RPT; ++i) {
-    const int r = warp + WARPS * i;
-    if (r < rows) load_cols4<VEC, 32>(v[i], w + (lo + r) * N, strip0, lane, N);
+  for (int i = 0; i < GROUP_RPT; ++i) {
+    const int r = rl + RL * i;
+    if (r < rows) load_cols4<VEC, LANES>(v[i], w + (lo + r) * N, strip0, lane, N);
     else v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
   }
   float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < RPT; ++i) max_cols4(m, v[i]);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) red[warp][lane + 32 * j] = m[j];  // [j][lane]: no bank conflict
+  for (int i = 0; i < GROUP_RPT; ++i) max_cols4(m, v[i]);
+  *reinterpret_cast<float4*>(&red[rl][lane * 4]) = make_float4(m[0], m[1], m[2], m[3]);
   __syncthreads();
-  float s[4], inv[4];
+  for (int i = threadIdx.x; i < COLS; i += LANES * RL) {  // slot i: column col_of(i / 4, i % 4)
+    float a = red[0][i];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    float a = red[0][lane + 32 * j];
-#pragma unroll
-    for (int l = 1; l < WARPS; ++l) a = fmaxf(a, red[l][lane + 32 * j]);
-    s[j] = scale_of(a);
-    inv[j] = __frcp_rn(s[j]);
+    for (int l = 1; l < RL; ++l) a = fmaxf(a, red[l][i]);
+    const float s = scale_of(a);
+    reinterpret_cast<float*>(scale_s)[i] = s;
+    reinterpret_cast<float*>(inv_s)[i] = __frcp_rn(s);
+    const int64_t c = col_of<VEC, LANES>(strip0, i / 4, i % 4);
+    if (c < N) scales[(int64_t)g * N + c] = s;
   }
-  if (warp == 0) {
+  __syncthreads();
+  const float4 i4 = inv_s[lane];
+  const float inv[4] = {i4.x, i4.y, i4.z, i4.w};
+  const float* s = reinterpret_cast<const float*>(scale_s) + lane * 4;  // (read for the few values near a half only)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t c = col_of<VEC, 32>(strip0, lane, j);
-      if (c < N) scales[(int64_t)g * N + c] = s[j];
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < RPT; ++i) {
-    const int r = warp + WARPS * i;
-    if (r < rows) store_codes4<VEC, 32>(v[i], s, inv, q + (lo + r) * N, strip0, lane, N);
+  for (int i = 0; i < GROUP_RPT; ++i) {
+    const int r = rl + RL * i;
+    if (r < rows) store_codes4<VEC, LANES>(v[i], s, inv, q + (lo + r) * N, strip0, lane, N);
   }
 }
 
@@ -208,8 +210,7 @@ quantize_tall_kernel(const float* __restrict__ w, int64_t K, int64_t N, int64_t 
   }
 }
 
-// The same in three passes over the whole grid, for matrices whose groups x strips are too few, or whose rows too
-// narrow, to fill the SMs above: maxima of 128 columns x up to 256 rows of one group merged by atomicMax on the bit
+// The same in three passes over the whole grid, for matrices whose groups x strips are too few to fill the SMs above: maxima of 128 columns x up to 256 rows of one group merged by atomicMax on the bit
 // pattern (non-negative floats order like unsigned integers, so the result does not depend on scheduling), scales in
 // place, codes.
 constexpr int CHUNK_ROWS = 256, CHUNK_LANES = 8;
@@ -435,6 +436,15 @@ int launch_quantize_tall(const float* w, int64_t K, int64_t N, int64_t G, int8_t
   return (int)cudaGetLastError();
 }
 
+template <bool VEC, int LANES, int RL>
+int launch_quantize_groups(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, float* scales, cudaStream_t s) {
+  const int64_t strips = (N + 4 * LANES - 1) / (4 * LANES), blocks = strips * ((K + G - 1) / G);
+  if (blocks > 0x7fffffffLL) return launch_quantize_passes(w, K, N, G, q, scales, s);
+  quantize_groups_kernel<VEC, LANES, RL><<<(unsigned)blocks, LANES * RL, 0, s>>>(w, K, N, (int)G, (unsigned)strips, q, scales);
+  count_launch();
+  return (int)cudaGetLastError();
+}
+
 // Where the lines lie (B200, us; the Python call costs about 15, so short ones are all launch):
 //   few tall items   a cluster walks K / 256 rows per lane whatever the width.  Eight items or fewer of more than
 //                    16384 rows, clusters / three passes: 16384 x 256 19.2 / 24.7, 32768 x 64 31.6 / 25.0, 65536 x 512
@@ -442,9 +452,10 @@ int launch_quantize_tall(const float* w, int64_t K, int64_t N, int64_t G, int8_t
 //   blocks per item  8192 x 14336, the cluster taken / clusters of eight / three passes: groups of 256 163 / 836 / 271, of
 //                    512 141 / 530 / 268 (one block), of 1024 148 / 279 / 268, of 2048 156 / 201 / 267 (two), of 4096 165 /
 //                    165 / 267; 2048 x 4096 by 256 17.4 / 56.4 / 32.1
-//   small items      a block of the groups kernel costs what its launch costs.  Groups kernel / three passes: 1048576 x 8 by
-//                    128 142 / 59, 262144 x 8 by 128 39.9 / 27.0, 262144 x 16 by 64 35.8 / 34.6, 262144 x 32 by 64 35.8 /
-//                    40.7, 262144 x 32 by 1 899 / 406, 65536 x 8 by 128 17.6 / 26.1; 4096 x 14336 by 1 1151 / 1048, by 2 598 / 598
+//   short groups     the groups kernel in blocks no taller than the group needs.  Blocks of 32 rows x 64 columns / of 16 x 64
+//                    (groups of 9 to 16) or 8 x 128 (up to 8) / three passes: 4096 x 14336 by 1 668 / 242 / 1049, by 8 105 /
+//                    54 / 240, by 16 66 / 51 / 199; 262144 x 32 by 1 205 / 150 / 476, by 8 33.0 / 33.0 / 92.3, by 16 21.3 / 17.2 /
+//                    69.3; 300000 x 100 by 8 71 / 37 / 148; narrow and tall, 1048576 x 8 by 128 26.9 / - / 71.9
 template <bool VEC>
 int launch_quantize(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, float* scales, cudaStream_t s) {
   const int64_t groups = (K + G - 1) / G;
@@ -458,14 +469,11 @@ int launch_quantize(const float* w, int64_t K, int64_t N, int64_t G, int8_t* q, 
            : ctas == 4 ? launch_quantize_tall<VEC, 4>(w, K, N, G, q, scales, s)
                        : launch_quantize_tall<VEC, 8>(w, K, N, G, q, scales, s);
   }
-  const int64_t strips = (N + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK;
-  if (groups > 1024 && (G == 1 || (N < COLS_PER_BLOCK && N * G <= 1024))) return launch_quantize_passes(w, K, N, G, q, scales, s);
-  const unsigned grid = (unsigned)(strips * groups), st = (unsigned)strips;
-  if (G <= 32) quantize_groups_kernel<VEC, 8, 4><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
-  else if (G <= 64) quantize_groups_kernel<VEC, 8, 8><<<grid, 256, 0, s>>>(w, K, N, (int)G, st, q, scales);
-  else quantize_groups_kernel<VEC, 16, 8><<<grid, 512, 0, s>>>(w, K, N, (int)G, st, q, scales);
-  count_launch();
-  return (int)cudaGetLastError();
+  if (G <= 8) return launch_quantize_groups<VEC, 32, 1>(w, K, N, G, q, scales, s);
+  if (G <= 16) return launch_quantize_groups<VEC, 16, 2>(w, K, N, G, q, scales, s);
+  if (G <= 32) return launch_quantize_groups<VEC, 16, 4>(w, K, N, G, q, scales, s);
+  if (G <= 64) return launch_quantize_groups<VEC, 16, 8>(w, K, N, G, q, scales, s);
+  return launch_quantize_groups<VEC, 8, 16>(w, K, N, G, q, scales, s);
 }
 
 }  // namespace

@@ -41,7 +41,7 @@ def test_row_quantiser_at_block_edges(rows, cols):
     (33000, 256, 1024), (16384, 252, 1024), (1281, 66, 700),  # clusters of two, four and two
     (4500, 130, 0), (4500, 132, 4097),                        # clusters of eight
     (16400, 132, 0), (16390, 67, 0),                          # three passes: few items
-    (20001, 8, 16), (20001, 7, 16), (1100, 100, 1), (1030, 260, 1),  # three passes: small items
+    (20001, 8, 16), (20001, 7, 16), (1100, 100, 1), (1030, 260, 1),  # many groups of few rows
     (300, 160, 64), (70, 264, 0), (513, 24, 100), (90, 520, 15), (90, 517, 15)])  # flat dequant: narrow, small groups
 def test_group_quantiser_forms(K, N, g):
     import torch
@@ -59,3 +59,20 @@ def test_group_quantiser_forms(K, N, g):
     nan = (ref & 0x7FFF) > 0x7F80  # code 0 x scale inf: any NaN pattern
     np.testing.assert_array_equal((out & 0x7FFF) > 0x7F80, nan)
     np.testing.assert_array_equal(out[~nan], ref[~nan])
+
+
+@pytest.mark.parametrize("g", [1, 2, 7, 8, 9, 16, 17, 32, 33, 64, 65, 127, 128])
+@pytest.mark.parametrize("N", [4, 31, 32, 36, 64, 65, 68, 128, 129, 132])
+def test_group_blocks_at_their_edges(g, N):
+    """Every block shape of the groups kernel (rows by group, columns by strip), with a ragged last group."""
+    import torch
+    from ateniaengine_b200 import quantize_per_group_i8
+    from oracle import oracle as orc
+    K = 3 * g + max(1, g // 2)
+    w = torch.randn((K, N), generator=torch.Generator().manual_seed(131 * g + N)) * 0.02
+    w[g - 1, 0], w[g, N - 1], w[2 * g, 1] = float("inf"), float("nan"), 0.0
+    w[K - 1, N // 2] = 3.0
+    q, s = quantize_per_group_i8(w.cuda(), g)
+    q_ref, s_ref = orc.absmax_per_group_symmetric(w.numpy(), g)
+    np.testing.assert_array_equal(s.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
+    np.testing.assert_array_equal(q.cpu().numpy(), q_ref)
