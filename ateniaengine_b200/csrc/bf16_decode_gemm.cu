@@ -15,7 +15,8 @@
 // shared memory (bf16 tiles, 128B swizzle, by TMA).
 //
 //   tile      = up to 128 tokens of one expert x { 128 gate rows + 128 up rows (kSwiGLU) | 256 down rows (kPlain) }
-//   k-block   = 64: two 16 KiB weight tiles + one 16 KiB token tile per stage, 4 stages
+//   k-block   = 64: two 16 KiB weight tiles + a token tile of 2 KiB (calls of at most 16 rows) or 16 KiB per stage, 6 or
+//               4 stages
 //   TMEM      = two buffers of two 128-column accumulators: the epilogue of a piece overlaps the
 //               main loop of the next
 //   warps     : 0 TMA, 1 MMA + TMEM alloc, 4..11 epilogue (two warps per TMEM lane quarter)
@@ -38,7 +39,7 @@
 // are four column blocks of ONE MMA (N = 4 x tokens rounded to 16), the int32 accumulators are exact,
 // and the epilogue folds them, v = a0 + 128 (a1 + 128 (a2 + 128 a3)), and multiplies by the weight
 // row's scale and the token's 2^(e - 26).  Per k-block of 128 codes a stage holds two 16 KiB weight tiles
-// and at most 16 KiB of digits; token tiles are 32 rows.
+// and 8 or 16 KiB of digits (5 or 4 stages); token tiles are 32 rows.
 #include "tc_common.cuh"
 
 namespace atenia {
@@ -47,19 +48,17 @@ using namespace tc;
 
 constexpr int DTN = 128;     // token tile (MMA N at most)
 constexpr int DROWS = 128;   // weight rows per A tile (MMA M)
-constexpr int D_STAGES = 4;
+constexpr int D_MAX_STAGES = 6;
 constexpr int D_W_BYTES = DROWS * BK * 2;  // 16 KiB
 constexpr int D_X_BYTES = DTN * BK * 2;    // 16 KiB
-constexpr int D_STAGE_BYTES = 2 * D_W_BYTES + D_X_BYTES;  // 48 KiB
 constexpr int D_THREADS = 384;
-constexpr int D_SMEM_BYTES = D_STAGES * D_STAGE_BYTES + 1024 + 256;
 constexpr int D_TMEM_COLS = 512;
 constexpr int D_SLOT_FLOATS = 2 * DTN * DROWS;  // [accumulator][token][feature]
 static_assert(D_SLOT_FLOATS == (int)kW8SplitKSlotFloats, "the layer sizes one workspace for both stream-K kernels");
 
 struct __align__(8) BarriersDec {
-  uint64_t full[D_STAGES];   // TMA landed (1 arrival + bytes)
-  uint64_t empty[D_STAGES];  // the MMAs that read the stage are done (commit)
+  uint64_t full[D_MAX_STAGES];   // TMA landed (1 arrival + bytes)
+  uint64_t empty[D_MAX_STAGES];  // the MMAs that read the stage are done (commit)
   uint64_t acc_full[2];      // all MMAs of the piece done (commit)
   uint64_t acc_empty[2];     // 8 epilogue warps drained the buffer
   uint32_t tmem_base;
@@ -88,6 +87,18 @@ __device__ __forceinline__ void tc_mma_i8_one(uint32_t d_tmem, uint64_t a_desc, 
 constexpr int ITOK = 32;        // INT8 form: token tile (four digit planes = 128 MMA columns)
 constexpr int IBK = 128;        // INT8 form: codes per k-block (128 bytes of a row, as for bf16)
 constexpr int kDigitPlanes = 4;
+
+// The ring.  A call of at most 16 rows (FEW) stages 16 token rows, not 128 (32 in four planes), and has room for two
+// stages more (one).  Bytes in flight decide here: DECIDE
+constexpr int kFewRows = 16;
+template <bool I8, bool FEW>
+struct DecRing {
+  static constexpr int X_BYTES = !FEW ? D_X_BYTES : I8 ? kDigitPlanes * kFewRows * IBK : kFewRows * BK * 2;
+  static constexpr int STAGE_BYTES = 2 * D_W_BYTES + X_BYTES;
+  static constexpr int STAGES = !FEW ? 4 : I8 ? 5 : 6;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+  static_assert(STAGES <= D_MAX_STAGES && STAGE_BYTES % 1024 == 0 && SMEM_BYTES <= 225 * 1024, "");
+};
 
 // Work of one CTA: whole tiles dealt round-robin, or (stream-K) one contiguous span of the flattened
 // (tile, k-block) list.  A span has at most one partial piece at its start (slot 0) and one at its end
@@ -161,24 +172,26 @@ struct DecPieces {
 // I8: tmap_x is the digit-plane map (uint8, box {128, 16}; plane p of row r at row p * plane_rows + r),
 // tmap_w0 / tmap_w1 are int8 maps with box {128, 128} and the 128-byte swizzle, scale0 / scale1 the
 // weight rows' scales per group and tok_scale the token rows' 2^(e - 26).
-template <int MODE, bool I8>
+template <int MODE, bool I8, bool FEW>
 __global__ void __launch_bounds__(D_THREADS, 1)
 grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUtensorMap* __restrict__ tmap_w0,
-                           const CUtensorMap* __restrict__ tmap_w1, const int32_t* __restrict__ group_offsets,
+                           const CUtensorMap* __restrict__ tmap_w1, const int32_t* __restrict__ group_offsets_g,
                            int num_groups, int N, int K, __nv_bfloat16* __restrict__ out, DeviceError* err,
                            int splitk, float* __restrict__ ws, const float* const* __restrict__ scale0,
                            const float* const* __restrict__ scale1, const float* __restrict__ tok_scale,
                            int plane_rows, unsigned int* __restrict__ tile_cnt) {
   extern __shared__ uint8_t smem_raw[];
+  __shared__ int32_t goff_s[kMaxGroupsShared + 1];
   constexpr int BN_OUT = (MODE == kSwiGLU) ? DROWS : 2 * DROWS;
   constexpr int BKE = I8 ? IBK : BK;      // k elements per k-block
   constexpr int TROWS = I8 ? ITOK : DTN;  // token rows per tile
   constexpr int ACOLS = DTN;              // tensor-memory columns of one accumulator
-  constexpr int STAGES = D_STAGES;
-  constexpr int STAGE_BYTES = D_STAGE_BYTES;
+  using Ring = DecRing<I8, FEW>;
+  constexpr int STAGES = Ring::STAGES;
+  constexpr int STAGE_BYTES = Ring::STAGE_BYTES;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
-  BarriersDec* bars = reinterpret_cast<BarriersDec*>(smem_aligned + D_STAGES * D_STAGE_BYTES);
+  BarriersDec* bars = reinterpret_cast<BarriersDec*>(smem_aligned + STAGES * STAGE_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = uniform_warp();
@@ -205,11 +218,13 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // before chain_wait(): the group offsets and, below, the first weights (see chain_wait)
+  stage_group_offsets(group_offsets_g, num_groups, goff_s);
+  const int32_t* group_offsets = goff_s;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  chain_wait();  // (everything above touches only this CTA's shared and tensor memory)
 
   DecPieces it;
   it.init(splitk != 0, num_kb, n_tiles, num_groups, BN_OUT, group_offsets, TROWS);
@@ -223,6 +238,8 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
       int last_group = -1;
       uint32_t armed = 0;
       bool ok = true;
+      int ahead = 0;        // k-blocks of the first piece whose weights were requested before the wait
+      bool waited = false;
       while (ok && it.next()) {
         const CUtensorMap* m0 = &tmap_w0[tc.group];
         const CUtensorMap* m1 = (MODE == kSwiGLU) ? &tmap_w1[tc.group] : m0;
@@ -233,38 +250,54 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
         }
         const int n1 = (MODE == kSwiGLU) ? tc.n0 : tc.n0 + DROWS;
         const int tokp = (it.rows() + 15) & ~15;
-        const uint32_t bytes = I8 ? 2 * D_W_BYTES + kDigitPlanes * tokp * 128 : (uint32_t)D_STAGE_BYTES;
+        const uint32_t bytes = I8 ? 2 * D_W_BYTES + kDigitPlanes * tokp * 128 : (uint32_t)STAGE_BYTES;
+        if (!waited) {
+          ahead = it.nkb < STAGES ? it.nkb : STAGES;
+          for (int i = 0; i < ahead; ++i) {
+            const uint32_t full = smem_u32(&bars->full[i]);
+            const uint32_t sw = smem_base + i * STAGE_BYTES;
+            mbar_expect_tx_one(full, bytes);
+            tma_load_2d_one(sw, m0, full, (it.kb0 + i) * BKE, tc.n0);
+            tma_load_2d_one(sw + D_W_BYTES, m1, full, (it.kb0 + i) * BKE, n1);
+          }
+          chain_wait();
+          waited = true;
+        }
         for (int kb = it.kb0; kb < it.kb0 + it.nkb; ++kb, ++idx) {
           const int stage = idx % STAGES;
           const uint32_t phase = (idx / STAGES) & 1u;
-          int got = 1;
-          if (lane == 0) got = mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag) ? 1 : 0;
-          got = __shfl_sync(0xffffffffu, got, 0);
-          if (!got) {
-            if (lane == 0) {
-              report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 2600 + stage);
-              *abort_flag = 1;
-            }
-            ok = false;
-            break;
-          }
           const uint32_t full = smem_u32(&bars->full[stage]);
           const uint32_t sw = smem_base + stage * STAGE_BYTES;
-          mbar_expect_tx_one(full, bytes);
-          tma_load_2d_one(sw, m0, full, kb * BKE, tc.n0);
-          tma_load_2d_one(sw + D_W_BYTES, m1, full, kb * BKE, n1);
+          if (idx >= (uint32_t)ahead) {  // (the first k-blocks' weights are on their way)
+            int got = 1;
+            if (lane == 0) got = mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag) ? 1 : 0;
+            got = __shfl_sync(0xffffffffu, got, 0);
+            if (!got) {
+              if (lane == 0) {
+                report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 2600 + stage);
+                *abort_flag = 1;
+              }
+              ok = false;
+              break;
+            }
+            mbar_expect_tx_one(full, bytes);
+            tma_load_2d_one(sw, m0, full, kb * BKE, tc.n0);
+            tma_load_2d_one(sw + D_W_BYTES, m1, full, kb * BKE, n1);
+          }
+          const uint32_t sx = sw + 2 * D_W_BYTES;
           if (I8) {
             // digit plane p, token rows cc .. cc + 15 of the tile: MMA columns p * tokp + cc ...
             for (int p = 0; p < kDigitPlanes; ++p)
               for (int cc = 0; cc < tokp; cc += 16)
-                tma_load_2d_one(sw + 2 * D_W_BYTES + (p * tokp + cc) * 128, &tmap_x, full, kb * BKE,
-                                p * plane_rows + tc.row0 + cc);
+                tma_load_2d_one(sx + (p * tokp + cc) * 128, &tmap_x, full, kb * BKE, p * plane_rows + tc.row0 + cc);
           } else {
-            tma_load_2d_one(sw + 2 * D_W_BYTES, &tmap_x, full, kb * BKE, tc.row0);
+            tma_load_2d_one(sx, &tmap_x, full, kb * BKE, tc.row0);
           }
           armed |= 1u << stage;
         }
       }
+      if (!waited) chain_wait();
+      chain_next();  // (every load is on its way: what follows may be launched)
       if (lane == 0 && *abort_flag) {
         const int stage = idx % STAGES;
         const uint32_t phase = (idx / STAGES) & 1u;
@@ -279,6 +312,7 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
   } else if (warp == 1) {
     // ================= MMA issuer =================
     // (the warp stays converged: see uniform_warp)
+    chain_wait();
     {
       uint32_t idx = 0;
       int acc = 0;
@@ -334,6 +368,7 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
     // Lane f of the two accumulators is output feature n0 + f (first weight tile) / the matching row
     // of the second tile; column t is token row0 + t.  For a fixed token the 32 lanes of a warp write
     // 64 contiguous bytes.
+    chain_wait();
     const int quarter = warp & 3;
     const int f = quarter * 32 + lane;
     const int half = (warp - 4) >> 2;  // which of the two warps of this lane quarter
@@ -353,17 +388,15 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
         // INT8 form: column p * tokp + t of an accumulator is digit plane p of token t (int32, exact)
         const int tokp = (rows + 15) & ~15;
         auto fold16 = [&](uint32_t t, int c, float (&v)[16]) {
-          uint32_t a[16];
-          tc_ld16(t + 3 * tokp + c, a);
+          uint32_t a[kDigitPlanes][16];
+#pragma unroll
+          for (int p = 0; p < kDigitPlanes; ++p) tc_ld16(t + p * tokp + c, a[p]);
           tc_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (float)(int32_t)a[j];
+          for (int j = 0; j < 16; ++j) {
+            v[j] = (float)(int32_t)a[kDigitPlanes - 1][j];
 #pragma unroll
-          for (int p = 2; p >= 0; --p) {
-            tc_ld16(t + p * tokp + c, a);
-            tc_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = fmaf(v[j], 128.0f, (float)(int32_t)a[j]);
+            for (int p = kDigitPlanes - 2; p >= 0; --p) v[j] = fmaf(v[j], 128.0f, (float)(int32_t)a[p][j]);
           }
         };
         const int n_lo = tc.n0 + f, n_hi = tc.n0 + DROWS + f;
@@ -466,13 +499,13 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
       // the whole-tile epilogue would.  Nothing waits for anything: a warp that is not last just goes on.
       if (tile_cnt != nullptr && it.slot >= 0) {
         const long long tkb = (long long)it.tile_id * num_kb;
-        const int c0 = (int)(tkb / it.span), c1 = (int)((tkb + num_kb - 1) / it.span);
+        const int p0 = (int)(tkb / it.span), p1 = (int)((tkb + num_kb - 1) / it.span);
         __threadfence();  // this thread's slot stores, before the count
         __syncwarp();
         int last = 0;
         if (lane == 0) {
           unsigned int* cnt = tile_cnt + (size_t)it.tile_id * 8 + (warp - 4);
-          last = atomicAdd(cnt, 1u) == (unsigned)(c1 - c0) ? 1 : 0;
+          last = atomicAdd(cnt, 1u) == (unsigned)(p1 - p0) ? 1 : 0;
           if (last) *cnt = 0u;  // ready for the next launch (and for graph replay)
         }
         last = __shfl_sync(0xffffffffu, last, 0);
@@ -487,15 +520,32 @@ grouped_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const CUt
           }
           __nv_bfloat16* obase = out + (size_t)tc.row0 * N;
 #pragma unroll 1
-          for (int c = half * 16; c < rows; c += 32) {
-            for (int j = 0; j < 16 && c + j < rows; ++j) {
-              float a = 0.f, b = 0.f;
-              for (int cc = c0; cc <= c1; ++cc) {
-                const int sl = (it.tile_id == (int)(((long long)cc * it.span) / num_kb)) ? 0 : 1;
-                const float* p = ws + ((size_t)cc * 2 + sl) * D_SLOT_FLOATS;
-                a += __ldcg(p + (size_t)(c + j) * DROWS + f);
-                b += __ldcg(p + (size_t)(DTN + c + j) * DROWS + f);
+          for (int c = half * 16; c < rows; c += (c & 8) ? 24 : 8) {
+            // (eight tokens at a time, the loads of a piece in flight together: token by token they were a chain of L2
+            // round trips; INT8, 8 / 16 tokens of the Mixtral shape 231 -> 224, 270 -> 255 us a forward)
+            float va[8], vb[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) va[j] = vb[j] = 0.f;
+#pragma unroll 1
+            for (int cc = p0; cc <= p1; ++cc) {
+              const int sl = (it.tile_id == (int)(((long long)cc * it.span) / num_kb)) ? 0 : 1;
+              const float* p = ws + ((size_t)cc * 2 + sl) * D_SLOT_FLOATS + (size_t)c * DROWS + f;
+              float xa[8], xb[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                xa[j] = c + j < rows ? __ldcg(p + (size_t)j * DROWS) : 0.f;
+                xb[j] = c + j < rows ? __ldcg(p + (size_t)(DTN + j) * DROWS) : 0.f;
               }
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                va[j] += xa[j];
+                vb[j] += xb[j];
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              if (c + j >= rows) continue;
+              float a = va[j], b = vb[j];
               if (I8) {
                 const float ts = tok_scale[tc.row0 + c + j];
                 a = a * sa * ts;
@@ -542,6 +592,8 @@ __global__ void __launch_bounds__(DROWS * kReduceTokLanes) decode_splitk_reduce_
   constexpr int TROWS = I8 ? ITOK : DTN;
   const int num_kb = (K + BKE - 1) / BKE;
   const int n_tiles = (N + BN_OUT - 1) / BN_OUT;
+  chain_next();
+  chain_wait();
   // the group offsets once, side by side, into shared memory: the walks below are chains of dependent reads
   __shared__ int32_t off_s[kReduceMaxGroups + 1];
   const bool in_smem = num_groups <= kReduceMaxGroups;
@@ -601,12 +653,13 @@ __global__ void __launch_bounds__(DROWS * kReduceTokLanes) decode_splitk_reduce_
 
 constexpr int kFixupMaxRows = 32;  // rows (tokens x top-k) up to which the kernel adds split tiles itself
 
-template <int MODE, bool I8>
+template <int MODE, bool I8, bool FEW>
 int launch_dec_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   static bool attr_set[kMaxDevices] = {};
+  constexpr int kSmem = DecRing<I8, FEW>::SMEM_BYTES;
   if (first_use_on_current_device(attr_set)) {
-    ATENIA_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_decode_kernel<MODE, I8>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, D_SMEM_BYTES));
+    ATENIA_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_decode_kernel<MODE, I8, FEW>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   }
   // stream-K where a workspace slot can hold every piece (bf16: every group fits one 128-token tile;
   // INT8: tiles are 32 tokens) and the tiles that can exist are too few to balance the SMs
@@ -623,15 +676,22 @@ int launch_dec_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   // hundred rows on the last warp's serial sum costs what the launch saved, so the reduce kernel stays.
   const bool fixup = splitk && a.splitk_cnt != nullptr && a.max_rows <= kFixupMaxRows &&
                      max_tok_tiles * n_tiles <= kSplitKMaxTiles;
-  int rc = launch_chained(a.chained, grouped_gemm_decode_kernel<MODE, I8>, dim3(num_sms), dim3(D_THREADS), D_SMEM_BYTES, s, a.tmap_a,
-                          a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K,
+  int rc = launch_chained(a.chained, grouped_gemm_decode_kernel<MODE, I8, FEW>, dim3(num_sms), dim3(D_THREADS), kSmem, s,
+                          FEW && !I8 ? a.pair_rows->box[0] : a.tmap_a, a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K,
                           a.out, a.err, splitk ? 1 : 0, a.splitk_ws, a.scale0, a.scale1, a.tok_scale, a.plane_rows,
                           fixup ? a.splitk_cnt : nullptr);
   if (rc || !splitk || fixup) return rc;
-  decode_splitk_reduce_kernel<MODE, I8><<<dim3(max_tok_tiles * n_tiles), dim3(DROWS, kReduceTokLanes), 0, s>>>(
-      a.group_offsets, a.num_groups, a.N, a.K, a.out, a.splitk_ws, num_sms, a.scale0, a.scale1, a.tok_scale);
   count_launch();
-  return (int)cudaGetLastError();
+  return launch_chained(a.chained, decode_splitk_reduce_kernel<MODE, I8>, dim3(max_tok_tiles * n_tiles), dim3(DROWS, kReduceTokLanes),
+                        0, s, a.group_offsets, a.num_groups, a.N, a.K, a.out, a.splitk_ws, num_sms, a.scale0, a.scale1,
+                        a.tok_scale);
+}
+
+template <bool I8>
+int launch_dec(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
+  if (a.max_rows <= kFewRows)
+    return a.mode == kSwiGLU ? launch_dec_one<kSwiGLU, I8, true>(a, num_sms, s) : launch_dec_one<kPlain, I8, true>(a, num_sms, s);
+  return a.mode == kSwiGLU ? launch_dec_one<kSwiGLU, I8, false>(a, num_sms, s) : launch_dec_one<kPlain, I8, false>(a, num_sms, s);
 }
 
 // One block per token row: the row's exponent, then its four digit planes (see the head of this file).
@@ -673,10 +733,14 @@ __device__ __forceinline__ void amax_of_vector(const uint4& q, float& amax, bool
 __global__ void __launch_bounds__(kQThreads) quantize_digits_kernel(DigitSource src,
                                                                     const int32_t* __restrict__ n_rows_dev, int n_rows,
                                                                     int K, int plane_rows, int8_t* __restrict__ planes,
-                                                                    float* __restrict__ tok_scale) {
+                                                                    float* __restrict__ tok_scale, bool between) {
   const int row = blockIdx.x;
+  // After the wait: the GEMM behind takes every SM, so it may come no earlier than these rows.  Between the two GEMMs
+  // of a layer it may: its blocks then start as those of the first leave (which were past their own wait when this
+  // kernel was launched, so the offsets that it reads early are complete).
+  if (between) chain_next();
   chain_wait();
-  chain_next();  // (after the wait: the GEMM behind takes every SM, so it may come no earlier than these rows)
+  if (!between) chain_next();
   // rows the dispatch did not place (invalid expert ids) hold nothing: skip them
   const int placed = n_rows_dev ? (*n_rows_dev < n_rows ? *n_rows_dev : n_rows) : n_rows;
   if (row >= placed) return;
@@ -747,8 +811,10 @@ __global__ void __launch_bounds__(kQThreads) quantize_digits_kernel(DigitSource 
 
 int launch_grouped_gemm_bf16_decode(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   if (a.num_groups <= 0) return ATENIA_OK;
-  if (a.N % 16 != 0 || a.K % 16 != 0) return ATENIA_ERR_SHAPE;
-  int rc = a.mode == kSwiGLU ? launch_dec_one<kSwiGLU, false>(a, num_sms, s) : launch_dec_one<kPlain, false>(a, num_sms, s);
+  if (a.N % 16 != 0 || a.K % 16 != 0 || a.num_groups > kMaxGroupsShared) return ATENIA_ERR_SHAPE;
+  static_assert(kFewRows == pair_box_rows(0), "few rows: the pair kernel's smallest box");
+  if (!a.pair_rows) return ATENIA_ERR_NULL;
+  int rc = launch_dec<false>(a, num_sms, s);
   count_launch();
   count_tcgen05_launch();
   return rc;
@@ -756,21 +822,21 @@ int launch_grouped_gemm_bf16_decode(const GroupedGemmArgs& a, int num_sms, cudaS
 
 int launch_grouped_gemm_w8_i8_decode(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   if (a.num_groups <= 0) return ATENIA_OK;
-  if (a.N % 16 != 0 || a.K % 16 != 0 || a.max_rows > kI8DecodeMaxRows) return ATENIA_ERR_SHAPE;
+  if (a.N % 16 != 0 || a.K % 16 != 0 || a.max_rows > kI8DecodeMaxRows || a.num_groups > kMaxGroupsShared) return ATENIA_ERR_SHAPE;
   if (!a.scale0 || (a.mode == kSwiGLU && !a.scale1) || !a.tok_scale || a.plane_rows < a.max_rows) return ATENIA_ERR_NULL;
-  int rc = a.mode == kSwiGLU ? launch_dec_one<kSwiGLU, true>(a, num_sms, s) : launch_dec_one<kPlain, true>(a, num_sms, s);
+  int rc = launch_dec<true>(a, num_sms, s);
   count_launch();
   count_tcgen05_launch();
   return rc;
 }
 
 int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, int n_rows, int K, int plane_rows,
-                           int8_t* planes, float* tok_scale, bool chained, cudaStream_t s) {
+                           int8_t* planes, float* tok_scale, bool between, bool chained, cudaStream_t s) {
   if (n_rows <= 0) return ATENIA_OK;
   if (K % 16 != 0 || n_rows > plane_rows || !src.x || (src.perm && src.k < 1)) return ATENIA_ERR_SHAPE;
   count_launch();
   return launch_chained(chained, quantize_digits_kernel, dim3(n_rows), dim3(kQThreads), 0, s, src, n_rows_dev, n_rows, K, plane_rows,
-                        planes, tok_scale);
+                        planes, tok_scale, between);
 }
 
 }  // namespace atenia

@@ -57,7 +57,8 @@ inline bool first_use_on_current_device(bool (&flags)[kMaxDevices]) {
 // launched plainly and wait for everything before them as usual.
 // One exception, the weights: a GEMM takes the group offsets and requests its first weight tiles before its
 // chain_wait().  The kernel before it writes neither (it gathers rows, makes digits, or is the GEMM before) and comes to
-// chain_next() only past its own chain_wait(), so whatever wrote them has completed before the GEMM's blocks start.
+// chain_next() only past its own chain_wait() -- or, between two GEMMs, was launched by one that had passed its -- so
+// whatever wrote them has completed before the GEMM's blocks start.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A kernel that takes whole SMs must not sit there waiting while another stream's work could run.  So the kernels
@@ -65,17 +66,13 @@ __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.laun
 // comes no earlier than the rows it reads are being written, and not already beside the router (one token of the
 // Mixtral shape 137.3 -> 134.8 us for it, other sizes the same).  Beside a layer's own shared expert the GEMMs are
 // not chained at all (`chained` false: Qwen1.5-MoE shape, 2048 tokens, in bursts after a pause, 342 -> 372 us when the
-// routed GEMM displaced the shared expert's), and a captured launch stays plain: a graph's own edges are as fast (eight INT8 layers, 8 tokens:
-// 1657 -> 1688 us chained).  Two layers on two streams, in all ms for the same calls, chained / plain: Mixtral shape of
-// 1024 tokens beside a 64-expert layer of 64 44.2 / 46.7, 4096 beside 64 42.5 / 49.2, 64 beside 16 33.5 / 35.6.
+// routed GEMM displaced the shared expert's).  A captured launch becomes a programmatic edge of the graph (eight INT8
+// layers, 8 tokens: 1609 -> 1573 us one graph after another, 1413 -> 1365 with three on their streams).  Two layers on
+// two streams, in all ms for the same calls, chained / plain: Mixtral shape of 1024 tokens beside a 64-expert layer of 64
+// 44.2 / 46.7, 4096 beside 64 42.5 / 49.2, 64 beside 16 33.5 / 35.6.
 // ATENIA_MOE_CHAINED=0 makes every launch of a layer plain.
 template <typename... P, typename... A>
 int launch_chained(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
-  if (chained) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) (void)cudaGetLastError();  // (the launch reports it)
-    chained = cap == cudaStreamCaptureStatusNone;
-  }
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -273,6 +270,7 @@ int launch_grouped_gemm_w8_i8_decode(const GroupedGemmArgs& a, int num_sms, cuda
 // planes [4][plane_rows][K] int8 and tok_scale [plane_rows] of n_rows rows; n_rows_dev (device, may be null)
 // bounds the rows that hold data.  Row r comes from row r of src.x, or -- with src.perm, the dispatch
 // permutation -- from token row perm[r] / k of the caller's batch (the row gather and the digits in one pass).
+// `between`: the launch before is the layer's first GEMM (the second may then be launched early).
 struct DigitSource {
   const void* x;        // [n_src_rows, K], bf16 or f32
   int x_is_f32;
@@ -281,7 +279,7 @@ struct DigitSource {
   int n_src_rows;
 };
 int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, int n_rows, int K, int plane_rows,
-                           int8_t* planes, float* tok_scale, bool chained, cudaStream_t s);
+                           int8_t* planes, float* tok_scale, bool between, bool chained, cudaStream_t s);
 // bf16 weights, CTA pairs (tcgen05 cta_group::2), transposed product: pair_rows describes the token rows (tmap_a
 // is not read), tmap_b0 / tmap_b1 have boxes of kPairWeightRows (kSwiGLU) or 128 (kPlain) weight rows
 constexpr int kPairWeightRows = 64;

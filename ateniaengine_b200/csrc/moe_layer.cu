@@ -107,7 +107,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   if (i8dec) {
     const DigitSource own{a_ptr, 0, nullptr, 1, max_rows};
     int rc = launch_quantize_digits(gather_here ? L->i8_src : own, group_offsets + num_groups, max_rows, c.d_model,
-                                    L->i8_rows, L->dq_x, L->dq_ts_x, L->gemm_chained, s);
+                                    L->i8_rows, L->dq_x, L->dq_ts_x, false, L->gemm_chained, s);
     if (rc) return rc;
     GroupedGemmArgs g1{};
     g1.chained = L->gemm_chained;
@@ -134,7 +134,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     if (L->timing) cudaEventRecord(L->ev[1], s);
     const DigitSource mid_rows{mid, 0, nullptr, 1, max_rows};
     rc = launch_quantize_digits(mid_rows, group_offsets + num_groups, max_rows, c.d_ff, L->i8_rows, L->dq_h, L->dq_ts_h,
-                                L->gemm_chained, s);
+                                true, L->gemm_chained, s);
     if (rc) return rc;
     GroupedGemmArgs g2 = g1;
     g2.tmap_a = L->tm_dq_h;
