@@ -108,17 +108,14 @@ struct RouterArgs {
   float* logits;       // [T, E] or null
   DeviceError* err;
   int variant;         // -1: by size; 0: CUDA-core f64 kernel (router.cu); 1: f64 tensor-core kernel
-                       // (router_dmma.cu); 2: split-k kernel (router_splitk.cu) when T <= sk_tokens
-  double* sk_part;     // variant 2 workspace (router_splitk_workspace), else null
-  double* sk_gate;
-  unsigned int* sk_counters;
-  int sk_tokens;       // largest batch the workspace serves
+                       // (router_dmma.cu); 2: split-k kernel (router_splitk.cu) up to kSplitkPinnedTokens
   bool chained;        // see launch_chained
 };
 int launch_router(const RouterArgs& a, cudaStream_t s);
 int launch_router_dmma(const RouterArgs& a, cudaStream_t s);  // same contract, E <= 128, k <= 8
-int launch_router_splitk(const RouterArgs& a, cudaStream_t s);  // same contract, T <= a.sk_tokens
-void router_splitk_workspace(int tokens, int d, int E, size_t* part_doubles, size_t* gate_doubles, size_t* counters);
+int launch_router_splitk(const RouterArgs& a, cudaStream_t s);  // same contract
+bool router_splitk_pays(int T, int E, int d);
+constexpr int kSplitkPinnedTokens = 1024;
 int launch_route_from_logits(const float* logits, int T, int E, int k, int renormalize,
                              int32_t* topk_idx, float* topk_w, DeviceError* err, cudaStream_t s);
 

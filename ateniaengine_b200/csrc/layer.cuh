@@ -43,12 +43,8 @@ struct AteniaMoeLayer {
   // (ATENIA_MOE_BF16_DECODE=1), 0 = never (=0, or INT8 weights)
   int bf16_decode = -1;
   // router kernel: -1 by size, 0 CUDA cores (router.cu), 1 f64 tensor cores (router_dmma.cu),
-  // 2 split-k for batches of at most sk_tokens (router_splitk.cu); see atenia_moe_create
+  // 2 split over a cluster for batches of at most kSplitkPinnedTokens (router_splitk.cu)
   int router_variant = -1;
-  double* sk_part = nullptr;
-  double* sk_gate = nullptr;
-  unsigned int* sk_counters = nullptr;
-  int sk_tokens = 0;
 
   // weights (device)
   float* d_router = nullptr;    // [E, d]

@@ -351,10 +351,8 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
     const int r = e ? std::atoi(e) : kGemvMaxRows;
     L->gemv_rows = r < 1 ? 1 : (r > 4 ? 4 : r);
   }
-  // Router kernel: by default the split-k kernel for batches of at most 128 tokens (many CTAs share one
-  // token block's dot products), the f64 tensor-core kernel for 32 experts and more, the CUDA-core
-  // kernel otherwise.  ATENIA_MOE_ROUTER = scalar | dmma | splitk pins one (tests, A/B runs); a pinned
-  // split-k serves batches up to 1024 tokens and hands larger ones to the CUDA-core kernel.
+  // Router kernel: by size (launch_router).  ATENIA_MOE_ROUTER = scalar | dmma | splitk pins one (tests, A/B runs); a
+  // pinned split-k serves batches up to 1024 tokens and hands larger ones to the CUDA-core kernel.
   {
     const char* rv = std::getenv("ATENIA_MOE_ROUTER");
     const std::string r(rv ? rv : "");
@@ -419,21 +417,6 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
         atenia_moe_destroy(L);
         return ATENIA_ERR_STATE;
       }
-    }
-  }
-  {
-    const int sk_cap = L->router_variant == 2 ? 1024 : (L->router_variant == -1 ? 128 : 0);
-    L->sk_tokens = c.max_tokens < sk_cap ? c.max_tokens : sk_cap;
-  }
-  if (L->sk_tokens > 0) {
-    size_t np = 0, ng = 0, nc = 0;
-    router_splitk_workspace(L->sk_tokens, c.d_model, c.num_experts, &np, &ng, &nc);
-    TRY_ALLOC(L->sk_part, np);
-    TRY_ALLOC(L->sk_gate, ng);
-    TRY_ALLOC(L->sk_counters, nc);
-    if (cudaMemset(L->sk_counters, 0, nc * sizeof(unsigned int)) != cudaSuccess) {
-      atenia_moe_destroy(L);
-      return ATENIA_ERR_STATE;
     }
   }
   if (c.weight_dtype == ATENIA_W_INT8_ROW) {
@@ -536,7 +519,7 @@ int atenia_moe_destroy(AteniaMoeLayer* L) {
                   L->splitk_ws, L->splitk_cnt, L->splitk_ws_shared, L->d_tm_gate_i8, L->d_tm_up_i8, L->d_tm_down_i8, L->dq_x, L->dq_h,
                   L->dq_ts_x, L->dq_ts_h, L->d_escore, L->logits_ws, L->recv_x, L->recv_h, L->recv_y, L->d_counts_all,
                   L->d_group_offsets, L->d_peer_recv_x, L->d_peer_y_perm, L->d_dst_base, L->d_src_base,
-                  L->d_gemm_offsets, L->d_bar, L->d_sync, L->d_peer_sync, L->d_ep_state, L->sk_part, L->sk_gate, L->sk_counters, L->block_normed};
+                  L->d_gemm_offsets, L->d_bar, L->d_sync, L->d_peer_sync, L->d_ep_state, L->block_normed};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (void* p : L->owned) cudaFree(p);
@@ -786,10 +769,6 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   ra.logits = (aux && aux->logits) ? aux->logits : (v3 ? L->logits_ws : nullptr);
   ra.err = L->d_err;
   ra.variant = L->router_variant;
-  ra.sk_part = L->sk_part;
-  ra.sk_gate = L->sk_gate;
-  ra.sk_counters = L->sk_counters;
-  ra.sk_tokens = L->sk_tokens;
   ra.chained = chained;
   int rc = launch_router(ra, s);
   if (rc) return rc;

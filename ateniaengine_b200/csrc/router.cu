@@ -351,8 +351,9 @@ int launch_v3_route(const float* logits, const float* e_score_bias, int T, int E
 int launch_router(const RouterArgs& a, cudaStream_t s) {
   if (a.T <= 0) return ATENIA_OK;
   if (a.k > kMaxK || a.E > 128) return ATENIA_ERR_UNSUPPORTED;
-  // variant -1: choose by size (see atenia_moe_create)
-  if ((a.variant == 2 || a.variant == -1) && a.T <= a.sk_tokens && a.sk_part) return launch_router_splitk(a, s);
+  // variant -1: choose by size
+  if (a.variant == 2 ? a.T <= kSplitkPinnedTokens && a.d % 16 == 0 : a.variant == -1 && router_splitk_pays(a.T, a.E, a.d))
+    return launch_router_splitk(a, s);
   if (a.variant == 1 || (a.variant == -1 && a.d % 16 == 0)) return launch_router_dmma(a, s);
   dim3 block(kRWarps * 32);
   // more tokens per CTA for many experts: the router matrix is re-read once per CTA

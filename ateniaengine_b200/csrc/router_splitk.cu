@@ -1,190 +1,229 @@
-// Router for small batches: the d-long dot products are cut into 128-wide slices over many CTAs.
+// Router for batches that do not fill the SMs with whole tokens: the d-long dot products are cut over a cluster.
 //
-// router.cu gives every 8 (or 16) tokens one CTA that walks all of d; a CTA takes tens of
-// microseconds however few tokens there are, so at decode sizes the router is a large part of a
-// layer and runs on one SM.  Here CTA (slice, token block) computes the f64 partial logits of 8 tokens
-// over k in [128 slice, 128 slice + 128) and leaves them in a workspace; the last CTA of a token block
-// to finish (an atomic counter decides) adds the slices in ascending order, adds the bias, rounds to
-// f32 and runs the same softmax + top-k (route_one_warp).  Every order of additions is fixed, so
-// results do not depend on scheduling; against router.cu only the order of f64 additions differs.
+// One cluster of eight (or four, or one) CTAs takes eight tokens.  Slice s of the k-range belongs to CTA s mod 8 of the
+// cluster and to one of its warp rows; the products are the f64 tensor-core products of router_dmma.cu (same fragments,
+// same permuted summation index).  The warps' partial sums are added in shared memory, the CTAs' through distributed
+// shared memory, CTA by CTA; the tokens of the block are finished (bias, rounding to f32, softmax, top-k) by one warp
+// each, spread over the CTAs.  Every order of additions is fixed.
 //
-//   warp w of a CTA owns experts w, w + 8, ...; lane l owns k = 128 slice + 4 l .. + 3 for all 8 tokens
-//   (x in registers as f64, loaded once per CTA; the router row is one coalesced 512-byte load per
-//   expert).  The eight tokens' sums are folded over the lanes together: at each of the first three levels of
-//   the tree a lane hands half of its tokens to its partner and keeps the other half (4 + 2 + 1 exchanges and
-//   two more levels for one token, against 5 exchanges for each of eight) -- the additions of the tree, and
-//   so the bits, are those of eight folds.  The last CTA loads 16 slices before it adds them.
-//   Bound by latency (loads, the fold, the counter, the slices' sum).  B200, 61 tokens, 64 experts of d = 2048:
-//   23.3 -> 16.3 us; 64 tokens, 8 experts of d = 512: 8.4 -> 7.2.
+// Bound by latency: two loads deep (the router rows are the layer's own, so they are requested before chain_wait()), the
+// products, two barriers, one softmax; from a few hundred tokens on by the f64 products.  B200, us, a form that left the
+// slices in a workspace for the last CTA to add (up to 128 tokens) or one CTA per eight tokens (above) / this one:
+//   8 experts, d 4096    8 tokens 8.0 / 4.3, 128 12.2 / 4.7, 256 7.5 / 5.0, 512 7.5 / 5.8, 2048 16.3 / 12.0
+//   64 experts, d 2048   8 tokens 12.1 / 6.6, 64 12.5 / 6.8, 256 18.3 / 8.5, 512 19.2 / 12.1, 2048 38.9 / 30.7
+//   128 experts, d 2048  8 tokens 18.0 / 9.3, 256 34.6 / 13.3, 512 34.6 / 20.3, 2048 70.1 / 58.7
+// Between 513 and 1184 tokens one CTA per eight tokens (router_dmma.cu) is as fast (64 experts, 1000 tokens 19.6 / 22 and
+// more), above 2368 its form of 16 tokens per CTA is (4096 tokens 54 / 58), and for a router matrix of 4096 words or less
+// it needs no cluster barriers (8 experts, d 512, 64 tokens 3.6 / 4.3): router_splitk_pays.
+#include "dmma.cuh"
 #include "route_warp.cuh"
 
 namespace atenia {
 namespace {
 
-constexpr int kSkTok = 8;     // tokens per CTA
-constexpr int kSkSlice = 128; // k values per CTA
+constexpr int kSkTok = 8;   // tokens per cluster
 constexpr int kSkWarps = 8;
+constexpr int kSkFewTokens = 512;
+constexpr int kSkSteps = 4;  // steps of 32 k whose router rows are in flight together
 
-template <int E_T>
-__global__ void __launch_bounds__(kSkWarps * 32) router_splitk_kernel(RouterArgs a, int ksplit, int n_tb) {
-  __shared__ float lg_s[kSkTok][E_T];
-  __shared__ double exps_s[kSkWarps][E_T];
-  __shared__ int32_t idx_s[kSkTok][kMaxK];
-  __shared__ float w_s[kSkTok][kMaxK];
-  __shared__ int s_last;
+template <int E_T, bool XF, int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kSkWarps * 32, 2)
+router_splitk_kernel(RouterArgs a, int kw) {
+  constexpr int NT = E_T / 8, NTW = NT < 2 ? NT : 2;  // 8-expert tiles, of which a warp owns NTW
+  constexpr int NW_N = NT / NTW, NW_K = kSkWarps / NW_N;
+  static_assert(NW_N * NW_K == kSkWarps, "warp arrangement");
+  constexpr int XW = XF ? 8 : 4;  // 32-bit words of a lane's eight x values
+  __shared__ double part_s[kSkWarps][NTW][32][2];
+  __shared__ double gpart_s[kSkWarps][kSkTok];
+  __shared__ double sum_s[kSkTok][E_T + 1];  // this CTA's share of the logits; column E_T: of the gate
+  constexpr int kMine = kSkTok / CTAS;  // tokens that a CTA finishes: rank, rank + CTAS, ...
+  __shared__ float lg_s[kMine][E_T];
+  __shared__ double exps_s[kMine][E_T];
+  __shared__ int32_t idx_s[kMine][kMaxK];
+  __shared__ float w_s[kMine][kMaxK];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int slice = blockIdx.x, tb = blockIdx.y;
-  const int t0 = tb * kSkTok;
+  const int ngrp = warp % NW_N, kslice = warp / NW_N;
+  const int r = lane >> 2, c = lane & 3;
+  const int rank = blockIdx.x % CTAS;
+  const int t0 = blockIdx.x / CTAS * kSkTok;
   const int d = a.d, E = a.E;
-  const int k0 = slice * kSkSlice + lane * 4;
-  const bool k_ok = k0 < d;  // d is a multiple of 16: four consecutive k are all in or all out
+  const int s0 = (kslice * CTAS + rank) * kw;
+  const int k_begin = s0 < d ? s0 : d, k_end = k_begin + kw < d ? k_begin + kw : d;
+  const int tg = t0 + r;
 
+  double acc[NTW][2], gacc = 0.0;
+#pragma unroll
+  for (int j = 0; j < NTW; ++j) acc[j][0] = acc[j][1] = 0.0;
+  uint32_t wq[kSkSteps][NTW][8], xq[2][XW];  // raw words: router rows of four steps, x of two
+  auto fetch_w = [&](int kb) {
+#pragma unroll
+    for (int i = 0; i < kSkSteps; ++i) {
+      const int k = kb + 32 * i + c * 8;
+      const bool k_ok = k < k_end;  // d and kw are multiples of 8: a lane's values are all in or all out
+#pragma unroll
+      for (int j = 0; j < NTW; ++j) {
+        const int e = (ngrp * NTW + j) * 8 + r;
+        zero_words(wq[i][j]);
+        if (k_ok && e < E) ld_words<8, true>(wq[i][j], a.w_router + (size_t)e * d + k);
+      }
+    }
+  };
+  auto fetch_x = [&](auto BUF, int kb) {
+    constexpr int b = decltype(BUF)::value;
+    const int k = kb + c * 8;
+    zero_words(xq[b]);
+    if (k < k_end && tg < a.T) {
+      if (XF) ld_words<XW, false>(xq[b], static_cast<const float*>(a.x) + (size_t)tg * d + k);
+      else ld_words<XW, false>(xq[b], static_cast<const __nv_bfloat16*>(a.x) + (size_t)tg * d + k);
+    }
+  };
+  auto multiply = [&](auto STEP) {
+    constexpr int i = decltype(STEP)::value, b = i & 1;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double xv = x_elem<XF>(xq[b], j);
+#pragma unroll
+      for (int jt = 0; jt < NTW; ++jt) dmma884(acc[jt], xv, (double)__uint_as_float(wq[i][jt][j]));
+    }
+  };
   chain_next();
+  fetch_w(k_begin);  // (the layer's copies: no kernel writes them)
+  // the dot product with the shared expert's gate vector: steps of 32 k dealt over all warps of the cluster
+  const int g_begin = (warp * CTAS + rank) * 32 + c * 8;
+  uint32_t gq[8];
+  zero_words(gq);
+  if (a.gate_vec && g_begin < d) ld_words<8, true>(gq, a.gate_vec + g_begin);
   chain_wait();
-  double xk[kSkTok][4];
+  for (int kb = k_begin; kb < k_end; kb += 32 * kSkSteps) {
+    if (kb != k_begin) fetch_w(kb);
+    fetch_x(Int<0>{}, kb);
+    fetch_x(Int<1>{}, kb + 32);
+    multiply(Int<0>{});  // (past k_end every word is zero)
+    fetch_x(Int<0>{}, kb + 64);
+    multiply(Int<1>{});
+    if (kb + 64 < k_end) {  // (uniform over the warp)
+      fetch_x(Int<1>{}, kb + 96);
+      multiply(Int<2>{});
+      multiply(Int<3>{});
+    }
+  }
 #pragma unroll
-  for (int t = 0; t < kSkTok; ++t) {
-    const int tg = t0 + t;
-    xk[t][0] = xk[t][1] = xk[t][2] = xk[t][3] = 0.0;
-    if (tg < a.T && k_ok) {
-      if (a.x_is_f32) {
-        const float4 v = *reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)tg * d + k0);
-        xk[t][0] = v.x; xk[t][1] = v.y; xk[t][2] = v.z; xk[t][3] = v.w;
-      } else {
-        const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a.x) + (size_t)tg * d + k0);
-        xk[t][0] = bf16lo(u.x); xk[t][1] = bf16hi(u.x); xk[t][2] = bf16lo(u.y); xk[t][3] = bf16hi(u.y);
+  for (int jt = 0; jt < NTW; ++jt) {
+    part_s[warp][jt][lane][0] = acc[jt][0];
+    part_s[warp][jt][lane][1] = acc[jt][1];
+  }
+  if (a.gate_vec) {
+    for (int k = g_begin; k < d; k += 32 * CTAS * kSkWarps) {
+      uint32_t xg[XW];
+      zero_words(xg);
+      if (tg < a.T) {
+        if (XF) ld_words<XW, false>(xg, static_cast<const float*>(a.x) + (size_t)tg * d + k);
+        else ld_words<XW, false>(xg, static_cast<const __nv_bfloat16*>(a.x) + (size_t)tg * d + k);
       }
-    }
-  }
-  double* part = a.sk_part + ((size_t)slice * n_tb + tb) * kSkTok * E_T;
-  // sums of eight tokens over the lanes; the lanes 4 t .. 4 t + 3 end with that of token t
-  static_assert(kSkTok == 8, "three halving levels");
-  auto fold8 = [&](double (&v)[kSkTok]) {
+      if (k != g_begin) ld_words<8, true>(gq, a.gate_vec + k);
 #pragma unroll
-    for (int o = 16, n = kSkTok / 2; o >= 4; o >>= 1, n >>= 1) {
-      const bool upper = (lane & o) != 0;
-#pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const double give = upper ? v[i] : v[n + i];
-        const double keep = upper ? v[n + i] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-      }
+      for (int j = 0; j < 8; ++j) gacc = fma((double)__uint_as_float(gq[j]), x_elem<XF>(xg, j), gacc);
     }
-    double r = v[0];
-    r += __shfl_xor_sync(0xffffffffu, r, 2);
-    r += __shfl_xor_sync(0xffffffffu, r, 1);
-    return r;
-  };
-  const int t_fold = lane >> 2;  // levels 16, 8, 4 chose bits 2, 1, 0 of the token
-  auto dots = [&](const double (&w)[4]) {
-    double acc[kSkTok];
-#pragma unroll
-    for (int t = 0; t < kSkTok; ++t) {
-      acc[t] = w[0] * xk[t][0];
-      acc[t] = fma(w[1], xk[t][1], acc[t]);
-      acc[t] = fma(w[2], xk[t][2], acc[t]);
-      acc[t] = fma(w[3], xk[t][3], acc[t]);
-    }
-    return fold8(acc);
-  };
-#pragma unroll 2
-  for (int e = warp; e < E; e += kSkWarps) {
-    double w[4] = {0.0, 0.0, 0.0, 0.0};
-    if (k_ok) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(a.w_router + (size_t)e * d + k0));
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    }
-    const double r = dots(w);
-    if ((lane & 3) == 0) part[t_fold * E_T + e] = r;
+    __syncwarp();
+    // the four lanes of a row hold the k-quarters of its dot product: fold them (fixed tree)
+    gacc += __shfl_xor_sync(0xffffffffu, gacc, 1);
+    gacc += __shfl_xor_sync(0xffffffffu, gacc, 2);
+    if (c == 0) gpart_s[warp][r] = gacc;
   }
-  if (a.gate_vec && warp == 0) {  // partial dot products with the shared expert's gate vector
-    double g[4] = {0.0, 0.0, 0.0, 0.0};
-    if (k_ok) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(a.gate_vec + k0));
-      g[0] = v.x; g[1] = v.y; g[2] = v.z; g[3] = v.w;
-    }
-    const double r = dots(g);
-    if ((lane & 3) == 0) a.sk_gate[((size_t)slice * n_tb + tb) * kSkTok + t_fold] = r;
-  }
-  // the last CTA of this token block to get here finishes the block
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = (atomicAdd(&a.sk_counters[tb], 1u) == (unsigned)(ksplit - 1)) ? 1 : 0;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // slices in ascending order, the loads of 16 in flight at once
-  auto sum_slices = [&](const double* p, size_t stride) {
+  for (int i = threadIdx.x; i < kSkTok * E_T; i += kSkWarps * 32) {
+    const int t = i / E_T, e = i - t * E_T;
+    const int nt = e >> 3, col = e & 7, og = nt / NTW, jt = nt - og * NTW;
     double v = 0.0;
-    for (int s0 = 0; s0 < ksplit; s0 += 16) {
-      double x[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) x[j] = s0 + j < ksplit ? __ldcg(p + (size_t)(s0 + j) * stride) : 0.0;
+    for (int ks = 0; ks < NW_K; ++ks) v += part_s[ks * NW_N + og][jt][t * 4 + (col >> 1)][col & 1];
+    sum_s[t][e] = v;
+  }
+  if (a.gate_vec && threadIdx.x < kSkTok) {
+    double v = 0.0;
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (s0 + j < ksplit) v += x[j];
+    for (int w = 0; w < kSkWarps; ++w) v += gpart_s[w][threadIdx.x];
+    sum_s[threadIdx.x][E_T] = v;
+  }
+  __syncwarp();  // (.aligned: the lanes of a warp arrive together)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  // this CTA's tokens: the shares of their logits in CTA order, then the bias, then the rounding to f32
+  for (int i = threadIdx.x; i < kMine * (E_T + 1); i += kSkWarps * 32) {
+    const int m = i / (E_T + 1), e = i - m * (E_T + 1), t = m * CTAS + rank, my = t0 + t;
+    if (my >= a.T || !(e < E || (e == E_T && a.gate_vec && a.gate_scale))) continue;
+    const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(&sum_s[t][e]));
+    double v[CTAS], sum = 0.0;
+#pragma unroll
+    for (int q = 0; q < CTAS; ++q) {
+      uint32_t theirs;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(q));
+      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v[q]) : "r"(theirs) : "memory");
     }
-    return v;
-  };
-  for (int i = threadIdx.x; i < kSkTok * E; i += blockDim.x) {
-    const int t = i / E, e = i - t * E;
-    double v = sum_slices(a.sk_part + ((size_t)tb * kSkTok + t) * E_T + e, (size_t)n_tb * kSkTok * E_T);
-    if (a.bias) v += (double)a.bias[e];  // the bias joins the f64 sum before the rounding to f32
-    const float f = (float)v;
-    lg_s[t][e] = f;
-    const int tg = t0 + t;
-    if (a.logits && tg < a.T) a.logits[(size_t)tg * E + e] = f;
+#pragma unroll
+    for (int q = 0; q < CTAS; ++q) sum += v[q];
+    if (e == E_T) {
+      a.gate_scale[my] = (float)(1.0 / (1.0 + exp(-sum)));
+    } else {
+      if (a.bias) sum += (double)a.bias[e];  // the bias joins the f64 sum before the rounding to f32
+      const float f = (float)sum;
+      lg_s[m][e] = f;
+      if (a.logits) a.logits[(size_t)my * E + e] = f;
+    }
   }
-  if (a.gate_vec && a.gate_scale && threadIdx.x < kSkTok) {
-    const int t = threadIdx.x, tg = t0 + t;
-    const double v = sum_slices(a.sk_gate + (size_t)tb * kSkTok + t, (size_t)n_tb * kSkTok);
-    if (tg < a.T) a.gate_scale[tg] = (float)(1.0 / (1.0 + exp(-v)));
-  }
+  // (waited for at the end: no CTA leaves while another may read its shares)
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   __syncthreads();
-  {
-    const int t = warp, tg = t0 + t;  // one warp per token
-    if (tg < a.T) {
-      int rc = route_one_warp<(E_T + 31) / 32>(lg_s[t], E, a.k, a.renormalize, lane, idx_s[t], w_s[t], exps_s[warp]);
-      if (rc) {
-        if (lane == 0) report_error(a.err, rc, 1004);
-        if (lane < a.k) {  // keep downstream kernels in bounds
-          idx_s[t][lane] = lane;
-          w_s[t][lane] = 0.f;
-        }
-      }
-      __syncwarp();
-      if (lane < a.k) {
-        a.topk_idx[(size_t)tg * a.k + lane] = idx_s[t][lane];
-        a.topk_w[(size_t)tg * a.k + lane] = w_s[t][lane];
+  const int my = t0 + warp * CTAS + rank;  // one warp per token
+  if (warp < kMine && my < a.T) {
+    const int rc = route_one_warp<(E_T + 31) / 32>(lg_s[warp], E, a.k, a.renormalize, lane, idx_s[warp], w_s[warp], exps_s[warp]);
+    if (rc) {
+      if (lane == 0) report_error(a.err, rc, 1004);
+      if (lane < a.k) {  // keep downstream kernels in bounds
+        idx_s[warp][lane] = lane;
+        w_s[warp][lane] = 0.f;
       }
     }
+    __syncwarp();
+    if (lane < a.k) {
+      a.topk_idx[(size_t)my * a.k + lane] = idx_s[warp][lane];
+      a.topk_w[(size_t)my * a.k + lane] = w_s[warp][lane];
+    }
   }
-  if (threadIdx.x == 0) a.sk_counters[tb] = 0u;  // ready for the next launch (and for graph replay)
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+template <int E_T, int CTAS>
+int launch_form(const RouterArgs& a, bool chained, cudaStream_t s) {
+  constexpr int NT = E_T / 8, NTW = NT < 2 ? NT : 2;
+  constexpr int kSlices = CTAS * (kSkWarps / (NT / NTW));
+  const int kw = ((a.d + kSlices - 1) / kSlices + 31) / 32 * 32;  // k-range of a slice: whole steps of 32
+  const dim3 grid((a.T + kSkTok - 1) / kSkTok * CTAS), block(kSkWarps * 32);
+  if (a.x_is_f32) return launch_chained(chained, router_splitk_kernel<E_T, true, CTAS>, grid, block, 0, s, a, kw);
+  return launch_chained(chained, router_splitk_kernel<E_T, false, CTAS>, grid, block, 0, s, a, kw);
+}
+
+// CTAs per cluster: as many as let every cluster run at once (two CTAs per SM).  From 1185 tokens on a cluster of one, a
+// plain launch (see router_dmma.cu).
 template <int E_T>
 int launch_one(const RouterArgs& a, cudaStream_t s) {
-  const int ksplit = (a.d + kSkSlice - 1) / kSkSlice;
-  const int n_tb = (a.T + kSkTok - 1) / kSkTok;
-  return launch_chained(a.chained, router_splitk_kernel<E_T>, dim3(ksplit, n_tb), dim3(kSkWarps * 32), 0, s, a, ksplit, n_tb);
+  if (a.T <= 256) return launch_form<E_T, 8>(a, a.chained, s);
+  if (a.T <= kSkFewTokens) return launch_form<E_T, 4>(a, a.chained, s);
+  return launch_form<E_T, 1>(a, false, s);
 }
 
 }  // namespace
 
-// Workspace a layer needs for batches of at most `tokens`: doubles for the partial logits and gate
-// dot products, counters (zero-initialised by the caller once).
-void router_splitk_workspace(int tokens, int d, int E, size_t* part_doubles, size_t* gate_doubles, size_t* counters) {
-  const size_t ksplit = (size_t)(d + kSkSlice - 1) / kSkSlice, n_tb = (size_t)(tokens + kSkTok - 1) / kSkTok;
-  const size_t e_t = E <= 8 ? 8 : E <= 16 ? 16 : E <= 32 ? 32 : E <= 64 ? 64 : 128;
-  *part_doubles = ksplit * n_tb * kSkTok * e_t;
-  *gate_doubles = ksplit * n_tb * kSkTok;
-  *counters = n_tb;
+bool router_splitk_pays(int T, int E, int d) {
+  if (d % 16 != 0 || (int64_t)E * d <= 4096) return false;
+  return T <= kSkFewTokens || (T > 8 * 148 && T <= 16 * 148);
 }
 
 int launch_router_splitk(const RouterArgs& a, cudaStream_t s) {
   if (a.T <= 0) return ATENIA_OK;
   if (a.k > kMaxK || a.E > 128 || a.d % 16 != 0) return ATENIA_ERR_UNSUPPORTED;
-  if (!a.sk_part || !a.sk_gate || !a.sk_counters || a.T > a.sk_tokens) return ATENIA_ERR_STATE;
   int rc;
   if (a.E <= 8) rc = launch_one<8>(a, s);
   else if (a.E <= 16) rc = launch_one<16>(a, s);
