@@ -109,6 +109,8 @@ struct RouterArgs {
   DeviceError* err;
   int variant;         // -1: by size; 0: CUDA-core f64 kernel (router.cu); 1: f64 tensor-core kernel
                        // (router_dmma.cu); 2: split-k kernel (router_splitk.cu) up to kSplitkPinnedTokens
+  const CUtensorMap* digit_map;  // integer router (router_i8.cu): digit planes of the router matrix (host pointer; null:
+  const double* digit_scale;     // the layer has none) and the scale of each of its rows
   bool chained;        // see launch_chained
 };
 int launch_router(const RouterArgs& a, cudaStream_t s);
@@ -116,6 +118,15 @@ int launch_router_dmma(const RouterArgs& a, cudaStream_t s);  // same contract, 
 int launch_router_splitk(const RouterArgs& a, cudaStream_t s);  // same contract
 bool router_splitk_pays(int T, int E, int d);
 constexpr int kSplitkPinnedTokens = 1024;
+// Integer router of bf16 activations: layers of at most 64 rows of w (experts, and the gate vector if the call wants it).
+// planes [kRouterDigitPlanes][kRouterDigitRows][d] int8, map with box {128, kRouterDigitPlanes * kRouterDigitRows / 2} and
+// the 128-byte swizzle; scale [kRouterDigitRows].
+constexpr int kRouterDigitRows = 64, kRouterDigitPlanes = 5;
+constexpr int kRouterDigitMaxK = 16384;  // (int32 sums of up to four products of 2^14 a k)
+// Does a layer get the planes?  (16 experts or fewer: the f64 routers are as fast)
+inline bool router_digits_built(int E, int d) { return E > 16 && E <= kRouterDigitRows && d <= kRouterDigitMaxK; }
+int launch_router_i8(const RouterArgs& a, cudaStream_t s);
+int launch_router_digits(const float* router, const float* gate, int E, int d, int8_t* planes, double* scale, cudaStream_t s);
 int launch_route_from_logits(const float* logits, int T, int E, int k, int renormalize,
                              int32_t* topk_idx, float* topk_w, DeviceError* err, cudaStream_t s);
 

@@ -48,6 +48,9 @@ struct AteniaMoeLayer {
 
   // weights (device)
   float* d_router = nullptr;    // [E, d]
+  int8_t* rd_planes = nullptr;  // integer router: digit planes of the router matrix and the gate vector, their scales
+  double* rd_scale = nullptr;
+  CUtensorMap tm_rd{};
   float* d_bias = nullptr;      // [E]
   float* d_gate_vec = nullptr;  // [d]
   float* d_escore = nullptr;    // [E] V3 e_score_correction_bias (zeros if none given)

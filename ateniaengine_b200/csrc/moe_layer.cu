@@ -377,6 +377,16 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
   TRY_ALLOC(L->d_router, E * d);
   TRY_ALLOC(L->d_bias, E);
   TRY_ALLOC(L->d_gate_vec, d);
+  if (router_digits_built(c.num_experts, c.d_model)) {
+    TRY_ALLOC(L->rd_planes, (size_t)kRouterDigitPlanes * kRouterDigitRows * d);
+    TRY_ALLOC(L->rd_scale, kRouterDigitRows);
+    rc = encode_tmap_2d_u8(&L->tm_rd, L->rd_planes, (uint64_t)kRouterDigitPlanes * kRouterDigitRows, d,
+                           kRouterDigitPlanes * kRouterDigitRows / 2, 128, 2);
+    if (rc) {
+      atenia_moe_destroy(L);
+      return rc;
+    }
+  }
   if (c.router_mode == ATENIA_ROUTER_V3) {
     TRY_ALLOC(L->d_escore, E);
     TRY_ALLOC(L->logits_ws, Tm * E);
@@ -510,7 +520,7 @@ int atenia_moe_destroy(AteniaMoeLayer* L) {
   if (!L) return ATENIA_OK;
   cudaDeviceSynchronize();
   ep_destroy(L);
-  void* ptrs[] = {L->d_router, L->d_bias, L->d_gate_vec, L->topk_idx, L->topk_w, L->gate_scale, L->perm,
+  void* ptrs[] = {L->d_router, L->rd_planes, L->rd_scale, L->d_bias, L->d_gate_vec, L->topk_idx, L->topk_w, L->gate_scale, L->perm,
                   L->inv_perm, L->expert_offsets, L->shared_offsets, L->block_counts, L->block_base, L->x_perm,
                   L->h, L->y_perm, L->x_bf16, L->h_shared, L->y_shared, L->d_err, L->d_tm_gate, L->d_tm_up,
                   L->d_tm_down, L->d_tm_shared, L->d_sc_gate, L->d_sc_up, L->d_sc_down, L->d_sc_shared,
@@ -563,6 +573,11 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
   L->has_gate_vec = L->gate_vec_bound && c.shared_gated;
   if (L->gate_vec_bound)
     ATENIA_CUDA_TRY(cudaMemcpy(L->d_gate_vec, w->shared_gate_vec, d * sizeof(float), cudaMemcpyDeviceToDevice));
+  if (L->rd_planes) {
+    int rrc = launch_router_digits(L->d_router, L->gate_vec_bound ? L->d_gate_vec : nullptr, c.num_experts, c.d_model,
+                                   L->rd_planes, L->rd_scale, nullptr);
+    if (rrc) return rrc;
+  }
 
   // INT8 matrices are borrowed as they are: their tensor maps describe bytes and the grouped GEMM
   // widens the codes to bf16 on chip.
@@ -769,6 +784,8 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   ra.logits = (aux && aux->logits) ? aux->logits : (v3 ? L->logits_ws : nullptr);
   ra.err = L->d_err;
   ra.variant = L->router_variant;
+  ra.digit_map = L->rd_planes ? &L->tm_rd : nullptr;
+  ra.digit_scale = L->rd_scale;
   ra.chained = chained;
   int rc = launch_router(ra, s);
   if (rc) return rc;

@@ -71,6 +71,10 @@ uint64_t layer_workspace_bytes(const AteniaMoeConfig& c, int world) {
   t.add(E * d * 4);           // router copy
   t.add(E * 4);               // bias
   t.add(d * 4);               // gate vector
+  if (router_digits_built(c.num_experts, c.d_model)) {  // digit planes of the router matrix
+    t.add((uint64_t)kRouterDigitPlanes * kRouterDigitRows * d);
+    t.add(kRouterDigitRows * 8);
+  }
   if (c.router_mode == ATENIA_ROUTER_V3) {
     t.add(E * 4);
     t.add(Tm * E * 4);
