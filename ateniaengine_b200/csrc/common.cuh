@@ -200,6 +200,7 @@ struct GroupedGemmArgs {
   DeviceError* err;
   int max_rows;  // upper bound on total rows (sizes nothing; used by the checking kernel's grid)
   const PairRowMaps* pair_rows;  // CTA-pair kernel only (host pointer, copied at the launch)
+  int pair_tokens;  // ... token rows of a tile at most: 64, 128, else 256 (pair_tokens_of)
   int w8;        // B matrices are int8 (tensor maps of bytes), widened to bf16 inside the kernel
   float* splitk_ws;  // W8 tensor-memory kernel: workspace for stream-K partial sums (null: whole tiles only)
   // stream-K decode kernels: zeroed counters [kSplitKMaxTiles * 8] with which the kernel finishes the split
@@ -291,6 +292,7 @@ int launch_quantize_digits(const DigitSource& src, const int32_t* n_rows_dev, in
 // bf16 weights, CTA pairs (tcgen05 cta_group::2), transposed product: pair_rows describes the token rows (tmap_a
 // is not read), tmap_b0 / tmap_b1 have boxes of kPairWeightRows (kSwiGLU) or 128 (kPlain) weight rows
 constexpr int kPairWeightRows = 64;
+inline int pair_f_tiles(int n, int mode) { return mode == kSwiGLU ? (n + 127) / 128 : (n + 255) / 256; }  // feature tiles
 int launch_grouped_gemm_2cta(const GroupedGemmArgs& a, int num_sms, cudaStream_t s);
 // bf16 weights, CTA pairs, token rows as the M side (grouped_gemm_pair_rows.cu): tensor maps of the single-CTA kernel
 int launch_grouped_gemm_pair_rows(const GroupedGemmArgs& a, int num_sms, cudaStream_t s);

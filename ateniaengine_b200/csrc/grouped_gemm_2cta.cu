@@ -7,16 +7,18 @@
 // tcgen05.mma.cta_group::2 (M256 x Nn x K16), which reads both operands from both CTAs' shared memory.
 //
 // Why transposed: the M side of an MMA costs 256 rows however few hold data, the N side costs what it is
-// wide.  A group of R rows is cut into ceil(R / 256) equal token tiles rounded up to 16 rows, so the padding
+// wide.  A group of R rows is cut into ceil(R / 256) (128, 64) equal token tiles rounded up to 16 rows, so the padding
 // is below 16 rows per tile.
 //
 //   kSwiGLU : 256 weight rows = 128 features; a CTA's 128 rows are 64 rows of W_gate and the same 64 of W_up,
 //             so the epilogue warps of lane quarters q and q + 2 hold gate and up of the same features and
 //             exchange them through shared memory (f32), each finishing half of the tokens
 //   kPlain  : 256 weight rows = 256 features
-//   k-block : 64 (one 128-byte swizzle row): 16 KiB of weights + at most 16 KiB of tokens per CTA, 6 stages
+//   k-block : 64 (one 128-byte swizzle row): 16 KiB of weights + 16, 8 or 4 KiB of tokens per CTA (tiles of at most 256, 128
+//             or 64 token rows, the launch's choice: pair_tokens_of), 6, 8 or 10 stages
 //
-// What bounds it: the tensor pipe and the board's power.  ncu, DeepSeek-V2-Lite shape, 8192 tokens, gate/up: the
+// What bounds it: below some hundred rows per group HBM's latency, that is, the weights in flight (10 stages hold 160 KiB per
+// SM: 16 tokens of the Mixtral shape 451 -> 422 us against 6 stages), above the tensor pipe and the board's power.  ncu, DeepSeek-V2-Lite shape, 8192 tokens, gate/up: the
 // pipe is busy 90 % of 524 k cycles (75 % of 626 k with the issuing lane under `lane == 0`, see uniform_warp;
 // 67 % of 701 k with two token tiles per weight tile and 16-byte stores through shared memory).  One forward on a
 // B200, before (token-major 256-row pair tiles from 512 rows per group, 128-row single-CTA tiles below) and now:
@@ -36,21 +38,27 @@ namespace {
 using namespace tc;
 
 constexpr int TN2 = kPairTokens;
-constexpr int STAGES2 = 6;
+constexpr int MAX_STAGES2 = 10;
 constexpr int ACC_BUFS2 = 2;
 constexpr int TMEM_COLS2 = 512;
 constexpr int W_BYTES2 = BM * BK * 2;         // 16 KiB: this CTA's 128 weight rows
-constexpr int X_BYTES2 = (TN2 / 2) * BK * 2;  // 16 KiB: this CTA's half of the token tile
-constexpr int STAGE_BYTES2 = W_BYTES2 + X_BYTES2;
 constexpr int EPI_WARPS2 = 8;
 constexpr int NUM_THREADS2 = 64 + EPI_WARPS2 * 32;
 constexpr int EPI_WARP_BYTES2 = 2 * 1024;  // kSwiGLU: two buffers of 8 tokens x 32 features of f32 per warp
 constexpr int EPI_BYTES2 = EPI_WARPS2 * EPI_WARP_BYTES2;
-constexpr int SMEM_BYTES2 = STAGES2 * STAGE_BYTES2 + EPI_BYTES2 + 1024 + 256;
+// The ring by the token rows of a tile at most.
+template <int TOK>
+struct PairRing {
+  static constexpr int X_BYTES = (TOK / 2) * BK * 2;  // this CTA's half of the token tile
+  static constexpr int STAGE_BYTES = W_BYTES2 + X_BYTES;
+  static constexpr int STAGES = TOK == 256 ? 6 : TOK == 128 ? 8 : 10;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES2 + 1024 + 256;
+  static_assert(STAGES <= MAX_STAGES2 && STAGE_BYTES % 1024 == 0 && SMEM_BYTES <= 225 * 1024, "");
+};
 
 struct __align__(8) Barriers2 {
-  uint64_t full[STAGES2];
-  uint64_t empty[STAGES2];
+  uint64_t full[MAX_STAGES2];
+  uint64_t empty[MAX_STAGES2];
   uint64_t acc_full[ACC_BUFS2];
   uint64_t acc_empty[ACC_BUFS2];
   uint32_t tmem_base;
@@ -70,13 +78,15 @@ struct PairTile {
   int group, row0, rows, f0;  // first row and rows of the tile, first feature
   int n;                      // MMA N: rows rounded up to 16
 };
+template <int TOK>
 __device__ __forceinline__ void pair_cursor_load(PairCursor& c, const int32_t* __restrict__ off) {
   c.row_begin = off[c.group];
   c.row_end = off[c.group + 1];
   const int rows = c.row_end - c.row_begin;
-  c.m_tiles = pair_tiles(rows);
+  c.m_tiles = pair_tiles(rows, TOK);
   c.tile_rows = pair_tile_rows(rows, c.m_tiles);
 }
+template <int TOK>
 __device__ __forceinline__ bool pair_cursor_seek(PairCursor& c, int tile, int f_tiles, int num_groups,
                                                  const int32_t* __restrict__ off, PairTile& out, int f_width) {
   while (c.group < num_groups) {
@@ -87,14 +97,14 @@ __device__ __forceinline__ bool pair_cursor_seek(PairCursor& c, int tile, int f_
       const int mt = local - ft * c.m_tiles;
       out.group = c.group;
       out.row0 = c.row_begin + mt * c.tile_rows;
-      out.rows = min(c.row_end - out.row0, c.tile_rows);  // >= 1: tile_rows <= 256, so no tile starts past the end
+      out.rows = min(c.row_end - out.row0, c.tile_rows);  // >= 1: m_tiles is the fewest of tile_rows
       out.n = pair_tile_n(out.rows);
       out.f0 = ft * f_width;
       return true;
     }
     c.base += here;
     c.group += 1;
-    if (c.group < num_groups) pair_cursor_load(c, off);
+    if (c.group < num_groups) pair_cursor_load<TOK>(c, off);
   }
   return false;
 }
@@ -159,7 +169,7 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
       : "memory");
 }
 
-template <int MODE>
+template <int MODE, int TOK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS2, 1)
 grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUtensorMap* __restrict__ tmap_w0,
                          const CUtensorMap* __restrict__ tmap_w1, const int32_t* __restrict__ group_offsets_g,
@@ -168,6 +178,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
   __shared__ int32_t goff_s[kMaxGroupsShared + 1];
   constexpr int F_CTA = (MODE == kSwiGLU) ? BM / 2 : BM;  // output features per CTA
   constexpr int F_PAIR = 2 * F_CTA;
+  constexpr int STAGES2 = PairRing<TOK>::STAGES, STAGE_BYTES2 = PairRing<TOK>::STAGE_BYTES;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
   uint8_t* epi = smem_aligned + STAGES2 * STAGE_BYTES2;
@@ -214,7 +225,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
   PairCursor cur;
   cur.group = 0;
   cur.base = 0;
-  if (num_groups > 0) pair_cursor_load(cur, group_offsets);
+  if (num_groups > 0) pair_cursor_load<TOK>(cur, group_offsets);
   PairTile tc;
 
   if (warp == 0) {
@@ -227,7 +238,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
     // Weights of the first tile's first k-blocks; their token rows follow after the wait.  B200, 64 tokens of a 512-wide
     // layer 37.7 -> 33.9 us, 256 Mixtral tokens 507 -> 497.
     int ahead = 0;
-    if (PairCursor c0 = cur; pair_cursor_seek(c0, pair, f_tiles, num_groups, group_offsets, tc, F_PAIR)) {
+    if (PairCursor c0 = cur; pair_cursor_seek<TOK>(c0, pair, f_tiles, num_groups, group_offsets, tc, F_PAIR)) {
       const CUtensorMap* m0 = &tmap_w0[tc.group];
       const CUtensorMap* m1 = MODE == kSwiGLU ? &tmap_w1[tc.group] : m0;
       tmap_acquire(m0);
@@ -246,7 +257,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
       }
     }
     chain_wait();
-    for (int tile = pair; ok && pair_cursor_seek(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
+    for (int tile = pair; ok && pair_cursor_seek<TOK>(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
          tile += num_pairs) {
       const CUtensorMap* m0 = &tmap_w0[tc.group];
       const CUtensorMap* m1 = MODE == kSwiGLU ? &tmap_w1[tc.group] : m0;
@@ -304,7 +315,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
       uint32_t acc_phase = 0;  // bit b: accumulator b
       int it = 0;
       bool ok = true;
-      for (int tile = pair; ok && pair_cursor_seek(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
+      for (int tile = pair; ok && pair_cursor_seek<TOK>(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
            tile += num_pairs, ++it) {
         const int acc = it & 1;
         if (!mbar_wait(smem_u32(&bars->acc_empty[acc]), ((acc_phase >> acc) & 1u) ^ 1u, abort_flag)) {
@@ -357,7 +368,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
     int flip = 0;
     uint32_t acc_phase = 0;
     int it = 0;
-    for (int tile = pair; pair_cursor_seek(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
+    for (int tile = pair; pair_cursor_seek<TOK>(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
          tile += num_pairs, ++it) {
       const int acc = it & 1;
       bool ready = mbar_wait(smem_u32(&bars->acc_full[acc]), (acc_phase >> acc) & 1u, abort_flag);
@@ -430,16 +441,23 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
   }
 }
 
-template <int MODE>
+template <int MODE, int TOK>
 int launch_2cta_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   static bool attr_set[kMaxDevices] = {};
   if (first_use_on_current_device(attr_set)) {
-    ATENIA_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_2cta_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES2));
+    ATENIA_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_2cta_kernel<MODE, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         PairRing<TOK>::SMEM_BYTES));
   }
   const int grid = num_sms & ~1;  // whole pairs
-  return launch_chained(a.chained, grouped_gemm_2cta_kernel<MODE>, dim3(grid), dim3(NUM_THREADS2), SMEM_BYTES2, s, *a.pair_rows, a.tmap_b0,
+  return launch_chained(a.chained, grouped_gemm_2cta_kernel<MODE, TOK>, dim3(grid), dim3(NUM_THREADS2), PairRing<TOK>::SMEM_BYTES, s, *a.pair_rows, a.tmap_b0,
                         MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out, a.err);
+}
+
+template <int MODE>
+int launch_2cta_tokens(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
+  if (a.pair_tokens == 64) return launch_2cta_one<MODE, 64>(a, num_sms, s);
+  if (a.pair_tokens == 128) return launch_2cta_one<MODE, 128>(a, num_sms, s);
+  return launch_2cta_one<MODE, kPairTokens>(a, num_sms, s);
 }
 
 }  // namespace
@@ -456,7 +474,7 @@ int launch_grouped_gemm_2cta(const GroupedGemmArgs& a, int num_sms, cudaStream_t
   if (a.N % 16 != 0 || a.K % 16 != 0 || a.num_groups > kMaxGroupsShared) return ATENIA_ERR_SHAPE;
   if (!a.pair_rows) return ATENIA_ERR_NULL;
   if (a.w8) return ATENIA_ERR_UNSUPPORTED;  // INT8 weights: w8_gemm.cu / w8_gemm_m256.cu
-  int rc = a.mode == kSwiGLU ? launch_2cta_one<kSwiGLU>(a, num_sms, s) : launch_2cta_one<kPlain>(a, num_sms, s);
+  int rc = a.mode == kSwiGLU ? launch_2cta_tokens<kSwiGLU>(a, num_sms, s) : launch_2cta_tokens<kPlain>(a, num_sms, s);
   count_launch();
   count_tcgen05_launch();
   return rc;

@@ -166,6 +166,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     g1.chained = L->gemm_chained;
     g1.tmap_a = tm_a.tile;
     g1.pair_rows = &tm_a.pair;
+    g1.pair_tokens = pair_tokens_of(max_rows, num_groups, pair_f_tiles(c.d_ff, kSwiGLU));
     g1.tmap_b0 = tmem ? L->d_tm_gate_sw : !q && !dec && bf1 == kBf16Pairs ? L->d_tm_gate_box : L->d_tm_gate;
     g1.tmap_b1 = tmem ? L->d_tm_up_sw : !q && !dec && bf1 == kBf16Pairs ? L->d_tm_up_box : L->d_tm_up;
     g1.group_offsets = group_offsets;
@@ -198,6 +199,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     g2.chained = L->gemm_chained;
     g2.tmap_a = tm_mid.tile;
     g2.pair_rows = &tm_mid.pair;
+    g2.pair_tokens = pair_tokens_of(max_rows, num_groups, pair_f_tiles(c.d_model, kPlain));
     g2.tmap_b0 = tmem ? L->d_tm_down_sw : L->d_tm_down;
     g2.tmap_b1 = g2.tmap_b0;
     g2.group_offsets = group_offsets;
@@ -260,10 +262,12 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   g1.chained = L->gemm_chained;
   // (the one group has T rows: only the boxes of its tiles, since the caller's x makes this part of every call)
   PairRowMaps x_rows{};
-  int rc = bf1 == kBf16Pairs ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model, pair_boxes_of_group(T))
+  const int tokens = pair_tokens_of(T, 1, pair_f_tiles(c.shared_d_ff, kSwiGLU));
+  int rc = bf1 == kBf16Pairs ? encode_pair_rows(&x_rows, xb, (uint64_t)T, (uint64_t)c.d_model, pair_boxes_of_group(T, tokens))
                              : encode_tmap_2d_bf16(&g1.tmap_a, xb, (uint64_t)T, (uint64_t)c.d_model, 128, 64);
   if (rc) return rc;
   g1.pair_rows = &x_rows;
+  g1.pair_tokens = tokens;
   g1.tmap_b0 = tmem ? L->d_tm_shared_sw : bf1 == kBf16Pairs ? L->d_tm_shared_box : L->d_tm_shared;
   g1.tmap_b1 = g1.tmap_b0 + 1;
   g1.group_offsets = L->shared_offsets;
@@ -286,6 +290,7 @@ int run_shared_gemms(AteniaMoeLayer* L, const __nv_bfloat16* xb, int T, cudaStre
   g2.chained = L->gemm_chained;
   g2.tmap_a = L->tm_h_shared.tile;
   g2.pair_rows = &L->tm_h_shared.pair;
+  g2.pair_tokens = pair_tokens_of(T, 1, pair_f_tiles(c.d_model, kPlain));
   g2.tmap_b0 = (tmem ? L->d_tm_shared_sw : L->d_tm_shared) + 2;
   g2.tmap_b1 = g2.tmap_b0;
   g2.group_offsets = L->shared_offsets;

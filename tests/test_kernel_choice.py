@@ -80,3 +80,22 @@ def test_the_benchmark_names_the_kernel_that_runs(lib):
                                 "grouped_gemm_pair_rows_kernel")[lib.choice_bf16(rows, E, d, 0)]
             else:
                 assert name == ("grouped_gemv_kernel" if rows <= 2 and rows * d * F < 1 << 26 else "grouped_gemm_decode_kernel")
+
+
+# rows, groups, feature tiles of the gate/up product, us of a forward with tiles of 256 / 128 / 64 token rows
+PAIR_TOKENS = [(32, 8, 112, 451, 432, 422), (240, 8, 112, 464, 444, 436), (512, 8, 112, 488, 466, 535),
+               (700, 8, 112, 519, 503, 584), (800, 8, 112, 530, 548, 602), (64, 60, 11, 147, 138, 137),
+               (600, 60, 11, 209, 197, 195), (1332, 60, 11, 237, 223, 228), (5200, 60, 11, 309, 297, 380),
+               (6800, 60, 11, 351, 356, 423), (366, 64, 11, 205, 196, 196), (5400, 64, 11, 272, 269, 317),
+               (7800, 64, 11, 306, 310, 380)]
+
+
+@pytest.mark.parametrize("rows,groups,f_tiles,t256,t128,t64", PAIR_TOKENS)
+def test_pair_tile_height_is_near_the_fastest_measured(lib, rows, groups, f_tiles, t256, t128, t64):
+    took = {256: t256, 128: t128, 64: t64}[lib.choice_pair_tokens(rows, groups, f_tiles)]
+    assert took <= 1.01 * min(t256, t128, t64)
+
+
+def test_pair_tile_height_of_one_group_holds_it_whole(lib):
+    assert [lib.choice_pair_tokens(r, 1, 100) for r in (1, 64, 65, 128, 129, 4096)] == [64, 64, 128, 128, 256, 256]
+    assert lib.choice_pair_tokens(4096, 8, 1) == 64  # fewer tiles than pairs of SMs

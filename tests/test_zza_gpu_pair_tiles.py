@@ -91,3 +91,11 @@ def _check_groups(sizes, d, F, int8):
         ref = (g * torch.sigmoid(g) * (xe @ weights("up", e).t())) @ weights("down", e).t()
         err = ((y[rows].double() - ref).norm() / ref.norm()).item()
         assert err <= TOL, (e, n, err)
+
+
+@pytest.mark.parametrize("sizes", [[63, 64, 65, 0, 1, 33, 20, 40],          # 35.75 rows a group: tiles of 64
+                                   [127, 128, 129, 0, 64, 65, 100, 155],    # 96: tiles of 128
+                                   [127, 128, 129, 0, 64, 65, 100, 156]])   # above: tiles of 256
+@pytest.mark.parametrize("d,F", [(272, 144), (2816, 1424)])  # few feature tiles (always 64), and enough for every pair
+def test_tile_heights_by_the_default_rule(sizes, d, F):
+    _check_groups(sizes, d, F, False)
