@@ -200,7 +200,7 @@ struct GroupedGemmArgs {
   DeviceError* err;
   int max_rows;  // upper bound on total rows (sizes nothing; used by the checking kernel's grid)
   const PairRowMaps* pair_rows;  // CTA-pair kernel only (host pointer, copied at the launch)
-  int pair_tokens;  // ... token rows of a tile at most: 64, 128, else 256 (pair_tokens_of)
+  int pair_tokens;  // ... token rows of a tile at most: 64, 128, 192, else 256 (pair_tokens_of)
   int w8;        // B matrices are int8 (tensor maps of bytes), widened to bf16 inside the kernel
   float* splitk_ws;  // W8 tensor-memory kernel: workspace for stream-K partial sums (null: whole tiles only)
   // stream-K decode kernels: zeroed counters [kSplitKMaxTiles * 8] with which the kernel finishes the split

@@ -7,15 +7,15 @@
 // tcgen05.mma.cta_group::2 (M256 x Nn x K16), which reads both operands from both CTAs' shared memory.
 //
 // Why transposed: the M side of an MMA costs 256 rows however few hold data, the N side costs what it is
-// wide.  A group of R rows is cut into ceil(R / 256) (128, 64) equal token tiles rounded up to 16 rows, so the padding
+// wide.  A group of R rows is cut into ceil(R / 256) (192, 128, 64) equal token tiles rounded up to 16 rows, so the padding
 // is below 16 rows per tile.
 //
 //   kSwiGLU : 256 weight rows = 128 features; a CTA's 128 rows are 64 rows of W_gate and the same 64 of W_up,
 //             so the epilogue warps of lane quarters q and q + 2 hold gate and up of the same features and
 //             exchange them through shared memory (f32), each finishing half of the tokens
 //   kPlain  : 256 weight rows = 256 features
-//   k-block : 64 (one 128-byte swizzle row): 16 KiB of weights + 16, 8 or 4 KiB of tokens per CTA (tiles of at most 256, 128
-//             or 64 token rows, the launch's choice: pair_tokens_of), 6, 8 or 10 stages
+//   k-block : 64 (one 128-byte swizzle row): 16 KiB of weights + 16, 12, 8 or 4 KiB of tokens per CTA (tiles of at most 256,
+//             192, 128 or 64 token rows, the launch's choice: pair_tokens_of), 6, 7, 8 or 10 stages
 //
 // What bounds it: below some hundred rows per group HBM's latency, that is, the weights in flight (10 stages hold 160 KiB per
 // SM: 16 tokens of the Mixtral shape 451 -> 422 us against 6 stages), above the tensor pipe and the board's power.  ncu, DeepSeek-V2-Lite shape, 8192 tokens, gate/up: the
@@ -51,7 +51,7 @@ template <int TOK>
 struct PairRing {
   static constexpr int X_BYTES = (TOK / 2) * BK * 2;  // this CTA's half of the token tile
   static constexpr int STAGE_BYTES = W_BYTES2 + X_BYTES;
-  static constexpr int STAGES = TOK == 256 ? 6 : TOK == 128 ? 8 : 10;
+  static constexpr int STAGES = TOK == 256 ? 6 : TOK == 192 ? 7 : TOK == 128 ? 8 : 10;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES2 + 1024 + 256;
   static_assert(STAGES <= MAX_STAGES2 && STAGE_BYTES % 1024 == 0 && SMEM_BYTES <= 225 * 1024, "");
 };
@@ -457,6 +457,7 @@ template <int MODE>
 int launch_2cta_tokens(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   if (a.pair_tokens == 64) return launch_2cta_one<MODE, 64>(a, num_sms, s);
   if (a.pair_tokens == 128) return launch_2cta_one<MODE, 128>(a, num_sms, s);
+  if (a.pair_tokens == 192) return launch_2cta_one<MODE, 192>(a, num_sms, s);
   return launch_2cta_one<MODE, kPairTokens>(a, num_sms, s);
 }
 

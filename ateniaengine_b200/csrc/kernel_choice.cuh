@@ -51,7 +51,7 @@ inline Bf16Kernel bf16_product_kernel(int rows, int groups, int k, bool beside) 
   return (int64_t)rows >= (int64_t)512 * groups ? kBf16PairRows : kBf16Single;
 }
 
-// Token rows of the CTA-pair kernel's tiles at most, and with them the depth of its ring: 256 (6 stages), 128 (8) or 64 (10).
+// Token rows of the CTA-pair kernel's tiles at most, and with them the depth of its ring: 256 (6 stages), 192 (7), 128 (8) or 64 (10).
 // With few rows per group the kernel streams weights, and what limits that is the bytes in flight (a stage holds 16 KiB of
 // weights per SM and 128, 64 or 32 token rows); a group of more rows than the tile passes its weights through twice.
 // One forward on a B200, 256 / 128 / 64, us (rows a group):
@@ -60,6 +60,10 @@ inline Bf16Kernel bf16_product_kernel(int rows, int groups, int k, bool beside) 
 //   60 of 2048 x 1408, shared   16 (1) 147 / 138 / 137, 150 (10) 209 / 197 / 195, 220 (15) 217 / 201 / 203, 333 (22) 237 / 223 / 228,
 //                               1300 (87) 309 / 297 / 380, 1500 (100) 315 / 296 / 370, 1700 (113) 351 / 356 / 423
 //   64 of 2048 x 1408, shared   61 (6) 205 / 196 / 196, 300 (28) 227 / 218 / 218, 900 (84) 272 / 269 / 317, 1300 (122) 306 / 310 / 380
+// ... and 256 / 192 / 128: 8 experts of 4096 x 14336, 350 tokens (87) 501 / 493 / 490, 400 (100) 512 / 502 / 543, 500 (125)
+// 594 / 549 / 606, 600 (150) 618 / 674 / 651; 60 of 2048 x 1408, 1300 (87) 297 / 292 / 292, 1700 (113) 341 / 334 / 337, 2048
+// (137) 372 / 372 / 410, 2500 (167) 429 / 442 / 491; 64, 1300 (122) 305 / 302 / 305, 1700 (159) 343 / 335 / 380, 2000 (187) 389
+// / 415 / 435.
 // A product of so few tiles that pairs of SMs go without one takes the smallest (8 experts of 512 x 1408, 600 / 1000 tokens
 // 38.3 / 35.2 / 35.2, 42.6 / 37.7 / 37.5).
 inline int pair_tokens_of(int rows, int groups, int f_tiles) {
@@ -68,7 +72,7 @@ inline int pair_tokens_of(int rows, int groups, int f_tiles) {
   if (groups == 1) return rows <= 64 ? 64 : rows <= 128 ? 128 : 256;
   const int64_t r = rows, g = groups;
   if (r <= 12 * g || (g <= 16 && r <= 36 * g)) return 64;
-  return r <= 96 * g ? 128 : 256;
+  return r <= 88 * g ? 128 : r <= 140 * g ? 192 : 256;
 }
 
 }  // namespace atenia

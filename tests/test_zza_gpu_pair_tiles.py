@@ -94,8 +94,9 @@ def _check_groups(sizes, d, F, int8):
 
 
 @pytest.mark.parametrize("sizes", [[63, 64, 65, 0, 1, 33, 20, 40],          # 35.75 rows a group: tiles of 64
-                                   [127, 128, 129, 0, 64, 65, 100, 155],    # 96: tiles of 128
-                                   [127, 128, 129, 0, 64, 65, 100, 156]])   # above: tiles of 256
+                                   [127, 128, 129, 0, 64, 65, 100, 91],     # 88: tiles of 128
+                                   [191, 192, 193, 0, 64, 65, 100, 315],    # 140: tiles of 192
+                                   [191, 192, 193, 0, 64, 65, 100, 316]])   # above: tiles of 256
 @pytest.mark.parametrize("d,F", [(272, 144), (2816, 1424)])  # few feature tiles (always 64), and enough for every pair
 def test_tile_heights_by_the_default_rule(sizes, d, F):
     _check_groups(sizes, d, F, False)
