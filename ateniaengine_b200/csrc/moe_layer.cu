@@ -743,7 +743,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   // The shared expert needs only this call's tokens, so its GEMMs run on the layer's second stream from
   // the start of the forward, beside the routing phase (an FP64-bound router, an HBM-bound gather: the
   // tensor cores are idle there) and, under expert parallelism, beside the exchanges; the combine waits
-  // for them.  f32 input is converted to bf16 first.  Calls of the matrix-vector kernel keep the one-stream
+  // for them.  f32 input is converted to bf16 there first.  Calls of the matrix-vector kernel keep the one-stream
   // order: there the two event hops cost what the overlap gives (DeepSeek-V2-Lite shape, 1 token: 89.3 us aside,
   // 88.6 in order; 3 tokens 99 / 126, 61 tokens 229 / 253; Qwen1.5-MoE shape, 16 tokens 172 / 198).
   // ATENIA_MOE_SHARED_ASIDE=0 turns it off.
@@ -757,13 +757,13 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   L->gemm_chained = L->chained && !shared_aside;
   if (shared_aside) {
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
-    if (x_f32) {
-      rc0 = launch_f32_to_bf16(static_cast<const float*>(x), L->x_bf16, (int64_t)T * c.d_model, s);
+    ATENIA_CUDA_TRY(cudaEventRecord(L->ev_fork, s));
+    ATENIA_CUDA_TRY(cudaStreamWaitEvent(L->aux_stream, L->ev_fork, 0));
+    if (x_f32) {  // (there too: the router reads x itself and need not wait for the copy)
+      rc0 = launch_f32_to_bf16(static_cast<const float*>(x), L->x_bf16, (int64_t)T * c.d_model, L->aux_stream);
       if (rc0) return rc0;
       xb = L->x_bf16;
     }
-    ATENIA_CUDA_TRY(cudaEventRecord(L->ev_fork, s));
-    ATENIA_CUDA_TRY(cudaStreamWaitEvent(L->aux_stream, L->ev_fork, 0));
     // (the dispatch kernels, which write the one-group offsets {0, T} otherwise, run later on `s`)
     rc0 = launch_set_pair(L->shared_offsets, 0, T, L->aux_stream);
     if (rc0) return rc0;
