@@ -201,6 +201,15 @@ struct GroupedGemmArgs {
   int max_rows;  // upper bound on total rows (sizes nothing; used by the checking kernel's grid)
   const PairRowMaps* pair_rows;  // CTA-pair kernel only (host pointer, copied at the launch)
   int pair_tokens;  // ... token rows of a tile at most: 64, 128, 192, else 256 (pair_tokens_of)
+  // CTA-pair kernel only: one more group in the same launch, with its own matrices, rows, sizes and output (the shared
+  // expert beside the routed ones).  rows 0: none.
+  struct Extra {
+    const PairRowMaps* x_rows;  // host pointer, copied at the launch
+    const CUtensorMap* tmap_b0;
+    const CUtensorMap* tmap_b1;
+    __nv_bfloat16* out;
+    int rows, N, K;
+  } extra;
   int w8;        // B matrices are int8 (tensor maps of bytes), widened to bf16 inside the kernel
   float* splitk_ws;  // W8 tensor-memory kernel: workspace for stream-K partial sums (null: whole tiles only)
   // stream-K decode kernels: zeroed counters [kSplitKMaxTiles * 8] with which the kernel finishes the split

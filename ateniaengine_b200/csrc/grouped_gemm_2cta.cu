@@ -31,6 +31,8 @@
 // Barriers: full[s] lives in the leader and collects the bytes of both CTAs; empty[s] and
 // acc_full[b] exist in both CTAs and are signalled by tcgen05.commit with a CTA mask; acc_empty[b]
 // lives in the leader and is arrived on by the epilogue warps of both CTAs.
+#include <type_traits>
+
 #include "tc_common.cuh"
 
 namespace atenia {
@@ -169,11 +171,22 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
       : "memory");
 }
 
-template <int MODE, int TOK>
+// One more group in the launch (GroupedGemmArgs::Extra): its tiles come first.
+struct PairExtra {
+  PairRowMaps x;
+  const CUtensorMap* w0;
+  const CUtensorMap* w1;
+  __nv_bfloat16* out;
+  int rows, N, K;
+};
+struct NoExtra {};
+
+template <int MODE, int TOK, bool EX>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS2, 1)
 grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUtensorMap* __restrict__ tmap_w0,
                          const CUtensorMap* __restrict__ tmap_w1, const int32_t* __restrict__ group_offsets_g,
-                         int num_groups, int N, int K, __nv_bfloat16* __restrict__ out, DeviceError* err) {
+                         int num_groups, int N, int K, __nv_bfloat16* __restrict__ out, DeviceError* err,
+                         const __grid_constant__ std::conditional_t<EX, PairExtra, NoExtra> ex) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int32_t goff_s[kMaxGroupsShared + 1];
   constexpr int F_CTA = (MODE == kSwiGLU) ? BM / 2 : BM;  // output features per CTA
@@ -227,24 +240,65 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
   cur.base = 0;
   if (num_groups > 0) pair_cursor_load<TOK>(cur, group_offsets);
   PairTile tc;
+  int ex_tiles = 0, ex_m = 1, ex_rows = 16, ex_kb = 0, ex_full = 0, ex_rest = 0, ex_weight = 1;
+  if constexpr (EX) {
+    ex_m = pair_tiles(ex.rows, TOK);
+    ex_rows = pair_tile_rows(ex.rows, ex_m);
+    ex_tiles = ex_m * ((ex.N + F_PAIR - 1) / F_PAIR);
+    ex_kb = (ex.K + BK - 1) / BK;
+    ex_full = ex_tiles / num_pairs;
+    ex_rest = ex_tiles - ex_full * num_pairs;
+    ex_weight = max(1, (ex_kb + num_kb / 2) / num_kb);
+  }
+  // This pair's i-th tile; false past its last.  Tiles are dealt round by round, the extra group's (group -1) first; where they
+  // are longer than the others, the pairs that have one in the last of their rounds miss as many rounds as it lasts.
+  auto seek = [&](PairCursor& c, int i) {
+    int tile = pair + i * num_pairs;
+    if constexpr (EX) {
+      const int m = i - ex_full;  // rounds after the full ones
+      if (m < 0 || (m == 0 && pair < ex_rest)) {
+        const int ft = tile / ex_m, mt = tile - ft * ex_m;
+        tc.group = -1;
+        tc.row0 = mt * ex_rows;
+        tc.rows = min(ex.rows - tc.row0, ex_rows);
+        tc.n = pair_tile_n(tc.rows);
+        tc.f0 = ft * F_PAIR;
+        return true;
+      }
+      const int others = num_pairs - ex_rest, late = ex_weight * others;
+      tile = pair < ex_rest ? late + (m - 1) * num_pairs + pair
+             : m < ex_weight ? m * others + pair - ex_rest : late + (m - ex_weight) * num_pairs + pair;
+    }
+    return pair_cursor_seek<TOK>(c, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
+  };
+  auto k_blocks = [&] { return EX && tc.group < 0 ? ex_kb : num_kb; };
+  auto weights0 = [&] {
+    if constexpr (EX) return tc.group < 0 ? ex.w0 : &tmap_w0[tc.group];
+    else return &tmap_w0[tc.group];
+  };
+  auto weights1 = [&] {
+    if constexpr (EX) return tc.group < 0 ? ex.w1 : &tmap_w1[tc.group];
+    else return &tmap_w1[tc.group];
+  };
 
   if (warp == 0) {
     // ================= TMA producer (both CTAs) =================
     int stage = 0;
     uint32_t phase = 0;
-    int last_group = -1;
+    int last_group = -2;
     uint32_t armed = 0;  // stages with a copy possibly in flight
     bool ok = true;
     // Weights of the first tile's first k-blocks; their token rows follow after the wait.  B200, 64 tokens of a 512-wide
     // layer 37.7 -> 33.9 us, 256 Mixtral tokens 507 -> 497.
     int ahead = 0;
-    if (PairCursor c0 = cur; pair_cursor_seek<TOK>(c0, pair, f_tiles, num_groups, group_offsets, tc, F_PAIR)) {
-      const CUtensorMap* m0 = &tmap_w0[tc.group];
-      const CUtensorMap* m1 = MODE == kSwiGLU ? &tmap_w1[tc.group] : m0;
+    if (PairCursor c0 = cur; seek(c0, 0)) {
+      const CUtensorMap* m0 = weights0();
+      const CUtensorMap* m1 = MODE == kSwiGLU ? weights1() : m0;
       tmap_acquire(m0);
       if (MODE == kSwiGLU) tmap_acquire(m1);
       last_group = tc.group;
-      ahead = num_kb < STAGES2 ? num_kb : STAGES2;
+      const int nkb = k_blocks();
+      ahead = nkb < STAGES2 ? nkb : STAGES2;
       const uint32_t tx = 2 * (W_BYTES2 + pair_box_rows(pair_tile_box(tc.n)) * BK * 2);
       const int f_row = tc.f0 + (int)rank * F_CTA;
       for (int kb = 0; kb < ahead; ++kb) {
@@ -257,10 +311,9 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
       }
     }
     chain_wait();
-    for (int tile = pair; ok && pair_cursor_seek<TOK>(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
-         tile += num_pairs) {
-      const CUtensorMap* m0 = &tmap_w0[tc.group];
-      const CUtensorMap* m1 = MODE == kSwiGLU ? &tmap_w1[tc.group] : m0;
+    for (int i = 0; ok && seek(cur, i); ++i) {
+      const CUtensorMap* m0 = weights0();
+      const CUtensorMap* m1 = MODE == kSwiGLU ? weights1() : m0;
       if (tc.group != last_group) {
         tmap_acquire(m0);
         if (MODE == kSwiGLU) tmap_acquire(m1);
@@ -268,10 +321,14 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
       }
       const int box = pair_tile_box(tc.n);
       const CUtensorMap* mx = &tmaps_x.box[box];
+      if constexpr (EX) {
+        if (tc.group < 0) mx = &ex.x.box[box];
+      }
+      const int nkb = k_blocks();
       const int f_row = tc.f0 + (int)rank * F_CTA;
       const int x_row = tc.row0 + (int)rank * (tc.n / 2);
       const uint32_t tx = 2 * (W_BYTES2 + pair_box_rows(box) * BK * 2);  // bytes of both CTAs
-      for (int kb = 0; kb < num_kb; ++kb) {
+      for (int kb = 0; kb < nkb; ++kb) {
         const uint32_t full_local = smem_u32(&bars->full[stage]);
         const uint32_t full_leader = mapa(full_local, 0);
         const uint32_t dst = smem_base + stage * STAGE_BYTES2;
@@ -315,9 +372,9 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
       uint32_t acc_phase = 0;  // bit b: accumulator b
       int it = 0;
       bool ok = true;
-      for (int tile = pair; ok && pair_cursor_seek<TOK>(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
-           tile += num_pairs, ++it) {
+      for (; ok && seek(cur, it); ++it) {
         const int acc = it & 1;
+        const int nkb = k_blocks();
         if (!mbar_wait(smem_u32(&bars->acc_empty[acc]), ((acc_phase >> acc) & 1u) ^ 1u, abort_flag)) {
           if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1200 + acc);
           *abort_flag = 1;
@@ -329,7 +386,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN2;
         const uint32_t idesc = kInstrDesc2 | (uint32_t(tc.n >> 3) << 17);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag)) {
             if (lane == 0) report_error(err, ATENIA_ERR_DEVICE_TIMEOUT, 1300 + stage);
             *abort_flag = 1;
@@ -368,8 +425,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
     int flip = 0;
     uint32_t acc_phase = 0;
     int it = 0;
-    for (int tile = pair; pair_cursor_seek<TOK>(cur, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
-         tile += num_pairs, ++it) {
+    for (; seek(cur, it); ++it) {
       const int acc = it & 1;
       bool ready = mbar_wait(smem_u32(&bars->acc_full[acc]), (acc_phase >> acc) & 1u, abort_flag);
       __syncwarp();  // (each lane polled by itself; the barriers and tensor-memory loads below want the warp as one)
@@ -394,16 +450,24 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
       acc_phase ^= 1u << acc;
       tc_fence_after();
       const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc * TN2;
-      const bool f_ok = tc.f0 + f_lane < N;
+      int ld = N;
+      __nv_bfloat16* base = out;
+      if constexpr (EX) {
+        if (tc.group < 0) {
+          ld = ex.N;
+          base = ex.out;
+        }
+      }
+      const bool f_ok = tc.f0 + f_lane < ld;
       const int t_half = up ? 8 : 0;
-      __nv_bfloat16* dst = out + (size_t)(tc.row0 + t_half) * N + tc.f0 + f_lane;
+      __nv_bfloat16* dst = base + (size_t)(tc.row0 + t_half) * ld + tc.f0 + f_lane;
       const int rows = f_ok ? tc.rows - t_half : 0;  // tokens of the tile this lane may store
 #pragma unroll 1
       for (int c = 16 * first; c < tc.n; c += 32) {
         uint32_t v[16];
         tc_ld16(taddr + c, v);
         tc_ld_wait();
-        __nv_bfloat16* d = dst + (size_t)c * N;
+        __nv_bfloat16* d = dst + (size_t)c * ld;
         if (MODE == kSwiGLU) {
           float* ex = mine + flip * 256;
 #pragma unroll
@@ -416,12 +480,12 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
             const float o = ox[j * 32 + lane];
             const float g = up ? o : __uint_as_float(v[j]);
             const float u = up ? __uint_as_float(v[8 + j]) : o;
-            if (c + j < rows) d[(size_t)j * N] = __float2bfloat16(silu_mul(g, u));
+            if (c + j < rows) d[(size_t)j * ld] = __float2bfloat16(silu_mul(g, u));
           }
         } else {
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (c + j < rows) d[(size_t)j * N] = __float2bfloat16(__uint_as_float(v[j]));
+            if (c + j < rows) d[(size_t)j * ld] = __float2bfloat16(__uint_as_float(v[j]));
         }
       }
       tc_fence_before();
@@ -441,16 +505,25 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
   }
 }
 
-template <int MODE, int TOK>
-int launch_2cta_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
+template <int MODE, int TOK, bool EX, typename E>
+int launch_2cta_form(const GroupedGemmArgs& a, int num_sms, cudaStream_t s, const E& ex) {
   static bool attr_set[kMaxDevices] = {};
   if (first_use_on_current_device(attr_set)) {
-    ATENIA_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_2cta_kernel<MODE, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    ATENIA_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_2cta_kernel<MODE, TOK, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          PairRing<TOK>::SMEM_BYTES));
   }
   const int grid = num_sms & ~1;  // whole pairs
-  return launch_chained(a.chained, grouped_gemm_2cta_kernel<MODE, TOK>, dim3(grid), dim3(NUM_THREADS2), PairRing<TOK>::SMEM_BYTES, s, *a.pair_rows, a.tmap_b0,
-                        MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0, a.group_offsets, a.num_groups, a.N, a.K, a.out, a.err);
+  return launch_chained(a.chained, grouped_gemm_2cta_kernel<MODE, TOK, EX>, dim3(grid), dim3(NUM_THREADS2),
+                        PairRing<TOK>::SMEM_BYTES, s, *a.pair_rows, a.tmap_b0, MODE == kSwiGLU ? a.tmap_b1 : a.tmap_b0,
+                        a.group_offsets, a.num_groups, a.N, a.K, a.out, a.err, ex);
+}
+
+template <int MODE, int TOK>
+int launch_2cta_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
+  if (a.extra.rows <= 0) return launch_2cta_form<MODE, TOK, false>(a, num_sms, s, NoExtra{});
+  const PairExtra ex{*a.extra.x_rows, a.extra.tmap_b0, MODE == kSwiGLU ? a.extra.tmap_b1 : a.extra.tmap_b0, a.extra.out,
+                     a.extra.rows, a.extra.N, a.extra.K};
+  return launch_2cta_form<MODE, TOK, true>(a, num_sms, s, ex);
 }
 
 template <int MODE>
@@ -474,6 +547,7 @@ int launch_grouped_gemm_2cta(const GroupedGemmArgs& a, int num_sms, cudaStream_t
   if (a.num_groups <= 0) return ATENIA_OK;
   if (a.N % 16 != 0 || a.K % 16 != 0 || a.num_groups > kMaxGroupsShared) return ATENIA_ERR_SHAPE;
   if (!a.pair_rows) return ATENIA_ERR_NULL;
+  if (a.extra.rows > 0 && (a.extra.N % 16 != 0 || a.extra.K % 16 != 0)) return ATENIA_ERR_SHAPE;
   if (a.w8) return ATENIA_ERR_UNSUPPORTED;  // INT8 weights: w8_gemm.cu / w8_gemm_m256.cu
   int rc = a.mode == kSwiGLU ? launch_2cta_tokens<kSwiGLU>(a, num_sms, s) : launch_2cta_tokens<kPlain>(a, num_sms, s);
   count_launch();

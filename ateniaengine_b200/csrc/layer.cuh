@@ -176,7 +176,10 @@ bool ep_ready(const AteniaMoeLayer* L);
 // ATENIA_ERR_NCCL, so a collective whose peer never arrives cannot block the host for ever.
 int ep_bounded_wait(AteniaMoeLayer* L, cudaStream_t s);
 void ep_destroy(AteniaMoeLayer* L);
+// shared_T > 0: the launches take the shared expert's group with them, shared_T rows described by shared_x (one GPU, bf16,
+// both products on the CTA-pair kernel: merges_shared)
 int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_mid,
                      const __nv_bfloat16* a_ptr, __nv_bfloat16* mid, __nv_bfloat16* out,
-                     const int32_t* group_offsets, int num_groups, int max_rows, cudaStream_t s);
+                     const int32_t* group_offsets, int num_groups, int max_rows, cudaStream_t s,
+                     const PairRowMaps* shared_x = nullptr, int shared_T = 0);
 }  // namespace atenia

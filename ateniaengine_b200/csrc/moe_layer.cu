@@ -64,11 +64,27 @@ int launch_bf16_product(Bf16Kernel kernel, const GroupedGemmArgs& a, int num_sms
                                    : launch_grouped_gemm_tcgen05(a, num_sms, s);
 }
 
+// Do the routed GEMMs of a forward of T tokens take the shared expert with them, one more group of the same two launches?
+// It saves two launches and the fork, every kernel of the forward is chained, and the shared expert's compute-bound tiles run
+// among weight streams.  It gives up running the shared expert beside the routing phase, which pays from some 1500 tokens on.
+// B200, on the second stream / merged, us: DeepSeek-V2-Lite shape 3 tokens 80.3 / 71.5, 16 156.9 / 146.9, 61 195.6 / 186.6, 300
+// 216.1 / 207.3, 1000 272.3 / 267.8, 2000 358.2 / 366.3; Qwen1.5-MoE shape 16 135.0 / 129.6, 64 184.5 / 179.0, 333 (block
+// step) 217.9 / 209.0, 1000 275.1 / 266.9, 1500 310.9 / 305.7, 2048 364.0 / 372.6.
+bool merges_shared(const AteniaMoeLayer* L, int T) {
+  const AteniaMoeConfig& c = L->cfg;
+  const int rows = T * c.experts_per_token;
+  if (c.weight_dtype != ATENIA_W_BF16 || c.ep_world > 1 || L->use_check_gemm || L->timing || T > 10 * L->num_sms) return false;
+  if (L->bf16_decode == 1 || (L->bf16_decode < 0 && rows <= 16)) return false;  // (the stream-K kernel's calls)
+  return bf16_kernel(L, rows, c.num_experts, c.d_model, false) == kBf16Pairs &&
+         bf16_kernel(L, rows, c.num_experts, c.d_ff, false) == kBf16Pairs;
+}
+
 }  // namespace
 
 int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_mid,
                      const __nv_bfloat16* a_ptr, __nv_bfloat16* mid, __nv_bfloat16* out,
-                     const int32_t* group_offsets, int num_groups, int max_rows, cudaStream_t s) {
+                     const int32_t* group_offsets, int num_groups, int max_rows, cudaStream_t s,
+                     const PairRowMaps* shared_x, int shared_T) {
   const AteniaMoeConfig& c = L->cfg;
   const bool q = c.weight_dtype == ATENIA_W_INT8_ROW;
   const bool large = max_rows >= 256 * num_groups;
@@ -182,6 +198,8 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     g1.w8 = q;
     g1.splitk_ws = L->splitk_ws;
     g1.splitk_cnt = L->splitk_cnt;
+    if (shared_T > 0)
+      g1.extra = {shared_x, L->d_tm_shared_box, L->d_tm_shared_box + 1, L->h_shared, shared_T, c.shared_d_ff, c.d_model};
     int rc = m256 ? launch_grouped_gemm_w8_m256(g1, L->num_sms, s)
                   : dec ? launch_grouped_gemm_bf16_decode(g1, L->num_sms, s)
                   : tmem ? launch_grouped_gemm_w8_tmem(g1, L->num_sms, s)
@@ -215,6 +233,8 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
     g2.w8 = q;
     g2.splitk_ws = L->splitk_ws;
     g2.splitk_cnt = L->splitk_cnt;
+    if (shared_T > 0)
+      g2.extra = {&L->tm_h_shared.pair, L->d_tm_shared + 2, nullptr, L->y_shared, shared_T, c.d_model, c.shared_d_ff};
     int rc = m256 ? launch_grouped_gemm_w8_m256(g2, L->num_sms, s)
                   : dec ? launch_grouped_gemm_bf16_decode(g2, L->num_sms, s)
                   : tmem ? launch_grouped_gemm_w8_tmem(g2, L->num_sms, s)
@@ -747,7 +767,10 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   // order: there the two event hops cost what the overlap gives (DeepSeek-V2-Lite shape, 1 token: 89.3 us aside,
   // 88.6 in order; 3 tokens 99 / 126, 61 tokens 229 / 253; Qwen1.5-MoE shape, 16 tokens 172 / 198).
   // ATENIA_MOE_SHARED_ASIDE=0 turns it off.
-  const bool shared_aside = L->has_shared && T > L->gemv_rows && L->aux_stream && L->shared_aside;
+  bool shared_aside = L->has_shared && T > L->gemv_rows && L->aux_stream && L->shared_aside;
+  // Up to some 1500 tokens the routed GEMMs take it with them instead (merges_shared).
+  const bool merged = shared_aside && merges_shared(L, T);
+  if (merged) shared_aside = false;
   // Blocks of a chained kernel sit on the SMs while they wait.  Beside a shared expert that is affordable up to about
   // four tokens per SM; from there on they keep its GEMMs out.  20 forwards after a pause, plain / chained routing kernels, us each:
   // DeepSeek-V2-Lite shape, 197 / 592 / 1578 tokens 233.9 / 228.0, 255.3 / 250.8, 313.7 / 340.1; Qwen1.5-MoE shape, 148 /
@@ -836,8 +859,15 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
 
   if (c.ep_world == 1) {
     if (L->timing) cudaEventRecord(L->ph[2], s);
+    PairRowMaps shared_x{};
+    if (merged) {
+      const __nv_bfloat16* xb = x_f32 ? L->x_bf16 : static_cast<const __nv_bfloat16*>(x);
+      const int tokens = pair_tokens_of(n, c.num_experts, pair_f_tiles(c.d_ff, kSwiGLU));
+      rc = encode_pair_rows(&shared_x, xb, (uint64_t)T, (uint64_t)c.d_model, pair_boxes_of_group(T, tokens));
+      if (rc) return rc;
+    }
     rc = run_expert_gemms(L, L->tm_x_perm, L->tm_h, L->x_perm, L->h, L->y_perm, L->expert_offsets,
-                          c.num_experts, n, s);
+                          c.num_experts, n, s, &shared_x, merged ? T : 0);
   } else if (L->ep_replicated) {
     rc = ep_forward_replicated(L, n, s);
   } else if (direct) {
@@ -855,7 +885,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
 
   if (shared_aside) {
     ATENIA_CUDA_TRY(cudaStreamWaitEvent(s, L->ev_join, 0));
-  } else if (L->has_shared && T > 0) {
+  } else if (L->has_shared && T > 0 && !merged) {
     const __nv_bfloat16* xb = x_f32 ? L->x_bf16 : static_cast<const __nv_bfloat16*>(x);
     rc = run_shared_gemms(L, xb, T, s);
     if (rc) return rc;

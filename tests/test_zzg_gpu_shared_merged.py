@@ -1,0 +1,64 @@
+"""The shared expert as one more group of the routed GEMMs' launches (bf16, up to ten tokens per SM) gives the bits it gives
+by launches of its own (ATENIA_MOE_SHARED_ASIDE=0: in order, after the routed experts): its width and k below and above
+the routed experts', token tiles of every height, k-blocks fewer than the ring, calls back to back and captured."""
+import pytest
+import torch
+
+from tests.test_gpu_parity import _synth, dev  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _layers(dev, monkeypatch, E, k, d, F, Fs, gated, T):
+    synth = _synth()
+    shape = synth.MoeShape("m", d, F, E, k, False, Fs, gated)
+    w = synth.make_weights(shape, E + Fs, dev)
+    merged = synth.build_layer(shape, w, max_tokens=T)
+    monkeypatch.setenv("ATENIA_MOE_SHARED_ASIDE", "0")
+    plain = synth.build_layer(shape, w, max_tokens=T)
+    monkeypatch.delenv("ATENIA_MOE_SHARED_ASIDE")
+    return shape, merged, plain
+
+
+# routed rows per group: 64-row tiles, 128, 192, 256; feature tiles fewer and more than pairs of SMs
+@pytest.mark.parametrize("E,k,d,F,Fs,gated", [(8, 2, 528, 400, 1040, True), (60, 4, 272, 144, 16, False),
+                                              (17, 4, 2064, 1040, 5632, True), (40, 2, 1040, 1424, 400, False)])
+@pytest.mark.parametrize("T", [9, 65, 257, 500, 1480])
+@pytest.mark.parametrize("io", [torch.bfloat16, torch.float32])
+def test_same_bits_as_launches_of_its_own(dev, monkeypatch, E, k, d, F, Fs, gated, T, io):
+    shape, merged, plain = _layers(dev, monkeypatch, E, k, d, F, Fs, gated, T)
+    x = _synth().make_activations(shape, T, dev, tokens=T, dtype=io)
+    want = plain.forward(x, out_dtype=torch.float32, sync=True)
+    outs = [torch.empty_like(want) for _ in range(4)]
+    for y in outs:  # nothing between the calls
+        merged.forward(x, out=y)
+    merged.check()
+    assert torch.isfinite(want).all() and want.abs().sum() > 0
+    assert all(torch.equal(y, want) for y in outs)
+
+
+def test_given_selections_with_empty_groups(dev, monkeypatch):
+    """All tokens on two experts, then on others: groups come and go, the shared rows stay."""
+    shape, merged, plain = _layers(dev, monkeypatch, 12, 2, 272, 1040, 528, False, 300)
+    for T, first in ((300, 0), (33, 10), (300, 5)):
+        x = _synth().make_activations(shape, first, dev, tokens=T)
+        idx = torch.tensor([[first, first + 1]], dtype=torch.int32, device=dev).repeat(T, 1)
+        w = torch.full((T, 2), 0.5, device=dev)
+        assert torch.equal(merged.forward_selected(x, idx, w, out_dtype=torch.float32), plain.forward_selected(x, idx, w, out_dtype=torch.float32))
+
+
+def test_captured(dev, monkeypatch):
+    shape, merged, plain = _layers(dev, monkeypatch, 24, 4, 528, 400, 1040, True, 200)
+    x = _synth().make_activations(shape, 1, dev, tokens=200, dtype=torch.float32)
+    want = plain.forward(x, sync=True)
+    out = torch.empty_like(want)
+    merged.forward(x, out=out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        merged.forward(x, out=out)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
