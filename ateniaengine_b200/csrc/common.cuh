@@ -112,11 +112,12 @@ struct RouterArgs {
   const CUtensorMap* digit_map;  // integer router (router_i8.cu): digit planes of the router matrix (host pointer; null:
   const double* digit_scale;     // the layer has none) and the scale of each of its rows
   bool chained;        // see launch_chained
+  bool beside;         // a shared expert's GEMMs run on another stream meanwhile
 };
 int launch_router(const RouterArgs& a, cudaStream_t s);
 int launch_router_dmma(const RouterArgs& a, cudaStream_t s);  // same contract, E <= 128, k <= 8
 int launch_router_splitk(const RouterArgs& a, cudaStream_t s);  // same contract
-bool router_splitk_pays(int T, int E, int d);
+bool router_splitk_pays(int T, int E, int d, bool beside);
 constexpr int kSplitkPinnedTokens = 1024;
 // Integer router of bf16 activations: layers of at most 64 rows of w (experts, and the gate vector if the call wants it).
 // planes [kRouterDigitPlanes][kRouterDigitRows][d] int8, map with box {128, kRouterDigitPlanes * kRouterDigitRows / 2} and

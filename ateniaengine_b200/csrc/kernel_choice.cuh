@@ -64,11 +64,12 @@ inline Bf16Kernel bf16_product_kernel(int rows, int groups, int k, bool beside) 
 // 594 / 549 / 606, 600 (150) 618 / 674 / 651; 60 of 2048 x 1408, 1300 (87) 297 / 292 / 292, 1700 (113) 341 / 334 / 337, 2048
 // (137) 372 / 372 / 410, 2500 (167) 429 / 442 / 491; 64, 1300 (122) 305 / 302 / 305, 1700 (159) 343 / 335 / 380, 2000 (187) 389
 // / 415 / 435.
-// A product of so few tiles that pairs of SMs go without one takes the smallest (8 experts of 512 x 1408, 600 / 1000 tokens
-// 38.3 / 35.2 / 35.2, 42.6 / 37.7 / 37.5).
+// A product whose tiles all run at once takes the lowest that still do (8 experts of 512 x 1408, 600 / 1000 tokens 38.3 / 35.2 /
+// 35.2, 42.6 / 37.7 / 37.5; but 333 rows of one group over 22 feature tiles, two rounds of 64-row tiles, 67.2 / - / 73.4).
 inline int pair_tokens_of(int rows, int groups, int f_tiles) {
-  constexpr int kPairs = 74;
-  if ((int64_t)f_tiles * (groups + rows / 128) <= kPairs) return 64;
+  constexpr int64_t kPairs = 74;
+  for (int t = 64; t <= 128; t += 64)
+    if (f_tiles * (int64_t)(groups == 1 ? (rows + t - 1) / t : groups + rows / t) <= kPairs) return t;
   if (groups == 1) return rows <= 64 ? 64 : rows <= 128 ? 128 : 256;
   const int64_t r = rows, g = groups;
   if (r <= 12 * g || (g <= 16 && r <= 36 * g)) return 64;

@@ -74,6 +74,7 @@ bool merges_shared(const AteniaMoeLayer* L, int T) {
   const AteniaMoeConfig& c = L->cfg;
   const int rows = T * c.experts_per_token;
   if (c.weight_dtype != ATENIA_W_BF16 || c.ep_world > 1 || L->use_check_gemm || L->timing || T > 10 * L->num_sms) return false;
+  if (rows > 140 * c.num_experts) return false;  // (groups that fill their tiles: the GEMMs are compute-bound themselves)
   if (L->bf16_decode == 1 || (L->bf16_decode < 0 && rows <= 16)) return false;  // (the stream-K kernel's calls)
   return bf16_kernel(L, rows, c.num_experts, c.d_model, false) == kBf16Pairs &&
          bf16_kernel(L, rows, c.num_experts, c.d_ff, false) == kBf16Pairs;
@@ -815,6 +816,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   ra.digit_map = L->rd_planes ? &L->tm_rd : nullptr;
   ra.digit_scale = L->rd_scale;
   ra.chained = chained;
+  ra.beside = shared_aside;
   int rc = launch_router(ra, s);
   if (rc) return rc;
   if (v3) {

@@ -361,7 +361,7 @@ int launch_router(const RouterArgs& a, cudaStream_t s) {
   if (a.k > kMaxK || a.E > 128) return ATENIA_ERR_UNSUPPORTED;
   // variant -1: choose by size
   if (a.variant == -1 && router_i8_pays(a)) return launch_router_i8(a, s);
-  if (a.variant == 2 ? a.T <= kSplitkPinnedTokens && a.d % 16 == 0 : a.variant == -1 && router_splitk_pays(a.T, a.E, a.d))
+  if (a.variant == 2 ? a.T <= kSplitkPinnedTokens && a.d % 16 == 0 : a.variant == -1 && router_splitk_pays(a.T, a.E, a.d, a.beside))
     return launch_router_splitk(a, s);
   if (a.variant == 1 || (a.variant == -1 && a.d % 16 == 0)) return launch_router_dmma(a, s);
   dim3 block(kRWarps * 32);

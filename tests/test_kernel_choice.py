@@ -101,4 +101,6 @@ def test_pair_tile_height_is_near_the_fastest_measured(lib, rows, groups, f_tile
 
 def test_pair_tile_height_of_one_group_holds_it_whole(lib):
     assert [lib.choice_pair_tokens(r, 1, 100) for r in (1, 64, 65, 128, 129, 4096)] == [64, 64, 128, 128, 256, 256]
-    assert lib.choice_pair_tokens(4096, 8, 1) == 64  # fewer tiles than pairs of SMs
+    # tiles that all run at once: the lowest that do
+    assert [lib.choice_pair_tokens(*a) for a in ((4096, 8, 1), (333, 1, 12), (333, 1, 13), (333, 1, 22), (333, 1, 25))] == [
+        64, 64, 128, 128, 256]
