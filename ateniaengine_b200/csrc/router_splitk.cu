@@ -14,7 +14,8 @@
 //   128 experts, d 2048  8 tokens 18.0 / 9.3, 256 34.6 / 13.3, 512 34.6 / 20.3, 2048 70.1 / 58.7
 // Between 513 and 1184 tokens one CTA per eight tokens (router_dmma.cu) is as fast (64 experts, 1000 tokens 19.6 / 22 and
 // more), above 2368 its form of 16 tokens per CTA is (4096 tokens 54 / 58), and for a router matrix of 4096 words or less
-// it needs no cluster barriers (8 experts, d 512, 64 tokens 3.6 / 4.3).  Clusters of one fill the register files, which keeps a
+// it needs no cluster barriers (8 experts, d 512, 64 tokens 3.6 / 4.3); nor does one of under 32768 words above 128 tokens
+// (forwards of 16 INT8 experts of d 1024, 256 / 500 tokens 84.5 / 86.5, 90.5 / 92.7).  Clusters of one fill the register files, which keeps a
 // shared expert's GEMMs off the SMs (64 INT8 experts, f32, 1500 tokens 432 / 446 a forward): not beside one.  router_splitk_pays.
 #include "dmma.cuh"
 #include "route_warp.cuh"
@@ -218,8 +219,10 @@ int launch_one(const RouterArgs& a, cudaStream_t s) {
 }  // namespace
 
 bool router_splitk_pays(int T, int E, int d, bool beside) {
-  if (d % 16 != 0 || (int64_t)E * d <= 4096) return false;
-  return T <= kSkFewTokens || (!beside && T > 8 * 148 && T <= 16 * 148);
+  const int64_t words = (int64_t)E * d;
+  if (d % 16 != 0 || words <= 4096) return false;
+  if (T <= kSkFewTokens) return T <= 128 || words >= 1 << 15;
+  return !beside && T > 8 * 148 && T <= 16 * 148;
 }
 
 int launch_router_splitk(const RouterArgs& a, cudaStream_t s) {
