@@ -20,7 +20,7 @@ def _stale(out, deps):
 
 
 def build(force=False, verbose=False):
-    headers = [os.path.join(HERE, h) for h in ("common.cuh", "layer.cuh", "tc_common.cuh", "v3_route.cuh", "route_warp.cuh", "dmma.cuh", "round_codes.cuh", "ep_plan.cuh", "pair_tiles.cuh", "kernel_choice.cuh")] + [
+    headers = [os.path.join(HERE, h) for h in ("common.cuh", "layer.cuh", "tc_common.cuh", "v3_route.cuh", "route_warp.cuh", "dmma.cuh", "router_digits.cuh", "round_codes.cuh", "ep_plan.cuh", "pair_tiles.cuh", "kernel_choice.cuh")] + [
         os.path.join(HERE, "..", "..", "include", "atenia_moe.h")]
     objs = []
     jobs = []

@@ -109,8 +109,8 @@ struct RouterArgs {
   DeviceError* err;
   int variant;         // -1: by size; 0: CUDA-core f64 kernel (router.cu); 1: f64 tensor-core kernel
                        // (router_dmma.cu); 2: split-k kernel (router_splitk.cu) up to kSplitkPinnedTokens
-  const CUtensorMap* digit_map;  // integer router (router_i8.cu): digit planes of the router matrix (host pointer; null:
-  const double* digit_scale;     // the layer has none) and the scale of each of its rows
+  const CUtensorMap* digit_map;  // integer router (router_i8.cu): digit planes of the router matrix (host pointer; null: the
+  const double* digit_scale;     // layer has none that hold it exactly) and the scale of each of its rows (NaN: row not held)
   bool chained;        // see launch_chained
   bool beside;         // a shared expert's GEMMs run on another stream meanwhile
 };

@@ -50,6 +50,7 @@ struct AteniaMoeLayer {
   float* d_router = nullptr;    // [E, d]
   int8_t* rd_planes = nullptr;  // integer router: digit planes of the router matrix and the gate vector, their scales
   double* rd_scale = nullptr;
+  bool rd_exact = false;        // every row is on its grid (else: the f64 routers)
   CUtensorMap tm_rd{};
   float* d_bias = nullptr;      // [E]
   float* d_gate_vec = nullptr;  // [d]

@@ -1,5 +1,6 @@
 // C ABI of the MoE block: layer life cycle, weight binding, the forward pass.
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -603,6 +604,10 @@ int atenia_moe_set_weights(AteniaMoeLayer* L, const AteniaMoeWeights* w) {
     int rrc = launch_router_digits(L->d_router, L->gate_vec_bound ? L->d_gate_vec : nullptr, c.num_experts, c.d_model,
                                    L->rd_planes, L->rd_scale, nullptr);
     if (rrc) return rrc;
+    double scale[kRouterDigitRows];
+    ATENIA_CUDA_TRY(cudaMemcpy(scale, L->rd_scale, sizeof(scale), cudaMemcpyDeviceToHost));
+    L->rd_exact = true;
+    for (double v : scale) L->rd_exact = L->rd_exact && !std::isnan(v);
   }
 
   // INT8 matrices are borrowed as they are: their tensor maps describe bytes and the grouped GEMM
@@ -813,7 +818,7 @@ static int forward_impl(AteniaMoeLayer* L, const void* x, int x_dtype, int T, vo
   ra.logits = (aux && aux->logits) ? aux->logits : (v3 ? L->logits_ws : nullptr);
   ra.err = L->d_err;
   ra.variant = L->router_variant;
-  ra.digit_map = L->rd_planes ? &L->tm_rd : nullptr;
+  ra.digit_map = L->rd_exact ? &L->tm_rd : nullptr;
   ra.digit_scale = L->rd_scale;
   ra.chained = chained;
   ra.beside = shared_aside;

@@ -1,24 +1,34 @@
-// Router of long bf16 prompts on the int8 tensor cores, with the exactness of the f64 sums.
+// Router of long bf16 prompts on the int8 tensor cores, with the f64 sums' precision for every input.
 //
 // The reference accumulates the router logits in f64, and the f64 tensor-core kernel (router_dmma.cu) is bound by the
 // f64 pipe and the conversions in front of it: 107 us for 8192 tokens, 64 experts, d = 2048, in which no expert GEMM
-// gets far.  Here both operands become integers on a grid of their row's largest magnitude and the products are exact:
-//   x[t, :] = 2^(ex - 30) X,  |X| < 2^30, four balanced base-256 digits (bf16 values within 2^-23 of the largest of the
-//             row's k-range are exact, below that the error is 2^-31 of it)
-//   w[e, :] = 2^(ew - 38) W,  |W| < 2^38, five digits (f32 values within 2^-15 of the row's largest are exact, below
-//             that the error is 2^-39 of it); made once per set_weights from the layer's copy
+// gets far.  Here both operands become integers on a grid of their row's largest magnitude and the products are exact
+// (router_digits.cuh has the grids):
+//   x[t, :] = 2^(ex - 30) X, four balanced base-256 digits; ex per token and k-range
+//   w[e, :] = 2^(ew - 38) W, five digits; made once per set_weights from the layer's copy
 //   logit   = 2^(ex + ew - 68) sum_s 256^(7 - s) A_s,  A_s = sum over i + j = s of the digit products, exact in int32
-// The eight A_s of 64 experts fill tensor memory; they are put together in f64 (three exact partial sums), so what
-// reaches the rounding to f32 differs from the f64 sum by far less than that rounding.
+// The eight A_s of 64 experts fill tensor memory; they are put together in f64 (three exact partial sums).
+//
+// Values off the grid (more than 2^22 below the largest of their k-range: of 2048 normal values there is one in a thousand
+// tokens) are not rounded away: a token that may have any is marked while its largest value is looked for, and what its
+// digits left out, x - 2^(ex - 30) X, is multiplied by the f32 router rows in f64 and added to its share, value by value.  B200,
+// 64 experts of d = 2048, normal activations, kernel without / with this, us: 1300 tokens 19.5 / 21.0, 2048 26.4 / 27.9, 8192
+// 44.4 / 46.2.  With a value 2^14 above the rest in every token (a few values a token off the grid) a forward of 8192 tokens
+// takes 10 us more and is still below the f64 router's; from 2^18 on, where no model's activations are, it is slower (2^18
+// 0.25 ms, all values off the grid 1.3 ms more).
+// A layer whose router rows or gate vector are not all on their grid (f32 values that bf16 does not hold) has a row scale
+// of NaN: launch_router keeps such a layer on the f64 routers, and a captured launch that meets it after new weights
+// computes those rows in f64 here.
 //
 // CTA = 128 tokens x one k-range of a cluster of 8, 4, 2 or 1; per k-block of 128 the 16 converting warps write the
 // four digit planes of the tokens (64 KiB, 128-byte swizzle), TMA brings the five planes of the experts (40 KiB), one
 // warp issues twenty M128 x N64 x K32 products per 32 k, plane i of x against plane j of w onto A_(i + j).  The f64
 // shares of the k-ranges meet in distributed shared memory in CTA order, then bias, rounding, softmax and top-k by one
-// warp per token. 
+// warp per token.
 // The shared expert's gate vector is one more row of w.  A token with an infinite or NaN value gets NaN logits, as from
 // the f64 sums.  All waits are bounded; a token block whose products did not finish gets NaN logits too.
 #include "route_warp.cuh"
+#include "router_digits.cuh"
 #include "tc_common.cuh"
 
 namespace atenia {
@@ -94,13 +104,10 @@ __device__ __forceinline__ void digits16(const uint4 (&q)[2], float mul, uint4 (
     const uint32_t w0 = g & 1 ? (g & 2 ? q[1].z : q[0].z) : (g & 2 ? q[1].x : q[0].x);
     const uint32_t w1 = g & 1 ? (g & 2 ? q[1].w : q[0].w) : (g & 2 ? q[1].y : q[0].y);
     uint32_t y[4];
-    y[0] = (uint32_t)__float2int_rn(bf16lo(w0) * mul);
-    y[1] = (uint32_t)__float2int_rn(bf16hi(w0) * mul);
-    y[2] = (uint32_t)__float2int_rn(bf16lo(w1) * mul);
-    y[3] = (uint32_t)__float2int_rn(bf16hi(w1) * mul);
-    // bytes of X + 0x80808080 are the balanced digits + 128
-#pragma unroll
-    for (int i = 0; i < 4; ++i) y[i] = (y[i] + 0x80808080u) ^ 0x80808080u;
+    y[0] = digits_x_bytes(__float2int_rn(bf16lo(w0) * mul));
+    y[1] = digits_x_bytes(__float2int_rn(bf16hi(w0) * mul));
+    y[2] = digits_x_bytes(__float2int_rn(bf16lo(w1) * mul));
+    y[3] = digits_x_bytes(__float2int_rn(bf16hi(w1) * mul));
     const uint32_t a = __byte_perm(y[0], y[1], 0x5140), b = __byte_perm(y[0], y[1], 0x7362);
     const uint32_t c = __byte_perm(y[2], y[3], 0x5140), d = __byte_perm(y[2], y[3], 0x7362);
     p[3][g] = __byte_perm(a, c, 0x5410);
@@ -112,12 +119,85 @@ __device__ __forceinline__ void digits16(const uint4 (&q)[2], float mul, uint4 (
   for (int i = 0; i < RPX; ++i) out[i] = make_uint4(p[i][0], p[i][1], p[i][2], p[i][3]);
 }
 
+// What the digits of one token left out of x[k_begin, k_end), times the rows of w; a row that the planes do not hold (off0, off1;
+// w_off: there are any) times all of x.  One warp, lane l rows l and l + 32; values are taken in the order of k.  (Short code: it
+// is seldom run, so every line of it is fetched anew.)
+__device__ __noinline__ double2 left_out(const __nv_bfloat16* __restrict__ x, int k_begin, int k_end, int ex,
+                                         const float* __restrict__ w_router, const float* __restrict__ gate_vec, int E, int d, bool off0,
+                                         bool off1, bool w_off, int lane) {
+  auto row_of = [&](int e) { return e < E ? w_router + (size_t)e * d : e == E ? gate_vec : nullptr; };
+  const float *row0 = row_of(lane), *row1 = row_of(lane + 32);
+  // (in f64: a small value next to a huge one would leave the range of f32 on the grid's scale)
+  const double mul = __longlong_as_double((long long)(30 - ex + 1023) << 52), unit = __longlong_as_double((long long)(ex - 30 + 1023) << 52);
+  const uint32_t edge = digits_x_edge(ex);  // below it a value may be off the grid
+  auto low = [&](uint32_t bits) { return bits != 0 && bits < edge; };
+  constexpr int U = 4;  // vectors of a lane in flight
+  double2 sum = make_double2(0.0, 0.0);
+#pragma unroll 1
+  for (int k0 = k_begin; k0 < k_end; k0 += U * 256) {
+    uint4 q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * 256 + lane * 8;
+      q[u] = k < k_end ? *reinterpret_cast<const uint4*>(x + k) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll 1
+    for (int u = 0; u < U; ++u) {
+      const uint4 own = q[0];
+#pragma unroll
+      for (int n = 1; n < U; ++n) q[n - 1] = q[n];
+      const int ku = k0 + u * 256;
+      const uint32_t ow[4] = {own.x, own.y, own.z, own.w};
+      bool some = w_off;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) some = some || low(ow[j] & 0x7fffu) || low(ow[j] >> 16 & 0x7fffu);
+      for (unsigned todo = __ballot_sync(0xffffffffu, some && ku + lane * 8 < k_end); todo; todo &= todo - 1) {
+        const int from = __ffs(todo) - 1, k = ku + from * 8;
+        // eight values: lane j (j < 8) makes its own ready
+        uint32_t word = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t v = __shfl_sync(0xffffffffu, ow[j], from);
+          if ((lane >> 1 & 3) == j) word = v;
+        }
+        const double v = lane & 1 ? bf16hi(word) : bf16lo(word), f = v * mul, left = (f - rint(f)) * unit;
+        unsigned which = __ballot_sync(0xffffffffu, lane < 8 && (w_off || left != 0.0));
+        if (__popc(which) > 2) {  // a token of many: all eight, their weights in flight together
+          float w0[8], w1[8];
+#pragma unroll
+          for (int j = 0; j < 8; j += 4) {
+            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 a = row0 ? *reinterpret_cast<const float4*>(row0 + k + j) : z, b = row1 ? *reinterpret_cast<const float4*>(row1 + k + j) : z;
+            w0[j] = a.x, w0[j + 1] = a.y, w0[j + 2] = a.z, w0[j + 3] = a.w;
+            w1[j] = b.x, w1[j + 1] = b.y, w1[j + 2] = b.z, w1[j + 3] = b.w;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const double vj = __shfl_sync(0xffffffffu, v, j), lj = __shfl_sync(0xffffffffu, left, j);
+            sum.x = fma(off0 ? vj : lj, (double)w0[j], sum.x);
+            sum.y = fma(off1 ? vj : lj, (double)w1[j], sum.y);
+          }
+          continue;
+        }
+        for (; which; which &= which - 1) {
+          const int j = __ffs(which) - 1;
+          const double vj = __shfl_sync(0xffffffffu, v, j), lj = __shfl_sync(0xffffffffu, left, j);
+          if (row0) sum.x = fma(off0 ? vj : lj, (double)row0[k + j], sum.x);
+          if (row1) sum.y = fma(off1 ? vj : lj, (double)row1[k + j], sum.y);
+        }
+      }
+    }
+  }
+  return sum;
+}
+
 template <int CTAS>
 __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(R_THREADS, 1)
 router_i8_kernel(RouterArgs a, const __grid_constant__ CUtensorMap tmap_w, const double* __restrict__ w_scale) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ BarriersR bars;
   __shared__ int row_exp[RM];  // ex of a token's k-range; kBad: a value is not finite
+  __shared__ bool row_off[RM];  // ... a value may be off the grid
   __shared__ int32_t idx_s[R_THREADS / 32][R_NT_MAX][kMaxK];
   __shared__ float w_s[R_THREADS / 32][R_NT_MAX][kMaxK];
   constexpr int kBad = 1 << 20;
@@ -236,8 +316,9 @@ router_i8_kernel(RouterArgs a, const __grid_constant__ CUtensorMap tmap_w, const
         }
       }
     };
-    // largest magnitude of each row over the k-range: bf16 bit patterns without the sign order like integers
-    uint32_t m[2] = {0u, 0u};
+    // largest and smallest (but zeros) magnitude of each row over the k-range: bf16 bit patterns without the sign order like
+    // integers
+    uint32_t m[2] = {0u, 0u}, key[2] = {0x7fff7fffu, 0x7fff7fffu};
     for (int i = 0; i < nkb; i += 4) {
       uint4 q[4][2][2];
 #pragma unroll
@@ -250,19 +331,29 @@ router_i8_kernel(RouterArgs a, const __grid_constant__ CUtensorMap tmap_w, const
           for (int v = 0; v < 2; ++v) {
             const uint32_t w[4] = {q[j][h][v].x, q[j][h][v].y, q[j][h][v].z, q[j][h][v].w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) m[h] = __vmaxu2(m[h], w[e] & 0x7fff7fffu);
+            for (int e = 0; e < 4; e += 2) {
+              const uint32_t w0 = w[e] & 0x7fff7fffu, w1 = w[e + 1] & 0x7fff7fffu;
+              m[h] = __vimax3_u16x2(m[h], w0, w1);
+              key[h] = __vimin3_s16x2(key[h], digits_keys(w0), digits_keys(w1));
+            }
           }
     }
     float mul[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      uint32_t v = max(m[h] & 0xffffu, m[h] >> 16);
+      uint32_t v = max(m[h] & 0xffffu, m[h] >> 16), kk = key[h];
 #pragma unroll
-      for (int o = 1; o < 8; o <<= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-      // |x| < 2^(field - 126); rows below 2^-89 keep that grid
-      const int field = (int)(v >> 7), ex = (field < 37 ? 37 : field) - 126;
+      for (int o = 1; o < 8; o <<= 1) {
+        v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+        kk = __vmins2(kk, __shfl_xor_sync(0xffffffffu, kk, o));
+      }
+      const int ex = digits_x_exponent(v);  // |x| < 2^ex
       const bool bad = v >= 0x7f80u;
-      if (c == 0) row_exp[row[h]] = bad ? kBad : ex;
+      const bool off = !bad && digits_x_off_grid(digits_of_key(__vmins2(kk, kk >> 16) & 0xffffu), ex);
+      if (c == 0) {
+        row_exp[row[h]] = bad ? kBad : ex;
+        row_off[row[h]] = off;
+      }
       mul[h] = bad ? 0.f : __uint_as_float((uint32_t)(30 - ex + 127) << 23);
     }
     bool ok = true;
@@ -305,7 +396,7 @@ router_i8_kernel(RouterArgs a, const __grid_constant__ CUtensorMap tmap_w, const
     }
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
-    asm volatile("bar.sync 1, %0;" ::"n"(R_CONV_WARPS * 32) : "memory");  // row_exp; nobody writes a stage any more
+    asm volatile("bar.sync 1, %0;" ::"n"(R_CONV_WARPS * 32) : "memory");  // row_exp, row_off; nobody writes a stage any more
     // a lane holds a token (row of the accumulators), a warp 16 experts of its lane quarter
     const int t = (warp & 3) * 32 + lane, e0 = (cw >> 2) * 16;
     const int ex = row_exp[t];
@@ -313,6 +404,7 @@ router_i8_kernel(RouterArgs a, const __grid_constant__ CUtensorMap tmap_w, const
     const double rs = (ex == kBad || !ok) ? nan : __longlong_as_double((long long)(ex + 1023) << 52);
     double* part = reinterpret_cast<double*>(smem) + (size_t)t * R_PART_LD;
     const uint32_t ta = tmem_base + (uint32_t((warp & 3) * 32) << 16);
+    bool w_off = false;  // a row of w that its planes do not hold
 #pragma unroll 1
     for (int e = e0; e < e0 + 16; e += 8) {
       int32_t A[8][8];
@@ -325,12 +417,30 @@ router_i8_kernel(RouterArgs a, const __grid_constant__ CUtensorMap tmap_w, const
       for (int j = 0; j < 8; ++j) {
         double v = 0.0;
         if (ok && nkb > 0) {
-          const long long p0 = ((long long)A[0][j] << 16) + ((long long)A[1][j] << 8) + A[2][j];
-          const long long p1 = ((long long)A[3][j] << 16) + ((long long)A[4][j] << 8) + A[5][j];
-          const long long p2 = ((long long)A[6][j] << 8) + A[7][j];
-          v = fma(to_double(p2), 0x1p-40, fma(to_double(p1), 0x1p-24, to_double(p0)));
+          const int32_t level[8] = {A[0][j], A[1][j], A[2][j], A[3][j], A[4][j], A[5][j], A[6][j], A[7][j]};
+          long long p[3];
+          digits_fold(level, p);
+          v = fma(to_double(p[2]), 0x1p-40, fma(to_double(p[1]), 0x1p-24, to_double(p[0])));
         }
-        part[e + j] = v * rs * w_scale[e + j];
+        const double ws = w_scale[e + j];
+        w_off = w_off || isnan(ws);
+        part[e + j] = v * rs * ws;
+      }
+    }
+    // what the digits left out, once the shares are written: does any token or row of w have some?
+    int some;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+                 : "=r"(some) : "r"((int)(w_off || row_off[t])), "n"(R_CONV_WARPS * 32) : "memory");
+    if (some && ok) {
+      const bool off0 = isnan(w_scale[lane]), off1 = isnan(w_scale[lane + 32]);
+      w_off = __any_sync(0xffffffffu, off0 || off1);
+      for (int r = cw; r < RM; r += R_CONV_WARPS) {
+        if (!(row_off[r] || w_off) || row_exp[r] == kBad || t0 + r >= a.T) continue;
+        const double2 v = left_out(static_cast<const __nv_bfloat16*>(a.x) + (size_t)(t0 + r) * d, kb0 * RKB, min(d, (kb0 + nkb) * RKB), row_exp[r],
+                                   a.w_router, a.gate_vec, E, d, off0, off1, w_off, lane);
+        double* share = reinterpret_cast<double*>(smem) + (size_t)r * R_PART_LD + lane;
+        share[0] = off0 ? v.x : share[0] + v.x;
+        share[32] = off1 ? v.y : share[32] + v.y;
       }
     }
   }
@@ -430,16 +540,19 @@ __global__ void __launch_bounds__(256) router_digits_kernel(const float* __restr
   for (int i = 1; i < 8; ++i) m = fmaxf(m, red[i]);
   const bool finite = m <= 3.402823466e38f;
   const int ew = finite && m > 0.f ? ilogbf(m) + 1 : 0;  // m < 2^ew
-  const double mul = finite ? ldexp(1.0, 38 - ew) : 0.0;
-  if (threadIdx.x == 0) scale[e] = finite ? ldexp(1.0, ew - 28) : __longlong_as_double(0x7ff8000000000000LL);
+  const double mul = ldexp(1.0, 38 - ew);
+  bool off = !finite;
+  for (int k = threadIdx.x; row && k < d; k += 256) {
+    const double v = (double)row[k] * mul;
+    off = off || v != rint(v);
+  }
+  off = __syncthreads_or(off);
+  // NaN: the row has values that are not finite or off the grid, and its planes are zero
+  if (threadIdx.x == 0) scale[e] = off ? __longlong_as_double(0x7ff8000000000000LL) : ldexp(1.0, ew - 28);
   for (int k = threadIdx.x; k < d; k += 256) {
-    long long X = row && finite ? __double2ll_rn((double)row[k] * mul) : 0;
+    long long W = row && !off ? __double2ll_rn((double)row[k] * mul) : 0;
 #pragma unroll
-    for (int p = RPW - 1; p >= 0; --p) {
-      const long long dg = ((X + 128) & 255) - 128;  // balanced digit in [-128, 127]
-      X = (X - dg) >> 8;
-      planes[((size_t)p * RE + e) * d + k] = (int8_t)dg;
-    }
+    for (int p = RPW - 1; p >= 0; --p) planes[((size_t)p * RE + e) * d + k] = digits_w_next(W);
   }
 }
 
