@@ -291,7 +291,14 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
     // Weights of the first tile's first k-blocks; their token rows follow after the wait.  B200, 64 tokens of a 512-wide
     // layer 37.7 -> 33.9 us, 256 Mixtral tokens 507 -> 497.
     int ahead = 0;
-    if (PairCursor c0 = cur; seek(c0, 0)) {
+    // (The loop's first seek finds the cursor where this one left it.  Walking the groups again there delays the token rows: 32
+    // experts of 512 x 1408, shared 2816 on the second stream, 333 / 500 / 1000 tokens 70.8 / 73.5 / 89.7 -> 67.2 / 70.5 / 86.1 us a
+    // forward.  With an extra group the tiles that follow are what counts, and the walk is repeated: once / twice 64 top-2 experts of
+    // 2048 x 1408, 24 tokens 112.1 / 111.2, 128 top-2 of 2048 x 768, 24 / 100 tokens 96.0 / 93.9, 171.6 / 170.1.)
+    PairCursor first = cur;
+    const bool any = seek(first, 0);
+    if constexpr (!EX) cur = first;
+    if (any) {
       const CUtensorMap* m0 = weights0();
       const CUtensorMap* m1 = MODE == kSwiGLU ? weights1() : m0;
       tmap_acquire(m0);
