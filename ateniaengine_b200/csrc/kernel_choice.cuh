@@ -66,14 +66,32 @@ inline Bf16Kernel bf16_product_kernel(int rows, int groups, int k, bool beside) 
 // / 415 / 435.
 // A product whose tiles all run at once takes the lowest that still do (8 experts of 512 x 1408, 600 / 1000 tokens 38.3 / 35.2 /
 // 35.2, 42.6 / 37.7 / 37.5; but 333 rows of one group over 22 feature tiles, two rounds of 64-row tiles, 67.2 / - / 73.4).
+constexpr int64_t kPairs = 74;
 inline int pair_tokens_of(int rows, int groups, int f_tiles) {
-  constexpr int64_t kPairs = 74;
   for (int t = 64; t <= 128; t += 64)
     if (f_tiles * (int64_t)(groups == 1 ? (rows + t - 1) / t : groups + rows / t) <= kPairs) return t;
   if (groups == 1) return rows <= 64 ? 64 : rows <= 128 ? 128 : 256;
   const int64_t r = rows, g = groups;
   if (r <= 12 * g || (g <= 16 && r <= 36 * g)) return 64;
   return r <= 88 * g ? 128 : r <= 140 * g ? 192 : 256;
+}
+
+// Does the shared expert's group, cut by the routed groups' tile height, ride along in their launches (merges_shared)?  It
+// passes its weights through once per tile of its rows: with many of them, above all low ones, its own launches on the second
+// stream, whose tiles are up to 256 rows high, are faster.  B200, a forward riding along / aside, us (in brackets the passes x
+// shared width against the routed weights' width, experts x F):
+//   64-row tiles   64 top-1 experts of 2048 x 1408, shared 1408, 300 tokens (0.08) 191 / 200; shared 5632, 100 (0.13) 152 / 157, 300
+//                  (0.3) 205 / 203, 600 (0.6) 237 / 230; shared 22528, 100 (0.5) 206 / 202, 300 (1.3) 276 / 261, 600 (2.5) 405 / 329;
+//                  128 top-1 of 2048 x 768, shared 3072, 300 (0.16) 211 / 214, 1000 (0.5) 273 / 261, 1480 (0.75) 309 / 308; shared 12288,
+//                  100 (0.25) 160 / 165, 600 (1.3) 325 / 287, 1000 (2) 399 / 340; 32 top-2 of 2048 x 1408, shared 11264, 100 (0.5) 136 / 145
+//   higher ones    64 top-1 of 2048 x 1408, shared 5632, 1000 (0.5) 257 / 263; shared 22528, 1000 (2) 423 / 405, 1480 (3) 572 / 530; 64 top-2,
+//                  shared 22528, 600 (1.3) 331 / 340, 1480 (3) 591 / 548; 16 top-1 of 2048 x 4096, shared 8192, 600 (0.6) 199 / 215,
+//                  1000 (1) 242 / 249; 32 top-2 of 2048 x 1408, shared 11264, 600 (1.25) 181 / 193, 1000 (2) 243 / 238
+// A group whose tiles all run at once rides along whatever its width (8 top-2 of 512 x 512, shared 1024, 333 tokens 30 / 41).
+inline bool shared_rides_along(int tokens, int tile, int experts, int F, int Fs) {
+  const int64_t passes = (tokens + tile - 1) / tile, f_tiles = (Fs + 127) / 128;
+  if (passes * f_tiles <= kPairs) return true;
+  return 4 * passes * Fs <= (tile == 64 ? 2 : 5) * (int64_t)experts * F;
 }
 
 }  // namespace atenia

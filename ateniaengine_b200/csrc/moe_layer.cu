@@ -77,6 +77,9 @@ bool merges_shared(const AteniaMoeLayer* L, int T) {
   if (c.weight_dtype != ATENIA_W_BF16 || c.ep_world > 1 || L->use_check_gemm || L->timing || T > 10 * L->num_sms) return false;
   if (rows > 140 * c.num_experts) return false;  // (groups that fill their tiles: the GEMMs are compute-bound themselves)
   if (L->bf16_decode == 1 || (L->bf16_decode < 0 && rows <= 16)) return false;  // (the stream-K kernel's calls)
+  // (a wide one beside many experts passes its weights through too often)
+  const int tile = pair_tokens_of(rows, c.num_experts, pair_f_tiles(c.d_ff, kSwiGLU));
+  if (!shared_rides_along(T, tile, c.num_experts, c.d_ff, c.shared_d_ff)) return false;
   return bf16_kernel(L, rows, c.num_experts, c.d_model, false) == kBf16Pairs &&
          bf16_kernel(L, rows, c.num_experts, c.d_ff, false) == kBf16Pairs;
 }

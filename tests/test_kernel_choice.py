@@ -104,3 +104,19 @@ def test_pair_tile_height_of_one_group_holds_it_whole(lib):
     # tiles that all run at once: the lowest that do
     assert [lib.choice_pair_tokens(*a) for a in ((4096, 8, 1), (333, 1, 12), (333, 1, 13), (333, 1, 22), (333, 1, 25))] == [
         64, 64, 128, 128, 256]
+
+
+# tokens, top-k, experts, F, shared width, us of a forward with the shared expert riding along / on its own stream
+SHARED_RIDES = [(300, 1, 64, 1408, 1408, 191, 200), (100, 1, 64, 1408, 5632, 152, 157), (600, 1, 64, 1408, 5632, 237, 230),
+                (300, 1, 64, 1408, 22528, 276, 261), (600, 1, 64, 1408, 22528, 405, 329), (1000, 1, 64, 1408, 22528, 423, 405),
+                (1480, 1, 64, 1408, 22528, 572, 530), (1000, 1, 64, 1408, 5632, 257, 263), (600, 2, 64, 1408, 22528, 331, 340),
+                (1480, 2, 64, 1408, 22528, 591, 548), (300, 1, 128, 768, 3072, 211, 214), (100, 1, 128, 768, 12288, 160, 165),
+                (600, 1, 128, 768, 12288, 325, 287), (1000, 1, 128, 768, 12288, 399, 340), (600, 1, 16, 4096, 8192, 199, 215),
+                (1000, 1, 16, 4096, 8192, 242, 249), (100, 2, 32, 1408, 11264, 136, 145), (600, 2, 32, 1408, 11264, 181, 193),
+                (1000, 2, 32, 1408, 11264, 243, 238), (333, 2, 8, 512, 1024, 30, 41), (333, 4, 60, 1408, 5632, 205, 215)]
+
+
+@pytest.mark.parametrize("tokens,k,experts,F,Fs,along,aside", SHARED_RIDES)
+def test_the_shared_expert_rides_along_where_that_is_faster(lib, tokens, k, experts, F, Fs, along, aside):
+    tile = lib.choice_pair_tokens(tokens * k, experts, (F + 127) // 128)
+    assert lib.choice_shared_rides(tokens, tile, experts, F, Fs) == (along < aside)
