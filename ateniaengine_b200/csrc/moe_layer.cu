@@ -74,7 +74,7 @@ int launch_bf16_product(Bf16Kernel kernel, const GroupedGemmArgs& a, int num_sms
 bool merges_shared(const AteniaMoeLayer* L, int T) {
   const AteniaMoeConfig& c = L->cfg;
   const int rows = T * c.experts_per_token;
-  if (c.weight_dtype != ATENIA_W_BF16 || c.ep_world > 1 || L->use_check_gemm || L->timing || T > 10 * L->num_sms) return false;
+  if (c.weight_dtype != ATENIA_W_BF16 || c.ep_world > 1 || L->use_check_gemm || T > 10 * L->num_sms) return false;
   if (rows > 140 * c.num_experts) return false;  // (groups that fill their tiles: the GEMMs are compute-bound themselves)
   if (L->bf16_decode == 1 || (L->bf16_decode < 0 && rows <= 16)) return false;  // (the stream-K kernel's calls)
   // (a wide one beside many experts passes its weights through too often)
@@ -249,6 +249,7 @@ int run_expert_gemms(AteniaMoeLayer* L, const RowMaps& tm_a, const RowMaps& tm_m
   if (L->timing) {
     cudaEventRecord(L->ev[2], s);
     L->ev_valid[0] = L->ev_valid[1] = true;
+    if (shared_T > 0) L->ev_valid[2] = L->ev_valid[3] = false;  // (part of these two launches)
   }
   return ATENIA_OK;
 }

@@ -659,6 +659,7 @@ def main():
     launches = int(_lib.lib().atenia_moe_counter(1) - launches0)
     layer.check()
     gemm1_ms, gemm2_ms = layer.last_gemm_ms(0), layer.last_gemm_ms(1)
+    shared_along = shape.shared_d_ff > 0 and layer.last_gemm_ms(2) < 0
     phases = [layer.last_phase_ms(i) for i in range(6)]
     recv_rows = layer.last_recv_rows() if args.gpus > 1 else T * shape.top_k
     layer.enable_timing(False)
@@ -757,7 +758,9 @@ def main():
     groups = (shape.num_experts // args.gpus) * (args.gpus if args.gpus > 1 and not direct else 1)
     kname = gate_up_kernel(shape, rows_slow, groups)
     # dominant kernel: the routed gate/up + SwiGLU grouped GEMM of the rank with the most rows
-    flops1 = 4.0 * rows_slow * shape.d_model * shape.d_ff  # gate and up: 2 * 2 * rows * d * F
+    # (a call whose shared expert rides along in the routed launches does its products in them too)
+    units = rows_slow * shape.d_ff + (T * shape.shared_d_ff if shared_along else 0)
+    flops1 = 4.0 * shape.d_model * units  # gate and up: 2 * 2 * rows * d * F
     achieved = flops1 / (g1_slow * 1e-3) / 1e12
     rl = layer_roofline(shape, T, touched if args.gpus == 1 else shape.num_experts // args.gpus, peaks, shape.int8)
     names = ("route_permute_gather", "rows_out", "routed_gemms", "rows_back", "shared_combine", "forward")
@@ -767,7 +770,7 @@ def main():
                 "frac_of_sustained_peak": achieved / peaks["bf16_tflops_sustained"],
                 "traffic": NCU_TRAFFIC_BYTES.get(f"{shape.name}:{T}:{kname}") if args.gpus == 1 else None,
                 "rows": rows_slow, "launch_ms": g1_slow, "down_gemm_ms": g2_slow,
-                "down_gemm_tflops": 2.0 * rows_slow * shape.d_model * shape.d_ff / (g2_slow * 1e-3) / 1e12,
+                "down_gemm_tflops": 2.0 * shape.d_model * units / (g2_slow * 1e-3) / 1e12,
                 "timed_inside": "the last step of the timed region (events on the launching stream)",
                 "phases_ms": {n: per_rank[slow][3 + i] for i, n in enumerate(names)},
                 "layer_frac_of_tensor_roofline": (T * shape.top_k * 6.0 * shape.d_model * shape.d_ff +

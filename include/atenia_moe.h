@@ -505,7 +505,8 @@ ATENIA_API uint64_t atenia_moe_counter(int which);
 
 /* Time of the most recent grouped-GEMM launches of this layer, measured with CUDA events on the
  * launching stream while timing is enabled (enable != 0).  `which`: 0 = routed gate/up + SwiGLU,
- * 1 = routed down, 2 = shared gate/up, 3 = shared down.  Returns milliseconds, or a negative value
+ * 1 = routed down, 2 = shared gate/up, 3 = shared down; where one launch does the routed and the shared
+ * product, 0 and 1 are its times and 2 and 3 are negative.  Returns milliseconds, or a negative value
  * if nothing was recorded.  Enabling timing adds event records to every forward. */
 ATENIA_API int atenia_moe_enable_timing(AteniaMoeLayer* layer, int enable);
 ATENIA_API float atenia_moe_last_gemm_ms(AteniaMoeLayer* layer, int which);

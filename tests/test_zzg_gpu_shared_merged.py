@@ -62,3 +62,25 @@ def test_captured(dev, monkeypatch):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
+
+
+def _launches(f):
+    from ateniaengine_b200 import _lib
+    before = _lib.lib().atenia_moe_counter(1)
+    f()
+    return _lib.lib().atenia_moe_counter(1) - before
+
+
+@pytest.mark.parametrize("T,along", [(200, True), (1500, False)])
+def test_timing_measures_the_launches_of_an_ordinary_forward(dev, monkeypatch, T, along):
+    shape, layer, _ = _layers(dev, monkeypatch, 24, 4, 528, 400, 1040, True, T)
+    x = _synth().make_activations(shape, 1, dev, tokens=T)
+    want = layer.forward(x, sync=True)
+    plain = _launches(lambda: layer.forward(x, sync=True))
+    layer.enable_timing(True)
+    got = []
+    assert _launches(lambda: got.append(layer.forward(x, sync=True))) == plain
+    assert torch.equal(got[0], want)
+    ms = [layer.last_gemm_ms(i) for i in range(4)]
+    assert min(ms[:2]) > 0 and (max(ms[2:]) < 0 if along else min(ms[2:]) > 0)
+    layer.enable_timing(False)
