@@ -528,9 +528,13 @@ int launch_2cta_form(const GroupedGemmArgs& a, int num_sms, cudaStream_t s, cons
 template <int MODE, int TOK>
 int launch_2cta_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   if (a.extra.rows <= 0) return launch_2cta_form<MODE, TOK, false>(a, num_sms, s, NoExtra{});
-  const PairExtra ex{*a.extra.x_rows, a.extra.tmap_b0, MODE == kSwiGLU ? a.extra.tmap_b1 : a.extra.tmap_b0, a.extra.out,
-                     a.extra.rows, a.extra.N, a.extra.K};
-  return launch_2cta_form<MODE, TOK, true>(a, num_sms, s, ex);
+  if constexpr (TOK == kPairTokens) {
+    return ATENIA_ERR_SHAPE;  // (merges_shared: an extra group rides with tiles of at most 192 rows)
+  } else {
+    const PairExtra ex{*a.extra.x_rows, a.extra.tmap_b0, MODE == kSwiGLU ? a.extra.tmap_b1 : a.extra.tmap_b0, a.extra.out,
+                       a.extra.rows, a.extra.N, a.extra.K};
+    return launch_2cta_form<MODE, TOK, true>(a, num_sms, s, ex);
+  }
 }
 
 template <int MODE>

@@ -75,7 +75,8 @@ bool merges_shared(const AteniaMoeLayer* L, int T) {
   const AteniaMoeConfig& c = L->cfg;
   const int rows = T * c.experts_per_token;
   if (c.weight_dtype != ATENIA_W_BF16 || c.ep_world > 1 || L->use_check_gemm || T > 10 * L->num_sms) return false;
-  if (rows > 140 * c.num_experts) return false;  // (groups that fill their tiles: the GEMMs are compute-bound themselves)
+  // (groups that fill their tiles: the GEMMs are compute-bound themselves; below that no tile is higher than 192 rows)
+  if (rows > (c.num_experts == 1 ? 128 : 140 * c.num_experts)) return false;
   if (L->bf16_decode == 1 || (L->bf16_decode < 0 && rows <= 16)) return false;  // (the stream-K kernel's calls)
   // (a wide one beside many experts passes its weights through too often)
   const int tile = pair_tokens_of(rows, c.num_experts, pair_f_tiles(c.d_ff, kSwiGLU));

@@ -20,12 +20,25 @@ def _layers(dev, monkeypatch, E, k, d, F, Fs, gated, T):
     return shape, merged, plain
 
 
-# routed rows per group: 64-row tiles, 128, 192, 256; feature tiles fewer and more than pairs of SMs
-@pytest.mark.parametrize("E,k,d,F,Fs,gated", [(8, 2, 528, 400, 1040, True), (60, 4, 272, 144, 16, False),
-                                              (17, 4, 2064, 1040, 5632, True), (40, 2, 1040, 1424, 400, False)])
-@pytest.mark.parametrize("T", [9, 65, 257, 500, 1480])
+def _launches(f):
+    from ateniaengine_b200 import _lib
+    before = _lib.lib().atenia_moe_counter(1)
+    f()
+    return _lib.lib().atenia_moe_counter(1) - before
+
+
+# routed rows per group: tiles of 64 rows, 128 and 192 (17 experts, 500 tokens); feature tiles fewer and more than pairs of SMs
+MERGED = [((8, 2, 528, 400, 1040, True), (9, 65, 257, 500)), ((60, 4, 272, 144, 16, False), (9, 65, 200, 255)),
+          ((17, 4, 2064, 1040, 5632, True), (9, 65, 257, 500)), ((40, 2, 1040, 1424, 400, False), (9, 65, 257, 500, 1480)),
+          ((1, 1, 528, 400, 1040, False), (17, 128))]
+# groups that fill their tiles, a product on the single-CTA kernel, a wide shared expert of many low tiles, decode calls
+ASIDE = [((8, 2, 528, 400, 1040, True), (8, 561, 1480)), ((60, 4, 272, 144, 16, False), (257, 1480)), ((17, 4, 2064, 1040, 5632, True), (1480,)),
+         ((40, 2, 1040, 1424, 400, False), (1481,)), ((32, 1, 272, 144, 9616, False), (300,)), ((1, 1, 528, 400, 1040, False), (129,))]
+
+
+@pytest.mark.parametrize("E,k,d,F,Fs,gated,T,merges", [(*s, T, m) for m, group in ((True, MERGED), (False, ASIDE)) for s, Ts in group for T in Ts])
 @pytest.mark.parametrize("io", [torch.bfloat16, torch.float32])
-def test_same_bits_as_launches_of_its_own(dev, monkeypatch, E, k, d, F, Fs, gated, T, io):
+def test_same_bits_as_launches_of_its_own(dev, monkeypatch, E, k, d, F, Fs, gated, T, merges, io):
     shape, merged, plain = _layers(dev, monkeypatch, E, k, d, F, Fs, gated, T)
     x = _synth().make_activations(shape, T, dev, tokens=T, dtype=io)
     want = plain.forward(x, out_dtype=torch.float32, sync=True)
@@ -33,6 +46,10 @@ def test_same_bits_as_launches_of_its_own(dev, monkeypatch, E, k, d, F, Fs, gate
     for y in outs:  # nothing between the calls
         merged.forward(x, out=y)
     merged.check()
+    # (in order the shared expert is two more launches; aside it has a launch for its offsets and, from f32, one that converts)
+    extra = _launches(lambda: merged.forward(x, out=outs[0])) - _launches(lambda: plain.forward(x, out=outs[0]))
+    assert extra == (-2 if merges else 1 if io == torch.bfloat16 else 2)
+    plain.check()
     assert torch.isfinite(want).all() and want.abs().sum() > 0
     assert all(torch.equal(y, want) for y in outs)
 
@@ -62,13 +79,6 @@ def test_captured(dev, monkeypatch):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
-
-
-def _launches(f):
-    from ateniaengine_b200 import _lib
-    before = _lib.lib().atenia_moe_counter(1)
-    f()
-    return _lib.lib().atenia_moe_counter(1) - before
 
 
 @pytest.mark.parametrize("T,along", [(200, True), (1500, False)])
