@@ -53,24 +53,30 @@ def _ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+# torch's current stream of a device as a plain handle (of torch's own code generators; torch.cuda.current_stream makes an object)
+_current_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+
+
 class _launching:
     """A call that launches on `device`: makes it the current one meanwhile and yields its current stream's handle.
-    What torch.cuda.device() and torch.cuda.current_stream() do, without their objects (6 us a call, of the 27 in which a
-    forward of six launches is issued)."""
-    __slots__ = ("index", "before")
+    Where it is the current one already, as it nearly always is, without torch's objects (6 us a call, of the 27 in which a
+    forward of six launches is issued); else torch.cuda.device changes it and puts the former back, which creates no
+    context on a device that has none."""
+    __slots__ = ("index", "other")
 
     def __init__(self, device):
         self.index = device.index
 
     def __enter__(self):
-        self.before = torch.cuda.current_device()
-        if self.before != self.index:
-            torch.cuda.set_device(self.index)
-        return torch._C._cuda_getCurrentRawStream(self.index)
+        self.other = None
+        if torch.cuda.current_device() != self.index:
+            self.other = torch.cuda.device(self.index)
+            self.other.__enter__()
+        return _current_stream(self.index)
 
     def __exit__(self, *exc):
-        if self.before != self.index:
-            torch.cuda.set_device(self.before)
+        if self.other is not None:
+            self.other.__exit__(*exc)
 
 
 def _io_dtype(t):
