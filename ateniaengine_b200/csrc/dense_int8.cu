@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(LANES * RL) quantize_groups_kernel(const float
                                                                      int G, unsigned strips, int8_t* __restrict__ q,
                                                                      float* __restrict__ scales) {
   constexpr int COLS = LANES * 4;
-  __shared__ float red[RL][COLS];
+  __shared__ __align__(16) float red[RL][COLS];
   __shared__ float4 scale_s[LANES], inv_s[LANES];
   const int lane = threadIdx.x % LANES, rl = threadIdx.x / LANES;
   const unsigned g = blockIdx.x / strips;
