@@ -36,9 +36,14 @@ namespace {
 // squares in index order; here they are added by a block reduction (fixed order), which can move inv_rms
 // by an ulp.  gamma == nullptr means unit gain.  One block per row; a thread keeps its (up
 // to two) float4 vectors in registers between the two passes, so a row of up to 8192 elements is read once.  Rows of at
-// most 2048 elements take 512 threads, of which four blocks fit an SM: the threads left out had nothing to add, so the
-// sum is the same (B200: with the bf16 copy for the shared expert made aside, the block step of 333 Qwen tokens 225 -> 219 us).
+// most 2048 elements that are read as vectors take 512 threads, of which four blocks fit an SM: the threads left out had
+// nothing to add, so the sum is the same (element by element it would not be, the stride is the block's; B200: with the bf16 copy for the shared expert made aside, the block step of 333 Qwen tokens 225 -> 219 us).
 constexpr int kNormVecs = 2;
+
+// 16-byte vectors when every row starts on a 16-byte boundary
+__host__ __device__ inline bool norm_in_vectors(const float* x, const float* y, int d) {
+  return (d & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+}
 
 template <int kNormThreads>
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float* __restrict__ x,
@@ -50,8 +55,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float*
   atenia::chain_wait();
   const float* row = x + (size_t)blockIdx.x * d;
   float* yrow = y + (size_t)blockIdx.x * d;
-  // 16-byte vectors when every row starts on a 16-byte boundary
-  const bool vec = (d & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  const bool vec = norm_in_vectors(x, y, d);
   const int nvec = vec ? d / 4 : 0;
   float4 keep[kNormVecs];
   float ss = 0.f;
@@ -106,7 +110,7 @@ int launch_rmsnorm_rows(const float* x, const float* gamma, float eps, float* y,
                         cudaStream_t s) {
   if (T <= 0) return ATENIA_OK;
   count_launch();
-  if (d <= 2048) return launch_chained(chained, rmsnorm_rows_kernel<512>, dim3(T), dim3(512), 0, s, x, gamma, eps, y, d);
+  if (d <= 2048 && norm_in_vectors(x, y, d)) return launch_chained(chained, rmsnorm_rows_kernel<512>, dim3(T), dim3(512), 0, s, x, gamma, eps, y, d);
   return launch_chained(chained, rmsnorm_rows_kernel<1024>, dim3(T), dim3(1024), 0, s, x, gamma, eps, y, d);
 }
 }  // namespace atenia
