@@ -240,23 +240,21 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
   cur.base = 0;
   if (num_groups > 0) pair_cursor_load<TOK>(cur, group_offsets);
   PairTile tc;
-  int ex_tiles = 0, ex_m = 1, ex_rows = 16, ex_kb = 0, ex_full = 0, ex_rest = 0, ex_weight = 1;
+  int ex_m = 1, ex_rows = 16, ex_kb = 0;
+  PairDeal deal{};
   if constexpr (EX) {
     ex_m = pair_tiles(ex.rows, TOK);
     ex_rows = pair_tile_rows(ex.rows, ex_m);
-    ex_tiles = ex_m * ((ex.N + F_PAIR - 1) / F_PAIR);
     ex_kb = (ex.K + BK - 1) / BK;
-    ex_full = ex_tiles / num_pairs;
-    ex_rest = ex_tiles - ex_full * num_pairs;
-    ex_weight = max(1, (ex_kb + num_kb / 2) / num_kb);
+    deal = pair_deal(num_pairs, ex_m * ((ex.N + F_PAIR - 1) / F_PAIR), ex_kb, num_kb);
   }
-  // This pair's i-th tile; false past its last.  Tiles are dealt round by round, the extra group's (group -1) first; where they
-  // are longer than the others, the pairs that have one in the last of their rounds miss as many rounds as it lasts.
+  // This pair's i-th tile (the extra group is group -1); false past its last.
   auto seek = [&](PairCursor& c, int i) {
     int tile = pair + i * num_pairs;
     if constexpr (EX) {
-      const int m = i - ex_full;  // rounds after the full ones
-      if (m < 0 || (m == 0 && pair < ex_rest)) {
+      bool extra;
+      tile = pair_deal_tile(deal, pair, i, extra);
+      if (extra) {
         const int ft = tile / ex_m, mt = tile - ft * ex_m;
         tc.group = -1;
         tc.row0 = mt * ex_rows;
@@ -265,9 +263,6 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
         tc.f0 = ft * F_PAIR;
         return true;
       }
-      const int others = num_pairs - ex_rest, late = ex_weight * others;
-      tile = pair < ex_rest ? late + (m - 1) * num_pairs + pair
-             : m < ex_weight ? m * others + pair - ex_rest : late + (m - ex_weight) * num_pairs + pair;
     }
     return pair_cursor_seek<TOK>(c, tile, f_tiles, num_groups, group_offsets, tc, F_PAIR);
   };

@@ -31,6 +31,25 @@ inline unsigned pair_boxes_of_group(int rows, int most = kPairTokens) {
   const unsigned of_last = 1u << pair_tile_box(pair_tile_n(last));
   return tiles > 1 ? of_last | 1u << pair_tile_box(pair_tile_n(full)) : of_last;
 }
+// How a launch deals its tiles to the pairs when one more group, whose tiles may be longer, comes with it: round by round, the
+// extra group's first; the pairs that have one in the last of their rounds miss as many rounds as it lasts (`weight`).
+struct PairDeal {
+  int pairs, full, rest, weight;  // pairs of SMs; rounds of extra tiles, and those of one more round
+};
+ATENIA_HD inline PairDeal pair_deal(int pairs, int extra_tiles, int extra_k_blocks, int k_blocks) {
+  const int full = extra_tiles / pairs, weight = (extra_k_blocks + k_blocks / 2) / k_blocks;
+  return PairDeal{pairs, full, extra_tiles - full * pairs, weight < 1 ? 1 : weight};
+}
+// The `i`-th tile of `pair`: of the extra group (`extra`), or of the others, counted from 0 each.
+ATENIA_HD inline int pair_deal_tile(const PairDeal& d, int pair, int i, bool& extra) {
+  const int m = i - d.full;  // rounds after the full ones
+  extra = m < 0 || (m == 0 && pair < d.rest);
+  if (extra) return pair + i * d.pairs;
+  const int others = d.pairs - d.rest, late = d.weight * others;
+  return pair < d.rest ? late + (m - 1) * d.pairs + pair
+         : m < d.weight ? m * others + pair - d.rest : late + (m - d.weight) * d.pairs + pair;
+}
+
 constexpr unsigned kPairAllBoxes = (1u << kPairBoxes) - 1u;  // rows known on the device only
 
 }  // namespace atenia

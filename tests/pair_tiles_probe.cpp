@@ -14,3 +14,9 @@ extern "C" int pair_probe_walk(int rows, int* row0, int* n_rows, int* box, int* 
   }
   return tiles;
 }
+// The kernel's deal of tiles beside an extra group: the i-th tile of a pair; returns 1 where it is the extra group's.
+extern "C" int pair_probe_deal(int pairs, int extra_tiles, int extra_kb, int kb, int pair, int i, int* tile) {
+  bool extra;
+  *tile = atenia::pair_deal_tile(atenia::pair_deal(pairs, extra_tiles, extra_kb, kb), pair, i, extra);
+  return extra;
+}
