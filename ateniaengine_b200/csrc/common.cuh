@@ -55,10 +55,13 @@ inline bool first_use_on_current_device(bool (&flags)[kMaxDevices]) {
 // one's chain_wait() has waited for the kernel before it, so nothing earlier is in flight either.  chain_next() lets
 // the next kernel's blocks start: what overlaps is its launch, not its work.  Kernels without chain_wait() are
 // launched plainly and wait for everything before them as usual.
-// One exception, the weights: a GEMM takes the group offsets and requests its first weight tiles before its
-// chain_wait().  The kernel before it writes neither (it gathers rows, makes digits, or is the GEMM before) and comes to
+// Two exceptions.  The cluster router requests rows of the layer's own copies of the router matrix and the gate vector, which
+// no kernel writes (set_weights synchronises).  And a GEMM takes the group offsets and requests its first weight tiles before
+// its chain_wait().  The kernel before it writes neither (it gathers rows, makes digits, or is the GEMM before) and comes to
 // chain_next() only past its own chain_wait() -- or, between two GEMMs, was launched by one that had passed its -- so
-// whatever wrote them has completed before the GEMM's blocks start.
+// whatever wrote them has completed before the GEMM's blocks start.  Under expert parallelism every kernel of ep.cu is launched
+// plainly and calls no chain_next(), and one of them (the scatter, or the host's read of the counts) comes between the kernel
+// that writes the offsets and the GEMM, whatever the collective right before it does.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A kernel that takes whole SMs must not sit there waiting while another stream's work could run.  So the kernels
