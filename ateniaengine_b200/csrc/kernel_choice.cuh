@@ -65,7 +65,9 @@ inline Bf16Kernel bf16_product_kernel(int rows, int groups, int k, bool beside) 
 // (137) 372 / 372 / 410, 2500 (167) 429 / 442 / 491; 64, 1300 (122) 305 / 302 / 305, 1700 (159) 343 / 335 / 380, 2000 (187) 389
 // / 415 / 435.
 // A product whose tiles all run at once takes the lowest that still do (8 experts of 512 x 1408, 600 / 1000 tokens 38.3 / 35.2 /
-// 35.2, 42.6 / 37.7 / 37.5; but 333 rows of one group over 22 feature tiles, two rounds of 64-row tiles, 67.2 / - / 73.4).
+// 35.2, 42.6 / 37.7 / 37.5).  Also beside others: a shared expert of 2816 on the second stream of 32 experts of 512 x 1408, 333 tokens
+// over 22 feature tiles (64-row tiles would take two rounds) 66.1 / 66.8 / 68.0; with both its products in 256-row tiles 500 / 700 /
+// 1480 tokens 73.4 -> 77.4, 82.5 -> 88.9, 105.1 -> 109.1.
 constexpr int64_t kPairs = 74;
 inline int pair_tokens_of(int rows, int groups, int f_tiles) {
   for (int t = 64; t <= 128; t += 64)

@@ -350,8 +350,8 @@ int launch_v3_route(const float* logits, const float* e_score_bias, int T, int E
 }
 
 // The integer router computes 64 rows whatever E is, and has a floor of some 15 us (B200, it / the f64 routers, us): 64
-// experts of d = 2048 1184 tokens 18.9 / 19.3, 1500 19.1 / 30.5, 2048 27.2 / 30.7, 4096 29.7 / 54, 8192 44.1 / 109; 32 experts
-// of d = 4096 2048 tokens 37.9 / 29.7, 3000 39.5 / 52, 4096 40.5 / 52.
+// experts of d = 2048 1185 tokens 21.1 / 19.3, 1500 21.1 / 30.5, 2048 27.9 / 30.7, 4096 30.3 / 54, 8192 46.6 / 104; 32 experts
+// of d = 4096 2048 tokens some 39 / 29.1, 3000 40.5 / 51.4, 4096 43.6 / 51.6.
 static bool router_i8_pays(const RouterArgs& a) {
   return a.digit_map && !a.x_is_f32 && (!a.gate_vec || a.E < kRouterDigitRows) && (a.T > 16 * 148 || (a.T > 8 * 148 && a.E > 32));
 }
