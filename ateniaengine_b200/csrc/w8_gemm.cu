@@ -444,10 +444,14 @@ grouped_gemm_w8_tmem_kernel(const __grid_constant__ CUtensorMap tmap_x, const CU
 }
 
 // Adds the partial pieces of every tile that stream-K cut across CTAs, in CTA order, and applies the
-// same scale / activation / store as the main kernel's epilogue.  One block per tile, one thread per
-// weight row (feature).
+// same scale / activation / store as the main kernel's epilogue.  One thread per weight row (feature); block (t, y) of a tile
+// takes every kReduceTokBlocks-th token, and a token's pieces are requested side by side.  One block per tile that walked tokens
+// and pieces one after another took most of a forward with a shared expert, whose second product has few tiles of many
+// pieces: 64 INT8 experts of 1024 x 2048 beside 8192, 52 tokens, 133 of 230 us (now some 30, under the routed GEMMs, of 171); 16 of
+// 256 x 2816 beside 5632, 24 tokens 100 of 147 (now 14 of 96).
+constexpr int kReduceTokBlocks = 16, kReducePieces = 8;
 template <int MODE>
-__global__ void __launch_bounds__(WROWS * 8) w8_splitk_reduce_kernel(const int32_t* __restrict__ group_offsets,
+__global__ void __launch_bounds__(WROWS) w8_splitk_reduce_kernel(const int32_t* __restrict__ group_offsets,
                                                                   int num_groups, int N, int K,
                                                                   __nv_bfloat16* __restrict__ out,
                                                                   const float* const* __restrict__ scale0,
@@ -488,14 +492,25 @@ __global__ void __launch_bounds__(WROWS * 8) w8_splitk_reduce_kernel(const int32
     s_a = ok_a ? sc0[n_lo] : 0.f;
     s_b = ok_b ? sc0[n_hi] : 0.f;
   }
-  // (thread (f, y) takes every blockDim.y-th token: few dependent loads per thread)
-  for (int tok = threadIdx.y; tok < rows; tok += blockDim.y) {
+  // CTA c0's piece is in its second slot unless its span starts in this tile; the others' spans all do
+  const int slot0 = (t == ((long long)c0 * span) / num_kb) ? 0 : 1;
+  for (int tok = blockIdx.y; tok < rows; tok += kReduceTokBlocks) {
+    const float* p = ws + (size_t)tok * WROWS + f;
     float a = 0.f, b = 0.f;
-    for (int c = c0; c <= c1; ++c) {
-      const int slot = (t == ((long long)c * span) / num_kb) ? 0 : 1;
-      const float* p = ws + ((size_t)c * 2 + slot) * SLOT_FLOATS;
-      a += p[(size_t)tok * WROWS + f];
-      b += p[(size_t)(TN + tok) * WROWS + f];
+    for (int c = c0; c <= c1; c += kReducePieces) {
+      float xa[kReducePieces], xb[kReducePieces];
+#pragma unroll
+      for (int j = 0; j < kReducePieces; ++j) {
+        const float* q = p + ((size_t)(c + j) * 2 + (c + j == c0 ? slot0 : 0)) * SLOT_FLOATS;
+        xa[j] = c + j <= c1 ? q[0] : 0.f;
+        xb[j] = c + j <= c1 ? q[(size_t)TN * WROWS] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < kReducePieces; ++j) {
+        if (c + j > c1) break;
+        a += xa[j];
+        b += xb[j];
+      }
     }
     __nv_bfloat16* orow = out + (size_t)(tc.row0 + tok) * N;
     if (MODE == kSwiGLU) {
@@ -528,7 +543,7 @@ int launch_w8_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   constexpr int BN_OUT = (MODE == kSwiGLU) ? WROWS : 2 * WROWS;
   const int n_tiles = (a.N + BN_OUT - 1) / BN_OUT;
   const int max_tiles = a.num_groups * n_tiles;  // every group has at most one token tile here
-  w8_splitk_reduce_kernel<MODE><<<dim3(max_tiles), dim3(WROWS, 8), 0, s>>>(a.group_offsets, a.num_groups, a.N, a.K, a.out,
+  w8_splitk_reduce_kernel<MODE><<<dim3(max_tiles, kReduceTokBlocks), dim3(WROWS), 0, s>>>(a.group_offsets, a.num_groups, a.N, a.K, a.out,
                                                                          a.scale0, a.scale1, a.splitk_ws, num_sms);
   count_launch();
   return (int)cudaGetLastError();
