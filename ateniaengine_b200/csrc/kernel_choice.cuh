@@ -79,21 +79,20 @@ inline int pair_tokens_of(int rows, int groups, int f_tiles) {
 }
 
 // Does the shared expert's group, cut by the routed groups' tile height, ride along in their launches (merges_shared)?  It
-// passes its weights through once per tile of its rows: with many of them, above all low ones, its own launches on the second
-// stream, whose tiles are up to 256 rows high, are faster.  B200, a forward riding along / aside, us (in brackets the passes x
-// shared width against the routed weights' width, experts x F):
-//   64-row tiles   64 top-1 experts of 2048 x 1408, shared 1408, 300 tokens (0.08) 191 / 200; shared 5632, 100 (0.13) 152 / 157, 300
-//                  (0.3) 205 / 203, 600 (0.6) 237 / 230; shared 22528, 100 (0.5) 206 / 202, 300 (1.3) 276 / 261, 600 (2.5) 405 / 329;
-//                  128 top-1 of 2048 x 768, shared 3072, 300 (0.16) 211 / 214, 1000 (0.5) 273 / 261, 1480 (0.75) 309 / 308; shared 12288,
-//                  100 (0.25) 160 / 165, 600 (1.3) 325 / 287, 1000 (2) 399 / 340; 32 top-2 of 2048 x 1408, shared 11264, 100 (0.5) 136 / 145
-//   higher ones    64 top-1 of 2048 x 1408, shared 5632, 1000 (0.5) 257 / 263; shared 22528, 1000 (2) 423 / 405, 1480 (3) 572 / 530; 64 top-2,
-//                  shared 22528, 600 (1.3) 331 / 340, 1480 (3) 591 / 548; 16 top-1 of 2048 x 4096, shared 8192, 600 (0.6) 199 / 215,
-//                  1000 (1) 242 / 249; 32 top-2 of 2048 x 1408, shared 11264, 600 (1.25) 181 / 193, 1000 (2) 243 / 238
-// A group whose tiles all run at once rides along whatever its width (8 top-2 of 512 x 512, shared 1024, 333 tokens 30 / 41).
-inline bool shared_rides_along(int tokens, int tile, int experts, int F, int Fs) {
-  const int64_t passes = (tokens + tile - 1) / tile, f_tiles = (Fs + 127) / 128;
-  if (passes * f_tiles <= kPairs) return true;
-  return 4 * passes * Fs <= (tile == 64 ? 2 : 5) * (int64_t)experts * F;
+// passes its weights through once per tile of its rows, its own launches on the second stream once per 256: the passes more are
+// traffic that its missing launches (some 8 us) and the interleaving have to pay for.  B200, a forward along / aside, us, by what
+// those passes read in MB:
+//   64-row tiles   64 top-1 experts of 2048 x 1408, shared 1408, 600 tokens (120) 209 / 222; shared 5632, 100 (70) 152 / 157, 300 (210)
+//                  205 / 203, 600 (480) 237 / 230; shared 22528, 100 (280) 206 / 202, 300 (830) 276 / 261, 600 (1940) 405 / 329; 128 top-1
+//                  of 2048 x 768, shared 768, 600 (66) 236 / 251; shared 3072, 1000 (450) 273 / 261; shared 12288, 100 (150) 160 / 165,
+//                  300 (450) 245 / 241, 600 (1060) 325 / 287; 16 top-1 of 1024 x 2816, shared 5632, 303 (100) 85 / 87, 500 (210) 87 / 93; 32
+//                  top-2 of 2048 x 1408, shared 11264, 100 (140) 136 / 145
+//   higher ones    64 top-1 of 2048 x 1408, shared 5632, 1000 (280) 257 / 263; shared 22528, 1000 (1110) 423 / 405, 1480 (1660) 572 / 530; 64
+//                  top-2, shared 22528, 1000 (1110) 424 / 412, 1480 (1660) 591 / 548; 16 top-1 of 2048 x 4096, shared 8192, 600 (200) 199 /
+//                  215, 1000 (400) 242 / 249; 32 top-2 of 2048 x 1408, shared 11264, 600 (280) 181 / 193
+inline bool shared_rides_along(int tokens, int tile, int d, int Fs) {
+  const int64_t more = (tokens + tile - 1) / tile - (tokens + 255) / 256;
+  return more * 6 * d * Fs <= (int64_t)(tile == 64 ? 240 : 576) * 1000000;
 }
 
 }  // namespace atenia

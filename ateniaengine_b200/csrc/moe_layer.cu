@@ -78,9 +78,9 @@ bool merges_shared(const AteniaMoeLayer* L, int T) {
   // (groups that fill their tiles: the GEMMs are compute-bound themselves; below that no tile is higher than 192 rows)
   if (rows > (c.num_experts == 1 ? 128 : 140 * c.num_experts)) return false;
   if (L->bf16_decode == 1 || (L->bf16_decode < 0 && rows <= 16)) return false;  // (the stream-K kernel's calls)
-  // (a wide one beside many experts passes its weights through too often)
+  // (a wide one in low tiles passes its weights through too often)
   const int tile = pair_tokens_of(rows, c.num_experts, pair_f_tiles(c.d_ff, kSwiGLU));
-  if (!shared_rides_along(T, tile, c.num_experts, c.d_ff, c.shared_d_ff)) return false;
+  if (!shared_rides_along(T, tile, c.d_model, c.shared_d_ff)) return false;
   return bf16_kernel(L, rows, c.num_experts, c.d_model, false) == kBf16Pairs &&
          bf16_kernel(L, rows, c.num_experts, c.d_ff, false) == kBf16Pairs;
 }

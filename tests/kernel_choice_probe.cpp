@@ -7,7 +7,7 @@ extern "C" int choice_i8_decode(int rows, int experts, int d, int F, int shared)
 extern "C" int choice_bf16(int rows, int groups, int k, int beside) {
   return atenia::bf16_product_kernel(rows, groups, k, beside != 0);
 }
-extern "C" int choice_shared_rides(int tokens, int tile, int experts, int F, int Fs) {
-  return atenia::shared_rides_along(tokens, tile, experts, F, Fs);
+extern "C" int choice_shared_rides(int tokens, int tile, int d, int Fs) {
+  return atenia::shared_rides_along(tokens, tile, d, Fs);
 }
 extern "C" int choice_pair_tokens(int rows, int groups, int f_tiles) { return atenia::pair_tokens_of(rows, groups, f_tiles); }

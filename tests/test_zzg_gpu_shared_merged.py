@@ -33,7 +33,7 @@ MERGED = [((8, 2, 528, 400, 1040, True), (9, 65, 257, 500)), ((60, 4, 272, 144, 
           ((1, 1, 528, 400, 1040, False), (17, 128))]
 # groups that fill their tiles, a product on the single-CTA kernel, a wide shared expert of many low tiles, decode calls
 ASIDE = [((8, 2, 528, 400, 1040, True), (8, 561, 1480)), ((60, 4, 272, 144, 16, False), (257, 1480)), ((17, 4, 2064, 1040, 5632, True), (1480,)),
-         ((40, 2, 1040, 1424, 400, False), (1481,)), ((32, 1, 272, 144, 9616, False), (300,)), ((1, 1, 528, 400, 1040, False), (129,))]
+         ((40, 2, 1040, 1424, 400, False), (1481,)), ((32, 1, 2064, 144, 9616, False), (300,)), ((1, 1, 528, 400, 1040, False), (129,))]
 
 
 @pytest.mark.parametrize("E,k,d,F,Fs,gated,T,merges", [(*s, T, m) for m, group in ((True, MERGED), (False, ASIDE)) for s, Ts in group for T in Ts])
