@@ -111,7 +111,8 @@ struct RouterArgs {
   float* logits;       // [T, E] or null
   DeviceError* err;
   int variant;         // -1: by size; 0: CUDA-core f64 kernel (router.cu); 1: f64 tensor-core kernel
-                       // (router_dmma.cu); 2: split-k kernel (router_splitk.cu) up to kSplitkPinnedTokens
+                       // (router_dmma.cu); 2: split-k kernel (router_splitk.cu) up to kSplitkPinnedTokens;
+                       // 3: integer router (router_i8.cu) wherever it can serve the call, else by size
   const CUtensorMap* digit_map;  // integer router (router_i8.cu): digit planes of the router matrix (host pointer; null: the
   const double* digit_scale;     // layer has none that hold it exactly) and the scale of each of its rows (NaN: row not held)
   bool chained;        // see launch_chained

@@ -95,4 +95,19 @@ inline bool shared_rides_along(int tokens, int tile, int d, int Fs) {
   return more * 6 * d * Fs <= (int64_t)(tile == 64 ? 240 : 576) * 1000000;
 }
 
+// Does the integer router (router_i8.cu) pay?  It computes 64 rows whatever E is, and has a floor of some 15 us; the f64 routers' time
+// follows T, d and E.  B200, router kernel, it / the f64 one of that size, us (forwards where the kernels are close):
+//   33 - 64 experts, 1185 - 2368 tokens   (64) d 2048, 1185 / 1600 / 2048 tokens 21.1 / 27.0, 21.0 / 30.5, 28.0 / 30.8; 1536, 1185 / 1600 /
+//            2368 20.5 / 21.3, 20.9 / 24.5, 25.3 / 25.0; 1024, 1300 / 2048 17.2 / 17.8, 21.8 / 19.4; 768, 1600 16.9 / 14.2; 256, 2048 16.7 / 8.9
+//   ... more tokens   d 2048, 4096 / 8192 30.3 / 54, 46.6 / 104; 1536, 2400 25.3 / 42.1; 768, 2400 21.1 / 24.9; 512, 3000 / 4096 forwards
+//            equal, 8192 128 / 138; 256, 4096 / 8192 forwards 80 / 76, 107 / 109
+//   17 - 32 experts, more than 2368   (32) d 4096, 3000 / 4096 40.5 / 51.4, 43.6 / 51.6; 2048, 2400 / 8192 26.0 / 28.0, 45.4 / 54.7;
+//            1536, 4096 / 8192 24.5 / 23.2, 38.3 / 43.8; 1024, 4096 / 8192 forwards 68 / 66, 102.5 / 104.3; 512, 8192 78 / 76
+inline bool router_i8_pays(int tokens, int d, int experts) {
+  const int64_t work = (int64_t)tokens * d;
+  if (tokens <= 8 * 148 || experts <= 16) return false;
+  if (tokens <= 16 * 148) return experts > 32 && d >= 1536;
+  return experts > 32 ? d >= 768 || work >= 1 << 21 : d >= 2048 || work >= 1 << 23;
+}
+
 }  // namespace atenia

@@ -383,12 +383,13 @@ int atenia_moe_create(const AteniaMoeConfig* cfg, AteniaMoeLayer** out) {
     const int r = e ? std::atoi(e) : kGemvMaxRows;
     L->gemv_rows = r < 1 ? 1 : (r > 4 ? 4 : r);
   }
-  // Router kernel: by size (launch_router).  ATENIA_MOE_ROUTER = scalar | dmma | splitk pins one (tests, A/B runs); a
-  // pinned split-k serves batches up to 1024 tokens and hands larger ones to the CUDA-core kernel.
+  // Router kernel: by size (launch_router).  ATENIA_MOE_ROUTER = scalar | dmma | splitk | int8 pins one (tests, A/B
+  // runs); a pinned split-k serves batches up to 1024 tokens and hands larger ones to the CUDA-core kernel, the integer router
+  // leaves what it cannot serve (f32 activations, router matrices off its grid, 16 experts or fewer, more than 64) to the others.
   {
     const char* rv = std::getenv("ATENIA_MOE_ROUTER");
     const std::string r(rv ? rv : "");
-    L->router_variant = r == "scalar" ? 0 : r == "dmma" ? 1 : r == "splitk" ? 2 : -1;
+    L->router_variant = r == "scalar" ? 0 : r == "dmma" ? 1 : r == "splitk" ? 2 : r == "int8" ? 3 : -1;
   }
   L->bf16_decode = c.weight_dtype != ATENIA_W_BF16 ? 0
                    : std::getenv("ATENIA_MOE_BF16_DECODE") ? (std::atoi(std::getenv("ATENIA_MOE_BF16_DECODE")) != 0 ? 1 : 0)

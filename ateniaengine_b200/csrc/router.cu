@@ -349,21 +349,17 @@ int launch_v3_route(const float* logits, const float* e_score_bias, int T, int E
   return (int)cudaGetLastError();
 }
 
-// The integer router computes 64 rows whatever E is, and has a floor of some 15 us (B200, it / the f64 routers, us): 64
-// experts of d = 2048 1185 tokens 21.1 / 19.3, 1500 21.1 / 30.5, 2048 27.9 / 30.7, 4096 30.3 / 54, 8192 46.6 / 104; 32 experts
-// of d = 4096 2048 tokens some 39 / 29.1, 3000 40.5 / 51.4, 4096 43.6 / 51.6.
-static bool router_i8_pays(const RouterArgs& a) {
-  return a.digit_map && !a.x_is_f32 && (!a.gate_vec || a.E < kRouterDigitRows) && (a.T > 16 * 148 || (a.T > 8 * 148 && a.E > 32));
-}
+static bool router_i8_can(const RouterArgs& a) { return a.digit_map && !a.x_is_f32 && (!a.gate_vec || a.E < kRouterDigitRows); }
 
 int launch_router(const RouterArgs& a, cudaStream_t s) {
   if (a.T <= 0) return ATENIA_OK;
   if (a.k > kMaxK || a.E > 128) return ATENIA_ERR_UNSUPPORTED;
-  // variant -1: choose by size
-  if (a.variant == -1 && router_i8_pays(a)) return launch_router_i8(a, s);
-  if (a.variant == 2 ? a.T <= kSplitkPinnedTokens && a.d % 16 == 0 : a.variant == -1 && router_splitk_pays(a.T, a.E, a.d, a.beside))
+  // variant -1: choose by size (3: but the integer router wherever it can serve the call)
+  if ((a.variant == 3 || (a.variant == -1 && router_i8_pays(a.T, a.d, a.E))) && router_i8_can(a)) return launch_router_i8(a, s);
+  const bool by_size = a.variant == -1 || a.variant == 3;
+  if (a.variant == 2 ? a.T <= kSplitkPinnedTokens && a.d % 16 == 0 : by_size && router_splitk_pays(a.T, a.E, a.d, a.beside))
     return launch_router_splitk(a, s);
-  if (a.variant == 1 || (a.variant == -1 && a.d % 16 == 0)) return launch_router_dmma(a, s);
+  if (a.variant == 1 || (by_size && a.d % 16 == 0)) return launch_router_dmma(a, s);
   dim3 block(kRWarps * 32);
   // more tokens per CTA for many experts: the router matrix is re-read once per CTA
   if (a.E <= 8) router_kernel<8, 8><<<(a.T + 7) / 8, block, 0, s>>>(a);

@@ -10,4 +10,5 @@ extern "C" int choice_bf16(int rows, int groups, int k, int beside) {
 extern "C" int choice_shared_rides(int tokens, int tile, int d, int Fs) {
   return atenia::shared_rides_along(tokens, tile, d, Fs);
 }
+extern "C" int choice_router_i8(int tokens, int d, int experts) { return atenia::router_i8_pays(tokens, d, experts); }
 extern "C" int choice_pair_tokens(int rows, int groups, int f_tiles) { return atenia::pair_tokens_of(rows, groups, f_tiles); }

@@ -125,3 +125,19 @@ def test_the_shared_expert_rides_along_where_that_is_faster(lib, tokens, k, expe
     tile = lib.choice_pair_tokens(tokens * k, experts, (F + 127) // 128)
     took = along if lib.choice_shared_rides(tokens, tile, d, Fs) else aside
     assert took <= 1.01 * min(along, aside)
+
+
+# tokens, d, experts, us of the router kernel (or the forward where they are close) with the integer router / the f64 one
+ROUTER_I8 = [(1185, 2048, 64, 21.1, 27.0), (1600, 2048, 64, 21.0, 30.5), (2368, 2048, 64, 28.1, 31.0), (4096, 2048, 64, 30.3, 54.0),
+             (8192, 2048, 64, 46.6, 104), (1185, 1536, 64, 20.5, 21.3), (2368, 1536, 64, 25.3, 25.0), (2400, 1536, 64, 25.3, 42.1),
+             (1600, 1536, 40, 19.4, 21.7), (2048, 1024, 64, 21.8, 19.4), (1600, 768, 64, 16.9, 14.2), (2400, 768, 64, 21.1, 24.9),
+             (2048, 512, 64, 18.3, 11.7), (3000, 512, 64, 84.2, 84.2), (4096, 512, 64, 90.4, 90.4), (8192, 512, 64, 128, 138),
+             (2048, 256, 64, 16.7, 8.9), (4096, 256, 64, 80, 76), (8192, 256, 64, 106.6, 109), (3000, 256, 40, 55.5, 51.4),
+             (3000, 4096, 32, 40.5, 51.4), (2400, 2048, 32, 26.0, 28.0), (8192, 2048, 32, 45.4, 54.7), (4096, 1536, 32, 24.5, 23.2),
+             (8192, 1536, 32, 38.3, 43.8), (4096, 1024, 32, 67.8, 65.7), (8192, 1024, 32, 102.5, 104.3), (8192, 512, 32, 77.7, 76.0),
+             (4096, 256, 32, 51.4, 43.3), (2400, 2048, 20, 24.0, 27.4)]
+
+
+@pytest.mark.parametrize("tokens,d,experts,i8,f64", ROUTER_I8)
+def test_the_integer_router_where_it_is_faster(lib, tokens, d, experts, i8, f64):
+    assert (i8 if lib.choice_router_i8(tokens, d, experts) else f64) <= 1.02 * min(i8, f64)

@@ -33,7 +33,7 @@ def _pair(dev, monkeypatch, E, k, d, gated, T, seed=0, bias="none"):
     x = synth.make_activations(shape, seed, dev, tokens=T)
     monkeypatch.setenv("ATENIA_MOE_ROUTER", "dmma")
     base = synth.build_layer(shape, w, max_tokens=T)
-    monkeypatch.delenv("ATENIA_MOE_ROUTER")
+    monkeypatch.setenv("ATENIA_MOE_ROUTER", "int8")
     return base, synth.build_layer(shape, w, max_tokens=T), x, w
 
 
@@ -59,6 +59,15 @@ def test_the_integer_router_runs(dev, monkeypatch):
     plain = _tcgen05_launches(lambda: base.forward(x, sync=True))
     assert _tcgen05_launches(lambda: layer.forward(x, sync=True)) == plain + 1
     assert _tcgen05_launches(lambda: layer.forward(x.float(), sync=True)) == plain  # f32 activations: an f64 router
+
+
+def test_the_default_takes_it_by_size(dev):
+    synth = _synth()
+    shape = synth.MoeShape("r", 1536, 64, 40, 3, True)
+    layer = synth.build_layer(shape, synth.make_weights(shape, 1, dev), max_tokens=1300)
+    for T, more in ((1184, 0), (1185, 1)):
+        x = synth.make_activations(shape, 1, dev, tokens=T)
+        assert _tcgen05_launches(lambda: layer.forward(x, sync=True)) == 2 + more
 
 
 def _assert_logits_as_from_f64(logits, x, router, bias=None):
@@ -99,7 +108,7 @@ def test_tokens_off_their_grid(dev, monkeypatch, T, d):
     shape = synth.MoeShape("r", d, 64, E, 4, True, 64, True)
     monkeypatch.setenv("ATENIA_MOE_ROUTER", "dmma")
     base = synth.build_layer(shape, w, max_tokens=T)
-    monkeypatch.delenv("ATENIA_MOE_ROUTER")
+    monkeypatch.setenv("ATENIA_MOE_ROUTER", "int8")
     layer = synth.build_layer(shape, w, max_tokens=T)
     y, a = base.forward(x, out_dtype=torch.float32, aux=True, sync=True)
     z, b = layer.forward(x, out_dtype=torch.float32, aux=True, sync=True)
@@ -118,6 +127,7 @@ def test_tokens_off_their_grid(dev, monkeypatch, T, d):
 def test_router_matrices_off_their_grid(dev, monkeypatch):
     """f32 weights that five digits do not hold: such a layer keeps the f64 router, and a graph captured before they came
     computes their rows in f64."""
+    monkeypatch.setenv("ATENIA_MOE_ROUTER", "int8")
     synth = _synth()
     E, k, d, T = 40, 3, 272, 1300
     shape = synth.MoeShape("r", d, 64, E, k, True)
@@ -179,11 +189,8 @@ def test_v3_selection(dev, monkeypatch):
     rule = {"n_group": 8, "topk_group": 4, "scaling": 2.5, "e_score_bias": torch.randn(64, generator=gen, device=dev) * 0.05}
     cfg = moe.MoeLayerConfig(64, 6, False, 528, 64)
     got = []
-    for pin in ("dmma", None):
-        if pin:
-            monkeypatch.setenv("ATENIA_MOE_ROUTER", pin)
-        else:
-            monkeypatch.delenv("ATENIA_MOE_ROUTER")
+    for pin in ("dmma", "int8"):
+        monkeypatch.setenv("ATENIA_MOE_ROUTER", pin)
         layer = moe.RealMoeLayer(cfg, w["router"], w["gate"], w["up"], w["down"], renormalize=True, max_tokens=1500, v3=rule)
         got.append(layer.forward(x, aux=True, sync=True)[1])
     a, b = got
