@@ -125,8 +125,7 @@ grouped_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const CU
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   chain_wait();  // (everything above touches only this CTA's shared and tensor memory)
-  stage_group_offsets(group_offsets_g, num_groups, goff_s);
-  const int32_t* group_offsets = goff_s;
+  const int32_t* group_offsets = staged_group_offsets(group_offsets_g, num_groups, goff_s);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -441,7 +440,7 @@ static int launch_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
 
 int launch_grouped_gemm_tcgen05(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   if (a.num_groups <= 0) return ATENIA_OK;
-  if (a.N % 16 != 0 || a.K % 16 != 0 || a.num_groups > kMaxGroupsShared) return ATENIA_ERR_SHAPE;
+  if (a.N % 16 != 0 || a.K % 16 != 0) return ATENIA_ERR_SHAPE;
   if (a.w8 && (!a.scale0 || (a.mode == kSwiGLU && !a.scale1))) return ATENIA_ERR_NULL;
   int rc;
   if (a.mode == kSwiGLU) rc = a.w8 ? launch_one<kSwiGLU, true>(a, num_sms, s) : launch_one<kSwiGLU, false>(a, num_sms, s);

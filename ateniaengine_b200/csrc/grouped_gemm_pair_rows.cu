@@ -135,8 +135,7 @@ grouped_gemm_pair_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   chain_wait();  // (everything above touches only this CTA's shared and tensor memory)
-  stage_group_offsets(group_offsets_g, num_groups, goff_s);
-  const int32_t* group_offsets = goff_s;
+  const int32_t* group_offsets = staged_group_offsets(group_offsets_g, num_groups, goff_s);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // barriers of both CTAs are initialised before anyone signals them
@@ -336,7 +335,7 @@ int launch_pair_rows_one(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) 
 
 int launch_grouped_gemm_pair_rows(const GroupedGemmArgs& a, int num_sms, cudaStream_t s) {
   if (a.num_groups <= 0) return ATENIA_OK;
-  if (a.N % 16 != 0 || a.K % 16 != 0 || a.num_groups > kMaxGroupsShared) return ATENIA_ERR_SHAPE;
+  if (a.N % 16 != 0 || a.K % 16 != 0) return ATENIA_ERR_SHAPE;
   if (a.w8) return ATENIA_ERR_UNSUPPORTED;  // INT8 weights: w8_gemm.cu / w8_gemm_m256.cu
   int rc = a.mode == kSwiGLU ? launch_pair_rows_one<kSwiGLU>(a, num_sms, s) : launch_pair_rows_one<kPlain>(a, num_sms, s);
   count_launch();

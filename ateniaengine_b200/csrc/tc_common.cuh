@@ -189,16 +189,26 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 // change (a persistent CTA's next tile is a grid width further on: with 60 experts of 20 tiles that is
 // seven groups, two dependent loads each).  From global memory that walk costs microseconds per tile and
 // the ring runs dry meanwhile, so kernels with many groups copy the offsets into shared memory first.
-// They index the array itself: through a pointer that may also be global the reads are generic loads, and the forwards
-// lose 1 to 3 us (B200, 64 tokens of a 512-wide layer 31.7 -> 28.6 us, 256 Mixtral tokens 490 -> 484).
-// The loads go past L1, so that a kernel may take the offsets before its chain_wait().
-constexpr int kMaxGroupsShared = 256;  // (a launch refuses more; a layer has at most 128)
+// The transposed pair kernel and the decode kernel index the array itself: through a pointer that may also be global the reads are
+// generic loads, and their forwards lose 1 to 3 us (B200, 64 tokens of a 512-wide layer 31.7 -> 28.6 us, 256 Mixtral tokens 490 ->
+// 484).  The loads go past L1, so that a kernel may take the offsets before its chain_wait().
+constexpr int kMaxGroupsShared = 256;  // (their launches refuse more; a layer has at most 128)
 __device__ __forceinline__ void stage_group_offsets(const int32_t* off_global, int num_groups, int32_t* off_shared) {
   for (int i = threadIdx.x; i <= num_groups; i += blockDim.x) {
     int32_t v;
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(off_global + i) : "memory");
     off_shared[i] = v;  // (valid after the caller's next block-wide barrier)
   }
+}
+
+// The kernels that take the offsets after their wait (one CTA a tile, token rows as the M side) walk them through such a pointer:
+// there the walk that the compiler makes of it is the faster one (128 experts top-6 of 512 x 768, 623 / 2940 tokens 105.8 / 168.0
+// through the array, 103.4 / 164.5 so; 96 top-8 of 1024 x 768, shared 768, 768 tokens 154.2 / 151.1).
+__device__ __forceinline__ const int32_t* staged_group_offsets(const int32_t* __restrict__ off_global, int num_groups,
+                                                               int32_t* off_shared) {
+  if (num_groups > kMaxGroupsShared) return off_global;
+  for (int i = threadIdx.x; i <= num_groups; i += blockDim.x) off_shared[i] = off_global[i];
+  return off_shared;  // (valid after the caller's next block-wide barrier)
 }
 
 struct TileCursor {
