@@ -288,11 +288,13 @@ grouped_gemm_2cta_kernel(const __grid_constant__ PairRowMaps tmaps_x, const CUte
     int ahead = 0;
     // (The loop's first seek finds the cursor where this one left it.  Walking the groups again there delays the token rows: 32
     // experts of 512 x 1408, shared 2816 on the second stream, 333 / 500 / 1000 tokens 70.8 / 73.5 / 89.7 -> 67.2 / 70.5 / 86.1 us a
-    // forward.  With an extra group the tiles that follow are what counts, and the walk is repeated: once / twice 64 top-2 experts of
-    // 2048 x 1408, 24 tokens 112.1 / 111.2, 128 top-2 of 2048 x 768, 24 / 100 tokens 96.0 / 93.9, 171.6 / 170.1.)
+    // forward.  In streams of weights, tiles of 64 rows or an extra group, the CTAs had better not start as one, and the walk is
+    // repeated: once / twice 64 top-2 experts of 2048 x 1408 and a shared one, 24 tokens 112.1 / 111.2, 128 top-2 of 2048 x 768 and a
+    // shared one, 24 / 100 tokens 96.0 / 93.9, 171.6 / 170.1; alone, 96 top-8 of 3072 x 1024, 3 tokens 99.7 / 96.6, 64 top-1 of 4096 x 512, 28
+    // tokens 88.5 / 86.6, 128 top-1 of 4096 x 1024, 31 tokens 155.3 / 152.4.)
     PairCursor first = cur;
     const bool any = seek(first, 0);
-    if constexpr (!EX) cur = first;
+    if constexpr (!EX && TOK > 64) cur = first;
     if (any) {
       const CUtensorMap* m0 = weights0();
       const CUtensorMap* m1 = MODE == kSwiGLU ? weights1() : m0;
