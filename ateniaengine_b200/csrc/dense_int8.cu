@@ -76,10 +76,16 @@ __device__ __forceinline__ void store_codes4(const float (&w)[4], const float* s
   }
 }
 
+// A NaN is skipped, as in the reference: fmaxf returns the other operand, and nothing compares greater for one.  The groups kernel is
+// faster with the first form, the tall one with the second (4096 x 14336 by 128 / 64 51.4 / 52.0, 49.9 / 51.9 us; 8192 x 14336 by
+// 512 / 1024 / 4096 143.5 / 140.7, 150.2 / 147.2, 167.2 / 163.6).
+template <bool COMPARE>
 __device__ __forceinline__ void max_cols4(float (&m)[4], const float (&v)[4]) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    m[j] = fmaxf(m[j], fabsf(v[j]));  // (fmaxf returns the other operand for a NaN: skipped, as in the reference)
+    const float a = fabsf(v[j]);
+    if (!COMPARE) m[j] = fmaxf(m[j], a);
+    else if (a > m[j]) m[j] = a;
   }
 }
 __device__ __forceinline__ float scale_of(float amax) { return fmaxf(__fdiv_rn(amax, 127.0f), 1e-12f); }
@@ -112,7 +118,7 @@ __global__ void __launch_bounds__(LANES * RL) quantize_groups_kernel(const float
   }
   float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < GROUP_RPT; ++i) max_cols4(m, v[i]);
+  for (int i = 0; i < GROUP_RPT; ++i) max_cols4<false>(m, v[i]);
   *reinterpret_cast<float4*>(&red[rl][lane * 4]) = make_float4(m[0], m[1], m[2], m[3]);
   __syncthreads();
   for (int i = threadIdx.x; i < COLS; i += LANES * RL) {  // slot i: column col_of(i / 4, i % 4)
@@ -158,12 +164,12 @@ quantize_tall_kernel(const float* __restrict__ w, int64_t K, int64_t N, int64_t 
 #pragma unroll
     for (int i = 0; i < 4; ++i) load_cols4<VEC, LANES>(v[i], w + (r + i * kStep) * N, strip0, lane, N);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) max_cols4(m, v[i]);
+    for (int i = 0; i < 4; ++i) max_cols4<true>(m, v[i]);
   }
   for (; r < hi; r += kStep) {
     float v[4];
     load_cols4<VEC, LANES>(v, w + r * N, strip0, lane, N);
-    max_cols4(m, v);
+    max_cols4<true>(m, v);
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) red[rl][lane + LANES * j] = m[j];
